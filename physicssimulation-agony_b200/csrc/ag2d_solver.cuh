@@ -1,16 +1,12 @@
 // Graph colouring + sequential-impulse solver as one device routine over a "team" of threads that share a barrier:
-// a thread-block cluster (hardware barrier.cluster, large single worlds), one CTA (batched small worlds) or a
-// cooperative grid (very large worlds). The per-constraint arithmetic (prep/warm/velocity/position) below is shared
-// by every variant.
+// one CTA (batched small worlds, single worlds of a few thousand bodies) or a cooperative grid (larger single worlds,
+// whose passes then run as a dataflow without barriers). The per-constraint arithmetic (prep/warm/velocity/position)
+// below is shared by every variant.
 #pragma once
-
-#include <cooperative_groups.h>
 
 #include "ag2d_kernels.cuh"
 
 namespace ag2d {
-
-namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------------------------------------------------------
 // Sequential-impulse solver (Solving/BodyCollisionSolver.cpp): computeConstraintData (:229-390), applyWarmStarting
@@ -137,10 +133,9 @@ __device__ __forceinline__ float impact_impulse(const Manifold& m, float4 vA, fl
     return impact;
 }
 
-template <class Bodies>
-__device__ __forceinline__ void warm_constraint(const Bodies& B, const Constraint& k)
+// The warm start of one constraint on its two bodies' velocities held in registers.
+__device__ __forceinline__ void warm_solve(const Constraint& k, float4& vA, float4& vB)
 {
-    float4 vA = B.v(k.bodyA), vB = B.v(k.bodyB);
     const float tx = -k.ny, ty = k.nx;
     const float jn0 = k.count > 0 ? k.jn0 : 0.0f, jt0 = k.count > 0 ? k.jt0 : 0.0f;
     const float jn1 = k.count > 1 ? k.jn1 : 0.0f, jt1 = k.count > 1 ? k.jt1 : 0.0f;
@@ -150,6 +145,13 @@ __device__ __forceinline__ void warm_constraint(const Bodies& B, const Constrain
     vB.x = vB.x + ix * k.imB; vB.y = vB.y + iy * k.imB;
     vA.z = vA.z - (jn0 * k.rAn0 + jt0 * k.rAt0 + jn1 * k.rAn1 + jt1 * k.rAt1) * k.iIA;
     vB.z = vB.z + (jn0 * k.rBn0 + jt0 * k.rBt0 + jn1 * k.rBn1 + jt1 * k.rBt1) * k.iIB;
+}
+
+template <class Bodies>
+__device__ __forceinline__ void warm_constraint(const Bodies& B, const Constraint& k)
+{
+    float4 vA = B.v(k.bodyA), vB = B.v(k.bodyB);
+    warm_solve(k, vA, vB);
     if (k.imA > 0.0f) B.setV(k.bodyA, vA);
     if (k.imB > 0.0f) B.setV(k.bodyB, vB);
 }
@@ -285,20 +287,28 @@ __device__ __forceinline__ void velocity_constraint(const Bodies& B, Constraint&
     if (k.imB > 0.0f) B.setV(k.bodyB, vB);
 }
 
+// One position step of one constraint on its two bodies' poses held in registers; false when it moves nothing.
+__device__ __forceinline__ bool position_solve(const Constraint& k, float4& pA, float4& pB)
+{
+    const float pen = k.penBase - ((pB.x - pA.x) * k.nx + (pB.y - pA.y) * k.ny);
+    if (pen <= 0.0f) return false;
+    const float imA = k.imA, imB = k.imB;
+    const float total = pen / (imA + imB) * 0.5f;
+    const float cA = imA * total, cB = imB * total;
+    const float cAx = k.nx * cA, cAy = k.ny * cA, cBx = k.nx * cB, cBy = k.ny * cB;
+    if (imA > 0.0f) { pA.x = pA.x - cAx; pA.y = pA.y - cAy; }
+    if (imB > 0.0f) { pB.x = pB.x + cBx; pB.y = pB.y + cBy; }
+    return true;
+}
+
 template <class Bodies>
 __device__ __forceinline__ void position_constraint(const Bodies& B, const Constraint& k)
 {
     float4 pA = B.p(k.bodyA), pB = B.p(k.bodyB);
-    const float pen = k.penBase - ((pB.x - pA.x) * k.nx + (pB.y - pA.y) * k.ny);
-    if (pen <= 0.0f) return;
-    const float imA = B.v(k.bodyA).w, imB = B.v(k.bodyB).w;
-    const float total = pen / (imA + imB) * 0.5f;
-    const float cA = imA * total, cB = imB * total;
-    const float cAx = k.nx * cA, cAy = k.ny * cA, cBx = k.nx * cB, cBy = k.ny * cB;
-    if (imA > 0.0f) { pA.x = pA.x - cAx; pA.y = pA.y - cAy; B.setP(k.bodyA, pA); }
-    if (imB > 0.0f) { pB.x = pB.x + cBx; pB.y = pB.y + cBy; B.setP(k.bodyB, pB); }
+    if (!position_solve(k, pA, pB)) return;
+    if (k.imA > 0.0f) B.setP(k.bodyA, pA);
+    if (k.imB > 0.0f) B.setP(k.bodyB, pB);
 }
-
 
 __device__ __forceinline__ uint32_t priority_hash(uint32_t x)
 {
@@ -317,6 +327,64 @@ constexpr uint32_t COLOR_SLOTS = MAX_COLORS + 4;
 // all 64 taken gets colour 64 + its round (unique to the round, so still conflict-free).
 constexpr uint32_t MAX_ROUNDS = MAX_COLORS - 64;
 
+// Solver records in global memory, structure of arrays: field f of record c at q[f * stride + c], so that a warp that
+// takes 32 consecutive records reads every field as four full lines. (As 128-byte structures a lane apart, each
+// 16-byte load of a warp touched 32 lines, and the load unit, not latency or bandwidth, bounded every pass: one CTA on
+// 3,265 manifolds took 4.5 us a colour.) A record with one contact point leaves out fields 5 and 6.
+struct ConsRecords {
+    float4* q;
+    float* pen;        // penetration base
+    uint32_t stride;
+    static constexpr uint32_t FIELDS = 7;
+    __device__ __forceinline__ ConsRecords from(uint32_t c) const { return ConsRecords{q + c, pen + c, stride}; }
+    __device__ __forceinline__ void store(uint32_t c, const Constraint& k) const
+    {
+        float4* r = q + c;
+        const size_t st = stride;
+        r[0] = make_float4(__uint_as_float(k.bodyA | min(k.count, 3u) << 30), __uint_as_float(k.bodyB), k.nx, k.ny);
+        r[st] = make_float4(k.imA, k.imB, k.iIA, k.iIB);
+        r[2 * st] = make_float4(k.jn0, k.jt0, k.sf, k.df);
+        r[3 * st] = make_float4(k.rAn0, k.rBn0, k.rAt0, k.rBt0);
+        r[4 * st] = make_float4(k.nm0, k.tm0, k.bias0, k.bias1);
+        if (k.count != 1u) {
+            r[5 * st] = make_float4(k.jn1, k.jt1, k.nm1, k.tm1);
+            r[6 * st] = make_float4(k.rAn1, k.rBn1, k.rAt1, k.rBt1);
+        }
+        pen[c] = k.penBase;
+    }
+    // The fields a position step reads: bodies, count, normal, masses, penetration base.
+    __device__ __forceinline__ void loadHead(uint32_t c, Constraint& k) const
+    {
+        const float4 h = q[c], ms = q[size_t(stride) + c];
+        k.bodyA = __float_as_uint(h.x) & 0x3FFFFFFFu;
+        k.count = __float_as_uint(h.x) >> 30;
+        k.bodyB = __float_as_uint(h.y);
+        k.nx = h.z; k.ny = h.w;
+        k.imA = ms.x; k.imB = ms.y; k.iIA = ms.z; k.iIB = ms.w;
+    }
+    __device__ __forceinline__ void load(uint32_t c, uint32_t kind, Constraint& k) const;
+    __device__ __forceinline__ void storeImpulses(uint32_t c, const Constraint& k) const
+    {
+        *reinterpret_cast<float2*>(q + 2 * size_t(stride) + c) = make_float2(k.jn0, k.jt0);
+        if (k.count != 1u) *reinterpret_cast<float2*>(q + 5 * size_t(stride) + c) = make_float2(k.jn1, k.jt1);
+    }
+    // The impulses (jn0, jt0, jn1, jt1); 'second' the ones a record with one point left out.
+    __device__ __forceinline__ float4 impulses(uint32_t c, float2 second) const
+    {
+        const float2 a = *reinterpret_cast<const float2*>(q + 2 * size_t(stride) + c);
+        float2 b = second;
+        if (__float_as_uint(q[c].x) >> 30 != 1u) b = *reinterpret_cast<const float2*>(q + 5 * size_t(stride) + c);
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+    // Pulls a warp's 32 records [c0, c0 + 32) into L1 ahead of the pass that reads them: a line a lane.
+    __device__ __forceinline__ void prefetch(uint32_t c0) const
+    {
+        const uint32_t lane = threadIdx.x & 31u;
+        if (lane < 4u * FIELDS)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(q + size_t(lane >> 2) * stride + c0 + (lane & 3u) * 8u));
+    }
+};
+
 // Scratch of one world's (or one team of worlds') colouring and solve.
 struct SolveScratch {
     uint32_t* color;                  // [manifolds]
@@ -325,7 +393,7 @@ struct SolveScratch {
     unsigned long long* bodyMask;     // [bodies] colours taken around each body, zeroed before the call
     uint32_t* colorCount;             // [COLOR_SLOTS], zeroed by the routine
     uint32_t* colorStart;             // [MAX_COLORS + 1]
-    Constraint* cons;                 // [manifolds]
+    ConsRecords cons;                 // [manifolds]
     const uint32_t* prio;             // [manifolds] colouring priorities, or null: priority_hash(index)
     uint4* listA;                     // [manifolds] uncoloured manifold records, ping
     uint4* listB;                     // [manifolds] uncoloured manifold records, pong
@@ -334,11 +402,7 @@ struct SolveScratch {
 };
 
 // Team barriers. ld() reads a colour counter written by other team members before the last barrier: global memory
-// through L2 for the multi-CTA teams, shared memory for one CTA.
-struct ClusterSync {
-    __device__ __forceinline__ bool operator()() const { cg::this_cluster().sync(); return true; }
-    static __device__ __forceinline__ uint32_t ld(const uint32_t* p) { return __ldcg(p); }
-};
+// through L2 for the grid, shared memory for one CTA.
 struct BlockSync {
     __device__ __forceinline__ bool operator()() const { __syncthreads(); return true; }
     static __device__ __forceinline__ uint32_t ld(const uint32_t* p) { return *static_cast<const volatile uint32_t*>(p); }
@@ -391,6 +455,11 @@ struct ConsSmem {
         k.tm1 = m1.x; k.bias1 = m1.y; k.sf = m1.z; k.df = m1.w;
         k.imA = ms.x; k.imB = ms.y; k.iIA = ms.z; k.iIB = ms.w;
     }
+    __device__ __forceinline__ void loadMasses(uint32_t c, Constraint& k) const
+    {
+        const float4 ms = q[6 * cap + c];
+        k.imA = ms.x; k.imB = ms.y;
+    }
     __device__ __forceinline__ void storeImpulses(uint32_t c, const Constraint& k) const
     {
         q[cap + c] = make_float4(k.jn0, k.jt0, k.jn1, k.jt1);
@@ -399,58 +468,52 @@ struct ConsSmem {
 };
 constexpr uint32_t CONS_SMEM_BYTES = ConsSmem::FIELDS * sizeof(float4);
 
-// Pulls the 128-byte constraint of slot c into L1 ahead of the pass that reads it.
-__device__ __forceinline__ void prefetch_l1(const void* p)
+// Phases of the solve: what a phase does with its records.
+constexpr uint32_t PHASE_WARM = 0, PHASE_VELOCITY = 1, PHASE_POSITION = 2;
+
+__device__ __forceinline__ void ConsRecords::load(uint32_t c, uint32_t kind, Constraint& k) const
 {
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+    loadHead(c, k);
+    if (kind == PHASE_POSITION) {
+        k.penBase = pen[c];
+        return;
+    }
+    const float4* r = q + c;
+    const size_t st = stride;
+    const float4 j = r[2 * st], r0 = r[3 * st], m0 = r[4 * st];
+    k.jn0 = j.x; k.jt0 = j.y; k.sf = j.z; k.df = j.w;
+    k.rAn0 = r0.x; k.rBn0 = r0.y; k.rAt0 = r0.z; k.rBt0 = r0.w;
+    k.nm0 = m0.x; k.tm0 = m0.y; k.bias0 = m0.z; k.bias1 = m0.w;
+    if (k.count != 1u) {
+        const float4 m1 = r[5 * st], r1 = r[6 * st];
+        k.jn1 = m1.x; k.jt1 = m1.y; k.nm1 = m1.z; k.tm1 = m1.w;
+        k.rAn1 = r1.x; k.rBn1 = r1.y; k.rAt1 = r1.z; k.rBt1 = r1.w;
+    } else {
+        k.jn1 = 0.0f; k.jt1 = 0.0f; k.nm1 = 0.0f; k.tm1 = 0.0f;
+        k.rAn1 = 0.0f; k.rBn1 = 0.0f; k.rAt1 = 0.0f; k.rBt1 = 0.0f;
+    }
 }
 
-// The constraint slot this thread handles first in colour 'col' (or nothing), prefetched before the barrier that
+// The records this thread's warp handles first in colour 'col' (or nothing), prefetched before the barrier that
 // precedes that colour's pass.
 template <class Sync>
 __device__ __forceinline__ void prefetch_colour(const SolveScratch& s, uint32_t col, uint32_t ncol, uint32_t rank)
 {
     if (col >= ncol) return;
-    const uint32_t c = Sync::ld(s.colorStart + col) + rank;
-    if (c < Sync::ld(s.colorStart + col + 1)) prefetch_l1(s.cons + c);
-}
-
-// Phases of the solve: what a phase does with its records.
-constexpr uint32_t PHASE_WARM = 0, PHASE_VELOCITY = 1, PHASE_POSITION = 2;
-
-// The fields a phase of 'kind' reads from global record c: the head (bodies, count, normal, masses) and, except
-// for a position phase, the rest; a position phase takes the penetration base instead.
-__device__ __forceinline__ void load_record(const Constraint* __restrict__ cons, uint32_t c, uint32_t kind,
-                                            Constraint& k)
-{
-    const float4* q = reinterpret_cast<const float4*>(cons + c);
-    const float4 h0 = q[0], h1 = q[1];
-    k.bodyA = __float_as_uint(h0.x); k.bodyB = __float_as_uint(h0.y); k.count = __float_as_uint(h0.z);
-    k.manifold = __float_as_uint(h0.w);
-    k.nx = h1.x; k.ny = h1.y; k.imA = h1.z; k.imB = h1.w;
-    if (kind == PHASE_POSITION) {
-        k.penBase = cons[c].penBase;
-        return;
-    }
-    const float4 h2 = q[2], j = q[3], r0 = q[4], m0 = q[5], r1 = q[6], m1 = q[7];
-    k.iIA = h2.x; k.iIB = h2.y; k.sf = h2.z; k.df = h2.w;
-    k.jn0 = j.x; k.jt0 = j.y; k.jn1 = j.z; k.jt1 = j.w;
-    k.rAn0 = r0.x; k.rBn0 = r0.y; k.rAt0 = r0.z; k.rBt0 = r0.w;
-    k.nm0 = m0.x; k.tm0 = m0.y; k.bias0 = m0.z; k.penBase = m0.w;
-    k.rAn1 = r1.x; k.rBn1 = r1.y; k.rAt1 = r1.z; k.rBt1 = r1.w;
-    k.nm1 = m1.x; k.tm1 = m1.y; k.bias1 = m1.z; k.pad = m1.w;
+    const uint32_t c0 = Sync::ld(s.colorStart + col) + (rank & ~31u);
+    if (c0 < Sync::ld(s.colorStart + col + 1)) s.cons.prefetch(c0);
 }
 
 // One phase's step on a record held in registers; a velocity step writes the record's impulses back.
 template <class Bodies>
-__device__ __forceinline__ void solve_record(const Bodies& B, Constraint* __restrict__ cons, uint32_t c, uint32_t kind,
+__device__ __forceinline__ void solve_record(const Bodies& B, const ConsRecords& cons, uint32_t c, uint32_t kind,
                                              Constraint& k)
 {
     if (kind == PHASE_WARM) {
         warm_constraint(B, k);
     } else if (kind == PHASE_VELOCITY) {
         velocity_constraint(B, k);
-        *reinterpret_cast<float4*>(&cons[c].jn0) = make_float4(k.jn0, k.jt0, k.jn1, k.jt1);
+        cons.storeImpulses(c, k);
     } else {
         position_constraint(B, k);
     }
@@ -476,7 +539,7 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
     uint32_t cNext = NO_REC;
     if (nPhase) {
         const uint32_t c0 = Sync::ld(s.colorStart) + rank;
-        if (c0 < Sync::ld(s.colorStart + 1)) { load_record(s.cons, c0, kindOf(0), nxt); cNext = c0; }
+        if (c0 < Sync::ld(s.colorStart + 1)) { s.cons.load(c0, kindOf(0), nxt); cNext = c0; }
     }
     for (uint32_t ph = 0; ph < nPhase; ph++) {
         const uint32_t col = ph % ncol, kind = kindOf(ph);
@@ -487,14 +550,14 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
         if (ph + 1 < nPhase) {
             const uint32_t col2 = (ph + 1) % ncol;
             const uint32_t c2 = Sync::ld(s.colorStart + col2) + rank;
-            if (c2 < Sync::ld(s.colorStart + col2 + 1)) { load_record(s.cons, c2, kindOf(ph + 1), nxt); cNext = c2; }
+            if (c2 < Sync::ld(s.colorStart + col2 + 1)) { s.cons.load(c2, kindOf(ph + 1), nxt); cNext = c2; }
         }
         while (c < end) {
             solve_record(B, s.cons, c, kind, k);
             // One colour: the next phase's record is this one, loaded before this phase's impulses.
             if (cNext == c) { nxt.jn0 = k.jn0; nxt.jt0 = k.jt0; nxt.jn1 = k.jn1; nxt.jt1 = k.jt1; }
             c += size;   // a colour larger than the team
-            if (c < end) load_record(s.cons, c, kind, k);
+            if (c < end) s.cons.load(c, kind, k);
         }
         if (!sync()) return false;
     }
@@ -516,11 +579,10 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
 // s.pairBodies words: body index | PAIR_DYNAMIC (finite mass) | PAIR_KEPT (first word: colour carried over).
 constexpr uint32_t PAIR_DYNAMIC = 0x80000000u, PAIR_KEPT = 0x40000000u, PAIR_BODY = 0x3FFFFFFFu;
 
-template <class Sync, class Bodies, bool PIPELINED = false>
-__device__ bool color_and_solve(const DeviceWorld& w, const Bodies& B, Manifold* __restrict__ m, uint32_t n,
-                                const SolveScratch& s, uint32_t velIters, uint32_t posIters, uint32_t rank,
-                                uint32_t size, Sync sync, uint32_t* __restrict__ outColors, uint32_t* __restrict__ status,
-                                ConsSmem cs = ConsSmem{})
+template <class Sync, class Bodies>
+__device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Manifold* __restrict__ m, uint32_t n,
+                                const SolveScratch& s, uint32_t rank, uint32_t size, Sync sync,
+                                uint32_t* __restrict__ outColors, uint32_t* __restrict__ status, uint32_t& ncolOut)
 {
     for (uint32_t c = rank; c < COLOR_SLOTS; c += size) s.colorCount[c] = 0;
     uint32_t* const nColors = s.colorCount + MAX_COLORS + 3;
@@ -615,7 +677,7 @@ __device__ bool color_and_solve(const DeviceWorld& w, const Bodies& B, Manifold*
         in = out;
     }
     if (len > 0) { if (rank == 0) atomicOr(status, STATUS_COLOR_OVERFLOW); return false; }
-    const uint32_t ncol = Sync::ld(nColors);
+    const uint32_t ncol = ncolOut = Sync::ld(nColors);
     if (rank == 0) {
         uint32_t run = 0;
         for (uint32_t c = 0; c < ncol; c++) { s.colorStart[c] = run; run += s.colorCount[c]; s.colorCount[c] = 0; }
@@ -627,7 +689,15 @@ __device__ bool color_and_solve(const DeviceWorld& w, const Bodies& B, Manifold*
         const uint32_t c = s.color[i] & COLOR_MASK;
         s.order[Sync::ld(s.colorStart + c) + atomicAdd(s.colorCount + c, 1u)] = i;
     }
-    if (!sync()) return false;
+    return sync();
+}
+
+// The colour-major solve of coloured manifolds (s.order, s.colorStart), with the team's barrier between colours.
+template <class Sync, class Bodies, bool PIPELINED = false>
+__device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* __restrict__ m, uint32_t n,
+                              const SolveScratch& s, uint32_t ncol, uint32_t velIters, uint32_t posIters,
+                              uint32_t rank, uint32_t size, Sync sync, ConsSmem cs = ConsSmem{})
+{
     // The colouring words are no longer needed: a lazily staged body cache is loaded over them now.
     if (B.stage(rank, size) && !sync()) return false;
     // Constraint build for every manifold before any velocity changes (computeConstraintData). The records go to
@@ -638,7 +708,7 @@ __device__ bool color_and_solve(const DeviceWorld& w, const Bodies& B, Manifold*
         Constraint k;
         prep_constraint(w, B, m[mi], mi, k);
         if (onChip) cs.store(c, k);
-        else s.cons[c] = k;
+        else s.cons.store(c, k);
     }
     if (!sync()) return false;
     bool passesDone = false;
@@ -652,70 +722,101 @@ __device__ bool color_and_solve(const DeviceWorld& w, const Bodies& B, Manifold*
         for (uint32_t col = 0; col < ncol; col++) {
             const uint32_t end = Sync::ld(s.colorStart + col + 1);
             for (uint32_t c = Sync::ld(s.colorStart + col) + rank; c < end; c += size) {
-                if (onChip) {
-                    Constraint k;
-                    cs.load(c, k);
-                    warm_constraint(B, k);
-                } else {
-                    warm_constraint(B, s.cons[c]);
-                }
+                Constraint k;
+                if (onChip) cs.load(c, k);
+                else s.cons.load(c, PHASE_WARM, k);
+                warm_constraint(B, k);
             }
             if (!sync()) return false;
         }
-        for (uint32_t it = 0; it < velIters; it++) {
+        // Position iteration 'it' runs beside velocity iteration 'it': the two touch different body state (poses and
+        // velocities), so a colour's position steps share the barrier interval of its velocity steps, on the threads
+        // that have no velocity step: 8 + 1 passes of barriers instead of 8 + 3 + 1 at the default counts.
+        const uint32_t iters = velIters > posIters ? velIters : posIters;
+        for (uint32_t it = 0; it < iters; it++) {
+            const bool vel = it < velIters, pos = it < posIters;
             for (uint32_t col = 0; col < ncol; col++) {
-                const uint32_t end = Sync::ld(s.colorStart + col + 1);
-                for (uint32_t c = Sync::ld(s.colorStart + col) + rank; c < end; c += size) {
+                const uint32_t begin = Sync::ld(s.colorStart + col), count = Sync::ld(s.colorStart + col + 1) - begin;
+                const uint32_t posBase = vel ? (count + 31u) & ~31u : 0u;   // a warp does one kind of step
+                const uint32_t total = pos ? posBase + count : count;
+                for (uint32_t j = rank; j < total; j += size) {
                     Constraint k;
-                    if (onChip) cs.load(c, k);
-                    else k = s.cons[c];
-                    velocity_constraint(B, k);
-                    if (onChip) cs.storeImpulses(c, k);
-                    else *reinterpret_cast<float4*>(&s.cons[c].jn0) = make_float4(k.jn0, k.jt0, k.jn1, k.jt1);
-                }
-                // The next pass's constraint: from the next colour, or colour 0 of the next iteration.
-                if (!onChip) prefetch_colour<Sync>(s, col + 1 < ncol ? col + 1 : 0, ncol, rank);
-                if (!sync()) return false;
-            }
-        }
-        for (uint32_t it = 0; it < posIters; it++) {
-            for (uint32_t col = 0; col < ncol; col++) {
-                const uint32_t end = Sync::ld(s.colorStart + col + 1);
-                for (uint32_t c = Sync::ld(s.colorStart + col) + rank; c < end; c += size) {
-                    if (onChip) {
-                        Constraint k;
-                        cs.loadHead(c, k);
+                    if (vel && j < count) {
+                        const uint32_t c = begin + j;
+                        if (onChip) cs.load(c, k);
+                        else s.cons.load(c, PHASE_VELOCITY, k);
+                        velocity_constraint(B, k);
+                        if (onChip) cs.storeImpulses(c, k);
+                        else s.cons.storeImpulses(c, k);
+                    } else if (j >= posBase) {
+                        const uint32_t c = begin + j - posBase;
+                        if (onChip) {
+                            cs.loadHead(c, k);
+                            cs.loadMasses(c, k);
+                        } else {
+                            s.cons.load(c, PHASE_POSITION, k);
+                        }
                         position_constraint(B, k);
-                    } else {
-                        position_constraint(B, s.cons[c]);
                     }
                 }
+                // The next interval's constraint: from the next colour, or colour 0 of the next iteration.
                 if (!onChip) prefetch_colour<Sync>(s, col + 1 < ncol ? col + 1 : 0, ncol, rank);
                 if (!sync()) return false;
             }
         }
     }
     for (uint32_t c = rank; c < n; c += size) {
-        if (onChip) {
-            const float4 j = cs.impulses(c);
-            Manifold& d = m[__ldcg(s.order + c)];
-            d.jn0 = j.x; d.jt0 = j.y; d.jn1 = j.z; d.jt1 = j.w;
-        } else {
-            const Constraint& k = s.cons[c];
-            Manifold& d = m[k.manifold];
-            d.jn0 = k.jn0; d.jt0 = k.jt0; d.jn1 = k.jn1; d.jt1 = k.jt1;
-        }
+        Manifold& d = m[__ldcg(s.order + c)];
+        const float4 j = onChip ? cs.impulses(c) : s.cons.impulses(c, make_float2(d.jn1, d.jt1));
+        d.jn0 = j.x; d.jt0 = j.y; d.jn1 = j.z; d.jt1 = j.w;
     }
     return true;
 }
 
-constexpr uint32_t SOLVE_CLUSTER_THREADS = 512;
+template <class Sync, class Bodies, bool PIPELINED = false>
+__device__ __forceinline__ bool color_and_solve(const DeviceWorld& w, const Bodies& B, Manifold* __restrict__ m,
+                                                uint32_t n, const SolveScratch& s, uint32_t velIters,
+                                                uint32_t posIters, uint32_t rank, uint32_t size, Sync sync,
+                                                uint32_t* __restrict__ outColors, uint32_t* __restrict__ status,
+                                                ConsSmem cs = ConsSmem{})
+{
+    uint32_t ncol = 0;
+    return color_manifolds(w, B, m, n, s, rank, size, sync, outColors, status, ncol) &&
+           solve_colored<Sync, Bodies, PIPELINED>(w, B, m, n, s, ncol, velIters, posIters, rank, size, sync, cs);
+}
 
-__global__ void __launch_bounds__(SOLVE_CLUSTER_THREADS, 1)
-k_color_solve_cluster(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, uint32_t velIters,
-                      uint32_t posIters, StepCounters* counters);
-__global__ void k_color_solve_grid(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, uint32_t velIters,
-                                   uint32_t posIters, uint32_t* bar, StepCounters* counters);
+// Single worlds whose bodies fit one CTA's shared memory (32 B each, up to BLOCK_SOLVE_BODIES): one CTA colours,
+// solves and links the islands, __syncthreads between colours.
+constexpr uint32_t BLOCK_SOLVE_BODIES = 6912;
+struct BlockSolve {
+    DeviceWorld w;
+    Manifold* m;
+    const uint32_t* nM;
+    SolveScratch s;            // colour counters in global memory, copied out for the readers of colour starts
+    uint32_t bodyCap;          // bodies of the shared-memory cache, >= w.nBodies
+    uint32_t velIters, posIters;
+    uint32_t* ufParent;        // [bodies] island roots out (smallest body index of the island)
+    uint32_t* ufFlag;          // [bodies] set to 1
+    StepCounters* counters;
+};
+// Host side: launches the one-CTA solver for about 'manifolds' manifolds.
+cudaError_t launch_color_solve_block(uint32_t manifolds, cudaStream_t stream, const BlockSolve& a);
+// Host side: raises the one-CTA solver's dynamic shared-memory limit (once per device).
+cudaError_t block_solver_init();
+
+// Larger single worlds: a cooperative grid colours the manifolds, then solves them as a dataflow over per-body
+// versions instead of barriers (k_color_solve_flow).
+constexpr uint32_t FLOW_VEL_WARPS = 16, FLOW_POS_WARPS = 4;   // warps of a CTA: velocity passes, position passes
+constexpr uint32_t FLOW_THREADS = 32 * (FLOW_VEL_WARPS + FLOW_POS_WARPS);
+struct FlowScratch {
+    float4* vel;       // [bodies] vx, vy, w, version
+    float4* pos;       // [bodies] x, y, -, version
+    Constraint* cons;  // [manifolds] records, 'pad' the rank and degree of a, of b: one byte each
+    float4* posRec;    // [2 x manifolds] position records: normal, penetration base, ranks; masses, bodies
+};
+__global__ void __launch_bounds__(FLOW_THREADS, 1)
+k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, FlowScratch f, uint32_t velIters,
+                   uint32_t posIters, uint32_t* bar, StepCounters* counters);
 
 // Batched worlds: teams of consecutive worlds (team k owns worlds [teamWorld[k], teamWorld[k + 1])), each coloured
 // and solved by one CTA with __syncthreads between colours. Teams are taken from the work counter *nextTeam (zeroed

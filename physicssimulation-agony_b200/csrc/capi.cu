@@ -199,8 +199,8 @@ struct Tree {
 
 struct DeviceInfo {
     int sms = 0;
-    int coopSolveBlocks = 0;   // co-resident CTAs of the grid solver
-    int solveCluster = 0;      // CTAs per cluster of the cluster solver (16 when the device allows it)
+    int flowBlocks = 0;        // co-resident CTAs of the grid solver
+    bool gridOnly = false;     // never the one-CTA solver
 };
 
 // glibc fmin / fmax (the reference's std::fmin / std::fmax on x86-64): the first argument unless the comparison
@@ -381,9 +381,6 @@ StagedWorld stage_world(const PackedArrays& a)
 // candidate pairs per collider; growing later synchronises the device and can take long on first touch of memory.
 constexpr uint32_t INITIAL_PAIRS_PER_COLLIDER = 8;
 
-// Manifold count above which the solver runs on the whole grid instead of one cluster.
-constexpr uint32_t GRID_SOLVE_THRESHOLD = 600000;
-
 }  // namespace
 
 // Launch limits of the solver kernels on a device (queried once per device and process).
@@ -396,39 +393,14 @@ static DeviceInfo probe_device(int device)
     if (it != cache.end()) return it->second;
     DeviceInfo dev;
     CK(cudaDeviceGetAttribute(&dev.sms, cudaDevAttrMultiProcessorCount, device));
+    CK(block_solver_init());
     int perSm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_color_solve_grid, 256, 0));
-    dev.coopSolveBlocks = std::max(1, perSm) * dev.sms;
-    // Largest cluster (16 non-portable, else 8, 4, 2) that can be resident.
-    dev.solveCluster = 1;
-    if (cudaFuncSetAttribute(k_color_solve_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-        cudaSuccess) {
-        for (int cl : {16, 8, 4, 2}) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(cl);
-            cfg.blockDim = dim3(SOLVE_CLUSTER_THREADS);
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = cl;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, k_color_solve_cluster, &cfg) == cudaSuccess &&
-                clusters >= 1) {
-                dev.solveCluster = cl;
-                break;
-            }
-        }
-    }
-    cudaGetLastError();
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_color_solve_flow, FLOW_THREADS, 0));
+    dev.flowBlocks = std::max(1, perSm) * dev.sms;
     // The narrow phase stages polygons in dynamic shared memory: up to 512 threads x NARROW_SMEM_PER_THREAD.
     CK(cudaFuncSetAttribute(k_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, int(512 * NARROW_SMEM_PER_THREAD)));
     // AG2D_SOLVER=grid forces the whole-grid solver (test hook for that variant).
-    if (const char* v = std::getenv("AG2D_SOLVER")) {
-        if (std::string(v) == "grid") dev.solveCluster = 1;
-    }
+    if (const char* v = std::getenv("AG2D_SOLVER")) dev.gridOnly = std::string(v) == "grid";
     cache[device] = dev;
     return dev;
 }
@@ -570,6 +542,8 @@ struct ag2d_world {
     bool hintsReady = false;   // this step's lookup wrote the hints
     DBuf<uint4> listA, listB;
     DBuf<unsigned long long> bodyMax, bodyMask;
+    DBuf<float4> flowVel, flowPos, flowPosRec;   // grid solver (FlowScratch)
+    DBuf<Constraint> flowCons;
     // Manifolds of sleeping islands (k_islands.cu): world-grouped records and the island (root body) of each, with
     // the back buffers the sleep pass scatters into. isleUpper bounds the count as the host knows it (0: empty).
     DBuf<Manifold> isle, bk_isle;
@@ -588,7 +562,8 @@ struct ag2d_world {
     DBuf<Manifold> sleepList;
     bool prevHoldsSleepers = false;   // the warm-start list still holds records moved to the store (compactPrev)
     bool islandsLinked = false;       // this step's team solver already linked the islands (phaseIslands skips it)
-    DBuf<Constraint> cons;
+    DBuf<float4> consQ;     // solver records (ConsRecords), their stride the manifold capacity they were sized for
+    DBuf<float> consPen;
     DBuf<uint2> pairBodies;
     // Islands.
     DBuf<uint32_t> ufParent, ufFlag, wakeIsland;
@@ -1380,7 +1355,8 @@ struct ag2d_world {
         listA.reserve(manifoldCap);
         listB.reserve(manifoldCap);
         pairBodies.reserve(manifoldCap);
-        cons.reserve(manifoldCap);
+        consQ.reserve(size_t(ConsRecords::FIELDS) * manifoldCap + 32);   // a warp prefetches whole lines
+        consPen.reserve(manifoldCap);
         hashCap = 16;
         while (hashCap < 2 * manifoldCap) hashCap <<= 1;
         hashKeys.reserve(hashCap);
@@ -1810,6 +1786,7 @@ struct ag2d_world {
     void phaseNarrow(bool warm = true)
     {
         const cudaStream_t s = stream;
+        islandsLinked = false;
         const uint32_t* nPairs = &dCounters.p->pairs;
         // Grid sized for the capacity, work bounded by the device-side pair count; the manifolds are compacted in
         // the same kernel.
@@ -2241,21 +2218,20 @@ struct ag2d_world {
     void phaseSolve()
     {
         const cudaStream_t s = stream;
-        CK(cudaMemsetAsync(bodyMax.p, 0, sizeof(unsigned long long) * std::max<uint32_t>(nBodies, 1), s));
-        CK(cudaMemsetAsync(bodyMask.p, 0, sizeof(unsigned long long) * std::max<uint32_t>(nBodies, 1), s));
-        CK(cudaMemsetAsync(bar.p, 0, 2 * sizeof(uint32_t), s));
         DeviceWorld w = view();
         Manifold* mm = manifolds.p;
         const uint32_t* nm = nManifolds.p;
-        SolveScratch scratch{color.p, order.p, bodyMax.p, bodyMask.p, colorCount.p, colorStart.p, cons.p, nullptr,
-                             listA.p, listB.p, pairBodies.p, hintsReady ? color.p : nullptr};
+        SolveScratch scratch{color.p, order.p, bodyMax.p, bodyMask.p, colorCount.p, colorStart.p,
+                             ConsRecords{consQ.p, consPen.p, manifoldCap}, nullptr, listA.p, listB.p, pairBodies.p, hintsReady ? color.p : nullptr};
         hintsReady = false;
         uint32_t vi = settings.velocity_iterations, pi = settings.position_iterations;
         StepCounters* ctr = dCounters.p;
         pbegin(10);
         if (nWorlds > 1) {
             // One CTA per world over the world-grouped manifold list; the teams also link their islands
-            // (phaseIslands then only decides sleep).
+            // (phaseIslands then only decides sleep). Teams too large for the body cache colour in global memory.
+            CK(cudaMemsetAsync(bodyMax.p, 0, sizeof(unsigned long long) * std::max<uint32_t>(nBodies, 1), s));
+            CK(cudaMemsetAsync(bodyMask.p, 0, sizeof(unsigned long long) * std::max<uint32_t>(nBodies, 1), s));
             CK(cudaMemsetAsync(nextWorld.p, 0, 2 * sizeof(uint32_t), s));
             k_island_init<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p);
             islandsLinked = true;
@@ -2284,28 +2260,26 @@ struct ag2d_world {
                 CK(cudaStreamWaitEvent(s, joinEvent, 0));
             }
             launches++;
-        } else if (lastManifolds <= GRID_SOLVE_THRESHOLD && dev.solveCluster > 1) {
-            // One thread-block cluster, hardware barriers between colours.
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(dev.solveCluster);
-            cfg.blockDim = dim3(SOLVE_CLUSTER_THREADS);
-            cfg.stream = s;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = dev.solveCluster;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            CK(cudaLaunchKernelEx(&cfg, k_color_solve_cluster, w, mm, nm, scratch, vi, pi, ctr));
+        } else if (nBodies <= BLOCK_SOLVE_BODIES && !dev.gridOnly) {
+            // One CTA, bodies in shared memory; it also links the islands.
+            const BlockSolve args{w, mm, nm, scratch, std::max<uint32_t>(nBodies, 1), vi, pi, ufParent.p, ufFlag.p, ctr};
+            CK(launch_color_solve_block(lastManifolds, s, args));
+            islandsLinked = true;
         } else {
-            // Whole-grid cooperative launch with the bounded software barrier.
+            // Whole-grid cooperative launch: about a warp of manifolds on each of a CTA's first four warps before a
+            // second CTA is added, up to every SM.
+            CK(cudaMemsetAsync(bodyMax.p, 0, sizeof(unsigned long long) * nBodies, s));
+            CK(cudaMemsetAsync(bodyMask.p, 0, sizeof(unsigned long long) * nBodies, s));
+            CK(cudaMemsetAsync(bar.p, 0, 2 * sizeof(uint32_t), s));
+            flowVel.reserve(nBodies); flowPos.reserve(nBodies); flowPosRec.reserve(2 * size_t(manifoldCap));
+            flowCons.reserve(manifoldCap);
+            FlowScratch flow{flowVel.p, flowPos.p, flowCons.p, flowPosRec.p};
             uint32_t* barp = bar.p;
             const uint32_t est = std::min<uint32_t>(manifoldCap, lastManifolds + lastManifolds / 2 + 1024);
-            const int grid = std::max(1, std::min<int>(dev.coopSolveBlocks, int(div_up(est, 256))));
-            void* args[] = {&w, &mm, &nm, &scratch, &vi, &pi, &barp, &ctr};
-            CK(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_color_solve_grid), dim3(grid), dim3(256), args,
-                                           0, s));
+            const int grid = std::max(1, std::min<int>(dev.flowBlocks, int(div_up(est, 128))));
+            void* args[] = {&w, &mm, &nm, &scratch, &flow, &vi, &pi, &barp, &ctr};
+            CK(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_color_solve_flow), dim3(grid), dim3(FLOW_THREADS),
+                                           args, 0, s));
         }
         pend(10);
         launches++;
@@ -4100,6 +4074,7 @@ int32_t ag2d_world_write(ag2d_world* world, int32_t field, const void* src, uint
             const uint32_t n = uint32_t(bytes / sizeof(Manifold));
             if (n > w.manifoldCap) w.reserveCapacities(std::max(n, w.pairCap), n);
             const bool prev = field == AG2D_PREV_MANIFOLDS;
+            w.islandsLinked = false;   // the solver's links are not this list's
             if (n) CK(cudaMemcpyAsync(prev ? w.prevManifolds.p : w.manifolds.p, src, bytes, cudaMemcpyHostToDevice, s));
             CK(cudaMemcpyAsync(prev ? w.nPrev.p : w.nManifolds.p, &n, 4, cudaMemcpyHostToDevice, s));
             if (prev) {

@@ -305,39 +305,238 @@ __global__ void k_wake_apply(DeviceWorld w, const uint32_t* __restrict__ wakeIsl
 // sequential Gauss-Seidel sweep in colour-major order.
 // ---------------------------------------------------------------------------------------------------------------
 
-// One thread-block cluster runs the whole colouring and solve with hardware cluster barriers between colours.
-__global__ void __launch_bounds__(SOLVE_CLUSTER_THREADS, 1)
-k_color_solve_cluster(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, uint32_t velIters,
-                      uint32_t posIters, StepCounters* counters)
+// A body's state and its version in one 16-byte word, read and written whole: a reader that sees the version it waits
+// for has the state that goes with it, without fences.
+__device__ __forceinline__ float4 flow_load(const float4* p)
 {
-    const cg::cluster_group cluster = cg::this_cluster();
-    const uint32_t rank = cluster.block_rank() * blockDim.x + threadIdx.x;
-    const uint32_t size = cluster.num_blocks() * blockDim.x;
-    color_and_solve(w, GlobalBodies{w.bvel, w.bpos, s.bodyMax, s.bodyMask}, m, *nM, s, velIters, posIters, rank, size,
-                    ClusterSync{},
-                    &counters->colors,
-                    &counters->status);
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 d;\n\tld.relaxed.gpu.global.b128 d, [%2];\n\tmov.b128 {%0, %1}, d;\n\t}"
+                 : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    return make_float4(__uint_as_float(uint32_t(lo)), __uint_as_float(uint32_t(lo >> 32)),
+                       __uint_as_float(uint32_t(hi)), __uint_as_float(uint32_t(hi >> 32)));
+}
+__device__ __forceinline__ void flow_store(float4* p, const float4& v)
+{
+    const unsigned long long lo = uint64_t(__float_as_uint(v.x)) | uint64_t(__float_as_uint(v.y)) << 32;
+    const unsigned long long hi = uint64_t(__float_as_uint(v.z)) | uint64_t(__float_as_uint(v.w)) << 32;
+    asm volatile("{\n\t.reg .b128 s;\n\tmov.b128 s, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], s;\n\t}"
+                 :: "l"(p), "l"(lo), "l"(hi) : "memory");
 }
 
-// Cooperative grid variant (bounded software grid barrier) for manifold counts beyond one cluster's reach.
-__global__ void k_color_solve_grid(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, uint32_t velIters,
-                                   uint32_t posIters, uint32_t* bar, StepCounters* counters)
+// One end of a constraint in the dataflow: waits until its body's version is 'need' (a body without a version, of
+// infinite mass, is always ready). Polled by a whole warp; false when the wait ran out somewhere on the grid.
+struct FlowEnd {
+    const float4* at;   // null: nothing to wait for
+    uint32_t need;
+};
+__device__ __forceinline__ bool flow_wait(const FlowEnd& a, const FlowEnd& b, float4& va, float4& vb,
+                                          const volatile uint32_t* status, uint32_t* statusOut)
+{
+    bool ra = a.at == nullptr, rb = b.at == nullptr;
+    for (uint32_t spins = 0;; spins++) {
+        if (!ra) { va = flow_load(a.at); ra = __float_as_uint(va.w) == a.need; }
+        if (!rb) { vb = flow_load(b.at); rb = __float_as_uint(vb.w) == b.need; }
+        if (__all_sync(0xffffffffu, ra && rb)) return true;
+        if ((spins & 1023u) == 1023u) {
+            const bool gone = (*status & STATUS_BARRIER_TIMEOUT) != 0;
+            if (__any_sync(0xffffffffu, gone)) return false;
+            if (spins > SPIN_LIMIT) { atomicOr(statusOut, STATUS_BARRIER_TIMEOUT); return false; }
+        }
+    }
+}
+
+// Whether slot c holds a record to solve. A record that names no body of the world is not one that the build above
+// wrote: it is reported and skipped, and the waits on it end.
+__device__ __forceinline__ bool flow_live(uint32_t c, const Constraint& k, uint32_t nBodies, uint32_t* status)
+{
+    if (c == 0xFFFFFFFFu) return false;
+    if (k.bodyA < nBodies && k.bodyB < nBodies) return true;
+    atomicOr(status, STATUS_BARRIER_TIMEOUT);
+    return false;
+}
+
+// Walks a warp's items of one pass: the manifolds in colour-major order, every colour padded to whole warps, chunk q
+// of 32 to warp q modulo the warps. A chunk has one colour, so its lanes never wait for one another.
+struct FlowWalk {
+    const uint32_t* start;    // colour starts (shared memory)
+    const uint32_t* chunk;    // first chunk of every colour (shared memory), [ncol] = the chunk count
+    uint32_t col;
+    __device__ __forceinline__ void seek(uint32_t q) { while (q >= chunk[col + 1]) col++; }
+    // This lane's slot of chunk q, or ~0u past the colour's end.
+    __device__ __forceinline__ uint32_t slot(uint32_t q) const
+    {
+        const uint32_t c = start[col] + (q - chunk[col]) * 32u + (threadIdx.x & 31u);
+        return c < start[col + 1] ? c : 0xFFFFFFFFu;
+    }
+};
+
+// Colouring and solve of a large single world on a cooperative grid. The passes have no barriers: a body's constraints
+// act on it in colour order, pass after pass, so its k-th update must follow its (k - 1)-th and nothing else. Every
+// body carries a version (the updates made so far) in the same 16-byte word as its velocity, and a constraint, the
+// r-th of the d around a body (both from the body's mask of colours), waits in pass p for version p d + r of each of
+// its moving bodies. Warps take the constraints in colour order within a pass and the passes in order, all warps are
+// resident, so the oldest unfinished constraint can always run. Velocity passes (warm start first) and position passes
+// touch different state and run on warps of their own. The order of the updates of every body is that of the
+// colour-major sweep, so the results are the same bit for bit.
+// Bound: the chain of updates along the contacts (a pass costs about one hop a colour, a hop one L2 round trip for
+// the store, half a poll and the arithmetic). With a grid barrier a colour instead, and on the sixteen SMs that one
+// thread-block cluster has, a pass over the pile of 100,000 bodies (128,000 manifolds, 14 colours) took 8 us a colour.
+// A colouring beyond the 64 first-fit colours has no rank in the masks: its passes run with the grid barrier.
+__global__ void __launch_bounds__(FLOW_THREADS, 1)
+k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, FlowScratch f, uint32_t velIters,
+                   uint32_t posIters, uint32_t* bar, StepCounters* counters)
 {
     const uint32_t rank = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t size = gridDim.x * blockDim.x;
-    color_and_solve(w, GlobalBodies{w.bvel, w.bpos, s.bodyMax, s.bodyMask}, m, *nM, s, velIters, posIters, rank,
-                    size, GridSync{bar, &counters->status},
-                    &counters->colors, &counters->status);
+    const uint32_t n = *nM;
+    const GlobalBodies B{w.bvel, w.bpos, s.bodyMax, s.bodyMask};
+    const GridSync sync{bar, &counters->status};
+    uint32_t ncol = 0;
+    if (!color_manifolds(w, B, m, n, s, rank, size, sync, &counters->colors, &counters->status, ncol)) return;
+    if (ncol > 64u) {
+        solve_colored(w, B, m, n, s, ncol, velIters, posIters, rank, size, sync);
+        return;
+    }
+    __shared__ uint32_t start[65], chunk[65];
+    for (uint32_t c = threadIdx.x; c <= ncol; c += blockDim.x) start[c] = __ldcg(s.colorStart + c);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t run = 0;
+        for (uint32_t c = 0; c < ncol; c++) { chunk[c] = run; run += (start[c + 1] - start[c] + 31u) >> 5; }
+        chunk[ncol] = run;
+    }
+    __syncthreads();
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t chunks = chunk[ncol];
+    const volatile uint32_t* status = &counters->status;
+    // Records of every manifold, before any velocity changes, each by the thread that solves it, and the bodies' words
+    // at version 0.
+    if (warp < FLOW_VEL_WARPS) {
+        FlowWalk walk{start, chunk, 0};
+        for (uint32_t q = warp * gridDim.x + blockIdx.x; q < chunks; q += FLOW_VEL_WARPS * gridDim.x) {
+            walk.seek(q);
+            const uint32_t c = walk.slot(q);
+            if (c == 0xFFFFFFFFu) continue;
+            const uint32_t mi = __ldcg(s.order + c);
+            Constraint k;
+            prep_constraint(w, B, m[mi], mi, k);
+            const unsigned long long below = (1ull << walk.col) - 1ull;
+            uint32_t ranks = 0;   // rank and degree of a, of b: one byte each
+            if (k.imA > 0.0f) {
+                const unsigned long long mask = __ldcg(s.bodyMask + k.bodyA);
+                ranks |= uint32_t(__popcll(mask & below)) | uint32_t(__popcll(mask)) << 8;
+            }
+            if (k.imB > 0.0f) {
+                const unsigned long long mask = __ldcg(s.bodyMask + k.bodyB);
+                ranks |= uint32_t(__popcll(mask & below)) << 16 | uint32_t(__popcll(mask)) << 24;
+            }
+            k.pad = __uint_as_float(ranks);
+            f.cons[c] = k;
+            f.posRec[2 * size_t(c)] = make_float4(k.nx, k.ny, k.penBase, __uint_as_float(ranks));
+            f.posRec[2 * size_t(c) + 1] = make_float4(k.imA, k.imB, __uint_as_float(k.bodyA), __uint_as_float(k.bodyB));
+        }
+    }
+    for (uint32_t b = rank; b < w.nBodies; b += size) {
+        const float4 v = w.bvel[b], p = w.bpos[b];
+        f.vel[b] = make_float4(v.x, v.y, v.z, 0.0f);
+        f.pos[b] = make_float4(p.x, p.y, 0.0f, 0.0f);
+    }
+    if (!sync()) return;
+    if (warp < FLOW_VEL_WARPS) {
+        const uint32_t q0 = warp * gridDim.x + blockIdx.x, qStep = FLOW_VEL_WARPS * gridDim.x;
+        if (q0 >= chunks) return;
+        const bool one = q0 + qStep >= chunks;   // one chunk: its records stay in registers
+        FlowWalk walk{start, chunk, 0};
+        walk.seek(q0);
+        uint32_t c = walk.slot(q0);
+        Constraint k, nxt;
+        if (c != 0xFFFFFFFFu) k = f.cons[c];
+        for (uint32_t pass = 0; pass <= velIters; pass++) {
+            for (uint32_t q = q0; q < chunks; q += qStep) {
+                // The next record is fetched while this one waits for its bodies.
+                uint32_t cNext = c;
+                if (!one) {
+                    uint32_t qn = q + qStep;
+                    if (qn >= chunks) { qn = q0; walk.col = 0; }
+                    walk.seek(qn);
+                    cNext = walk.slot(qn);
+                    if (cNext != 0xFFFFFFFFu) nxt = f.cons[cNext];
+                }
+                const bool live = flow_live(c, k, w.nBodies, &counters->status);
+                const uint32_t ranks = live ? __float_as_uint(k.pad) : 0u;
+                const bool mA = live && k.imA > 0.0f, mB = live && k.imB > 0.0f;
+                const FlowEnd a{mA ? f.vel + k.bodyA : nullptr, pass * ((ranks >> 8) & 255u) + (ranks & 255u)};
+                const FlowEnd b{mB ? f.vel + k.bodyB : nullptr, pass * (ranks >> 24) + ((ranks >> 16) & 255u)};
+                float4 vA = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vB = vA;
+                if (live && !mA) vA = w.bvel[k.bodyA];
+                if (live && !mB) vB = w.bvel[k.bodyB];
+                if (!flow_wait(a, b, vA, vB, status, &counters->status)) return;
+                if (live) {
+                    vA.w = k.imA;
+                    vB.w = k.imB;
+                    if (pass == 0) {
+                        warm_solve(k, vA, vB);
+                    } else {
+                        velocity_solve(k, vA, vB);
+                        if (!one) *reinterpret_cast<float4*>(&f.cons[c].jn0) = make_float4(k.jn0, k.jt0, k.jn1, k.jt1);
+                    }
+                    if (mA) {
+                        flow_store(f.vel + k.bodyA, make_float4(vA.x, vA.y, vA.z, __uint_as_float(a.need + 1u)));
+                        if (pass == velIters && (ranks & 255u) + 1u == ((ranks >> 8) & 255u)) w.bvel[k.bodyA] = vA;
+                    }
+                    if (mB) {
+                        flow_store(f.vel + k.bodyB, make_float4(vB.x, vB.y, vB.z, __uint_as_float(b.need + 1u)));
+                        if (pass == velIters && ((ranks >> 16) & 255u) + 1u == ranks >> 24) w.bvel[k.bodyB] = vB;
+                    }
+                    if (pass == velIters) {
+                        Manifold& d = m[k.manifold];
+                        d.jn0 = k.jn0; d.jt0 = k.jt0; d.jn1 = k.jn1; d.jt1 = k.jt1;
+                    }
+                }
+                if (!one) { k = nxt; c = cNext; }
+            }
+        }
+    } else {
+        const uint32_t q0 = (warp - FLOW_VEL_WARPS) * gridDim.x + blockIdx.x, qStep = FLOW_POS_WARPS * gridDim.x;
+        for (uint32_t pass = 0; pass < posIters; pass++) {
+            FlowWalk walk{start, chunk, 0};
+            for (uint32_t q = q0; q < chunks; q += qStep) {
+                walk.seek(q);
+                const uint32_t c = walk.slot(q);
+                Constraint k;
+                uint32_t ranks = 0;
+                k.imA = k.imB = 0.0f;
+                if (c != 0xFFFFFFFFu) {
+                    const float4 r0 = __ldcg(f.posRec + 2 * size_t(c)), r1 = __ldcg(f.posRec + 2 * size_t(c) + 1);
+                    k.nx = r0.x; k.ny = r0.y; k.penBase = r0.z; ranks = __float_as_uint(r0.w);
+                    k.imA = r1.x; k.imB = r1.y; k.bodyA = __float_as_uint(r1.z); k.bodyB = __float_as_uint(r1.w);
+                }
+                const bool live = flow_live(c, k, w.nBodies, &counters->status);
+                const bool mA = live && k.imA > 0.0f, mB = live && k.imB > 0.0f;
+                const FlowEnd a{mA ? f.pos + k.bodyA : nullptr, pass * ((ranks >> 8) & 255u) + (ranks & 255u)};
+                const FlowEnd b{mB ? f.pos + k.bodyB : nullptr, pass * (ranks >> 24) + ((ranks >> 16) & 255u)};
+                float4 pA = make_float4(0.0f, 0.0f, 0.0f, 0.0f), pB = pA;
+                if (live && !mA) pA = w.bpos[k.bodyA];
+                if (live && !mB) pB = w.bpos[k.bodyB];
+                if (!flow_wait(a, b, pA, pB, status, &counters->status)) return;
+                if (live) {
+                    position_solve(k, pA, pB);
+                    if (mA) {
+                        flow_store(f.pos + k.bodyA, make_float4(pA.x, pA.y, 0.0f, __uint_as_float(a.need + 1u)));
+                        if (pass + 1u == posIters && (ranks & 255u) + 1u == ((ranks >> 8) & 255u))
+                            *reinterpret_cast<float2*>(w.bpos + k.bodyA) = make_float2(pA.x, pA.y);
+                    }
+                    if (mB) {
+                        flow_store(f.pos + k.bodyB, make_float4(pB.x, pB.y, 0.0f, __uint_as_float(b.need + 1u)));
+                        if (pass + 1u == posIters && ((ranks >> 16) & 255u) + 1u == ranks >> 24)
+                            *reinterpret_cast<float2*>(w.bpos + k.bodyB) = make_float2(pB.x, pB.y);
+                    }
+                }
+            }
+        }
+    }
 }
 
-// Batched worlds: each CTA takes the next team of consecutive worlds, whose manifolds are one contiguous range of
-// the world-grouped list, and colours + solves that range as one problem (the worlds share no body, so their
-// colour classes simply merge). Priorities are world-local indices: every world gets the colouring, hence the
-// solving order, it has when stepped on its own, whichever team it is in. A team whose bodies fit the dynamic
-// shared memory (bodyCap bodies) keeps their velocities, poses and colouring words there. The solver is bound by
-// load latency and barriers, so what counts is how many teams an SM holds at once: the colouring words share the
-// body cache when the records stay in global memory (32 B of shared memory a body), and the unpipelined variant is
-// held to 64 registers a thread (1024 threads an SM).
 // Union-find over a parent array in shared or global memory (generic addressing; volatile reads see other SMs'
 // links), linking the larger root under the smaller, so every island's root is its smallest body index whatever
 // the order of the links (IslandManager's islands, the same roots k_island_union gives).
@@ -363,6 +562,89 @@ __device__ __forceinline__ void team_union(uint32_t* par, uint32_t a, uint32_t b
     }
 }
 
+// A single world in one CTA: bodies in shared memory (colouring words first, SharedBodies lazy), then its islands.
+template <uint32_t THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_color_solve_block(BlockSolve a)
+{
+    extern __shared__ float4 teamCache[];
+    __shared__ uint32_t colorCount[COLOR_SLOTS];
+    __shared__ uint32_t colorStart[MAX_COLORS + 1];
+    const DeviceWorld& w = a.w;
+    const uint32_t n = *a.nM, nb = w.nBodies;
+    uint32_t* par = reinterpret_cast<uint32_t*>(teamCache);
+    if (n > 0) {
+        float4* vel = teamCache;
+        float4* pos = teamCache + a.bodyCap;
+        auto* maxW = reinterpret_cast<unsigned long long*>(teamCache);
+        unsigned long long* maskW = maxW + a.bodyCap;
+        for (uint32_t i = threadIdx.x; i < nb; i += THREADS) {
+            maxW[i] = 0ull;
+            maskW[i] = 0ull;
+        }
+        __syncthreads();
+        SharedBodies sb{vel, pos, maxW, maskW, 0u};
+        sb.count = nb;
+        sb.gvel = w.bvel;
+        sb.gpos = w.bpos;
+        SolveScratch s = a.s;
+        s.colorCount = colorCount;
+        s.colorStart = colorStart;
+        const bool solved = color_and_solve<BlockSync, SharedBodies>(w, sb, a.m, n, s, a.velIters, a.posIters,
+                                                                     threadIdx.x, THREADS, BlockSync{},
+                                                                     &a.counters->colors, &a.counters->status);
+        __syncthreads();
+        if (!solved) return;   // the step is redone or fails: the bodies stay as they were
+        for (uint32_t i = threadIdx.x; i < nb; i += THREADS) {
+            w.bvel[i] = vel[i];
+            w.bpos[i] = pos[i];
+        }
+        const uint32_t colors = min(__ldcg(&a.counters->colors), MAX_COLORS);
+        for (uint32_t c = threadIdx.x; c <= colors; c += THREADS) a.s.colorStart[c] = colorStart[c];
+        __syncthreads();
+    }
+    for (uint32_t i = threadIdx.x; i < nb; i += THREADS) par[i] = i;
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < n; j += THREADS) {
+        const uint2 q = a.s.pairBodies[j];
+        const uint32_t x = q.x & PAIR_BODY, y = q.y & PAIR_BODY;
+        if (w.bstate[x] == STATE_DYNAMIC && w.bstate[y] == STATE_DYNAMIC) team_union(par, x, y);
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < nb; i += THREADS) {
+        a.ufParent[i] = team_find(par, i);
+        a.ufFlag[i] = 1u;
+    }
+}
+
+cudaError_t block_solver_init()
+{
+    const int bytes = int(team_smem_bytes(BLOCK_SOLVE_BODIES, 0));
+    for (const void* k : {reinterpret_cast<const void*>(k_color_solve_block<128>),
+                          reinterpret_cast<const void*>(k_color_solve_block<512>),
+                          reinterpret_cast<const void*>(k_color_solve_block<1024>)}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_color_solve_block(uint32_t manifolds, cudaStream_t stream, const BlockSolve& a)
+{
+    const size_t smem = team_smem_bytes(a.bodyCap, 0);
+    if (manifolds <= 512) k_color_solve_block<128><<<1, 128, smem, stream>>>(a);
+    else if (manifolds <= 4096) k_color_solve_block<512><<<1, 512, smem, stream>>>(a);
+    else k_color_solve_block<1024><<<1, 1024, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
+// Batched worlds: each CTA takes the next team of consecutive worlds, whose manifolds are one contiguous range of
+// the world-grouped list, and colours + solves that range as one problem (the worlds share no body, so their
+// colour classes simply merge). Priorities are world-local indices: every world gets the colouring, hence the
+// solving order, it has when stepped on its own, whichever team it is in. A team whose bodies fit the dynamic
+// shared memory (bodyCap bodies) keeps their velocities, poses and colouring words there. The solver is bound by
+// load latency and barriers, so what counts is how many teams an SM holds at once: the colouring words share the
+// body cache when the records stay in global memory (32 B of shared memory a body), and the unpipelined variant is
+// held to 64 registers a thread (1024 threads an SM).
 template <uint32_t THREADS, bool PIPELINED>
 __global__ void __launch_bounds__(THREADS, PIPELINED ? 1 : 1024 / THREADS) k_color_solve_teams(TeamLaunch a)
 {
@@ -388,7 +670,7 @@ __global__ void __launch_bounds__(THREADS, PIPELINED ? 1 : 1024 / THREADS) k_col
         for (uint32_t i = lo + threadIdx.x; i < hi; i += THREADS)
             prio[i] = priority_hash(i - a.manSeg[w.bodyWorld[w.cbody[m[i].a]]]);
         const SolveScratch ls{a.s.color + lo, a.s.order + lo, a.s.bodyMax, a.s.bodyMask, colorCount, colorStart,
-                              a.s.cons + lo, prio + lo, a.s.listA + lo, a.s.listB + lo, a.s.pairBodies + lo,
+                              a.s.cons.from(lo), prio + lo, a.s.listA + lo, a.s.listB + lo, a.s.pairBodies + lo,
                               a.s.hint ? a.s.hint + lo : nullptr};
         const uint32_t b0 = w.worldBodyStart[w0], nb = w.worldBodyStart[w1] - b0;
         if (nb <= a.bodyCap) {

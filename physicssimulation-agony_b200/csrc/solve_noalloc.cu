@@ -25,8 +25,9 @@ constexpr uint32_t NOALLOC_MAX_BODIES = AG2D_SOLVE_NOALLOC_MAX_BODIES;
 constexpr uint32_t NOALLOC_THREADS = 512;
 
 // Scratch layout (byte offsets; every part 256-byte aligned).
-constexpr size_t NA_CONS = 0;                                                         // Constraint[M]
-constexpr size_t NA_COLOR = NA_CONS + size_t(NOALLOC_MAX_MANIFOLDS) * sizeof(Constraint);   // u32[M]
+constexpr size_t NA_CONS = 0;                                                         // float4[7 M], ConsRecords::q
+constexpr size_t NA_PEN = NA_CONS + size_t(NOALLOC_MAX_MANIFOLDS) * 16 * ConsRecords::FIELDS;   // float[M]
+constexpr size_t NA_COLOR = NA_PEN + size_t(NOALLOC_MAX_MANIFOLDS) * 4;               // u32[M]
 constexpr size_t NA_ORDER = NA_COLOR + size_t(NOALLOC_MAX_MANIFOLDS) * 4;            // u32[M]
 constexpr size_t NA_LIST_A = NA_ORDER + size_t(NOALLOC_MAX_MANIFOLDS) * 4;           // uint4[M]
 constexpr size_t NA_LIST_B = NA_LIST_A + size_t(NOALLOC_MAX_MANIFOLDS) * 16;         // uint4[M]
@@ -61,7 +62,9 @@ k_color_solve_static(DeviceWorld w, Manifold* m, uint32_t n, unsigned char* scra
     }
     __syncthreads();
     const SolveScratch s{reinterpret_cast<uint32_t*>(scratch + NA_COLOR), reinterpret_cast<uint32_t*>(scratch + NA_ORDER),
-                         bodyMax, bodyMask, colorCount, colorStart, reinterpret_cast<Constraint*>(scratch + NA_CONS),
+                         bodyMax, bodyMask, colorCount, colorStart,
+                         ConsRecords{reinterpret_cast<float4*>(scratch + NA_CONS), reinterpret_cast<float*>(scratch + NA_PEN),
+                                     NOALLOC_MAX_MANIFOLDS},
                          nullptr, reinterpret_cast<uint4*>(scratch + NA_LIST_A),
                          reinterpret_cast<uint4*>(scratch + NA_LIST_B), reinterpret_cast<uint2*>(scratch + NA_PAIRS)};
     color_and_solve(w, GlobalBodies{w.bvel, w.bpos, bodyMax, bodyMask}, m, n, s, velIters, posIters, threadIdx.x,
