@@ -156,8 +156,26 @@ __device__ __forceinline__ void warm_constraint(const Bodies& B, const Constrain
     if (k.imB > 0.0f) B.setV(k.bodyB, vB);
 }
 
+// What the block solve of a two-point contact takes from its record alone, the same in every iteration: the 2x2
+// matrix and the reciprocal of its determinant, negative where the matrix is too ill-conditioned to use it.
+struct BlockMatrix {
+    float K00, K01, K11, invDet;
+};
+__device__ __forceinline__ BlockMatrix block_matrix(const Constraint& k)
+{
+    BlockMatrix b;
+    const float effMass = k.imA + k.imB;
+    b.K00 = effMass + k.rAn0 * k.rAn0 * k.iIA + k.rBn0 * k.rBn0 * k.iIB;
+    b.K11 = effMass + k.rAn1 * k.rAn1 * k.iIA + k.rBn1 * k.rBn1 * k.iIB;
+    b.K01 = effMass + k.rAn0 * k.rAn1 * k.iIA + k.rBn0 * k.rBn1 * k.iIB;
+    const float det = b.K00 * b.K11 - b.K01 * b.K01;
+    const float maxK = rfmaxf(b.K00, b.K11);
+    b.invDet = maxK * maxK < 1000.0f * det ? 1.0f / det : -1.0f;
+    return b;
+}
+
 // One velocity iteration of one constraint on its two bodies' velocities held in registers.
-__device__ __forceinline__ void velocity_solve(Constraint& k, float4& vA, float4& vB)
+__device__ __forceinline__ void velocity_solve(Constraint& k, const BlockMatrix& bm, float4& vA, float4& vB)
 {
     const float imA = k.imA, imB = k.imB, iIA = k.iIA, iIB = k.iIB;
     const float nx = k.nx, ny = k.ny, tx = -ny, ty = nx;
@@ -193,7 +211,6 @@ __device__ __forceinline__ void velocity_solve(Constraint& k, float4& vA, float4
             vB.z = vB.z + dj * k.rBt0 * iIB;
         }
     } else {
-        const float effMass = imA + imB;
         float jnArr0 = 0.0f, jnArr1 = 0.0f;
         bool ok = false;
         {
@@ -201,17 +218,13 @@ __device__ __forceinline__ void velocity_solve(Constraint& k, float4& vA, float4
             const float vn0 = dvn + k.rBn0 * vB.z - k.rAn0 * vA.z;
             const float vn1 = dvn + k.rBn1 * vB.z - k.rAn1 * vA.z;
             const float a0 = k.jn0, a1 = k.jn1;
-            const float K00 = effMass + k.rAn0 * k.rAn0 * iIA + k.rBn0 * k.rBn0 * iIB;
-            const float K11 = effMass + k.rAn1 * k.rAn1 * iIA + k.rBn1 * k.rBn1 * iIB;
-            const float K01 = effMass + k.rAn0 * k.rAn1 * iIA + k.rBn0 * k.rBn1 * iIB;
+            const float K00 = bm.K00, K11 = bm.K11, K01 = bm.K01;
             const float b0 = k.bias0 - vn0 + K00 * a0 + K01 * a1;
             const float b1 = k.bias1 - vn1 + K01 * a0 + K11 * a1;
             const float EPS = 1e-6f;
             float x0 = 0.0f, x1 = 0.0f;
-            const float det = K00 * K11 - K01 * K01;
-            const float maxK = rfmaxf(K00, K11);
-            if (maxK * maxK < 1000.0f * det) {
-                const float invDet = 1.0f / det;
+            if (bm.invDet >= 0.0f) {
+                const float invDet = bm.invDet;
                 const float s0 = (K11 * b0 - K01 * b1) * invDet;
                 const float s1 = (K00 * b1 - K01 * b0) * invDet;
                 if (s0 >= -EPS && s1 >= -EPS) { x0 = rfmaxf(s0, 0.0f); x1 = rfmaxf(s1, 0.0f); ok = true; }
@@ -279,10 +292,10 @@ __device__ __forceinline__ void velocity_solve(Constraint& k, float4& vA, float4
 }
 
 template <class Bodies>
-__device__ __forceinline__ void velocity_constraint(const Bodies& B, Constraint& k)
+__device__ __forceinline__ void velocity_constraint(const Bodies& B, Constraint& k, const BlockMatrix& bm)
 {
     float4 vA = B.v(k.bodyA), vB = B.v(k.bodyB);
-    velocity_solve(k, vA, vB);
+    velocity_solve(k, bm, vA, vB);
     if (k.imA > 0.0f) B.setV(k.bodyA, vA);
     if (k.imB > 0.0f) B.setV(k.bodyB, vB);
 }
@@ -321,8 +334,9 @@ constexpr uint32_t COLOR_AGE_SHIFT = 24;
 constexpr uint32_t COLOR_MASK = (1u << COLOR_AGE_SHIFT) - 1u;
 constexpr uint32_t COLOR_KEEP_STEPS = 16;
 
-// Colour counters: one per colour, then the lengths of the two uncoloured lists, then the colour count.
-constexpr uint32_t COLOR_SLOTS = MAX_COLORS + 4;
+// Colour counters: one per colour, then the lengths of the two uncoloured lists, then the colour count, then a second
+// counter per colour (one-point contacts placed from the colour's end).
+constexpr uint32_t COLOR_SLOTS = 2 * MAX_COLORS + 4;
 // Colours 0..63 are chosen first-fit from a body's 64-bit mask of neighbouring colours; a manifold whose bodies see
 // all 64 taken gets colour 64 + its round (unique to the round, so still conflict-free).
 constexpr uint32_t MAX_ROUNDS = MAX_COLORS - 64;
@@ -330,12 +344,12 @@ constexpr uint32_t MAX_ROUNDS = MAX_COLORS - 64;
 // Solver records in global memory, structure of arrays: field f of record c at q[f * stride + c], so that a warp that
 // takes 32 consecutive records reads every field as four full lines. (As 128-byte structures a lane apart, each
 // 16-byte load of a warp touched 32 lines, and the load unit, not latency or bandwidth, bounded every pass: one CTA on
-// 3,265 manifolds took 4.5 us a colour.) A record with one contact point leaves out fields 5 and 6.
+// 3,265 manifolds took 4.5 us a colour.) A record with one contact point leaves out fields 5 to 7.
 struct ConsRecords {
     float4* q;
     float* pen;        // penetration base
     uint32_t stride;
-    static constexpr uint32_t FIELDS = 7;
+    static constexpr uint32_t FIELDS = 8;
     __device__ __forceinline__ ConsRecords from(uint32_t c) const { return ConsRecords{q + c, pen + c, stride}; }
     __device__ __forceinline__ void store(uint32_t c, const Constraint& k) const
     {
@@ -349,6 +363,8 @@ struct ConsRecords {
         if (k.count != 1u) {
             r[5 * st] = make_float4(k.jn1, k.jt1, k.nm1, k.tm1);
             r[6 * st] = make_float4(k.rAn1, k.rBn1, k.rAt1, k.rBt1);
+            const BlockMatrix b = block_matrix(k);
+            r[7 * st] = make_float4(b.K00, b.K01, b.K11, b.invDet);
         }
         pen[c] = k.penBase;
     }
@@ -362,7 +378,7 @@ struct ConsRecords {
         k.nx = h.z; k.ny = h.w;
         k.imA = ms.x; k.imB = ms.y; k.iIA = ms.z; k.iIB = ms.w;
     }
-    __device__ __forceinline__ void load(uint32_t c, uint32_t kind, Constraint& k) const;
+    __device__ __forceinline__ void load(uint32_t c, uint32_t kind, Constraint& k, BlockMatrix& bm) const;
     __device__ __forceinline__ void storeImpulses(uint32_t c, const Constraint& k) const
     {
         *reinterpret_cast<float2*>(q + 2 * size_t(stride) + c) = make_float2(k.jn0, k.jt0);
@@ -380,8 +396,7 @@ struct ConsRecords {
     __device__ __forceinline__ void prefetch(uint32_t c0) const
     {
         const uint32_t lane = threadIdx.x & 31u;
-        if (lane < 4u * FIELDS)
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(q + size_t(lane >> 2) * stride + c0 + (lane & 3u) * 8u));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(q + size_t(lane >> 2) * stride + c0 + (lane & 3u) * 8u));
     }
 };
 
@@ -471,7 +486,7 @@ constexpr uint32_t CONS_SMEM_BYTES = ConsSmem::FIELDS * sizeof(float4);
 // Phases of the solve: what a phase does with its records.
 constexpr uint32_t PHASE_WARM = 0, PHASE_VELOCITY = 1, PHASE_POSITION = 2;
 
-__device__ __forceinline__ void ConsRecords::load(uint32_t c, uint32_t kind, Constraint& k) const
+__device__ __forceinline__ void ConsRecords::load(uint32_t c, uint32_t kind, Constraint& k, BlockMatrix& bm) const
 {
     loadHead(c, k);
     if (kind == PHASE_POSITION) {
@@ -488,6 +503,10 @@ __device__ __forceinline__ void ConsRecords::load(uint32_t c, uint32_t kind, Con
         const float4 m1 = r[5 * st], r1 = r[6 * st];
         k.jn1 = m1.x; k.jt1 = m1.y; k.nm1 = m1.z; k.tm1 = m1.w;
         k.rAn1 = r1.x; k.rBn1 = r1.y; k.rAt1 = r1.z; k.rBt1 = r1.w;
+        if (kind == PHASE_VELOCITY) {
+            const float4 b = r[7 * st];
+            bm.K00 = b.x; bm.K01 = b.y; bm.K11 = b.z; bm.invDet = b.w;
+        }
     } else {
         k.jn1 = 0.0f; k.jt1 = 0.0f; k.nm1 = 0.0f; k.tm1 = 0.0f;
         k.rAn1 = 0.0f; k.rBn1 = 0.0f; k.rAt1 = 0.0f; k.rBt1 = 0.0f;
@@ -507,12 +526,12 @@ __device__ __forceinline__ void prefetch_colour(const SolveScratch& s, uint32_t 
 // One phase's step on a record held in registers; a velocity step writes the record's impulses back.
 template <class Bodies>
 __device__ __forceinline__ void solve_record(const Bodies& B, const ConsRecords& cons, uint32_t c, uint32_t kind,
-                                             Constraint& k)
+                                             Constraint& k, const BlockMatrix& bm)
 {
     if (kind == PHASE_WARM) {
         warm_constraint(B, k);
     } else if (kind == PHASE_VELOCITY) {
-        velocity_constraint(B, k);
+        velocity_constraint(B, k, bm);
         cons.storeImpulses(c, k);
     } else {
         position_constraint(B, k);
@@ -536,28 +555,30 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
     };
     constexpr uint32_t NO_REC = 0xFFFFFFFFu;
     Constraint nxt;
+    BlockMatrix nxtBm;
     uint32_t cNext = NO_REC;
     if (nPhase) {
         const uint32_t c0 = Sync::ld(s.colorStart) + rank;
-        if (c0 < Sync::ld(s.colorStart + 1)) { s.cons.load(c0, kindOf(0), nxt); cNext = c0; }
+        if (c0 < Sync::ld(s.colorStart + 1)) { s.cons.load(c0, kindOf(0), nxt, nxtBm); cNext = c0; }
     }
     for (uint32_t ph = 0; ph < nPhase; ph++) {
         const uint32_t col = ph % ncol, kind = kindOf(ph);
         const uint32_t end = Sync::ld(s.colorStart + col + 1);
         Constraint k = nxt;
+        BlockMatrix bm = nxtBm;
         uint32_t c = cNext;   // NO_REC (above every end) when this thread has no record in the phase
         cNext = NO_REC;
         if (ph + 1 < nPhase) {
             const uint32_t col2 = (ph + 1) % ncol;
             const uint32_t c2 = Sync::ld(s.colorStart + col2) + rank;
-            if (c2 < Sync::ld(s.colorStart + col2 + 1)) { s.cons.load(c2, kindOf(ph + 1), nxt); cNext = c2; }
+            if (c2 < Sync::ld(s.colorStart + col2 + 1)) { s.cons.load(c2, kindOf(ph + 1), nxt, nxtBm); cNext = c2; }
         }
         while (c < end) {
-            solve_record(B, s.cons, c, kind, k);
+            solve_record(B, s.cons, c, kind, k, bm);
             // One colour: the next phase's record is this one, loaded before this phase's impulses.
             if (cNext == c) { nxt.jn0 = k.jn0; nxt.jt0 = k.jt0; nxt.jn1 = k.jn1; nxt.jt1 = k.jt1; }
             c += size;   // a colour larger than the team
-            if (c < end) s.cons.load(c, kind, k);
+            if (c < end) s.cons.load(c, kind, k, bm);
         }
         if (!sync()) return false;
     }
@@ -576,8 +597,9 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
 // cannot share a dynamic body: their predecessors were coloured together last step, and a body's dynamic flag
 // (finite mass) does not change between steps. The other manifolds run the Jones-Plassmann rounds around the kept
 // colours. With no hints every manifold runs the rounds. s.color holds colour | age << COLOR_AGE_SHIFT.
-// s.pairBodies words: body index | PAIR_DYNAMIC (finite mass) | PAIR_KEPT (first word: colour carried over).
-constexpr uint32_t PAIR_DYNAMIC = 0x80000000u, PAIR_KEPT = 0x40000000u, PAIR_BODY = 0x3FFFFFFFu;
+// s.pairBodies words: body index | PAIR_DYNAMIC (finite mass) | PAIR_KEPT (first word: colour carried over) or
+// PAIR_TWO (second word: not a one-point contact).
+constexpr uint32_t PAIR_DYNAMIC = 0x80000000u, PAIR_KEPT = 0x40000000u, PAIR_TWO = 0x40000000u, PAIR_BODY = 0x3FFFFFFFu;
 
 template <class Sync, class Bodies>
 __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Manifold* __restrict__ m, uint32_t n,
@@ -604,7 +626,7 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
             if (dA) atomicOr(B.maskWord(bA), 1ull << h);
             if (dB) atomicOr(B.maskWord(bB), 1ull << h);
         }
-        s.pairBodies[i] = make_uint2(bA | (dA ? DYN : 0u) | (kept ? KEPT : 0u), bB | (dB ? DYN : 0u));
+        s.pairBodies[i] = make_uint2(bA | (dA ? DYN : 0u) | (kept ? KEPT : 0u), bB | (dB ? DYN : 0u) | (m[i].count != 1u ? PAIR_TWO : 0u));
     }
     if (s.hint) {
         for (int o = 16; o > 0; o >>= 1) keptTop = max(keptTop, __shfl_xor_sync(0xffffffffu, keptTop, o));
@@ -636,8 +658,8 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
                 if (j0 + u * size >= len) break;
                 if (e[u].z & KEPT) continue;
                 const unsigned long long key = tag | e[u].y;
-                if (e[u].z & DYN) atomicMax(B.maxWord(e[u].z & ~DYN), key);
-                if (e[u].w & DYN) atomicMax(B.maxWord(e[u].w & ~DYN), key);
+                if (e[u].z & DYN) atomicMax(B.maxWord(e[u].z & PAIR_BODY), key);
+                if (e[u].w & DYN) atomicMax(B.maxWord(e[u].w & PAIR_BODY), key);
             }
         }
         if (!sync()) return false;
@@ -652,7 +674,7 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
                 if (e[u].z & KEPT) continue;
                 const uint32_t i = e[u].x;
                 const unsigned long long key = tag | e[u].y;
-                const uint32_t bA = e[u].z & ~DYN, bB = e[u].w & ~DYN;
+                const uint32_t bA = e[u].z & PAIR_BODY, bB = e[u].w & PAIR_BODY;
                 const bool dA = (e[u].z & DYN) != 0, dB = (e[u].w & DYN) != 0;
                 if ((!dA || B.ldWord(B.maxWord(bA)) == key) && (!dB || B.ldWord(B.maxWord(bB)) == key)) {
                     const unsigned long long used = (dA ? B.ldWord(B.maskWord(bA)) : 0ull) |
@@ -685,9 +707,14 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
         atomicMax(outColors, ncol);
     }
     if (!sync()) return false;
+    // Within a colour (independent contacts, any order) two-point contacts come first and one-point contacts last, so
+    // that few warps run both solves.
     for (uint32_t i = rank; i < n; i += size) {
         const uint32_t c = s.color[i] & COLOR_MASK;
-        s.order[Sync::ld(s.colorStart + c) + atomicAdd(s.colorCount + c, 1u)] = i;
+        const uint32_t at = s.pairBodies[i].y & PAIR_TWO
+                                ? Sync::ld(s.colorStart + c) + atomicAdd(s.colorCount + c, 1u)
+                                : Sync::ld(s.colorStart + c + 1) - 1u - atomicAdd(s.colorCount + MAX_COLORS + 4 + c, 1u);
+        s.order[at] = i;
     }
     return sync();
 }
@@ -723,8 +750,9 @@ __device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* _
             const uint32_t end = Sync::ld(s.colorStart + col + 1);
             for (uint32_t c = Sync::ld(s.colorStart + col) + rank; c < end; c += size) {
                 Constraint k;
+                BlockMatrix bm;
                 if (onChip) cs.load(c, k);
-                else s.cons.load(c, PHASE_WARM, k);
+                else s.cons.load(c, PHASE_WARM, k, bm);
                 warm_constraint(B, k);
             }
             if (!sync()) return false;
@@ -741,11 +769,16 @@ __device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* _
                 const uint32_t total = pos ? posBase + count : count;
                 for (uint32_t j = rank; j < total; j += size) {
                     Constraint k;
+                    BlockMatrix bm;
                     if (vel && j < count) {
                         const uint32_t c = begin + j;
-                        if (onChip) cs.load(c, k);
-                        else s.cons.load(c, PHASE_VELOCITY, k);
-                        velocity_constraint(B, k);
+                        if (onChip) {
+                            cs.load(c, k);
+                            bm = block_matrix(k);
+                        } else {
+                            s.cons.load(c, PHASE_VELOCITY, k, bm);
+                        }
+                        velocity_constraint(B, k, bm);
                         if (onChip) cs.storeImpulses(c, k);
                         else s.cons.storeImpulses(c, k);
                     } else if (j >= posBase) {
@@ -754,7 +787,7 @@ __device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* _
                             cs.loadHead(c, k);
                             cs.loadMasses(c, k);
                         } else {
-                            s.cons.load(c, PHASE_POSITION, k);
+                            s.cons.load(c, PHASE_POSITION, k, bm);
                         }
                         position_constraint(B, k);
                     }

@@ -463,6 +463,7 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
                     if (cNext != 0xFFFFFFFFu) nxt = f.cons[cNext];
                 }
                 const bool live = flow_live(c, k, w.nBodies, &counters->status);
+                const BlockMatrix bm = block_matrix(k);   // needs no body: done before the wait
                 const uint32_t ranks = live ? __float_as_uint(k.pad) : 0u;
                 const bool mA = live && k.imA > 0.0f, mB = live && k.imB > 0.0f;
                 const FlowEnd a{mA ? f.vel + k.bodyA : nullptr, pass * ((ranks >> 8) & 255u) + (ranks & 255u)};
@@ -477,7 +478,7 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
                     if (pass == 0) {
                         warm_solve(k, vA, vB);
                     } else {
-                        velocity_solve(k, vA, vB);
+                        velocity_solve(k, bm, vA, vB);
                         if (!one) *reinterpret_cast<float4*>(&f.cons[c].jn0) = make_float4(k.jn0, k.jt0, k.jn1, k.jt1);
                     }
                     if (mA) {

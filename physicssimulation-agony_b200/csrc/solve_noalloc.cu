@@ -25,7 +25,7 @@ constexpr uint32_t NOALLOC_MAX_BODIES = AG2D_SOLVE_NOALLOC_MAX_BODIES;
 constexpr uint32_t NOALLOC_THREADS = 512;
 
 // Scratch layout (byte offsets; every part 256-byte aligned).
-constexpr size_t NA_CONS = 0;                                                         // float4[7 M], ConsRecords::q
+constexpr size_t NA_CONS = 0;                                                         // float4[8 M], ConsRecords::q
 constexpr size_t NA_PEN = NA_CONS + size_t(NOALLOC_MAX_MANIFOLDS) * 16 * ConsRecords::FIELDS;   // float[M]
 constexpr size_t NA_COLOR = NA_PEN + size_t(NOALLOC_MAX_MANIFOLDS) * 4;               // u32[M]
 constexpr size_t NA_ORDER = NA_COLOR + size_t(NOALLOC_MAX_MANIFOLDS) * 4;            // u32[M]
@@ -34,7 +34,7 @@ constexpr size_t NA_LIST_B = NA_LIST_A + size_t(NOALLOC_MAX_MANIFOLDS) * 16;    
 constexpr size_t NA_BODY_MAX = NA_LIST_B + size_t(NOALLOC_MAX_MANIFOLDS) * 16;       // u64[B]
 constexpr size_t NA_BODY_MASK = NA_BODY_MAX + size_t(NOALLOC_MAX_BODIES) * 8;        // u64[B]
 constexpr size_t NA_PAIRS = NA_BODY_MASK + size_t(NOALLOC_MAX_BODIES) * 8;           // uint2[M]
-constexpr size_t NA_BYTES = NA_PAIRS + size_t(NOALLOC_MAX_MANIFOLDS) * 8;             // 3.1 MiB
+constexpr size_t NA_BYTES = NA_PAIRS + size_t(NOALLOC_MAX_MANIFOLDS) * 8;             // 3.4 MiB
 static_assert(NA_COLOR % 256 == 0 && NA_BODY_MAX % 256 == 0 && NA_BODY_MASK % 256 == 0 && NA_PAIRS % 256 == 0,
               "256-byte parts");
 static_assert(sizeof(ag2d_manifold) == sizeof(Manifold), "ag2d_manifold is the device Manifold record");
