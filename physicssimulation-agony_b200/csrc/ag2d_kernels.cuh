@@ -142,10 +142,10 @@ __global__ void k_scan(const uint32_t* in, uint32_t* out, uint32_t n, const uint
 constexpr uint32_t NARROW_SMEM_PER_THREAD =
     uint32_t(sizeof(Manifold) + sizeof(uint32_t) + 2 * MAX_POLYGON_VERTICES * sizeof(V2) / NARROW_GROUP);
 // Narrow phase + manifold compaction: manifolds of the hit pairs, in pair order, into out; tileState [tiles + 1] and
-// tileCounter zeroed before the launch (tiles: blockDim.x pairs each).
+// tileCounter zeroed before the launch (tiles: blockDim.x / 32 x perWarp pairs each, perWarp at most 32).
 __global__ void k_narrow(DeviceWorld w, const uint2* pairs, const uint32_t* nPairs, uint32_t pairCap, Manifold* out,
                          uint32_t manifoldCap, uint32_t* nOut, StepCounters* counters, uint32_t* tileState,
-                         uint32_t* tileCounter);
+                         uint32_t* tileCounter, uint32_t perWarp);
 __global__ void k_warm_insert(const Manifold* prev, const uint32_t* nPrev, unsigned long long* keys,
                               uint32_t* vals, uint32_t capacity, const uint32_t* seg, const uint32_t* colWorld,
                               uint32_t* status);

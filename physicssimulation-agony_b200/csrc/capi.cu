@@ -487,6 +487,7 @@ struct ag2d_world {
     uint32_t pairCap = 0, manifoldCap = 0, hashCap = 0;
     uint32_t lastManifolds = 0;
     uint32_t lastPairs = 0;   // candidate pairs of the last step
+    uint32_t pairsSeen = 0;   // candidate pairs of the last pass that found any (pairEstimate)
     uint32_t prevCount = 0;   // manifolds in prevManifolds (the warm-start source), as the host knows them
 
     // Bodies.
@@ -640,8 +641,8 @@ struct ag2d_world {
     // The collision-detection pass (AG2D_PHASE_COLLIDE) as a captured CUDA graph, replayed while its launch shapes
     // hold (list sizes, capacities, block sizes, whether the static tree is rebuilt).
     cudaGraphExec_t collideExec = nullptr;
-    uint64_t collideKey[9] = {};
-    uint64_t collideSeen[9] = {};   // the shape of the last pass run without a graph
+    uint64_t collideKey[10] = {};
+    uint64_t collideSeen[10] = {};  // the shape of the last pass run without a graph
     uint64_t collideLaunches = 0;
     cudaEvent_t ev[NPHASE][2] = {};
     bool evPending[NPHASE] = {};
@@ -1192,6 +1193,7 @@ struct ag2d_world {
         if (known) {
             lastManifolds = h.lastManifolds;
             lastPairs = h.lastPairs;
+            pairsSeen = h.lastPairs;
             reserveCapacities(uint32_t(std::min<uint64_t>(std::max<uint64_t>(3ull * h.lastPairs, 4096), 1ull << 30)),
                               uint32_t(std::min<uint64_t>(std::max<uint64_t>({3ull * h.lastManifolds, h.nPrev, 4096}),
                                                           1ull << 30)));
@@ -1330,7 +1332,7 @@ struct ag2d_world {
         pairCap = pairCapNew;
         manifoldCap = manCapNew;
         pairs.reserve(pairCap);
-        narrowState.reserve(size_t(div_up(pairCap, 64)) + 2);
+        narrowState.reserve(size_t(div_up(pairCap, 16)) + 2);   // the smallest tile: 4 warps of 4 pairs
         // Manifold arrays keep their contents (the previous step's manifolds are the warm-start source).
         auto grow_keep = [&](DBuf<Manifold>& b, uint32_t cap) {
             if (b.n >= cap && b.p) return;
@@ -1783,20 +1785,40 @@ struct ag2d_world {
         pend(4);
     }
 
+    // Candidate pairs to size launches for: the last pass's count, a quarter on top, rounded up to a power of two (so
+    // that a captured pass keeps its shape); the capacity when no pass has run.
+    uint32_t pairEstimate() const
+    {
+        const uint64_t want = pairsSeen ? uint64_t(pairsSeen) + pairsSeen / 4 + 64 : pairCap;
+        uint64_t p = 64;
+        while (p < want) p <<= 1;
+        return uint32_t(std::min<uint64_t>(p, std::max<uint32_t>(pairCap, 1)));
+    }
+    // Pairs a warp of the narrow phase takes: a warp works polygon pairs four at a time, one round after the other, so
+    // the fewest that still leave no SM more than 16 warps (about one wave); 32 above that, where throughput counts.
+    uint32_t narrowPerWarp() const
+    {
+        for (uint32_t p : {4u, 8u, 16u})
+            if (pairEstimate() <= p * 16u * uint32_t(dev.sms)) return p;
+        return 32u;
+    }
+
     void phaseNarrow(bool warm = true)
     {
         const cudaStream_t s = stream;
         islandsLinked = false;
         const uint32_t* nPairs = &dCounters.p->pairs;
-        // Grid sized for the capacity, work bounded by the device-side pair count; the manifolds are compacted in
-        // the same kernel.
-        const uint32_t gn = gridFor(pairCap, narrowThreads);
-        const uint32_t tilesCap = std::max<uint32_t>(div_up(pairCap, narrowThreads), 1);
+        // Work bounded by the device-side pair count (the tile states for the capacity); grid and pairs per warp
+        // from the last count; the manifolds are compacted in the same kernel.
+        const uint32_t perWarp = narrowPerWarp(), tilePairs = narrowThreads / 32 * perWarp;
+        const uint32_t gn = std::min(gridFor(uint64_t(pairEstimate()) * 32 / perWarp, narrowThreads),
+                                     gridFor(uint64_t(pairCap) * 32 / perWarp, narrowThreads));
+        const uint32_t tilesCap = std::max<uint32_t>(div_up(pairCap, tilePairs), 1);
         pbegin(5);
         CK(cudaMemsetAsync(narrowState.p, 0, (size_t(tilesCap) + 1) * sizeof(uint32_t), s));
         k_narrow<<<gn, narrowThreads, narrowThreads * NARROW_SMEM_PER_THREAD, s>>>(
             view(), pairs.p, nPairs, pairCap, manifolds.p, manifoldCap, nManifolds.p, dCounters.p, narrowState.p,
-            narrowState.p + tilesCap);
+            narrowState.p + tilesCap, perWarp);
         CK(cudaGetLastError());
         pend(5);
         launches += 1;
@@ -2313,6 +2335,7 @@ struct ag2d_world {
         const auto t0 = std::chrono::steady_clock::now();
         CK(cudaStreamSynchronize(stream));
         syncMs += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+        if (hCounters->pairs) pairsSeen = hCounters->pairs;
         pcollect();
     }
 
@@ -4153,20 +4176,20 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
             // The pass's launches depend on these only; the kernels read their counts on the device.
             auto shape = [&](uint64_t* k) {
                 // Any device reallocation (a buffer a captured kernel points at) changes the allocation count.
-                const uint64_t v[9] = {w.nDynCol, w.nOther, w.pairCap, w.manifoldCap, w.queryThreads,
+                const uint64_t v[10] = {w.nDynCol, w.nOther, w.pairCap, w.manifoldCap, w.queryThreads,
                                        w.narrowThreads, uint64_t(w.otherDirty), uint64_t(w.nColliders),
-                                       g_deviceAllocs.load(std::memory_order_relaxed)};
-                std::copy(v, v + 9, k);
+                                       g_deviceAllocs.load(std::memory_order_relaxed), w.pairEstimate()};
+                std::copy(v, v + 10, k);
             };
-            uint64_t key[9];
+            uint64_t key[10];
             shape(key);
-            if (w.collideExec && std::equal(key, key + 9, w.collideKey)) {
+            if (w.collideExec && std::equal(key, key + 10, w.collideKey)) {
                 CK(cudaGraphLaunch(w.collideExec, w.stream));
                 w.launches += w.collideLaunches;
                 break;
             }
             if (w.collideExec) { CK(cudaGraphExecDestroy(w.collideExec)); w.collideExec = nullptr; }
-            if (!std::equal(key, key + 9, w.collideSeen)) {
+            if (!std::equal(key, key + 10, w.collideSeen)) {
                 // A new shape: one pass as it is (it may grow buffers or rebuild the static tree), remembered.
                 pass();
                 shape(w.collideSeen);
@@ -4188,7 +4211,7 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
             cudaGraphDestroy(graph);
             CK(ie);
             w.collideLaunches = w.launches - before;
-            std::copy(key, key + 9, w.collideKey);
+            std::copy(key, key + 10, w.collideKey);
             CK(cudaGraphLaunch(w.collideExec, w.stream));
             break;
         }

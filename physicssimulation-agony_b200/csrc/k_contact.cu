@@ -49,10 +49,12 @@ __device__ __forceinline__ void write_slot(const Contact& ct, uint32_t a, uint32
     *slot = m;
 }
 
-// Narrow phase with the manifold compaction fused in. Blocks take tiles of blockDim.x consecutive pairs in ticket
-// order (tileState and the ticket counter zeroed before the launch); in a tile each warp takes 32 pairs, one per
-// lane. Pairs of other shape types run one per lane; then the warp's polygon-polygon pairs run four at a time, one
-// per group of NARROW_GROUP lanes (collide_polygon_polygon_group). Each pair's manifold goes to its slot in shared
+// Narrow phase with the manifold compaction fused in. Blocks take tiles of consecutive pairs in ticket order (tileState
+// and the ticket counter zeroed before the launch); in a tile each warp takes perWarp pairs (at most 32), one per
+// lane. Pairs of other shape types run one per lane; the warp's polygon-polygon pairs search their axes four at a time,
+// one per group of NARROW_GROUP lanes (collide_polygon_polygon_group), and are then clipped one per lane. A group's
+// search takes about 1.5 us, so a step with few pairs spreads them over more warps (perWarp 4 is one search a warp)
+// and one with many keeps every lane of the one-per-lane parts busy. Each pair's manifold goes to its slot in shared
 // memory; the tile's hits are then counted (warp ballots, then a scan of the warps' counts), its output offset
 // comes from the decoupled look-back over the preceding tiles, and the hit pairs' manifolds are copied straight to
 // their places: manifolds come out in pair order. The last tile writes the manifold count. Launched with a
@@ -60,7 +62,7 @@ __device__ __forceinline__ void write_slot(const Contact& ct, uint32_t a, uint32
 __global__ void k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairs,
                          uint32_t pairCap, Manifold* __restrict__ out, uint32_t manifoldCap,
                          uint32_t* __restrict__ nOut, StepCounters* counters, uint32_t* __restrict__ tileState,
-                         uint32_t* __restrict__ tileCounter)
+                         uint32_t* __restrict__ tileCounter, uint32_t perWarp)
 {
     extern __shared__ __align__(16) unsigned char narrowSmem[];
     // [blockDim] manifold slots, [blockDim] hit flags, then per group A's vertices and B's (in A's frame).
@@ -74,8 +76,9 @@ __global__ void k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const u
         if (blockIdx.x == 0 && threadIdx.x == 0) { *nOut = 0u; counters->manifolds = 0u; }
         return;
     }
-    const uint32_t tiles_n = (n + blockDim.x - 1) / blockDim.x;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = blockDim.x >> 5;
+    const uint32_t tilePairs = nWarps * perWarp;
+    const uint32_t tiles_n = (n + tilePairs - 1) / tilePairs;
     const uint32_t group = lane / NARROW_GROUP, gl = lane % NARROW_GROUP;
     const uint32_t gmask = ((1u << NARROW_GROUP) - 1u) << (group * NARROW_GROUP);
     V2* const sA = tiles + (threadIdx.x / NARROW_GROUP) * 2 * MAX_POLYGON_VERTICES;
@@ -86,8 +89,8 @@ __global__ void k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const u
         __syncthreads();
         const uint32_t tile = tileSlot;
         if (tile >= tiles_n) return;
-        const uint32_t p = tile * blockDim.x + threadIdx.x;
-        const bool valid = p < n;
+        const uint32_t p = tile * tilePairs + warp * perWarp + lane;
+        const bool valid = lane < perWarp && p < n;
         uint32_t a = 0, b = 0;
         bool pp = false;
         hitS[threadIdx.x] = 0u;
@@ -117,16 +120,26 @@ __global__ void k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const u
             for (uint32_t k = 0; k < 32 / NARROW_GROUP && todo; k++) todo &= todo - 1;
             if (has) {
                 const ColliderView A = collider_view(w, ga), B = collider_view(w, gb);
-                Contact ct;
-                const bool h = collide_polygon_polygon_group(A, B, ct, gl, gmask, sA, sB);
+                float depth;
+                uint32_t edges;
+                const bool h = collide_polygon_polygon_group(A, B, depth, edges, gl, gmask, sA, sB);
                 if (gl == 0 && h) {
                     hitS[warpFirst + src] = 1u;
-                    write_slot(ct, ga, gb, slot + warpFirst + src);
+                    slot[warpFirst + src].depth = depth;
+                    slot[warpFirst + src].id0 = edges;
                 }
                 __syncwarp(gmask);   // the group's tiles are reused by its next pair
             }
         }
         __syncwarp();
+        if (pp && hitS[threadIdx.x]) {
+            const ColliderView A = collider_view(w, a), B = collider_view(w, b);
+            Contact ct;
+            if (collide_polygon_polygon_clip(A, B, slot[threadIdx.x].depth, slot[threadIdx.x].id0, ct))
+                write_slot(ct, a, b, slot + threadIdx.x);
+            else
+                hitS[threadIdx.x] = 0u;
+        }
         const bool h = hitS[threadIdx.x] != 0u;
         // Output offsets: the tile's hits in pair order after those of the preceding tiles.
         const uint32_t hits = __ballot_sync(0xffffffffu, h);
