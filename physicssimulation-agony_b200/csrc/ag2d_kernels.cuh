@@ -32,7 +32,6 @@ static_assert(sizeof(NodeRec) == 48, "NodeRec is 48 bytes");
 struct TreeView {
     int n;
     const int2* child;
-    const int2* range;
     const float4* nodeAabb;
     const float4* leafAabb;       // AABBs in sorted (leaf) order
     const uint32_t* vals;         // collider index of each leaf
@@ -66,13 +65,30 @@ __global__ void k_sort_digit_scan(uint32_t* hist);
 __global__ void k_sort_pass(const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut, uint32_t* valsOut,
                             uint32_t n, uint32_t shift, const uint32_t* digitBase, uint32_t* tileState,
                             uint32_t* tileCounter, uint32_t* status);
-// Segments up to SEGMENT_SORT_MAX keys are sorted in shared memory (k_segment_sort), in two size classes.
-constexpr uint32_t SEGMENT_SORT_SMALL = 2048;
-constexpr uint32_t SEGMENT_SORT_MAX = 16384;
-__global__ void k_segment_sort(const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut, uint32_t* valsOut,
-                               const uint32_t* segStart, uint32_t worlds, uint32_t minSize, uint32_t maxSize);
+// Trees of up to TREE_SEGMENT_MAX leaves are built by one CTA each (k_tree_segments), in three size classes.
+constexpr uint32_t TREE_SEGMENT_SMALL = 256;
+constexpr uint32_t TREE_SEGMENT_MEDIUM = 2048;
+constexpr uint32_t TREE_SEGMENT_MAX = 16384;
+struct TreeBuild {
+    const float4* caabb;
+    const uint32_t* list;       // colliders, world-grouped
+    const uint32_t* segStart;   // [worlds + 1], or null: one segment of n
+    uint32_t worlds, n;
+    uint32_t *vals, *keys;      // sorted colliders and their Morton keys
+    uint32_t* sortedWorld;      // or null
+    float4* leafAabb;
+    float4* nodeAabb;           // or null: the boxes in the records are enough for the pair query
+    int2* child;                // or null, likewise
+    NodeRec* rec;
+};
+// Host side: builds every segment's tree; 'largest' bounds the segment sizes (at most TREE_SEGMENT_MAX). Adds the
+// kernels launched to *launches.
+cudaError_t launch_tree_segments(const TreeBuild& t, uint32_t largest, uint32_t sms, cudaStream_t stream,
+                                 uint32_t* launches);
+// Host side: raises the builder's dynamic shared-memory limit (once per device).
+cudaError_t tree_segments_init();
 __global__ void k_lbvh_build(const uint32_t* keys, const uint32_t* sortedWorld, const uint32_t* segStart, int n,
-                             int2* child, int2* range, int* parent, int* leafParent, float4* meet, NodeRec* rec);
+                             int2* child, int* parent, int* leafParent, float4* meet, NodeRec* rec);
 __global__ void k_lbvh_refit(int n, const int2* child, const int* parent, const int* leafParent,
                              const float4* leafAabb, float4* nodeAabb, float4* meet, NodeRec* rec);
 // Empty marker of a refit meeting slot (min x bits): a NaN no arithmetic produces.

@@ -167,7 +167,7 @@ struct Scanner {
 
 struct Tree {
     DBuf<uint32_t> keys, vals, keys2, vals2;
-    DBuf<int2> child, range;
+    DBuf<int2> child;
     DBuf<int> parent, leafParent;
     DBuf<float4> leafAabb, nodeAabb;
     DBuf<NodeRec> rec;
@@ -181,7 +181,7 @@ struct Tree {
     {
         worlds = nWorlds;
         keys.reserve(cap); vals.reserve(cap); keys2.reserve(cap); vals2.reserve(cap);
-        child.reserve(cap); range.reserve(cap); parent.reserve(cap); leafParent.reserve(cap);
+        child.reserve(cap); parent.reserve(cap); leafParent.reserve(cap);
         leafAabb.reserve(cap); nodeAabb.reserve(cap); meet.reserve(cap); rec.reserve(cap);
         bounds.reserve(4 * size_t(nWorlds)); hist.reserve(4 * 256); tileCounter.reserve(4);
         tileState.reserve(size_t(div_up(std::max<uint32_t>(cap, 1), SORT_TILE)) * 256 * 4);
@@ -192,7 +192,7 @@ struct Tree {
     TreeView view() const
     {
         const bool seg = worlds > 1;
-        return TreeView{n, child.p, range.p, nodeAabb.p, leafAabb.p, vals.p, seg ? sortedWorld.p : nullptr,
+        return TreeView{n, child.p, nodeAabb.p, leafAabb.p, vals.p, seg ? sortedWorld.p : nullptr,
                         seg ? segStart.p : nullptr, rec.p};
     }
 };
@@ -394,6 +394,7 @@ static DeviceInfo probe_device(int device)
     DeviceInfo dev;
     CK(cudaDeviceGetAttribute(&dev.sms, cudaDevAttrMultiProcessorCount, device));
     CK(block_solver_init());
+    CK(tree_segments_init());
     int perSm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_color_solve_flow, FLOW_THREADS, 0));
     dev.flowBlocks = std::max(1, perSm) * dev.sms;
@@ -575,7 +576,6 @@ struct ag2d_world {
     uint32_t teamBodyCap = 2048;           // bodies of a team staged in shared memory (larger teams use global)
     uint32_t teamConsCap = 0;              // constraint records a team keeps in shared memory (more: global)
     uint32_t maxWorldCols = 0;             // colliders of the largest world of a batch (segmented-sort class)
-    bool segSortReady = false;
     uint32_t bigConsCap = 0;
     bool consOnChip = false;               // team constraint records in shared memory when they fit (tunable)
     uint32_t nTeams = 0;
@@ -1662,6 +1662,12 @@ struct ag2d_world {
         launches += 2 + passes;
     }
 
+    uint32_t treeSingleMax() const
+    {
+        if (const char* v = std::getenv("AG2D_TREE_SINGLE")) return uint32_t(atoi(v));
+        return 4096;
+    }
+
     // Tree over the colliders of 'list' (Morton keys from the world's bounds, sorted, Karras build, refit). With
     // several worlds the order is (world, Morton key) and every world gets its own tree over its segment.
     void buildTree(Tree& t, const uint32_t* list, uint32_t n)
@@ -1672,38 +1678,29 @@ struct ag2d_world {
         const uint32_t W = nWorlds;
         const bool seg = W > 1;
         const uint32_t* cw = seg ? colWorld.p : nullptr;
+        const bool isDyn = &t == &dynTree;
+        if (seg ? maxWorldCols <= TREE_SEGMENT_MAX : n <= treeSingleMax()) {
+            // One CTA a segment builds its whole tree. Continuous collision traverses the static and sleeping tree by
+            // its node boxes and child links; the pair query needs neither.
+            const TreeBuild b{caabb.p, list, seg ? t.segStart.p : nullptr, W, n, t.vals.p,
+                              seg ? t.sortedKey.p : t.keys.p, seg ? t.sortedWorld.p : nullptr, t.leafAabb.p,
+                              isDyn ? nullptr : t.nodeAabb.p, isDyn ? nullptr : t.child.p, t.rec.p};
+            uint32_t count = 0;
+            if (isDyn) pbegin(13);
+            CK(launch_tree_segments(b, seg ? std::min(maxWorldCols, n) : n, uint32_t(std::max(dev.sms, 1)), s, &count));
+            if (isDyn) pend(13);
+            launches += count;
+            return;
+        }
         launches += 5 + (n > 1 ? 1 : 0);
         k_bounds_init<<<gridFor(W), 256, 0, s>>>(t.bounds.p, W);
         k_bounds<<<gridFor(n), 256, 0, s>>>(caabb.p, list, n, cw, t.bounds.p);
         k_morton<<<gridFor(n), 256, 0, s>>>(caabb.p, list, n, cw, t.bounds.p, t.keys.p, t.vals.p,
                                              seg ? t.keyOf.p : nullptr);
         CK(cudaGetLastError());
-        const bool isDyn = &t == &dynTree;
         if (isDyn) pbegin(12);
-        if (seg && maxWorldCols <= SEGMENT_SORT_MAX) {
-            // Every world's segment sorted in shared memory, small and large segments by separate launches.
-            if (!segSortReady) {
-                CK(cudaFuncSetAttribute(k_segment_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(SEGMENT_SORT_MAX * sizeof(unsigned long long))));
-                segSortReady = true;
-            }
-            const uint32_t grid = std::min<uint32_t>(W, uint32_t(dev.sms) * 8);
-            k_segment_sort<<<grid, 256, SEGMENT_SORT_SMALL * sizeof(unsigned long long), s>>>(
-                t.keys.p, t.vals.p, t.keys2.p, t.vals2.p, t.segStart.p, W, 0, SEGMENT_SORT_SMALL);
-            launches++;
-            if (maxWorldCols > SEGMENT_SORT_SMALL) {
-                k_segment_sort<<<std::min<uint32_t>(W, uint32_t(dev.sms)), 1024,
-                                 SEGMENT_SORT_MAX * sizeof(unsigned long long), s>>>(
-                    t.keys.p, t.vals.p, t.keys2.p, t.vals2.p, t.segStart.p, W, SEGMENT_SORT_SMALL, SEGMENT_SORT_MAX);
-                launches++;
-            }
-            CK(cudaGetLastError());
-            swap_bufs(t.keys, t.keys2);
-            swap_bufs(t.vals, t.vals2);
-        } else {
-            sortPasses(t, n, 4);
-        }
-        if (seg && maxWorldCols > SEGMENT_SORT_MAX) {
+        sortPasses(t, n, 4);
+        if (seg) {
             // Stable passes on the world id: order (world, Morton key, collider).
             uint32_t passes = 1;
             while (passes < 4 && (W - 1) >> (8 * passes)) passes++;
@@ -1718,7 +1715,7 @@ struct ag2d_world {
                                                   seg ? t.sortedKey.p : nullptr, seg ? t.sortedWorld.p : nullptr,
                                                   t.leafAabb.p);
         k_lbvh_build<<<gridFor(n), 256, 0, s>>>(seg ? t.sortedKey.p : t.keys.p, seg ? t.sortedWorld.p : nullptr,
-                                                 seg ? t.segStart.p : nullptr, int(n), t.child.p, t.range.p,
+                                                 seg ? t.segStart.p : nullptr, int(n), t.child.p,
                                                  t.parent.p, t.leafParent.p, t.meet.p, t.rec.p);
         CK(cudaGetLastError());
         if (n > 1) {

@@ -402,6 +402,7 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
     const uint32_t rank = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t size = gridDim.x * blockDim.x;
     const uint32_t n = *nM;
+    if (n == 0) return;
     const GlobalBodies B{w.bvel, w.bpos, s.bodyMax, s.bodyMask};
     const GridSync sync{bar, &counters->status};
     uint32_t ncol = 0;

@@ -1,6 +1,8 @@
 // Spatial phase kernels: integration, collider poses + AABBs, Morton keys, onesweep radix sort, Karras LBVH build
 // and refit, and the candidate-pair query. Reference routines cited per kernel (paths relative to
 // PhysicsSimulation-Agony/PS_AGONY2D/).
+#include <algorithm>
+
 #include "ag2d_ccd.cuh"
 #include "ag2d_kernels.cuh"
 
@@ -255,6 +257,27 @@ __global__ void k_simd_flags(const uint32_t* __restrict__ list, uint32_t n, cons
 // Morton keys: transformCentroids + computeMortonCodes (BvhTree.cpp:191-280). 2 x centroid scaled into [0, 65535]
 // per axis by the tree bounds, truncated, bits interleaved (y in the odd bits): a 32-bit key.
 // ---------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t morton_key(const float4& a, float bminX, float bminY, float bmaxX, float bmaxY)
+{
+    const float kEps = 1e-5f;
+    const float maxX = rfmaxf(bmaxX, bminX + kEps);
+    const float maxY = rfmaxf(bmaxY, bminY + kEps);
+    const float clampMax = 65535.0f;
+    const float scaleX = clampMax / (maxX - bminX);
+    const float scaleY = clampMax / (maxY - bminY);
+    const float negScaledMinX = -bminX * scaleX;
+    const float negScaledMinY = -bminY * scaleY;
+    const float halfScaleX = scaleX * 0.5f;
+    const float halfScaleY = scaleY * 0.5f;
+    const float cx = a.x + a.z;
+    const float cy = a.y + a.w;
+    float tx = cx * halfScaleX + negScaledMinX;
+    float ty = cy * halfScaleY + negScaledMinY;
+    tx = tx < 0.0f ? 0.0f : (tx > clampMax ? clampMax : tx);
+    ty = ty < 0.0f ? 0.0f : (ty > clampMax ? clampMax : ty);
+    return (part1by1(uint32_t(ty)) << 1) | part1by1(uint32_t(tx));
+}
+
 __global__ void k_morton(const float4* __restrict__ aabb, const uint32_t* __restrict__ list, uint32_t n,
                          const uint32_t* __restrict__ colWorld, const uint32_t* __restrict__ bounds,
                          uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* __restrict__ keyOf)
@@ -262,26 +285,8 @@ __global__ void k_morton(const float4* __restrict__ aabb, const uint32_t* __rest
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const uint32_t c = list ? list[k] : k;
         const uint32_t* b = bounds + 4 * (colWorld ? colWorld[c] : 0u);
-        const float bminX = ordered_to_float(b[0]), bminY = ordered_to_float(b[1]);
-        const float bmaxX = ordered_to_float(b[2]), bmaxY = ordered_to_float(b[3]);
-        const float kEps = 1e-5f;
-        const float maxX = rfmaxf(bmaxX, bminX + kEps);
-        const float maxY = rfmaxf(bmaxY, bminY + kEps);
-        const float clampMax = 65535.0f;
-        const float scaleX = clampMax / (maxX - bminX);
-        const float scaleY = clampMax / (maxY - bminY);
-        const float negScaledMinX = -bminX * scaleX;
-        const float negScaledMinY = -bminY * scaleY;
-        const float halfScaleX = scaleX * 0.5f;
-        const float halfScaleY = scaleY * 0.5f;
-        const float4 a = aabb[c];
-        const float cx = a.x + a.z;
-        const float cy = a.y + a.w;
-        float tx = cx * halfScaleX + negScaledMinX;
-        float ty = cy * halfScaleY + negScaledMinY;
-        tx = tx < 0.0f ? 0.0f : (tx > clampMax ? clampMax : tx);
-        ty = ty < 0.0f ? 0.0f : (ty > clampMax ? clampMax : ty);
-        const uint32_t key = (part1by1(uint32_t(ty)) << 1) | part1by1(uint32_t(tx));
+        const uint32_t key = morton_key(aabb[c], ordered_to_float(b[0]), ordered_to_float(b[1]), ordered_to_float(b[2]),
+                                        ordered_to_float(b[3]));
         keys[k] = key;
         vals[k] = c;
         if (keyOf) keyOf[c] = key;
@@ -521,10 +526,34 @@ __device__ __forceinline__ int lbvh_delta(const uint32_t* keys, int lo, int hi, 
     return 32 + __clz(uint32_t(i - lo) ^ uint32_t(j - lo));
 }
 
+// Internal node i of a tree with prefix lengths delta(i, j) (-1 outside the segment): its range and split.
+struct KarrasNode {
+    int first, last, gamma;
+};
+template <class Delta>
+__device__ __forceinline__ KarrasNode karras_node(int i, Delta delta)
+{
+    const int d = (delta(i, i + 1) - delta(i, i - 1)) >= 0 ? 1 : -1;
+    const int dmin = delta(i, i - d);
+    int lmax = 2;
+    while (delta(i, i + lmax * d) > dmin) lmax <<= 1;
+    int l = 0;
+    for (int t = lmax >> 1; t >= 1; t >>= 1)
+        if (delta(i, i + (l + t) * d) > dmin) l += t;
+    const int j = i + l * d;
+    const int dnode = delta(i, j);
+    int s = 0, t = l;
+    do {
+        t = (t + 1) >> 1;
+        if (delta(i, i + (s + t) * d) > dnode) s += t;
+    } while (t > 1);
+    return KarrasNode{i < j ? i : j, i < j ? j : i, i + s * d + (d < 0 ? -1 : 0)};
+}
+
 // sortedWorld/segStart null: one segment [0, n).
 __global__ void k_lbvh_build(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ sortedWorld,
                              const uint32_t* __restrict__ segStart, int n, int2* __restrict__ child,
-                             int2* __restrict__ range, int* __restrict__ parent, int* __restrict__ leafParent,
+                             int* __restrict__ parent, int* __restrict__ leafParent,
                              float4* __restrict__ meet, NodeRec* __restrict__ rec)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -538,26 +567,11 @@ __global__ void k_lbvh_build(const uint32_t* __restrict__ keys, const uint32_t* 
         if (i >= hi - 1) continue;
         meet[i] = make_float4(__uint_as_float(MEET_EMPTY), 0.0f, 0.0f, 0.0f);
         if (i == lo) parent[i] = -1;
-        const int d = (lbvh_delta(keys, lo, hi, i, i + 1) - lbvh_delta(keys, lo, hi, i, i - 1)) >= 0 ? 1 : -1;
-        const int dmin = lbvh_delta(keys, lo, hi, i, i - d);
-        int lmax = 2;
-        while (lbvh_delta(keys, lo, hi, i, i + lmax * d) > dmin) lmax <<= 1;
-        int l = 0;
-        for (int t = lmax >> 1; t >= 1; t >>= 1)
-            if (lbvh_delta(keys, lo, hi, i, i + (l + t) * d) > dmin) l += t;
-        const int j = i + l * d;
-        const int dnode = lbvh_delta(keys, lo, hi, i, j);
-        int s = 0, t = l;
-        do {
-            t = (t + 1) >> 1;
-            if (lbvh_delta(keys, lo, hi, i, i + (s + t) * d) > dnode) s += t;
-        } while (t > 1);
-        const int gamma = i + s * d + (d < 0 ? -1 : 0);
-        const int first = i < j ? i : j, last = i < j ? j : i;
+        const KarrasNode k = karras_node(i, [&](int a, int b) { return lbvh_delta(keys, lo, hi, a, b); });
+        const int first = k.first, last = k.last, gamma = k.gamma;
         const int left = (first == gamma) ? ~gamma : gamma;
         const int right = (last == gamma + 1) ? ~(gamma + 1) : gamma + 1;
         child[i] = make_int2(left, right);
-        range[i] = make_int2(first, last);
         rec[i].child = make_int2(left, right);
         rec[i].last = make_int2(gamma, last);
         if (left < 0) leafParent[~left] = i; else parent[left] = i;
@@ -579,45 +593,153 @@ __device__ __forceinline__ float4 exchange_box(float4* slot, float4 v)
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Segmented sort of a world-grouped tree list: every world segment [segStart[w], segStart[w + 1]) is sorted by its
-// Morton key in shared memory, one CTA per segment, by a bitonic network over (key << 32 | position) so that equal
-// keys keep their list order: the result equals the stable (world, key, position) order of the global radix passes.
-// A CTA takes only the segments of its size class (minSize, maxSize]; every segment of the list is written to the
-// output arrays by exactly one class.
+// The whole tree of a segment in one CTA: bounds, Morton keys, sort, leaf gather, Karras build and refit, over every
+// world segment [segStart[w], segStart[w + 1]) of a world-grouped list (or the one segment [0, n)) whose size is in
+// (minSize, maxSize]. The results are those of the kernels above and below run one after the other: the sort is a
+// bitonic network over (key << 32 | position), so equal keys keep their list order; steps between elements at most 32
+// apart stay within a warp's 64 elements and need no block barrier. The two subtrees of a node meet by a flag in shared
+// memory, their boxes in the node's record.
+// Bound: barriers and shared-memory latency; one CTA a segment and one launch in place of seven over all segments
+// (bounds, keys, sort, gather, build, refit and their clears), which took 460 us a step on 4,096 worlds and 70 to
+// 95 us on a single world of 64 to 2,048 colliders, most of it launches waiting for one another.
 // ---------------------------------------------------------------------------------------------------------------
-__global__ void k_segment_sort(const uint32_t* __restrict__ keysIn, const uint32_t* __restrict__ valsIn,
-                               uint32_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut,
-                               const uint32_t* __restrict__ segStart, uint32_t worlds, uint32_t minSize,
-                               uint32_t maxSize)
+template <uint32_t THREADS>
+__global__ void __launch_bounds__(THREADS) k_tree_segments(TreeBuild t, uint32_t minSize, uint32_t maxSize)
 {
-    extern __shared__ unsigned long long sortTile[];
-    for (uint32_t w = blockIdx.x; w < worlds; w += gridDim.x) {
-        const uint32_t lo = segStart[w], n = segStart[w + 1] - lo;
+    // [m] sort words (keys stay in their upper halves through the build, then the meeting flags), m the next power of
+    // two, then per node and per leaf the parent << 1 | side (16 bits each).
+    extern __shared__ unsigned long long treeTile[];
+    __shared__ float4 part[THREADS / 32];
+    constexpr uint32_t NO_PARENT = 0xFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint32_t w = blockIdx.x; w < t.worlds; w += gridDim.x) {
+        const uint32_t lo = t.segStart ? t.segStart[w] : 0u, n = t.segStart ? t.segStart[w + 1] - lo : t.n;
         if (n <= minSize || n > maxSize) continue;
         uint32_t m = 1;
         while (m < n) m <<= 1;
-        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x)
-            sortTile[i] = i < n ? (static_cast<unsigned long long>(keysIn[lo + i]) << 32 | i) : ~0ull;
+        uint16_t* const nodeUp = reinterpret_cast<uint16_t*>(treeTile + m);
+        uint16_t* const leafUp = nodeUp + n;
+        const uint32_t* const list = t.list + lo;
+        // Bounds of the segment's boxes.
+        float4 bb = make_float4(FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX);
+        for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
+            const float4 a = t.caabb[list[i]];
+            bb = make_float4(fminf(bb.x, a.x), fminf(bb.y, a.y), fmaxf(bb.z, a.z), fmaxf(bb.w, a.w));
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            bb.x = fminf(bb.x, __shfl_xor_sync(0xffffffffu, bb.x, o));
+            bb.y = fminf(bb.y, __shfl_xor_sync(0xffffffffu, bb.y, o));
+            bb.z = fmaxf(bb.z, __shfl_xor_sync(0xffffffffu, bb.z, o));
+            bb.w = fmaxf(bb.w, __shfl_xor_sync(0xffffffffu, bb.w, o));
+        }
+        if (lane == 0) part[warp] = bb;
+        __syncthreads();
+        for (uint32_t k = 0; k < THREADS / 32; k++) {
+            const float4 q = part[k];
+            bb = make_float4(fminf(bb.x, q.x), fminf(bb.y, q.y), fmaxf(bb.z, q.z), fmaxf(bb.w, q.w));
+        }
+        for (uint32_t i = threadIdx.x; i < m; i += THREADS) {
+            unsigned long long e = ~0ull;
+            if (i < n) e = static_cast<unsigned long long>(morton_key(t.caabb[list[i]], bb.x, bb.y, bb.z, bb.w)) << 32 | i;
+            treeTile[i] = e;
+        }
         __syncthreads();
         for (uint32_t k = 2; k <= m; k <<= 1) {
             for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-                    const uint32_t p = i ^ j;
-                    if (p > i) {
-                        const unsigned long long a = sortTile[i], b = sortTile[p];
-                        if ((a > b) == ((i & k) == 0)) { sortTile[i] = b; sortTile[p] = a; }
-                    }
+                for (uint32_t p = threadIdx.x; p < m / 2; p += THREADS) {
+                    const uint32_t i = ((p & ~(j - 1u)) << 1) | (p & (j - 1u));
+                    const unsigned long long a = treeTile[i], b = treeTile[i + j];
+                    if ((a > b) == ((i & k) == 0)) { treeTile[i] = b; treeTile[i + j] = a; }
                 }
-                __syncthreads();
+                if (j > 32u || (j == 1u && k > 32u)) __syncthreads();
+                else __syncwarp();
             }
         }
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const unsigned long long e = sortTile[i];
-            keysOut[lo + i] = uint32_t(e >> 32);
-            valsOut[lo + i] = valsIn[lo + uint32_t(e)];
-        }
         __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
+            const unsigned long long e = treeTile[i];
+            const uint32_t c = list[uint32_t(e)];
+            t.vals[lo + i] = c;
+            t.keys[lo + i] = uint32_t(e >> 32);
+            if (t.sortedWorld) t.sortedWorld[lo + i] = w;
+            t.leafAabb[lo + i] = t.caabb[c];
+        }
+        if (n > 1) {
+            const int hi = int(n);
+            auto delta = [&](int i, int j) {
+                if (j < 0 || j >= hi) return -1;
+                const uint32_t a = uint32_t(treeTile[i] >> 32), b = uint32_t(treeTile[j] >> 32);
+                return a != b ? __clz(a ^ b) : 32 + __clz(uint32_t(i) ^ uint32_t(j));
+            };
+            for (int i = int(threadIdx.x); i < hi - 1; i += int(THREADS)) {
+                const KarrasNode k = karras_node(i, delta);
+                const int left = k.first == k.gamma ? ~(int(lo) + k.gamma) : int(lo) + k.gamma;
+                const int right = k.last == k.gamma + 1 ? ~(int(lo) + k.gamma + 1) : int(lo) + k.gamma + 1;
+                if (t.child) t.child[lo + i] = make_int2(left, right);
+                t.rec[lo + i].child = make_int2(left, right);
+                t.rec[lo + i].last = make_int2(int(lo) + k.gamma, int(lo) + k.last);
+                (left < 0 ? leafUp : nodeUp)[k.gamma] = uint16_t(i << 1);
+                (right < 0 ? leafUp : nodeUp)[k.gamma + 1] = uint16_t(i << 1 | 1);
+                if (i == 0) nodeUp[0] = NO_PARENT;
+            }
+            __syncthreads();
+            uint32_t* const met = reinterpret_cast<uint32_t*>(treeTile);
+            for (uint32_t i = threadIdx.x; i < n; i += THREADS) met[i] = 0u;
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
+                float4 box = t.leafAabb[lo + i];   // written by this thread
+                uint32_t up = leafUp[i];
+                while (up != NO_PARENT) {
+                    const uint32_t node = up >> 1, side = up & 1u;
+                    NodeRec* const r = t.rec + lo + node;
+                    r->box[side] = box;
+                    __threadfence_block();
+                    if (atomicExch(met + node, 1u) == 0u) break;   // the sibling carries on
+                    __threadfence_block();
+                    const float4 o = r->box[side ^ 1u];
+                    box = make_float4(fminf(box.x, o.x), fminf(box.y, o.y), fmaxf(box.z, o.z), fmaxf(box.w, o.w));
+                    if (t.nodeAabb) t.nodeAabb[lo + node] = box;
+                    up = nodeUp[node];
+                }
+            }
+        }
+        __syncthreads();   // the tile is reused by the next segment
     }
+}
+
+size_t tree_segment_smem(uint32_t n)
+{
+    size_t m = 1;
+    while (m < n) m <<= 1;
+    return m * sizeof(unsigned long long) + 2 * size_t(n) * sizeof(uint16_t) + 16;
+}
+
+cudaError_t tree_segments_init()
+{
+    return cudaFuncSetAttribute(k_tree_segments<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(tree_segment_smem(TREE_SEGMENT_MAX)));
+}
+
+cudaError_t launch_tree_segments(const TreeBuild& t, uint32_t largest, uint32_t sms, cudaStream_t stream,
+                                 uint32_t* launches)
+{
+    // Three size classes, each with the CTA that its largest segment keeps busy: segments of a ragged batch differ by a
+    // factor of a hundred, and a small one in a wide CTA waits at barriers with most warps idle.
+    const uint32_t small = std::min(largest, TREE_SEGMENT_SMALL), medium = std::min(largest, TREE_SEGMENT_MEDIUM);
+    const bool one = t.segStart == nullptr;
+    if (!one || largest <= TREE_SEGMENT_SMALL) {
+        k_tree_segments<128><<<std::min(t.worlds, sms * 16u), 128, tree_segment_smem(small), stream>>>(t, 0u, small);
+        ++*launches;
+    }
+    if (largest > TREE_SEGMENT_SMALL && (!one || largest <= TREE_SEGMENT_MEDIUM)) {
+        k_tree_segments<512><<<std::min(t.worlds, sms * 4u), 512, tree_segment_smem(medium), stream>>>(t, small, medium);
+        ++*launches;
+    }
+    if (largest > TREE_SEGMENT_MEDIUM) {
+        k_tree_segments<1024><<<std::min(t.worlds, sms), 1024, tree_segment_smem(largest), stream>>>(t, medium, largest);
+        ++*launches;
+    }
+    return cudaGetLastError();
 }
 
 // Bottom-up AABB refit (BvhTree::fitNodes equivalent). The two subtrees of a node meet in its slot: each swaps its
