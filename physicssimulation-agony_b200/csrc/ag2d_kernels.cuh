@@ -65,10 +65,11 @@ __global__ void k_sort_digit_scan(uint32_t* hist);
 __global__ void k_sort_pass(const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut, uint32_t* valsOut,
                             uint32_t n, uint32_t shift, const uint32_t* digitBase, uint32_t* tileState,
                             uint32_t* tileCounter, uint32_t* status);
-// Trees of up to TREE_SEGMENT_MAX leaves are built by one CTA each (k_tree_segments), in three size classes.
-constexpr uint32_t TREE_SEGMENT_SMALL = 256;
-constexpr uint32_t TREE_SEGMENT_MEDIUM = 2048;
+// Trees of up to TREE_SEGMENT_MAX leaves are built by one CTA each (k_tree_segments), in size classes.
 constexpr uint32_t TREE_SEGMENT_MAX = 16384;
+// A single tree of more leaves is built by the whole GPU in a dozen launches: 108 us at 6,000 and at 8,000 leaves,
+// where one CTA takes 89 and 113 us (40 against 95 at 2,000).
+constexpr uint32_t TREE_SINGLE_MAX = 7168;
 struct TreeBuild {
     const float4* caabb;
     const uint32_t* list;       // colliders, world-grouped
@@ -80,12 +81,13 @@ struct TreeBuild {
     float4* nodeAabb;           // or null: the boxes in the records are enough for the pair query
     int2* child;                // or null, likewise
     NodeRec* rec;
+    float4* meet;               // [2 x leaves] meeting boxes of the largest class
 };
-// Host side: builds every segment's tree; 'largest' bounds the segment sizes (at most TREE_SEGMENT_MAX). Adds the
-// kernels launched to *launches.
+// Host side: builds every segment's tree; 'largest' bounds the segment sizes (at most TREE_SEGMENT_MAX); *launches: the
+// kernels launched.
 cudaError_t launch_tree_segments(const TreeBuild& t, uint32_t largest, uint32_t sms, cudaStream_t stream,
                                  uint32_t* launches);
-// Host side: raises the builder's dynamic shared-memory limit (once per device).
+// Host side: raises the builders' dynamic shared-memory limit (once per device).
 cudaError_t tree_segments_init();
 __global__ void k_lbvh_build(const uint32_t* keys, const uint32_t* sortedWorld, const uint32_t* segStart, int n,
                              int2* child, int* parent, int* leafParent, float4* meet, NodeRec* rec);

@@ -171,7 +171,7 @@ struct Tree {
     DBuf<int> parent, leafParent;
     DBuf<float4> leafAabb, nodeAabb;
     DBuf<NodeRec> rec;
-    DBuf<float4> meet;   // refit meeting slots, one per internal node
+    DBuf<float4> meet;   // refit meeting slots: one per internal node, or (one CTA a tree) two per split
     DBuf<uint32_t> bounds, hist, tileState, tileCounter;
     // World-segmented trees: Morton key per collider, sorted keys / worlds, segment starts (filled with the lists).
     DBuf<uint32_t> keyOf, sortedKey, sortedWorld, segStart;
@@ -182,7 +182,7 @@ struct Tree {
         worlds = nWorlds;
         keys.reserve(cap); vals.reserve(cap); keys2.reserve(cap); vals2.reserve(cap);
         child.reserve(cap); parent.reserve(cap); leafParent.reserve(cap);
-        leafAabb.reserve(cap); nodeAabb.reserve(cap); meet.reserve(cap); rec.reserve(cap);
+        leafAabb.reserve(cap); nodeAabb.reserve(cap); meet.reserve(2 * size_t(cap)); rec.reserve(cap);
         bounds.reserve(4 * size_t(nWorlds)); hist.reserve(4 * 256); tileCounter.reserve(4);
         tileState.reserve(size_t(div_up(std::max<uint32_t>(cap, 1), SORT_TILE)) * 256 * 4);
         if (nWorlds > 1) {
@@ -1662,12 +1662,6 @@ struct ag2d_world {
         launches += 2 + passes;
     }
 
-    uint32_t treeSingleMax() const
-    {
-        if (const char* v = std::getenv("AG2D_TREE_SINGLE")) return uint32_t(atoi(v));
-        return 4096;
-    }
-
     // Tree over the colliders of 'list' (Morton keys from the world's bounds, sorted, Karras build, refit). With
     // several worlds the order is (world, Morton key) and every world gets its own tree over its segment.
     void buildTree(Tree& t, const uint32_t* list, uint32_t n)
@@ -1679,12 +1673,12 @@ struct ag2d_world {
         const bool seg = W > 1;
         const uint32_t* cw = seg ? colWorld.p : nullptr;
         const bool isDyn = &t == &dynTree;
-        if (seg ? maxWorldCols <= TREE_SEGMENT_MAX : n <= treeSingleMax()) {
+        if (seg ? maxWorldCols <= TREE_SEGMENT_MAX : n <= TREE_SINGLE_MAX) {
             // One CTA a segment builds its whole tree. Continuous collision traverses the static and sleeping tree by
             // its node boxes and child links; the pair query needs neither.
             const TreeBuild b{caabb.p, list, seg ? t.segStart.p : nullptr, W, n, t.vals.p,
                               seg ? t.sortedKey.p : t.keys.p, seg ? t.sortedWorld.p : nullptr, t.leafAabb.p,
-                              isDyn ? nullptr : t.nodeAabb.p, isDyn ? nullptr : t.child.p, t.rec.p};
+                              isDyn ? nullptr : t.nodeAabb.p, isDyn ? nullptr : t.child.p, t.rec.p, t.meet.p};
             uint32_t count = 0;
             if (isDyn) pbegin(13);
             CK(launch_tree_segments(b, seg ? std::min(maxWorldCols, n) : n, uint32_t(std::max(dev.sms, 1)), s, &count));

@@ -366,6 +366,21 @@ __global__ void k_sort_histogram(const uint32_t* __restrict__ keys, uint32_t n, 
         if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
+// The lanes of a full warp that hold the same 8-bit digit as this one (among the valid): one ballot a bit. match.any
+// serves one distinct value after the other, and the digits of a warp mostly differ: with it the ranking of 2,000 keys
+// in one CTA took 4,100 cycles a pass.
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool valid)
+{
+    uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (uint32_t b = 0; b < 8; b++) {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t with = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? with : ~with;
+    }
+    return peers;
+}
+
 // In-place exclusive scan of each 256-bin digit histogram; launched with 4 blocks of 256 threads.
 __global__ void k_sort_digit_scan(uint32_t* hist)
 {
@@ -411,8 +426,8 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
         const bool valid = idx < n;
         key[k] = valid ? keysIn[idx] : 0u;
         val[k] = valid ? valsIn[idx] : 0u;
-        const uint32_t d = valid ? ((key[k] >> shift) & 0xFFu) : 256u;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t d = (key[k] >> shift) & 0xFFu;
+        const uint32_t peers = digit_peers(d, valid);
         const uint32_t before = __popc(peers & ltMask);
         uint32_t base = 0;
         if (valid) base = warpHist[warp][d];
@@ -593,37 +608,64 @@ __device__ __forceinline__ float4 exchange_box(float4* slot, float4 v)
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// The whole tree of a segment in one CTA: bounds, Morton keys, sort, leaf gather, Karras build and refit, over every
-// world segment [segStart[w], segStart[w + 1]) of a world-grouped list (or the one segment [0, n)) whose size is in
-// (minSize, maxSize]. The results are those of the kernels above and below run one after the other: the sort is a
-// bitonic network over (key << 32 | position), so equal keys keep their list order; steps between elements at most 32
-// apart stay within a warp's 64 elements and need no block barrier. The two subtrees of a node meet by a flag in shared
-// memory, their boxes in the node's record.
-// Bound: barriers and shared-memory latency; one CTA a segment and one launch in place of seven over all segments
-// (bounds, keys, sort, gather, build, refit and their clears), which took 460 us a step on 4,096 worlds and 70 to
-// 95 us on a single world of 64 to 2,048 colliders, most of it launches waiting for one another.
+// The whole tree of a segment in one CTA: bounds, Morton keys, sort, leaf gather and the nodes with their boxes, over
+// every world segment [segStart[w], segStart[w + 1]) of a world-grouped list (or the one segment [0, n)) whose size is
+// in (minSize, maxSize], maxSize at most THREADS x E. The results are those of the kernels above and below run one
+// after the other.
+// Sort: four 8-bit radix passes in shared memory, ranked per warp as k_sort_pass ranks a tile, so equal keys keep their
+// list order.
+// Nodes: bottom up from the leaves. A subtree over [l, r] is the left child of the node that splits after r when the
+// keys r and r + 1 share more bits than l - 1 and l do, else the right child of the one that splits after l - 1. Both
+// children leave their boxes at the split; the second one to arrive there (a meeting word) takes the whole range and
+// carries on. The records are written afterwards, split by split; a node is numbered as Karras numbers it (r as a left
+// child, l as a right child, the root 0).
+// Bound: shared-memory latency and instruction issue of one CTA. One launch a size class in place of seven or more over
+// all segments (bounds, keys, sort, gather, build, refit, their clears), which took 460 us a step on 4,096 worlds and 70
+// to 95 us on one world of 64 to 2,048 colliders; now 250 and 16 to 40. Cycles at 2,000 leaves: sort 15,700, nodes and
+// boxes 22,000, records 6,200. With a bitonic network and Karras's searches in shared memory it was 32,000 for the
+// sort, 21,000 for the nodes and 29,000 for the boxes; the network in registers and shuffles took 20,700.
 // ---------------------------------------------------------------------------------------------------------------
-template <uint32_t THREADS>
-__global__ void __launch_bounds__(THREADS) k_tree_segments(TreeBuild t, uint32_t minSize, uint32_t maxSize)
+// Acquire-release fence of the CTA's memory order (__threadfence_block is the sequentially consistent one).
+__device__ __forceinline__ void fence_cta() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
+
+template <uint32_t THREADS, uint32_t E, bool MEET_SHARED>
+struct TreeSmem {
+    static constexpr uint32_t WARPS = THREADS / 32, CAP = THREADS * E;
+    // The sort's words, and (MEET_SHARED) over them the boxes of both children of every split.
+    static constexpr size_t SORT = (WARPS + 1) * 256 * sizeof(uint32_t) + CAP * (sizeof(uint32_t) + sizeof(uint16_t));
+    __host__ __device__ static constexpr size_t front(uint32_t maxSize)
+    {
+        return MEET_SHARED && size_t(maxSize) * 32 > SORT ? size_t(maxSize) * 32 : SORT;
+    }
+    // Behind them the meeting words and the bits shared by each split's two keys.
+    __host__ __device__ static constexpr size_t bytes(uint32_t maxSize) { return front(maxSize) + 5 * size_t(maxSize) + 16; }
+};
+
+template <uint32_t THREADS, uint32_t E, bool MEET_SHARED>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_tree_segments(TreeBuild t, uint32_t minSize, uint32_t maxSize)
 {
-    // [m] sort words (keys stay in their upper halves through the build, then the meeting flags), m the next power of
-    // two, then per node and per leaf the parent << 1 | side (16 bits each).
-    extern __shared__ unsigned long long treeTile[];
-    __shared__ float4 part[THREADS / 32];
-    constexpr uint32_t NO_PARENT = 0xFFFFu;
+    // The classes work on different segments: the next class's launch need not wait for this one.
+    asm volatile("griddepcontrol.launch_dependents;");
+    using Smem = TreeSmem<THREADS, E, MEET_SHARED>;
+    constexpr uint32_t WARPS = Smem::WARPS;
+    extern __shared__ float4 treeTile[];
+    __shared__ float4 part[WARPS];
+    uint32_t* const hist = reinterpret_cast<uint32_t*>(treeTile);        // [WARPS][256]
+    uint32_t* const digit = hist + WARPS * 256;                          // [256]
+    uint32_t* const sortKey = digit + 256;                               // [CAP]
+    uint16_t* const sortPos = reinterpret_cast<uint16_t*>(sortKey + Smem::CAP);   // [CAP]
+    uint32_t* const met = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(treeTile) + Smem::front(maxSize));
+    uint8_t* const shared = reinterpret_cast<uint8_t*>(met + maxSize);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t ltMask = (1u << lane) - 1u;
     for (uint32_t w = blockIdx.x; w < t.worlds; w += gridDim.x) {
         const uint32_t lo = t.segStart ? t.segStart[w] : 0u, n = t.segStart ? t.segStart[w + 1] - lo : t.n;
         if (n <= minSize || n > maxSize) continue;
-        uint32_t m = 1;
-        while (m < n) m <<= 1;
-        uint16_t* const nodeUp = reinterpret_cast<uint16_t*>(treeTile + m);
-        uint16_t* const leafUp = nodeUp + n;
         const uint32_t* const list = t.list + lo;
         // Bounds of the segment's boxes.
         float4 bb = make_float4(FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX);
         for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
-            const float4 a = t.caabb[list[i]];
+            const float4 a = __ldg(t.caabb + __ldg(list + i));
             bb = make_float4(fminf(bb.x, a.x), fminf(bb.y, a.y), fmaxf(bb.z, a.z), fmaxf(bb.w, a.w));
         }
         for (int o = 16; o > 0; o >>= 1) {
@@ -634,112 +676,220 @@ __global__ void __launch_bounds__(THREADS) k_tree_segments(TreeBuild t, uint32_t
         }
         if (lane == 0) part[warp] = bb;
         __syncthreads();
-        for (uint32_t k = 0; k < THREADS / 32; k++) {
+        for (uint32_t k = 0; k < WARPS; k++) {
             const float4 q = part[k];
             bb = make_float4(fminf(bb.x, q.x), fminf(bb.y, q.y), fmaxf(bb.z, q.z), fmaxf(bb.w, q.w));
         }
-        for (uint32_t i = threadIdx.x; i < m; i += THREADS) {
-            unsigned long long e = ~0ull;
-            if (i < n) e = static_cast<unsigned long long>(morton_key(t.caabb[list[i]], bb.x, bb.y, bb.z, bb.w)) << 32 | i;
-            treeTile[i] = e;
+        // This thread's elements: one a stretch of 32, the stretches of a warp consecutive (list order by warp, then
+        // stretch, then lane). 'per' stretches a warp cover the segment.
+        const uint32_t per = (n + THREADS - 1) / THREADS, base = warp * per * 32u + lane;
+        uint32_t key[E], pos[E], rank[E];
+#pragma unroll
+        for (uint32_t k = 0; k < E; k++) {
+            const uint32_t i = base + k * 32u;
+            pos[k] = i;
+            key[k] = 0u;
+            if (k < per && i < n) key[k] = morton_key(__ldg(t.caabb + __ldg(list + i)), bb.x, bb.y, bb.z, bb.w);
         }
-        __syncthreads();
-        for (uint32_t k = 2; k <= m; k <<= 1) {
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t p = threadIdx.x; p < m / 2; p += THREADS) {
-                    const uint32_t i = ((p & ~(j - 1u)) << 1) | (p & (j - 1u));
-                    const unsigned long long a = treeTile[i], b = treeTile[i + j];
-                    if ((a > b) == ((i & k) == 0)) { treeTile[i] = b; treeTile[i + j] = a; }
+        for (uint32_t shift = 0; shift < 32; shift += 8) {
+            for (uint32_t i = threadIdx.x; i < WARPS * 256; i += THREADS) hist[i] = 0u;
+            __syncthreads();
+            uint32_t* const mine = hist + warp * 256;
+#pragma unroll
+            for (uint32_t k = 0; k < E; k++) {
+                if (k >= per) break;
+                const bool valid = base + k * 32u < n;
+                const uint32_t d = (key[k] >> shift) & 255u;
+                const uint32_t peers = digit_peers(d, valid);
+                const uint32_t before = __popc(peers & ltMask);
+                uint32_t first = 0;
+                if (valid) first = mine[d];
+                __syncwarp();
+                if (valid && before == 0) mine[d] = first + __popc(peers);
+                __syncwarp();
+                rank[k] = first + before;
+            }
+            __syncthreads();
+            for (uint32_t d = threadIdx.x; d < 256; d += THREADS) {
+                uint32_t run = 0;
+#pragma unroll 8
+                for (uint32_t wi = 0; wi < WARPS; wi++) {
+                    const uint32_t c = hist[wi * 256 + d];
+                    hist[wi * 256 + d] = run;
+                    run += c;
                 }
-                if (j > 32u || (j == 1u && k > 32u)) __syncthreads();
-                else __syncwarp();
+                digit[d] = run;
+            }
+            __syncthreads();
+            if (warp == 0) {   // exclusive scan of the digit counts, eight a lane
+                uint32_t local[8], sum = 0;
+#pragma unroll
+                for (uint32_t j = 0; j < 8; j++) { local[j] = digit[lane * 8 + j]; sum += local[j]; }
+                uint32_t incl = sum;
+                for (uint32_t o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                uint32_t excl = incl - sum;
+#pragma unroll
+                for (uint32_t j = 0; j < 8; j++) { digit[lane * 8 + j] = excl; excl += local[j]; }
+            }
+            __syncthreads();
+#pragma unroll
+            for (uint32_t k = 0; k < E; k++) {
+                if (k < per && base + k * 32u < n) {
+                    const uint32_t d = (key[k] >> shift) & 255u;
+                    const uint32_t at = digit[d] + mine[d] + rank[k];
+                    sortKey[at] = key[k];
+                    sortPos[at] = uint16_t(pos[k]);
+                }
+            }
+            __syncthreads();
+            if (shift < 24) {
+#pragma unroll
+                for (uint32_t k = 0; k < E; k++) {
+                    const uint32_t i = base + k * 32u;
+                    if (k < per && i < n) { key[k] = sortKey[i]; pos[k] = sortPos[i]; }
+                }
             }
         }
-        __syncthreads();
+        // Leaves in sorted order; thread i % THREADS takes leaf i from here on.
         for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
-            const unsigned long long e = treeTile[i];
-            const uint32_t c = list[uint32_t(e)];
+            const uint32_t k = sortKey[i], c = __ldg(list + sortPos[i]);
             t.vals[lo + i] = c;
-            t.keys[lo + i] = uint32_t(e >> 32);
+            t.keys[lo + i] = k;
             if (t.sortedWorld) t.sortedWorld[lo + i] = w;
-            t.leafAabb[lo + i] = t.caabb[c];
+            t.leafAabb[lo + i] = __ldg(t.caabb + c);
+            if (i + 1 < n) {
+                const uint32_t x = k ^ sortKey[i + 1];
+                shared[i] = uint8_t(x ? __clz(x) : 32 + __clz(i ^ (i + 1)));
+                met[i] = 0u;
+            }
         }
+        __syncthreads();
         if (n > 1) {
-            const int hi = int(n);
-            auto delta = [&](int i, int j) {
-                if (j < 0 || j >= hi) return -1;
-                const uint32_t a = uint32_t(treeTile[i] >> 32), b = uint32_t(treeTile[j] >> 32);
-                return a != b ? __clz(a ^ b) : 32 + __clz(uint32_t(i) ^ uint32_t(j));
+            float4* const meet = MEET_SHARED ? treeTile : t.meet + 2 * size_t(lo);
+            // Bits shared across the ends of a leaf's stretch, one more than they are; 0 beyond the segment. The subtree
+            // over [l, r] is the left child of its parent (side 0, split after r) when it shares more on its right.
+            auto bits_left = [&](uint32_t l) { return l > 0 ? uint32_t(shared[l - 1]) + 1u : 0u; };
+            auto bits_right = [&](uint32_t r) { return r + 1 < n ? uint32_t(shared[r]) + 1u : 0u; };
+            for (uint32_t i = threadIdx.x; i < n; i += THREADS)
+                meet[bits_right(i) > bits_left(i) ? 2 * i : 2 * i - 1] = t.leafAabb[lo + i];   // written by this thread
+            __syncthreads();
+            // One loop over this thread's leaves and their way up: a lane whose sibling carries on takes its next leaf
+            // while the others of its warp climb. A subtree leaves its outer bound and the bits shared there in the
+            // meeting word, so that its sibling knows the node's place from the exchange alone.
+            uint32_t i = threadIdx.x, l = i, r = i, bl = 0, br = 0;
+            float4 box;
+            auto leaf = [&] {
+                l = r = i;
+                bl = bits_left(i);
+                br = bits_right(i);
+                box = meet[br > bl ? 2 * i : 2 * i - 1];
             };
-            for (int i = int(threadIdx.x); i < hi - 1; i += int(THREADS)) {
-                const KarrasNode k = karras_node(i, delta);
-                const int left = k.first == k.gamma ? ~(int(lo) + k.gamma) : int(lo) + k.gamma;
-                const int right = k.last == k.gamma + 1 ? ~(int(lo) + k.gamma + 1) : int(lo) + k.gamma + 1;
-                if (t.child) t.child[lo + i] = make_int2(left, right);
-                t.rec[lo + i].child = make_int2(left, right);
-                t.rec[lo + i].last = make_int2(int(lo) + k.gamma, int(lo) + k.last);
-                (left < 0 ? leafUp : nodeUp)[k.gamma] = uint16_t(i << 1);
-                (right < 0 ? leafUp : nodeUp)[k.gamma + 1] = uint16_t(i << 1 | 1);
-                if (i == 0) nodeUp[0] = NO_PARENT;
+            if (i < n) leaf();
+            while (i < n) {
+                const bool right = br <= bl;             // this subtree's side
+                const uint32_t g = right ? l - 1 : r;
+                const uint32_t word = right ? (r + 1u) | br << 24 : (l + 1u) | bl << 24;
+                const uint32_t other = atomicExch(met + g, word);
+                bool up = other != 0u;                   // second here
+                if (up) {
+                    fence_cta();
+                    const float4 o = meet[right ? 2 * g : 2 * g + 1];
+                    if (right) { l = (other & 0xFFFFFFu) - 1u; bl = other >> 24; }
+                    else { r = (other & 0xFFFFFFu) - 1u; br = other >> 24; }
+                    met[g] = l | r << 16;                // the word now holds the node's range
+                    const float4 a = right ? o : box, b = right ? box : o;
+                    box = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
+                    up = (bl | br) != 0u;                // not the root
+                    if (up) {
+                        meet[br > bl ? 2 * r : 2 * l - 1] = box;
+                        fence_cta();
+                    }
+                }
+                if (!up) {
+                    i += THREADS;
+                    if (i < n) leaf();
+                }
             }
             __syncthreads();
-            uint32_t* const met = reinterpret_cast<uint32_t*>(treeTile);
-            for (uint32_t i = threadIdx.x; i < n; i += THREADS) met[i] = 0u;
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
-                float4 box = t.leafAabb[lo + i];   // written by this thread
-                uint32_t up = leafUp[i];
-                while (up != NO_PARENT) {
-                    const uint32_t node = up >> 1, side = up & 1u;
-                    NodeRec* const r = t.rec + lo + node;
-                    r->box[side] = box;
-                    __threadfence_block();
-                    if (atomicExch(met + node, 1u) == 0u) break;   // the sibling carries on
-                    __threadfence_block();
-                    const float4 o = r->box[side ^ 1u];
-                    box = make_float4(fminf(box.x, o.x), fminf(box.y, o.y), fmaxf(box.z, o.z), fmaxf(box.w, o.w));
-                    if (t.nodeAabb) t.nodeAabb[lo + node] = box;
-                    up = nodeUp[node];
-                }
+            for (uint32_t g = threadIdx.x; g + 1 < n; g += THREADS) {
+                const uint32_t l = met[g] & 0xFFFFu, r = met[g] >> 16;
+                const bool root = l == 0 && r + 1 == n;
+                const uint32_t node = lo + (root ? 0u : (bits_right(r) > bits_left(l) ? r : l));
+                const int left = l == g ? ~int(lo + g) : int(lo + g);
+                const int right = r == g + 1 ? ~int(lo + g + 1) : int(lo + g + 1);
+                const float4 a = meet[2 * g], b = meet[2 * g + 1];
+                NodeRec* const rec = t.rec + node;
+                rec->box[0] = a;
+                rec->box[1] = b;
+                rec->child = make_int2(left, right);
+                rec->last = make_int2(int(lo + g), int(lo + r));
+                if (t.child) t.child[node] = make_int2(left, right);
+                if (t.nodeAabb)
+                    t.nodeAabb[node] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
             }
         }
         __syncthreads();   // the tile is reused by the next segment
     }
+    // This launch is done only when the class before it is: what follows waits for both.
+    if (threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-size_t tree_segment_smem(uint32_t n)
+template <uint32_t THREADS, uint32_t E, bool MEET_SHARED>
+static cudaError_t launch_tree_class(const TreeBuild& t, uint32_t minSize, uint32_t maxSize, uint32_t sms,
+                                     cudaStream_t stream, uint32_t* launches)
 {
-    size_t m = 1;
-    while (m < n) m <<= 1;
-    return m * sizeof(unsigned long long) + 2 * size_t(n) * sizeof(uint16_t) + 16;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::min(t.worlds, sms * std::max(1u, 2048u / THREADS)));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = TreeSmem<THREADS, E, MEET_SHARED>::bytes(maxSize);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = *launches > 0 ? 1 : 0;   // beside the class launched before it
+    ++*launches;
+    return cudaLaunchKernelEx(&cfg, k_tree_segments<THREADS, E, MEET_SHARED>, t, minSize, maxSize);
+}
+
+template <uint32_t THREADS, uint32_t E, bool MEET_SHARED>
+static cudaError_t tree_class_init(uint32_t maxSize)
+{
+    return cudaFuncSetAttribute(k_tree_segments<THREADS, E, MEET_SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(TreeSmem<THREADS, E, MEET_SHARED>::bytes(maxSize)));
 }
 
 cudaError_t tree_segments_init()
 {
-    return cudaFuncSetAttribute(k_tree_segments<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(tree_segment_smem(TREE_SEGMENT_MAX)));
+    cudaError_t e = tree_class_init<512, 4, true>(2048);
+    if (e == cudaSuccess) e = tree_class_init<1024, 4, true>(4096);
+    if (e == cudaSuccess) e = tree_class_init<1024, 8, false>(8192);
+    if (e == cudaSuccess) e = tree_class_init<1024, 16, false>(TREE_SEGMENT_MAX);
+    return e;
 }
 
 cudaError_t launch_tree_segments(const TreeBuild& t, uint32_t largest, uint32_t sms, cudaStream_t stream,
                                  uint32_t* launches)
 {
-    // Three size classes, each with the CTA that its largest segment keeps busy: segments of a ragged batch differ by a
-    // factor of a hundred, and a small one in a wide CTA waits at barriers with most warps idle.
-    const uint32_t small = std::min(largest, TREE_SEGMENT_SMALL), medium = std::min(largest, TREE_SEGMENT_MEDIUM);
-    const bool one = t.segStart == nullptr;
-    if (!one || largest <= TREE_SEGMENT_SMALL) {
-        k_tree_segments<128><<<std::min(t.worlds, sms * 16u), 128, tree_segment_smem(small), stream>>>(t, 0u, small);
-        ++*launches;
-    }
-    if (largest > TREE_SEGMENT_SMALL && (!one || largest <= TREE_SEGMENT_MEDIUM)) {
-        k_tree_segments<512><<<std::min(t.worlds, sms * 4u), 512, tree_segment_smem(medium), stream>>>(t, small, medium);
-        ++*launches;
-    }
-    if (largest > TREE_SEGMENT_MEDIUM) {
-        k_tree_segments<1024><<<std::min(t.worlds, sms), 1024, tree_segment_smem(largest), stream>>>(t, medium, largest);
-        ++*launches;
-    }
-    return cudaGetLastError();
+    // Size classes, each with the CTA that its largest segment keeps busy: segments of a ragged batch differ by a
+    // factor of a hundred, and a small one in a wide CTA waits at barriers with most warps idle. The longest run first
+    // and the classes overlap. Those up to 4,096 leaves keep the meeting boxes in shared memory (32 B a leaf), the two
+    // above in global memory.
+    const bool one = t.segStart == nullptr;   // one segment of 'largest' leaves: its class alone
+    cudaError_t e = cudaSuccess;
+    *launches = 0;
+    auto takes = [&](uint32_t from, uint32_t to) { return e == cudaSuccess && largest > from && (!one || largest <= to); };
+    auto top = [&](uint32_t to) { return std::min(largest, to); };
+    if (takes(8192, TREE_SEGMENT_MAX)) e = launch_tree_class<1024, 16, false>(t, 8192, largest, sms, stream, launches);
+    if (takes(4096, 8192)) e = launch_tree_class<1024, 8, false>(t, 4096, top(8192), sms, stream, launches);
+    if (takes(2048, 4096)) e = launch_tree_class<1024, 4, true>(t, 2048, top(4096), sms, stream, launches);
+    if (takes(1024, 2048)) e = launch_tree_class<512, 4, true>(t, 1024, top(2048), sms, stream, launches);
+    if (takes(256, 1024)) e = launch_tree_class<256, 4, true>(t, 256, top(1024), sms, stream, launches);
+    if (takes(0, 256)) e = launch_tree_class<128, 2, true>(t, 0, top(256), sms, stream, launches);
+    return e;
 }
 
 // Bottom-up AABB refit (BvhTree::fitNodes equivalent). The two subtrees of a node meet in its slot: each swaps its
