@@ -26,6 +26,29 @@ struct alignas(16) NodeRec {
 };
 static_assert(sizeof(NodeRec) == 48, "NodeRec is 48 bytes");
 
+// Warm start: the previous step's manifolds in an open-addressing table keyed by the unordered collider pair, those
+// with a non-zero impulse on an active contact flagged (bit 31 of the value: the reference caches only these,
+// rebuildContactCache, NarrowPhaseCollisionDetector.cpp:272-297; makePairKey .h:216-219); each new manifold of the
+// same ordered pair takes the flagged manifold's impulses of the contacts with equal ids (finalizeResults,
+// :749-766). Every new manifold whose pair was there also takes that manifold's colour as its colouring hint.
+// One region of the table per world of a batch, [2 seg[w], 2 seg[w + 1]) for the world's seg[w + 1] - seg[w] previous
+// manifolds (seg: the previous list's world starts), so a probe stays in its world's few kilobytes and hits in cache;
+// a single world (seg null) uses the whole power-of-two table. Which region holds a pair changes nothing but where
+// it is found.
+constexpr uint32_t WARM_CACHED = 0x80000000u;   // the manifold had a non-zero impulse
+struct WarmTable {
+    unsigned long long* keys;   // all ones: empty; null: no warm start
+    uint32_t* vals;
+    uint32_t capacity;
+    const uint32_t* seg;
+    const uint32_t* colWorld;
+    const Manifold* prev;
+    const uint32_t* nPrev;
+    const uint32_t* prevColor;   // or null
+    uint32_t* hint;              // colouring hints of the new manifolds out, or null
+    uint32_t* status;
+};
+
 // Read-only view of one LBVH over n leaves in sorted order. A single tree has n - 1 internal nodes and root 0; a
 // world-segmented tree (sortedWorld non-null) holds one tree per world segment [segStart[w], segStart[w + 1]),
 // rooted at internal node segStart[w].
@@ -41,10 +64,41 @@ struct TreeView {
 };
 
 // Spatial kernels (k_spatial.cu).
-__global__ void k_integrate(DeviceWorld w, const uint32_t* dynBody, const uint8_t* dynSimd, uint32_t nDyn, float dt,
-                            float gx, float gy, float dampHalf, uint32_t phase);
+struct IntegrateParams {
+    float dt, gx, gy;
+    float dampHalf;   // damping^(dt/2), or >= 1 when damping is off
+};
+__global__ void k_integrate(DeviceWorld w, const uint32_t* dynBody, const uint8_t* dynSimd, uint32_t nDyn,
+                            IntegrateParams ip, uint32_t phase);
+// A 16-byte aligned buffer to fill with a value, or (iota) with its indices.
+struct FillRegion {
+    uint32_t* p;
+    uint32_t words, value, iota;
+};
+constexpr uint32_t MAX_FILLS = 12;
+struct StepBegin {
+    DeviceWorld w;
+    float4 *snapVel, *snapPos;
+    float2* snapRot;
+    float *snapWrap, *snapTimer;
+    uint8_t* snapState;
+    uint32_t* snapIsland;
+    const uint32_t* dynBody;   // the dynamic bodies
+    const uint8_t* dynSimd;
+    uint32_t nDyn;
+    uint32_t both;             // both halves of the integration, else the first
+    IntegrateParams ip;
+    float4* copyDst;           // collider poses to save (or bring back) for continuous collision
+    const float4* copySrc;
+    uint32_t copyCount;
+    uint32_t fills;
+    FillRegion fill[MAX_FILLS];
+    const uint32_t* nIsle;
+    StepCounters* counters;
+};
+__global__ void k_step_begin(StepBegin a);
 __global__ void k_collider_pose(DeviceWorld w, const uint32_t* list, const uint8_t* listSimd, uint32_t n,
-                                const uint32_t* worldMask);
+                                const uint32_t* worldMask, WarmTable insert);
 __global__ void k_bounds_init(uint32_t* bounds, uint32_t worlds);
 __global__ void k_bounds(const float4* aabb, const uint32_t* list, uint32_t n, const uint32_t* colWorld,
                          uint32_t* bounds);
@@ -139,16 +193,51 @@ __device__ __forceinline__ uint32_t scan_lookback(uint32_t tile, uint32_t* tileS
     return prefix;
 }
 
-// Contact-cache key of an unordered collider pair, and its home slot in a power-of-two open-addressing table.
+// Contact-cache key of an unordered collider pair, and the region of the table that holds it.
 __device__ __forceinline__ unsigned long long pair_key(uint32_t a, uint32_t b)
 {
     const uint32_t lo = a < b ? a : b, hi = a < b ? b : a;
     return (static_cast<unsigned long long>(lo) << 32) | hi;
 }
-__device__ __forceinline__ uint32_t slot_of(unsigned long long key, uint32_t capacity)
+struct WarmRegion {
+    uint32_t base, size;   // size 0: the world had no manifolds
+    __device__ __forceinline__ uint32_t home(unsigned long long key) const
+    {
+        return base + uint32_t(((key * 0x9E3779B97F4A7C15ull) >> 32) % size);
+    }
+    __device__ __forceinline__ uint32_t next(uint32_t s) const { return s + 1 == base + size ? base : s + 1; }
+};
+__device__ __forceinline__ WarmRegion warm_region(const WarmTable& t, uint32_t a)
 {
-    const uint32_t shift = 64u - (31u - __clz(capacity));   // capacity is a power of two
-    return static_cast<uint32_t>((key * 0x9E3779B97F4A7C15ull) >> shift) & (capacity - 1u);
+    if (!t.seg) return WarmRegion{0u, t.capacity};
+    const uint32_t wd = t.colWorld[a];
+    const uint32_t lo = t.seg[wd], hi = t.seg[wd + 1];
+    if (hi < lo || 2ull * hi > t.capacity) return WarmRegion{0u, 0u};   // not a valid segmentation: no region
+    return WarmRegion{2u * lo, 2u * (hi - lo)};
+}
+// Puts the previous manifolds into the (empty) table, grid-stride over all threads of the launch.
+__device__ __forceinline__ void warm_insert(const WarmTable& t)
+{
+    const uint32_t n = *t.nPrev;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint2 pair = *reinterpret_cast<const uint2*>(&t.prev[i].a);
+        const uint32_t count = t.prev[i].count;
+        const float4 j = *reinterpret_cast<const float4*>(&t.prev[i].jn0);
+        uint32_t mask = uint32_t(j.x != 0.0f) | uint32_t(j.y != 0.0f) << 1 | uint32_t(j.z != 0.0f) << 2 |
+                        uint32_t(j.w != 0.0f) << 3;
+        mask &= (1u << (2u * count)) - 1u;
+        const unsigned long long key = pair_key(pair.x, pair.y);
+        const WarmRegion r = warm_region(t, pair.x);
+        if (r.size == 0) { atomicOr(t.status, STATUS_HASH_FULL); continue; }   // cannot happen: m is in its world
+        uint32_t s = r.home(key);
+        uint32_t probes = 0;
+        for (;;) {
+            const unsigned long long old = atomicCAS(t.keys + s, ~0ull, key);
+            if (old == ~0ull || old == key) { t.vals[s] = i | (mask ? WARM_CACHED : 0u); break; }
+            s = r.next(s);
+            if (++probes >= r.size) { atomicOr(t.status, STATUS_HASH_FULL); break; }
+        }
+    }
 }
 
 // Exclusive scan of in[0, min(n, *nDev)) into out (nDev may be null), total = the sum (may be null).
@@ -163,15 +252,8 @@ constexpr uint32_t NARROW_SMEM_PER_THREAD =
 // tileCounter zeroed before the launch (tiles: blockDim.x / 32 x perWarp pairs each, perWarp at most 32).
 __global__ void k_narrow(DeviceWorld w, const uint2* pairs, const uint32_t* nPairs, uint32_t pairCap, Manifold* out,
                          uint32_t manifoldCap, uint32_t* nOut, StepCounters* counters, uint32_t* tileState,
-                         uint32_t* tileCounter, uint32_t perWarp);
-__global__ void k_warm_insert(const Manifold* prev, const uint32_t* nPrev, unsigned long long* keys,
-                              uint32_t* vals, uint32_t capacity, const uint32_t* seg, const uint32_t* colWorld,
-                              uint32_t* status);
-constexpr uint32_t WARM_CACHED = 0x80000000u;   // contact-cache value flag: the manifold had a non-zero impulse
-__global__ void k_warm_lookup(const Manifold* prev, Manifold* cur, const uint32_t* nCur,
-                              const unsigned long long* keys, const uint32_t* vals, uint32_t capacity,
-                              const uint32_t* seg, const uint32_t* colWorld, StepCounters* counters,
-                              const uint32_t* prevColor, uint32_t* hint);
+                         uint32_t* tileCounter, uint32_t perWarp, WarmTable warm, uint32_t* wakeIsland);
+__global__ void k_warm_insert(WarmTable t);
 __global__ void k_wake(DeviceWorld w, const Manifold* m, const uint32_t* nM, uint32_t* wakeIsland,
                        StepCounters* counters);
 __global__ void k_wake_apply(DeviceWorld w, const uint32_t* wakeIsland, StepCounters* counters);
@@ -179,9 +261,19 @@ __global__ void k_island_init(DeviceWorld w, uint32_t* parent, uint32_t* flag);
 __global__ void k_island_union(DeviceWorld w, const Manifold* m, const uint32_t* nM, uint32_t* parent);
 __global__ void k_island_quiet(DeviceWorld w, uint32_t* parent, uint32_t* flag, float dt, float speedThreshold,
                                float timeThreshold);
-__global__ void k_island_sleep(DeviceWorld w, uint32_t* parent, const uint32_t* flag, StepCounters* counters);
+// The end of a step on the device, by the last block of its last kernel: the warm-start count (a step without error
+// bits becomes the next one's source) and the counters written to page-locked host memory. done: blocks finished,
+// zeroed before the launch; null host: not the end of a step.
+struct StepEnd {
+    StepCounters* host;
+    uint32_t* done;
+    const uint32_t* nManifolds;
+    uint32_t* nPrev;
+};
+__global__ void k_island_sleep(DeviceWorld w, uint32_t* parent, const uint32_t* flag, StepCounters* counters,
+                               StepEnd end);
 __global__ void k_state_flags(const uint8_t* bstate, const uint32_t* cbody, uint32_t nBodies, uint32_t nColliders,
-                              uint32_t* bodyDyn, uint32_t* colDyn, uint32_t* colOther);
+                              uint32_t* bodyDyn, uint32_t* colDyn, uint32_t* colOther, uint32_t* sleeping);
 __global__ void k_scatter_list(const uint32_t* flag, const uint32_t* offset, uint32_t n, uint32_t* list);
 
 // Sleeping-island manifold store (k_islands.cu): restore at wake, move at sleep.

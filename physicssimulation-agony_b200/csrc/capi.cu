@@ -564,6 +564,9 @@ struct ag2d_world {
     DBuf<Manifold> sleepList;
     bool prevHoldsSleepers = false;   // the warm-start list still holds records moved to the store (compactPrev)
     bool islandsLinked = false;       // this step's team solver already linked the islands (phaseIslands skips it)
+    bool anySleeping = false;         // a body sleeps, as of the last list rebuild
+    bool begun = false;               // k_step_begin ran for this step: its clears and the warm-start table are there
+    DBuf<uint32_t> stepDone;          // blocks of the step's last kernel that have finished
     DBuf<float4> consQ;     // solver records (ConsRecords), their stride the manifold capacity they were sized for
     DBuf<float> consPen;
     DBuf<uint2> pairBodies;
@@ -1309,7 +1312,8 @@ struct ag2d_world {
         nPrev.reserve(1);
         nIsle.reserve(1);
         isleCounts.reserve(8);
-        listCounts.reserve(3);
+        listCounts.reserve(4);
+        stepDone.reserve(4);
         colorCount.reserve(COLOR_SLOTS);
         colorStart.reserve(MAX_COLORS + 1);
         CK(cudaMemsetAsync(nPrev.p, 0, sizeof(uint32_t), stream));
@@ -1532,7 +1536,9 @@ struct ag2d_world {
         listRebuilds++;
         const cudaStream_t s = stream;
         const uint32_t nmax = std::max(nBodies, nColliders);
-        k_state_flags<<<gridFor(nmax), 256, 0, s>>>(bstate.p, cbody.p, nBodies, nColliders, flagA.p, flagB.p, flagC.p);
+        CK(cudaMemsetAsync(listCounts.p + 3, 0, sizeof(uint32_t), s));
+        k_state_flags<<<gridFor(nmax), 256, 0, s>>>(bstate.p, cbody.p, nBodies, nColliders, flagA.p, flagB.p, flagC.p,
+                                                    listCounts.p + 3);
         CK(cudaGetLastError());
         scanner.run(flagA.p, offA.p, nBodies, listCounts.p + 0, s);
         scanner.run(flagB.p, offB.p, nColliders, listCounts.p + 1, s);
@@ -1551,12 +1557,13 @@ struct ag2d_world {
             CK(cudaGetLastError());
             launches += 2;
         }
-        uint32_t counts[3] = {0, 0, 0};
+        uint32_t counts[4] = {0, 0, 0, 0};
         CK(cudaMemcpyAsync(counts, listCounts.p, sizeof(counts), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         nDynBody = counts[0];
         nDynCol = counts[1];
         nOther = counts[2];
+        anySleeping = counts[3] != 0;
         if (nWorlds > 1) {
             // SIMD-path flag of each entry: its rank within its world's part of the list against (count & ~7).
             const uint32_t W = nWorlds;
@@ -1595,42 +1602,145 @@ struct ag2d_world {
     }
 
     // ---- phases ----
-    void phaseIntegrate()
+    IntegrateParams integrateParams() const
     {
         const float damp = settings.angular_damping;
         const float dampHalf = (damp >= 0.0f && damp < 1.0f) ? std::pow(damp, settings.dt * 0.5f) : 2.0f;
-        if (nDynBody) {
-            pbegin(0);
-            const uint8_t* simd = nWorlds > 1 ? dynSimd.p : nullptr;
-            if (jointsActive()) {
-                // The constraints between the halves (Simulation::integrateAndApplyConstraints, :392-407).
-                k_integrate<<<gridFor(nDynBody), 256, 0, stream>>>(view(), dynBody.p, simd, nDynBody, settings.dt,
-                                                                  settings.gravity_x, settings.gravity_y, dampHalf, 1u);
-                launchJoints();
-                k_integrate<<<gridFor(nDynBody), 256, 0, stream>>>(view(), dynBody.p, simd, nDynBody, settings.dt,
-                                                                  settings.gravity_x, settings.gravity_y, dampHalf, 2u);
-                launches += 2;
-            } else {
-                k_integrate<<<gridFor(nDynBody), 256, 0, stream>>>(view(), dynBody.p, simd, nDynBody, settings.dt,
-                                                                  settings.gravity_x, settings.gravity_y, dampHalf, 3u);
-                launches++;
-            }
-            CK(cudaGetLastError());
-            pend(0);
+        return IntegrateParams{settings.dt, settings.gravity_x, settings.gravity_y, dampHalf};
+    }
+
+    void integrateHalves(uint32_t phase)
+    {
+        k_integrate<<<gridFor(nDynBody), 256, 0, stream>>>(view(), dynBody.p, nWorlds > 1 ? dynSimd.p : nullptr, nDynBody,
+                                                          integrateParams(), phase);
+        CK(cudaGetLastError());
+        launches++;
+    }
+
+    void phaseIntegrate()
+    {
+        if (!nDynBody) return;
+        pbegin(0);
+        if (jointsActive()) {
+            // The constraints between the halves (Simulation::integrateAndApplyConstraints, :392-407).
+            integrateHalves(1u);
+            launchJoints();
+            integrateHalves(2u);
+        } else {
+            integrateHalves(3u);
         }
+        pend(0);
+    }
+
+    // The start of a step (k_step_begin), with the constraints and the integration's second half where there are any.
+    // 'again': the step is being redone (continuous collision starts from the saved poses).
+    void phaseBegin(bool again)
+    {
+        const cudaStream_t s = stream;
+        pbegin(0);
+        if (motorsOnDevice)
+            CK(cudaMemcpyAsync(snapMotorImpulse.p, motorImpulse.p, motorsOnDevice * sizeof(float),
+                               cudaMemcpyDeviceToDevice, s));
+        const bool joints = nDynBody && jointsActive();
+        StepBegin a{};
+        a.w = view();
+        a.snapVel = snapVel.p; a.snapPos = snapPos.p; a.snapRot = snapRot.p; a.snapWrap = snapWrap.p;
+        a.snapTimer = snapTimer.p; a.snapState = snapState.p; a.snapIsland = snapIsland.p;
+        a.dynBody = dynBody.p;
+        a.dynSimd = nWorlds > 1 ? dynSimd.p : nullptr;
+        a.nDyn = nDynBody;
+        a.both = joints ? 0u : 1u;
+        a.ip = integrateParams();
+        if (settings.ccd && nColliders) {
+            // The poses continuous collision sweeps from; a retried step starts again from the same poses.
+            a.copyDst = again ? cpose.p : prevPose.p;
+            a.copySrc = again ? prevPose.p : cpose.p;
+            a.copyCount = nColliders;
+        }
+        uint64_t most = std::max(nBodies, nColliders);
+        auto fill = [&](auto* p, uint64_t words, uint32_t value, uint32_t iota = 0u) {
+            if (!words) return;
+            a.fill[a.fills++] = FillRegion{reinterpret_cast<uint32_t*>(p), uint32_t(words), value, iota};
+            most = std::max(most, iota ? words : words / 4);
+        };
+        const uint64_t nb = std::max<uint32_t>(nBodies, 1);
+        fill(wakeIsland.p, nb, 0u);
+        fill(stepDone.p, 1, 0u);
+        if (nDynCol) {
+            queryState.reserve(size_t(queryTiles()) + 1);
+            fill(queryState.p, uint64_t(queryTiles()) + 1, 0u);
+        }
+        fill(narrowState.p, uint64_t(narrowTiles()) + 1, 0u);
+        fill(hashKeys.p, 2ull * warmSlots(), 0xFFFFFFFFu);
+        if (!blockSolver()) {
+            fill(bodyMax.p, 2 * nb, 0u);
+            fill(bodyMask.p, 2 * nb, 0u);
+            fill(bar.p, 2, 0u);
+            fill(ufParent.p, nb, 0u, 1u);
+            fill(ufFlag.p, nb, 1u);
+            if (nWorlds > 1) fill(nextWorld.p, 2, 0u);
+        }
+        a.nIsle = nIsle.p;
+        a.counters = dCounters.p;
+        k_step_begin<<<gridFor(most), 256, 0, s>>>(a);
+        CK(cudaGetLastError());
+        launches++;
+        if (joints) {
+            launchJoints();
+            integrateHalves(2u);
+        }
+        pend(0);
+        begun = true;
     }
 
     // full: every collider (or, with 'changedWorlds', those of the worlds whose bodies changed state this step).
-    void phasePose(bool full, bool changedWorlds = false)
+    void phasePose(bool full, bool changedWorlds = false, const WarmTable& insert = WarmTable{})
     {
         const uint32_t n = full ? nColliders : nDynCol;
-        if (n == 0) return;
+        if (n == 0) {
+            if (insert.keys) warmInsert(insert);
+            return;
+        }
         pbegin(1);
         const uint32_t* mask = (full && changedWorlds && nWorlds > 1) ? worldDirty.p : nullptr;
-        k_collider_pose<<<gridFor(n), 256, 0, stream>>>(view(), full ? nullptr : dynCol.p,
-                                                         (full || nWorlds == 1) ? nullptr : dynColSimd.p, n, mask);
+        k_collider_pose<<<gridFor(std::max(n, insert.keys ? prevCount : 0u)), 256, 0, stream>>>(
+            view(), full ? nullptr : dynCol.p, (full || nWorlds == 1) ? nullptr : dynColSimd.p, n, mask, insert);
         CK(cudaGetLastError());
         pend(1);
+        launches++;
+    }
+
+    // Warm-start table size: for the manifolds actually stored (load <= 1/2), not the buffer capacity: a smaller table
+    // is cheaper to clear and stays in L2.
+    uint32_t warmSlots() const
+    {
+        uint32_t slots = 1024;
+        while (slots < 2 * prevCount && slots < hashCap) slots <<= 1;
+        return std::min(slots, hashCap);
+    }
+    // The table over the previous step's manifolds. A batch keeps one region per world (the previous list's world
+    // starts, kept from the last step's solve or recomputed when the list changed since).
+    WarmTable warmTable()
+    {
+        const uint32_t* seg = nullptr;
+        if (nWorlds > 1) {
+            prevSeg.reserve(nWorlds + 1);
+            if (!prevSegValid) {
+                k_manifold_segments<<<gridFor(manifoldCap), 256, 0, stream>>>(prevManifolds.p, nPrev.p, cbody.p,
+                                                                              bodyWorld.p, nWorlds, prevSeg.p);
+                CK(cudaGetLastError());
+                launches++;
+                prevSegValid = true;
+            }
+            seg = prevSeg.p;
+        }
+        return WarmTable{hashKeys.p, hashVals.p, warmSlots(), seg, colWorld.p, prevManifolds.p, nPrev.p, prevColor.p,
+                         color.p, &dCounters.p->status};
+    }
+    void warmInsert(const WarmTable& t)
+    {
+        k_warm_insert<<<gridFor(std::max<uint32_t>(prevCount, 1)), 256, 0, stream>>>(t);
+        CK(cudaGetLastError());
         launches++;
     }
 
@@ -1746,6 +1856,8 @@ struct ag2d_world {
         launches += 3;
     }
 
+    uint32_t queryTiles() const { return div_up(nDynCol, queryThreads); }
+
     void phaseBroad()
     {
         const cudaStream_t s = stream;
@@ -1767,9 +1879,11 @@ struct ag2d_world {
         pbegin(4);
         launches += 1;
         const uint32_t gq = gridFor(nDynCol, queryThreads);
-        const uint32_t tiles = div_up(nDynCol, queryThreads);
-        queryState.reserve(size_t(tiles) + 1);
-        CK(cudaMemsetAsync(queryState.p, 0, (size_t(tiles) + 1) * sizeof(uint32_t), s));
+        const uint32_t tiles = queryTiles();
+        if (!begun) {
+            queryState.reserve(size_t(tiles) + 1);
+            CK(cudaMemsetAsync(queryState.p, 0, (size_t(tiles) + 1) * sizeof(uint32_t), s));
+        }
         k_query<<<gq, queryThreads, 0, s>>>(dynTree.view(), otherTree.view(), cbody.p, pairs.p, pairCap, total,
                                             &dCounters.p->status, queryState.p, queryState.p + tiles);
         CK(cudaGetLastError());
@@ -1794,66 +1908,58 @@ struct ag2d_world {
         return 32u;
     }
 
+    uint32_t narrowTiles() const
+    {
+        return std::max<uint32_t>(div_up(pairCap, narrowThreads / 32 * narrowPerWarp()), 1);
+    }
+
+    // The narrow phase with the warm start of its manifolds (not for a collision-detection pass alone). Within a step
+    // (begun) the clears and the table are there already and the manifolds mark the sleeping islands they wake.
     void phaseNarrow(bool warm = true)
     {
         const cudaStream_t s = stream;
         islandsLinked = false;
         const uint32_t* nPairs = &dCounters.p->pairs;
+        WarmTable table{};
+        if (warm) table = warmTable();
+        if (!begun) {
+            CK(cudaMemsetAsync(narrowState.p, 0, (size_t(narrowTiles()) + 1) * sizeof(uint32_t), s));
+            if (warm) {
+                CK(cudaMemsetAsync(hashKeys.p, 0xFF, size_t(table.capacity) * sizeof(unsigned long long), s));
+                warmInsert(table);
+            }
+        }
         // Work bounded by the device-side pair count (the tile states for the capacity); grid and pairs per warp
         // from the last count; the manifolds are compacted in the same kernel.
-        const uint32_t perWarp = narrowPerWarp(), tilePairs = narrowThreads / 32 * perWarp;
+        const uint32_t perWarp = narrowPerWarp();
         const uint32_t gn = std::min(gridFor(uint64_t(pairEstimate()) * 32 / perWarp, narrowThreads),
                                      gridFor(uint64_t(pairCap) * 32 / perWarp, narrowThreads));
-        const uint32_t tilesCap = std::max<uint32_t>(div_up(pairCap, tilePairs), 1);
         pbegin(5);
-        CK(cudaMemsetAsync(narrowState.p, 0, (size_t(tilesCap) + 1) * sizeof(uint32_t), s));
         k_narrow<<<gn, narrowThreads, narrowThreads * NARROW_SMEM_PER_THREAD, s>>>(
             view(), pairs.p, nPairs, pairCap, manifolds.p, manifoldCap, nManifolds.p, dCounters.p, narrowState.p,
-            narrowState.p + tilesCap, perWarp);
+            narrowState.p + narrowTiles(), perWarp, table, begun && anySleeping ? wakeIsland.p : nullptr);
         CK(cudaGetLastError());
         pend(5);
         launches += 1;
-        if (!warm) return;
-        pbegin(7);
-        // Warm start from the previous step's manifolds.
-        // Table sized for the manifolds actually stored (load <= 1/2), not the buffer capacity: a smaller table is
-        // cheaper to clear and stays in L2.
-        uint32_t slotsUsed = 1024;
-        while (slotsUsed < 2 * prevCount && slotsUsed < hashCap) slotsUsed <<= 1;
-        slotsUsed = std::min(slotsUsed, hashCap);
-        CK(cudaMemsetAsync(hashKeys.p, 0xFF, size_t(slotsUsed) * sizeof(unsigned long long), s));
-        // A batch keeps one table region per world (the previous list's world starts, kept from the last step's
-        // solve or recomputed when the list changed since).
-        const uint32_t* seg = nullptr;
-        if (nWorlds > 1) {
-            prevSeg.reserve(nWorlds + 1);
-            if (!prevSegValid) {
-                k_manifold_segments<<<gridFor(manifoldCap), 256, 0, s>>>(prevManifolds.p, nPrev.p, cbody.p,
-                                                                         bodyWorld.p, nWorlds, prevSeg.p);
-                launches++;
-            }
-            seg = prevSeg.p;
-        }
-        k_warm_insert<<<gridFor(manifoldCap), 256, 0, s>>>(prevManifolds.p, nPrev.p, hashKeys.p, hashVals.p, slotsUsed,
-                                                           seg, colWorld.p, &dCounters.p->status);
-        k_warm_lookup<<<gridFor(manifoldCap), 256, 0, s>>>(prevManifolds.p, manifolds.p, nManifolds.p, hashKeys.p,
-                                                           hashVals.p, slotsUsed, seg, colWorld.p, dCounters.p,
-                                                           prevColor.p, color.p);
-        hintsReady = true;
-        CK(cudaGetLastError());
-        pend(7);
+        hintsReady = warm;
     }
 
+    // Sleeping islands that the step's manifolds touch wake. Within a step the narrow phase has marked them, and there
+    // is nothing to wake when no body sleeps.
     void phaseWake()
     {
+        if (begun && !anySleeping) return;
         const cudaStream_t s = stream;
         pbegin(8);
-        launches += 2;
-        CK(cudaMemsetAsync(wakeIsland.p, 0, sizeof(uint32_t) * std::max<uint32_t>(nBodies, 1), s));
-        k_wake<<<gridFor(manifoldCap), 256, 0, s>>>(view(), manifolds.p, nManifolds.p, wakeIsland.p, dCounters.p);
+        if (!begun) {
+            CK(cudaMemsetAsync(wakeIsland.p, 0, sizeof(uint32_t) * std::max<uint32_t>(nBodies, 1), s));
+            k_wake<<<gridFor(manifoldCap), 256, 0, s>>>(view(), manifolds.p, nManifolds.p, wakeIsland.p, dCounters.p);
+            launches++;
+        }
         k_wake_apply<<<gridFor(nBodies), 256, 0, s>>>(view(), wakeIsland.p, dCounters.p);
         CK(cudaGetLastError());
         pend(8);
+        launches++;
     }
 
     // Manifolds of the islands that woke this step join the list (k_islands.cu, restore): fresh manifolds of their
@@ -1861,7 +1967,7 @@ struct ag2d_world {
     // merged into mergeMan / mergeHint, which then become 'manifolds' / 'color').
     void phaseRestore()
     {
-        if (isleUpper == 0) return;
+        if (isleUpper == 0 || (begun && !anySleeping)) return;
         const cudaStream_t s = stream;
         const DeviceWorld wv = view();
         reserveIsleScratch(isleUpper);
@@ -2228,6 +2334,9 @@ struct ag2d_world {
         }
     }
 
+    // A single world small enough for one CTA's solver.
+    bool blockSolver() const { return nWorlds == 1 && nBodies <= BLOCK_SOLVE_BODIES && !dev.gridOnly; }
+
     void phaseSolve()
     {
         const cudaStream_t s = stream;
@@ -2243,12 +2352,14 @@ struct ag2d_world {
         if (nWorlds > 1) {
             // One CTA per world over the world-grouped manifold list; the teams also link their islands
             // (phaseIslands then only decides sleep). Teams too large for the body cache colour in global memory.
-            CK(cudaMemsetAsync(bodyMax.p, 0, sizeof(unsigned long long) * std::max<uint32_t>(nBodies, 1), s));
-            CK(cudaMemsetAsync(bodyMask.p, 0, sizeof(unsigned long long) * std::max<uint32_t>(nBodies, 1), s));
-            CK(cudaMemsetAsync(nextWorld.p, 0, 2 * sizeof(uint32_t), s));
-            k_island_init<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p);
+            if (!begun) {
+                CK(cudaMemsetAsync(bodyMax.p, 0, sizeof(unsigned long long) * std::max<uint32_t>(nBodies, 1), s));
+                CK(cudaMemsetAsync(bodyMask.p, 0, sizeof(unsigned long long) * std::max<uint32_t>(nBodies, 1), s));
+                CK(cudaMemsetAsync(nextWorld.p, 0, 2 * sizeof(uint32_t), s));
+                k_island_init<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p);
+                launches++;
+            }
             islandsLinked = true;
-            launches++;
             k_manifold_segments<<<gridFor(manifoldCap), 256, 0, s>>>(mm, nm, cbody.p, bodyWorld.p, nWorlds,
                                                                       manSeg.p);
             scratch.prio = prio.p;
@@ -2273,7 +2384,7 @@ struct ag2d_world {
                 CK(cudaStreamWaitEvent(s, joinEvent, 0));
             }
             launches++;
-        } else if (nBodies <= BLOCK_SOLVE_BODIES && !dev.gridOnly) {
+        } else if (blockSolver()) {
             // One CTA, bodies in shared memory; it also links the islands.
             const BlockSolve args{w, mm, nm, scratch, std::max<uint32_t>(nBodies, 1), vi, pi, ufParent.p, ufFlag.p, ctr};
             CK(launch_color_solve_block(lastManifolds, s, args));
@@ -2281,9 +2392,11 @@ struct ag2d_world {
         } else {
             // Whole-grid cooperative launch: about a warp of manifolds on each of a CTA's first four warps before a
             // second CTA is added, up to every SM.
-            CK(cudaMemsetAsync(bodyMax.p, 0, sizeof(unsigned long long) * nBodies, s));
-            CK(cudaMemsetAsync(bodyMask.p, 0, sizeof(unsigned long long) * nBodies, s));
-            CK(cudaMemsetAsync(bar.p, 0, 2 * sizeof(uint32_t), s));
+            if (!begun) {
+                CK(cudaMemsetAsync(bodyMax.p, 0, sizeof(unsigned long long) * nBodies, s));
+                CK(cudaMemsetAsync(bodyMask.p, 0, sizeof(unsigned long long) * nBodies, s));
+                CK(cudaMemsetAsync(bar.p, 0, 2 * sizeof(uint32_t), s));
+            }
             flowVel.reserve(nBodies); flowPos.reserve(nBodies); flowPosRec.reserve(2 * size_t(manifoldCap));
             flowCons.reserve(manifoldCap);
             FlowScratch flow{flowVel.p, flowPos.p, flowCons.p, flowPosRec.p};
@@ -2303,9 +2416,13 @@ struct ag2d_world {
         const cudaStream_t s = stream;
         const DeviceWorld w = view();
         pbegin(11);
-        launches += islandsLinked ? 2 : 4;
+        launches += 2;
         if (!islandsLinked) {
-            k_island_init<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p);
+            if (!begun) {
+                k_island_init<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p);
+                launches++;
+            }
+            launches++;
             k_island_union<<<gridFor(manifoldCap), 256, 0, s>>>(w, manifolds.p, nManifolds.p, ufParent.p);
         }
         if (nJointEdges) {   // after the teams' links too: union-find links in any order
@@ -2315,14 +2432,18 @@ struct ag2d_world {
         islandsLinked = false;
         k_island_quiet<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p, settings.dt, settings.sleep_speed,
                                                         settings.sleep_time);
-        k_island_sleep<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p, dCounters.p);
+        // Within a step this is its last kernel: it leaves the counters in page-locked memory.
+        const StepEnd end{begun ? hCounters : nullptr, stepDone.p, nManifolds.p, nPrev.p};
+        k_island_sleep<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p, dCounters.p, end);
         CK(cudaGetLastError());
         pend(11);
     }
 
     void readCounters()
     {
-        CK(cudaMemcpyAsync(hCounters, dCounters.p, sizeof(StepCounters), cudaMemcpyDeviceToHost, stream));
+        if (!begun)
+            CK(cudaMemcpyAsync(hCounters, dCounters.p, sizeof(StepCounters), cudaMemcpyDeviceToHost, stream));
+        begun = false;
         const auto t0 = std::chrono::steady_clock::now();
         CK(cudaStreamSynchronize(stream));
         syncMs += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -2842,26 +2963,27 @@ struct ag2d_world {
             if (attempt > 0) retries++;
             if (listsDirty) rebuildLists();
             const cudaStream_t s = stream;
-            CK(cudaMemsetAsync(dCounters.p, 0, sizeof(StepCounters), s));
-            CK(cudaMemcpyAsync(&dCounters.p->stored, nIsle.p, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-            snapshot(false);
-            if (settings.ccd && nColliders) {
-                // The poses continuous collision sweeps from; a retried step starts again from the same poses.
-                if (attempt == 0)
-                    CK(cudaMemcpyAsync(prevPose.p, cpose.p, sizeof(float4) * nColliders, cudaMemcpyDeviceToDevice, s));
-                else
-                    CK(cudaMemcpyAsync(cpose.p, prevPose.p, sizeof(float4) * nColliders, cudaMemcpyDeviceToDevice, s));
-            }
             const bool fullPoseThisStep = fullPose;
             const bool otherDirtyThisStep = otherDirty;
-            CK(cudaMemsetAsync(wrapCount.p, 0, sizeof(float) * std::max<uint32_t>(nBodies, 1), s));   // preUpdate
-            phaseIntegrate();
-            phasePose(fullPose);
+            struct Begun {   // an error on the way leaves no step begun
+                bool& b;
+                ~Begun() { b = false; }
+            } endBegun{begun};
+            phaseBegin(attempt > 0);
+            {
+                const WarmTable table = warmTable();
+                // Few manifolds go into the table beside the poses, which saves a launch; many in a launch of their
+                // own (2.7 M: 220 us with the poses in two launches, 343 in one).
+                const bool beside = prevCount <= 65536;
+                if (!beside) warmInsert(table);
+                phasePose(fullPose, false, beside ? table : WarmTable{});
+            }
             if (newWorldsPending && !fullPose) {
                 // Worlds that joined a server batch: their first step poses every collider, as alone.
                 const DeviceWorld wv = view();
                 k_collider_pose<<<gridFor(nColliders), 256, 0, s>>>(wv, nullptr, nullptr, nColliders,
-                                                                    nWorlds > 1 ? newWorldMask.p : nullptr);
+                                                                    nWorlds > 1 ? newWorldMask.p : nullptr,
+                                                                    WarmTable{});
                 CK(cudaGetLastError());
                 launches++;
             }
@@ -2917,11 +3039,8 @@ struct ag2d_world {
             swap_bufs(color, prevColor);   // this step's colours: next step's hints
             newWorldsPending = false;
             manSegFresh = nWorlds > 1;
-            CK(cudaMemcpyAsync(nPrev.p, nManifolds.p, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
             if (nWorlds > 1) {   // the solve's world starts describe the list that is now the warm-start list
-                prevSeg.reserve(nWorlds + 1);
-                CK(cudaMemcpyAsync(prevSeg.p, manSeg.p, (size_t(nWorlds) + 1) * sizeof(uint32_t),
-                                   cudaMemcpyDeviceToDevice, s));
+                swap_bufs(prevSeg, manSeg);
                 prevSegValid = true;
             }
             lastManifolds = hCounters->manifolds;

@@ -49,6 +49,48 @@ __device__ __forceinline__ void write_slot(const Contact& ct, uint32_t a, uint32
     *slot = m;
 }
 
+// The warm start of new manifold 'm' (index o of the step's list): its pair's impulses and colour of the last step. True
+// when it took an impulse.
+__device__ __forceinline__ bool warm_take(const WarmTable& t, Manifold& m, uint32_t o)
+{
+    const unsigned long long key = pair_key(m.a, m.b);
+    const WarmRegion r = warm_region(t, m.a);
+    uint32_t idx = NO_COLOR;
+    if (r.size) {
+        uint32_t s = r.home(key);
+        for (uint32_t probes = 0; probes < r.size; probes++) {
+            const unsigned long long k = t.keys[s];
+            if (k == key) { idx = t.vals[s]; break; }
+            if (k == ~0ull) break;
+            s = r.next(s);
+        }
+    }
+    if (t.hint) t.hint[o] = (idx != NO_COLOR && t.prevColor) ? t.prevColor[idx & ~WARM_CACHED] : NO_COLOR;
+    if (idx == NO_COLOR || !(idx & WARM_CACHED)) return false;
+    const Manifold p = t.prev[idx & ~WARM_CACHED];
+    if (p.a != m.a || p.b != m.b) return false;
+    bool any = false;
+    for (uint32_t k = 0; k < m.count; k++) {
+        const uint32_t id = k == 0 ? m.id0 : m.id1;
+        float jn, jt;
+        if (p.count > 0 && id == p.id0) { jn = p.jn0; jt = p.jt0; }
+        else if (p.count > 1 && id == p.id1) { jn = p.jn1; jt = p.jt1; }
+        else continue;
+        if (k == 0) { m.jn0 = jn; m.jt0 = jt; } else { m.jn1 = jn; m.jt1 = jt; }
+        any = true;
+    }
+    return any;
+}
+
+// Marks the islands of a manifold's sleeping bodies to wake. Island ids are body indices (the island's root);
+// anything else is ignored rather than written.
+__device__ __forceinline__ void mark_wakes(const DeviceWorld& w, const Manifold& m, uint32_t* wakeIsland)
+{
+    const uint32_t bA = w.cbody[m.a], bB = w.cbody[m.b];
+    if (w.bstate[bA] == STATE_SLEEPING && w.sleepIsland[bA] < w.nBodies) wakeIsland[w.sleepIsland[bA]] = 1u;
+    if (w.bstate[bB] == STATE_SLEEPING && w.sleepIsland[bB] < w.nBodies) wakeIsland[w.sleepIsland[bB]] = 1u;
+}
+
 // Narrow phase with the manifold compaction fused in. Blocks take tiles of consecutive pairs in ticket order (tileState
 // and the ticket counter zeroed before the launch); in a tile each warp takes perWarp pairs (at most 32), one per
 // lane. Pairs of other shape types run one per lane; the warp's polygon-polygon pairs search their axes four at a time,
@@ -62,7 +104,8 @@ __device__ __forceinline__ void write_slot(const Contact& ct, uint32_t a, uint32
 __global__ void k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairs,
                          uint32_t pairCap, Manifold* __restrict__ out, uint32_t manifoldCap,
                          uint32_t* __restrict__ nOut, StepCounters* counters, uint32_t* __restrict__ tileState,
-                         uint32_t* __restrict__ tileCounter, uint32_t perWarp)
+                         uint32_t* __restrict__ tileCounter, uint32_t perWarp, WarmTable warm,
+                         uint32_t* __restrict__ wakeIsland)
 {
     extern __shared__ __align__(16) unsigned char narrowSmem[];
     // [blockDim] manifold slots, [blockDim] hit flags, then per group A's vertices and B's (in A's frame).
@@ -176,106 +219,17 @@ __global__ void k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const u
         __syncthreads();
         if (h) {
             const uint32_t o = tileBase + warpBase[warp] + __popc(hits & ((1u << lane) - 1u));
-            if (o < manifoldCap) out[o] = slot[threadIdx.x];
+            if (o < manifoldCap) {
+                if (warm.keys && warm_take(warm, slot[threadIdx.x], o)) atomicAdd(&counters->warmHits, 1u);
+                if (wakeIsland) mark_wakes(w, slot[threadIdx.x], wakeIsland);
+                out[o] = slot[threadIdx.x];
+            }
         }
         __syncthreads();   // tileSlot, tileBase, warpBase, the slots and the vertex tiles are reused by the next tile
     }
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// Warm start: the previous step's manifolds go into an open-addressing table keyed by the unordered collider pair,
-// those with a non-zero impulse on an active contact flagged (bit 31 of the value: the reference caches only these,
-// rebuildContactCache, NarrowPhaseCollisionDetector.cpp:272-297; makePairKey .h:216-219); each new manifold of the
-// same ordered pair takes the flagged manifold's impulses of the contacts with equal ids (finalizeResults,
-// :749-766). Every new manifold whose pair was there also takes that manifold's colour as its colouring hint.
-// ---------------------------------------------------------------------------------------------------------------
-
-// The table: one open-addressing region per world of a batch, [2 seg[w], 2 seg[w + 1]) for the world's
-// seg[w + 1] - seg[w] previous manifolds (seg: the previous list's world starts), so a warm-start probe stays in its
-// world's few kilobytes and hits in cache; a single world (seg null) uses the whole power-of-two table. Which
-// region holds a pair changes nothing but where it is found.
-struct WarmRegion {
-    uint32_t base, size;   // size 0: the world had no manifolds
-    __device__ __forceinline__ uint32_t home(unsigned long long key) const
-    {
-        return base + uint32_t(((key * 0x9E3779B97F4A7C15ull) >> 32) % size);
-    }
-    __device__ __forceinline__ uint32_t next(uint32_t s) const { return s + 1 == base + size ? base : s + 1; }
-};
-__device__ __forceinline__ WarmRegion warm_region(const uint32_t* seg, const uint32_t* colWorld, uint32_t a,
-                                                  uint32_t capacity)
-{
-    if (!seg) return WarmRegion{0u, capacity};
-    const uint32_t wd = colWorld[a];
-    const uint32_t lo = seg[wd], hi = seg[wd + 1];
-    if (hi < lo || 2ull * hi > capacity) return WarmRegion{0u, 0u};   // not a valid segmentation: no region
-    return WarmRegion{2u * lo, 2u * (hi - lo)};
-}
-
-__global__ void k_warm_insert(const Manifold* __restrict__ prev, const uint32_t* __restrict__ nPrev,
-                              unsigned long long* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t capacity,
-                              const uint32_t* __restrict__ seg, const uint32_t* __restrict__ colWorld,
-                              uint32_t* __restrict__ status)
-{
-    const uint32_t n = *nPrev;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const Manifold m = prev[i];
-        uint32_t mask = uint32_t(m.jn0 != 0.0f) | uint32_t(m.jt0 != 0.0f) << 1 | uint32_t(m.jn1 != 0.0f) << 2 |
-                        uint32_t(m.jt1 != 0.0f) << 3;
-        mask &= (1u << (2u * m.count)) - 1u;
-        const unsigned long long key = pair_key(m.a, m.b);
-        const WarmRegion r = warm_region(seg, colWorld, m.a, capacity);
-        if (r.size == 0) { atomicOr(status, STATUS_HASH_FULL); continue; }   // cannot happen: m is in its world
-        uint32_t s = r.home(key);
-        uint32_t probes = 0;
-        for (;;) {
-            const unsigned long long old = atomicCAS(keys + s, ~0ull, key);
-            if (old == ~0ull || old == key) { vals[s] = i | (mask ? WARM_CACHED : 0u); break; }
-            s = r.next(s);
-            if (++probes >= r.size) { atomicOr(status, STATUS_HASH_FULL); break; }
-        }
-    }
-}
-
-__global__ void k_warm_lookup(const Manifold* __restrict__ prev, Manifold* __restrict__ cur,
-                              const uint32_t* __restrict__ nCur, const unsigned long long* __restrict__ keys,
-                              const uint32_t* __restrict__ vals, uint32_t capacity, const uint32_t* __restrict__ seg,
-                              const uint32_t* __restrict__ colWorld, StepCounters* counters,
-                              const uint32_t* __restrict__ prevColor, uint32_t* __restrict__ hint)
-{
-    const uint32_t n = *nCur;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        Manifold& c = cur[i];
-        const unsigned long long key = pair_key(c.a, c.b);
-        const WarmRegion r = warm_region(seg, colWorld, c.a, capacity);
-        uint32_t idx = NO_COLOR;
-        if (r.size) {
-            uint32_t s = r.home(key);
-            for (uint32_t probes = 0; probes < r.size; probes++) {
-                const unsigned long long k = keys[s];
-                if (k == key) { idx = vals[s]; break; }
-                if (k == ~0ull) break;
-                s = r.next(s);
-            }
-        }
-        if (hint) hint[i] = (idx != NO_COLOR && prevColor) ? prevColor[idx & ~WARM_CACHED] : NO_COLOR;
-        if (idx == NO_COLOR || !(idx & WARM_CACHED)) continue;
-        idx &= ~WARM_CACHED;
-        const Manifold p = prev[idx];
-        if (p.a != c.a || p.b != c.b) continue;
-        bool any = false;
-        for (uint32_t k = 0; k < c.count; k++) {
-            const uint32_t id = k == 0 ? c.id0 : c.id1;
-            float jn, jt;
-            if (p.count > 0 && id == p.id0) { jn = p.jn0; jt = p.jt0; }
-            else if (p.count > 1 && id == p.id1) { jn = p.jn1; jt = p.jt1; }
-            else continue;
-            if (k == 0) { c.jn0 = jn; c.jt0 = jt; } else { c.jn1 = jn; c.jt1 = jt; }
-            any = true;
-        }
-        if (any) atomicAdd(&counters->warmHits, 1u);
-    }
-}
+__global__ void k_warm_insert(WarmTable t) { warm_insert(t); }
 
 // ---------------------------------------------------------------------------------------------------------------
 // Wake: every sleeping body in a manifold wakes its whole island (ObjectManager::wakeIslandsOfContacts,
@@ -285,12 +239,8 @@ __global__ void k_wake(DeviceWorld w, const Manifold* __restrict__ m, const uint
                        uint32_t* __restrict__ wakeIsland, StepCounters* counters)
 {
     const uint32_t n = *nM;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t bA = w.cbody[m[i].a], bB = w.cbody[m[i].b];
-        // Island ids are body indices (the island's root); anything else is ignored rather than written.
-        if (w.bstate[bA] == STATE_SLEEPING && w.sleepIsland[bA] < w.nBodies) wakeIsland[w.sleepIsland[bA]] = 1u;
-        if (w.bstate[bB] == STATE_SLEEPING && w.sleepIsland[bB] < w.nBodies) wakeIsland[w.sleepIsland[bB]] = 1u;
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        mark_wakes(w, m[i], wakeIsland);
 }
 
 __global__ void k_wake_apply(DeviceWorld w, const uint32_t* __restrict__ wakeIsland, StepCounters* counters)
@@ -608,7 +558,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_color_solve_block(BlockSolve a)
                                                                      threadIdx.x, THREADS, BlockSync{},
                                                                      &a.counters->colors, &a.counters->status);
         __syncthreads();
-        if (!solved) return;   // the step is redone or fails: the bodies stay as they were
+        if (!solved) {   // the step is redone or fails: the bodies stay as they were, every one its own island
+            for (uint32_t i = threadIdx.x; i < nb; i += THREADS) {
+                a.ufParent[i] = i;
+                a.ufFlag[i] = 1u;
+            }
+            return;
+        }
         for (uint32_t i = threadIdx.x; i < nb; i += THREADS) {
             w.bvel[i] = vel[i];
             w.bpos[i] = pos[i];
@@ -873,8 +829,29 @@ __global__ void k_island_quiet(DeviceWorld w, uint32_t* __restrict__ parent, uin
     }
 }
 
+// Last thing of a step: see StepEnd. Called by every thread of the launch's blocks, after their own work.
+__device__ __forceinline__ void step_end(const StepEnd& e, StepCounters* counters)
+{
+    if (!e.host) return;
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(e.done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    constexpr uint32_t WORDS = sizeof(StepCounters) / sizeof(uint32_t);
+    if (threadIdx.x < WORDS)
+        reinterpret_cast<volatile uint32_t*>(e.host)[threadIdx.x] =
+            __ldcg(reinterpret_cast<const uint32_t*>(counters) + threadIdx.x);
+    if (threadIdx.x == 0 && __ldcg(&counters->status) == 0u) *e.nPrev = __ldcg(e.nManifolds);
+    __threadfence_system();
+}
+
 __global__ void k_island_sleep(DeviceWorld w, uint32_t* __restrict__ parent, const uint32_t* __restrict__ flag,
-                               StepCounters* counters)
+                               StepCounters* counters, StepEnd end)
 {
     uint32_t slept = 0;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nBodies; b += gridDim.x * blockDim.x) {
@@ -893,16 +870,22 @@ __global__ void k_island_sleep(DeviceWorld w, uint32_t* __restrict__ parent, con
         atomicAdd(&counters->slept, slept);
         counters->topoDirty = 1u;
     }
+    step_end(end, counters);
 }
 
 // Work-list flags from body states: dynamic bodies, dynamic colliders, static + sleeping colliders.
 __global__ void k_state_flags(const uint8_t* __restrict__ bstate, const uint32_t* __restrict__ cbody,
                               uint32_t nBodies, uint32_t nColliders, uint32_t* __restrict__ bodyDyn,
-                              uint32_t* __restrict__ colDyn, uint32_t* __restrict__ colOther)
+                              uint32_t* __restrict__ colDyn, uint32_t* __restrict__ colOther,
+                              uint32_t* __restrict__ sleeping)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nBodies; b += stride)
+    bool any = false;
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nBodies; b += stride) {
         bodyDyn[b] = bstate[b] == STATE_DYNAMIC;
+        any |= bstate[b] == STATE_SLEEPING;
+    }
+    if (any) *sleeping = 1u;
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nColliders; c += stride) {
         const uint8_t st = bstate[cbody[c]];
         colDyn[c] = st == STATE_DYNAMIC;

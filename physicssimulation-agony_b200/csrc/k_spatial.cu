@@ -16,50 +16,109 @@ namespace ag2d {
 // phase: 3 both halves; 1 the first (half kick and damping: Integrator::integratePhase1_VelocityVerlet +
 // dampAngularVelocities); 2 the second (position step, half kick, damping, wrap, cos/sin). The body constraints
 // run between the two (Simulation.cpp:399-404).
+__device__ __forceinline__ void integrate_kick(float4& v, const float4& p, bool simd, float gdx, float gdy,
+                                               float dampHalf /* damping^(dt/2), or >= 1 when damping is off */)
+{
+    const bool movable = v.w != 0.0f;
+    const bool angMovable = p.w != 0.0f;
+    if (simd) { v.x += movable ? gdx : 0.0f; v.y += movable ? gdy : 0.0f; }
+    else { v.x += gdx * float(movable); v.y += gdy * float(movable); }
+    if (dampHalf < 1.0f) {
+        const float nv = v.z * dampHalf;
+        if (simd) v.z = angMovable ? nv : v.z;
+        else { const float m = float(angMovable); v.z = m * nv + (1.0f - m) * v.z; }
+    }
+}
+
+// The second half; wrap holds the body's wrap count in and out.
+__device__ __forceinline__ void integrate_move(const DeviceWorld& w, uint32_t b, float4 v, float4 p, float wrap, bool simd,
+                                               const IntegrateParams& ip)
+{
+    p.x = v.x * ip.dt + p.x;
+    p.y = v.y * ip.dt + p.y;
+    p.z = v.z * ip.dt + p.z;
+    const float halfDT = ip.dt * 0.5f;
+    integrate_kick(v, p, simd, ip.gx * halfDT, ip.gy * halfDT, ip.dampHalf);
+    float wraps;
+    p.z = wrap_angle(p.z, simd, wraps);
+    w.wrapCount[b] = wrap + wraps;
+    float c, s;
+    fast_cos_sin(p.z, simd, c, s);
+    w.bvel[b] = v;
+    w.bpos[b] = p;
+    w.brot[b] = make_float2(c, s);
+}
+
 __global__ void k_integrate(DeviceWorld w, const uint32_t* __restrict__ dynBody, const uint8_t* __restrict__ dynSimd,
-                            uint32_t nDyn, float dt, float gx, float gy,
-                            float dampHalf /* damping^(dt/2), or >= 1 when damping is off */, uint32_t phase)
+                            uint32_t nDyn, IntegrateParams ip, uint32_t phase)
 {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nDyn; k += gridDim.x * blockDim.x) {
         const uint32_t b = dynBody[k];
         const bool simd = dynSimd ? dynSimd[k] != 0 : k < (nDyn & ~7u);
         float4 v = w.bvel[b];
-        float4 p = w.bpos[b];
-        const float halfDT = dt * 0.5f;
-        const float gdx = gx * halfDT, gdy = gy * halfDT;
-        const bool movable = v.w != 0.0f;
-        const bool angMovable = p.w != 0.0f;
-        if (phase & 1u) {
-            if (simd) { v.x += movable ? gdx : 0.0f; v.y += movable ? gdy : 0.0f; }
-            else { v.x += gdx * float(movable); v.y += gdy * float(movable); }
-            if (dampHalf < 1.0f) {
-                const float nv = v.z * dampHalf;
-                if (simd) v.z = angMovable ? nv : v.z;
-                else { const float m = float(angMovable); v.z = m * nv + (1.0f - m) * v.z; }
-            }
-            if (!(phase & 2u)) {
-                w.bvel[b] = v;
-                continue;
-            }
+        const float4 p = w.bpos[b];
+        const float halfDT = ip.dt * 0.5f;
+        if (phase & 1u) integrate_kick(v, p, simd, ip.gx * halfDT, ip.gy * halfDT, ip.dampHalf);
+        if (phase & 2u) integrate_move(w, b, v, p, w.wrapCount[b], simd, ip);
+        else w.bvel[b] = v;
+    }
+}
+
+// The start of a step in one launch: the body state saved (a step that overflows a buffer is redone from it), wrap
+// counts cleared, the integration (both halves, or the first when body constraints follow), the step's counters reset
+// and every buffer that the step's kernels expect cleared. As separate copies, clears and kernels these were twenty
+// operations of two to three microseconds each, most of a small world's step; by bytes it is one pass over the bodies.
+__global__ void k_step_begin(StepBegin a)
+{
+    const DeviceWorld& w = a.w;
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (first == 0) {
+        StepCounters c = {};
+        c.stored = *a.nIsle;
+        *a.counters = c;
+    }
+    // Bodies that are not dynamic (the dynamic ones are the list's, below).
+    for (uint32_t b = first; b < w.nBodies; b += stride) {
+        const uint8_t st = w.bstate[b];
+        a.snapState[b] = st;
+        a.snapTimer[b] = w.sleepTimer[b];
+        a.snapIsland[b] = w.sleepIsland[b];
+        if (st == STATE_DYNAMIC) continue;
+        a.snapVel[b] = w.bvel[b];
+        a.snapPos[b] = w.bpos[b];
+        a.snapRot[b] = w.brot[b];
+        a.snapWrap[b] = w.wrapCount[b];
+        w.wrapCount[b] = 0.0f;
+    }
+    const float halfDT = a.ip.dt * 0.5f;
+    for (uint32_t k = first; k < a.nDyn; k += stride) {
+        const uint32_t b = a.dynBody[k];
+        const bool simd = a.dynSimd ? a.dynSimd[k] != 0 : k < (a.nDyn & ~7u);
+        float4 v = w.bvel[b];
+        const float4 p = w.bpos[b];
+        a.snapVel[b] = v;
+        a.snapPos[b] = p;
+        a.snapRot[b] = w.brot[b];
+        a.snapWrap[b] = w.wrapCount[b];
+        integrate_kick(v, p, simd, a.ip.gx * halfDT, a.ip.gy * halfDT, a.ip.dampHalf);
+        if (a.both) {
+            integrate_move(w, b, v, p, 0.0f, simd, a.ip);
+        } else {
+            w.bvel[b] = v;
+            w.wrapCount[b] = 0.0f;
         }
-        p.x = v.x * dt + p.x;
-        p.y = v.y * dt + p.y;
-        p.z = v.z * dt + p.z;
-        if (simd) { v.x += movable ? gdx : 0.0f; v.y += movable ? gdy : 0.0f; }
-        else { v.x += gdx * float(movable); v.y += gdy * float(movable); }
-        if (dampHalf < 1.0f) {
-            const float nv = v.z * dampHalf;
-            if (simd) v.z = angMovable ? nv : v.z;
-            else { const float m = float(angMovable); v.z = m * nv + (1.0f - m) * v.z; }
+    }
+    for (uint32_t i = first; i < a.copyCount; i += stride) a.copyDst[i] = a.copySrc[i];
+    for (uint32_t f = 0; f < a.fills; f++) {
+        const FillRegion r = a.fill[f];
+        if (r.iota) {
+            for (uint32_t i = first; i < r.words; i += stride) r.p[i] = i;
+            continue;
         }
-        float wraps;
-        p.z = wrap_angle(p.z, simd, wraps);
-        w.wrapCount[b] = w.wrapCount[b] + wraps;
-        float c, s;
-        fast_cos_sin(p.z, simd, c, s);
-        w.bvel[b] = v;
-        w.bpos[b] = p;
-        w.brot[b] = make_float2(c, s);
+        const uint32_t quads = r.words / 4;
+        uint4* const q = reinterpret_cast<uint4*>(r.p);
+        for (uint32_t i = first; i < quads; i += stride) q[i] = make_uint4(r.value, r.value, r.value, r.value);
+        if (first < r.words - 4 * quads) r.p[4 * quads + first] = r.value;
     }
 }
 
@@ -107,9 +166,12 @@ __device__ __forceinline__ float4 collider_aabb(const DeviceWorld& w, uint32_t c
     }
 }
 
+// insert: the warm-start table filled beside the poses (one launch for two passes that touch nothing in common), or a
+// table without keys.
 __global__ void k_collider_pose(DeviceWorld w, const uint32_t* __restrict__ list, const uint8_t* __restrict__ listSimd,
-                                uint32_t n, const uint32_t* __restrict__ worldMask)
+                                uint32_t n, const uint32_t* __restrict__ worldMask, WarmTable insert)
 {
+    if (insert.keys) warm_insert(insert);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const uint32_t c = list ? list[k] : k;
         if (worldMask && !worldMask[w.colWorld[c]]) continue;
