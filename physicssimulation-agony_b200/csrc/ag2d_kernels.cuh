@@ -311,12 +311,23 @@ __global__ void k_isle_add_count(uint32_t* nIsle, const uint32_t* nMove);
 __global__ void k_isle_list_scatter(const Manifold* m, const uint32_t* color, const uint32_t* nM,
                                     const uint32_t* stay, const uint32_t* stayOff, Manifold* out,
                                     uint32_t* colorOut);
-__global__ void k_query_shape(const float4* caabb, const uint32_t* cbody, const uint8_t* bstate, uint32_t n,
-                              uint32_t shape, float4 q, uint32_t trees, uint32_t* flag);
-__global__ void k_circle_contacts(DeviceWorld w, float x, float y, float radius, uint32_t trees, uint32_t* flag,
-                                  float* dist);
-__global__ void k_scatter_contacts(const uint32_t* flag, const uint32_t* offset, const float* dist, uint32_t n,
-                                   uint32_t* list, float* listDist);
+// Spatial queries: kind, the box (min x, min y, max x, max y) or circle (x, y, radius), tree selection; tileState
+// [tiles + 1] (tiles of QUERY_SELECT_THREADS colliders, then the ticket counter) clear, nextState cleared for the next
+// query; results to list / dist and the first hostCap of them to page-locked host: {count, timeout, indices, distances}.
+constexpr uint32_t QUERY_SELECT_THREADS = 256;
+enum QuerySelectKind : uint32_t { QUERY_SELECT_AABB = 0, QUERY_SELECT_CIRCLE = 1, QUERY_SELECT_CONTACTS = 2 };
+struct QuerySelect {
+    uint32_t kind, trees;
+    float4 shape;
+    uint32_t* tileState;
+    uint32_t* nextState;
+    uint32_t* list;
+    float* dist;
+    uint32_t* host;
+    uint32_t hostCap;
+    uint32_t* status;
+};
+__global__ void k_query_select(DeviceWorld w, QuerySelect q);
 
 // Body constraints (k_joints.cu): springs (kind 0), revolute (1), prismatic (2) and slider (3) joints and motors
 // (4), the reference's ConstraintType order, each kind's active
@@ -367,6 +378,16 @@ __global__ void k_fill_u32(uint32_t* out, uint32_t n, uint32_t value);
 enum ExtractKind : uint32_t {
     EXTRACT_DIRECT = 0, EXTRACT_F4_COMP, EXTRACT_F4_XYZ, EXTRACT_F2_COMP, EXTRACT_U8_U32, EXTRACT_ISLAND
 };
+struct SectionCopy {
+    uint8_t* dst;
+    const uint8_t* src;
+    uint64_t bytes;
+};
+struct SectionCopies {
+    uint32_t count;
+    SectionCopy c[32];
+};
+__global__ void k_copy_sections(SectionCopies a);
 __global__ void k_extract(const void* src, uint32_t lo, uint32_t n, uint32_t kind, uint32_t comp, uint32_t bias,
                           void* out);
 

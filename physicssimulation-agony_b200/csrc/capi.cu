@@ -426,6 +426,35 @@ static float reference_angle(float rotA, float rotB)
     return a;
 }
 
+// Host memory the device can copy into directly: page-locked by cudaHostAlloc or cudaHostRegister (any CUDA runtime
+// of the process; the driver tracks it).
+static bool page_locked(const void* p)
+{
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+}
+// Where kernels reach page-locked host memory that is aligned to 'align' bytes; null for any other memory.
+static void* kernel_reach(const void* p, size_t align)
+{
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    if (a.type != cudaMemoryTypeHost || reinterpret_cast<uintptr_t>(a.devicePointer) % align) return nullptr;
+    return a.devicePointer;
+}
+
+// Transfers up to this size go between page-locked host memory and the device inside a kernel (packed reads, small
+// checkpoints): a copy operation adds about eight microseconds to a kernel that is there anyway, and above it the copy
+// engine's bandwidth counts.
+constexpr uint64_t HOST_DIRECT_BYTES = 256 << 10;
+
+
 // A deferred body command (ObjectManager::ObjectCommand, SimulationImpl/ObjectManager.h:45): queued by destroy and the
 // setters in call order, applied at the start of the next step (Simulation::update -> flushCommands,
 // Simulation.cpp:39; ObjectManager::applyCommand, ObjectManager.cpp:662-790). Stale handles are dropped.
@@ -615,6 +644,7 @@ struct ag2d_world {
     // of the previous one) into pageable memory.
     DBuf<uint8_t> readStage;
     PinnedBuf readBounce;
+    PinnedBuf hostWord;   // element counts on their way to the host
     cudaEvent_t readEv[2] = {nullptr, nullptr};
     // Asynchronous reads: a ring of device staging buffers; each read packs on the engine stream and copies on
     // copyStream, so the copy overlaps the steps launched after it.
@@ -627,8 +657,13 @@ struct ag2d_world {
     AsyncSlot asyncSlot[NASYNC];
     uint32_t asyncNext = 0;
     cudaStream_t copyStream = nullptr;
-    DBuf<uint32_t> queryFlag, queryOffset, queryList, queryCount;   // spatial query scratch
-    DBuf<float> queryDist, queryListDist;
+    // Spatial queries: tile states (one query clears the other's), results on the device and the first of them in
+    // page-locked memory.
+    static constexpr uint32_t QUERY_HOST = 4096;
+    DBuf<uint32_t> selectState[2], queryList, queryStatus;
+    DBuf<float> queryListDist;
+    PinnedBuf queryHost;
+    uint32_t selectTurn = 0, selectTiles = 0;
     DBuf<GatherSeg> gatherSegs;
     bool newWorldsPending = false;   // joined worlds take a full pose pass in their first step
     // Shape table sizes of the last upload.
@@ -1172,9 +1207,19 @@ struct ag2d_world {
         nBodies = h.nBodies; nColliders = h.nColliders; nCircles = h.nCircles; nBoxes = h.nBoxes;
         nPolygons = h.nPolygons; nPolyVerts = h.nPolyVerts; nMaterialRows = h.nMaterialRows; nStatic = h.nStatic;
         nWorlds = std::max<uint32_t>(h.nWorlds, 1);
+        // A small page-locked checkpoint goes over in one kernel that reads the sections where they lie, a large or
+        // pageable one in a copy a section.
+        const void* const mapped = h.totalBytes <= 4 * HOST_DIRECT_BYTES ? kernel_reach(src, 16) : nullptr;
+        SectionCopies sections{};
+        auto put = [&](void* dst, uint32_t k) {
+            if (!h.len[k]) return;
+            if (!mapped) CK(cudaMemcpyAsync(dst, src + h.off[k], h.len[k], cudaMemcpyHostToDevice, s));
+            else sections.c[sections.count++] = SectionCopy{static_cast<uint8_t*>(dst),
+                                                            static_cast<const uint8_t*>(mapped) + h.off[k], h.len[k]};
+        };
         auto up = [&](auto& buf, uint32_t k, size_t count) {
             buf.reserve(std::max<size_t>(count, 1));
-            if (h.len[k]) CK(cudaMemcpyAsync(buf.p, src + h.off[k], h.len[k], cudaMemcpyHostToDevice, s));
+            put(buf.p, k);
         };
         up(bvel, CK_VEL, nBodies); up(bpos, CK_POS, nBodies); up(brot, CK_ROT, nBodies);
         up(wrapCount, CK_WRAP, nBodies); up(boundRadius, CK_BOUND, nBodies); up(sleepTimer, CK_TIMER, nBodies);
@@ -1203,10 +1248,8 @@ struct ag2d_world {
         }
         sizeFor(known);
         if (h.nPrev > manifoldCap) reserveCapacities(std::max(h.nPrev, pairCap), h.nPrev);
-        if (h.len[CK_PREV])
-            CK(cudaMemcpyAsync(prevManifolds.p, src + h.off[CK_PREV], h.len[CK_PREV], cudaMemcpyHostToDevice, s));
-        if (h.len[CK_PREVCOLOR])
-            CK(cudaMemcpyAsync(prevColor.p, src + h.off[CK_PREVCOLOR], h.len[CK_PREVCOLOR], cudaMemcpyHostToDevice, s));
+        put(prevManifolds.p, CK_PREV);
+        put(prevColor.p, CK_PREVCOLOR);
         prevCount = h.nPrev;
         prevSegValid = false;
         CK(cudaMemcpyAsync(nPrev.p, &prevCount, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
@@ -1220,6 +1263,10 @@ struct ag2d_world {
         }
         up(isle, CK_ISLE, h.nIsle);
         up(isleId, CK_ISLEID, h.nIsle);
+        if (sections.count) {
+            k_copy_sections<<<gridFor(h.totalBytes / 16), 256, 0, s>>>(sections);
+            CK(cudaGetLastError());
+        }
         isleUpper = h.nIsle;
         CK(cudaMemcpyAsync(nIsle.p, &isleUpper, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
         const uint32_t ones = std::max<uint32_t>(nBodies, 1);
@@ -3834,19 +3881,6 @@ int32_t ag2d_world_body_count(ag2d_world* world, uint32_t* out_bodies, uint32_t*
 }  // extern "C"
 
 // Field access ---------------------------------------------------------------------------------------------------
-
-// Host memory the device can copy into directly: page-locked by cudaHostAlloc or cudaHostRegister (any CUDA runtime
-// of the process; the driver tracks it).
-static bool page_locked(const void* p)
-{
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeHost;
-}
-
 // How a per-body or per-collider field is read: its device array and how k_extract packs it.
 struct FieldSpec {
     const void* src = nullptr;
@@ -3930,6 +3964,13 @@ static uint64_t read_packed(ag2d_world& w, const FieldSpec& f, uint32_t lo, uint
     const uint64_t bytes = uint64_t(n) * f.outBytes;
     if (!bytes) return 0;
     const void* src = static_cast<const uint8_t*>(f.src) + size_t(lo) * f.outBytes;
+    void* const mapped = f.kind != EXTRACT_DIRECT && bytes <= HOST_DIRECT_BYTES ? kernel_reach(dst, 4) : nullptr;
+    if (mapped) {
+        k_extract<<<w.gridFor(n), 256, 0, w.stream>>>(f.src, lo, n, f.kind, f.comp, bias, mapped);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(w.stream));
+        return bytes;
+    }
     if (f.kind != EXTRACT_DIRECT) {
         w.readStage.reserve(bytes);
         k_extract<<<w.gridFor(n), 256, 0, w.stream>>>(f.src, lo, n, f.kind, f.comp, bias, w.readStage.p);
@@ -3972,40 +4013,93 @@ static void read_async(ag2d_world& w, const FieldSpec& f, uint32_t lo, uint32_t 
 }
 
 
-// The phase-tap fields (Morton order, pairs, manifolds, solve order, colour starts): element count from the device
-// counters where the count lives there. With sizeOnly the bytes are counted but not read.
-static std::vector<uint8_t> read_field(ag2d_world& w, int32_t field, bool sizeOnly, uint64_t* bytesOut)
+// The phase-tap fields (Morton order, pairs, manifolds, solve order, colour starts) as they lie on the device: the
+// element count comes from the device counters where the count lives there.
+struct TapField {
+    const void* src;
+    uint64_t bytes;
+};
+static TapField tap_field(ag2d_world& w, int32_t field)
 {
-    const cudaStream_t s = w.stream;
-    auto pack = [](const auto& v) {
-        std::vector<uint8_t> out(v.size() * sizeof(v[0]));
-        if (!v.empty()) std::memcpy(out.data(), v.data(), out.size());
-        return out;
-    };
     auto devCount = [&](const uint32_t* p) {
-        uint32_t n = 0;
-        CK(cudaMemcpyAsync(&n, p, 4, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        return n;
+        w.hostWord.reserve(sizeof(uint32_t));
+        CK(cudaMemcpyAsync(w.hostWord.p, p, 4, cudaMemcpyDeviceToHost, w.stream));
+        CK(cudaStreamSynchronize(w.stream));
+        return *reinterpret_cast<const uint32_t*>(w.hostWord.p);
     };
-    auto get = [&](const auto* p, size_t n) {
-        *bytesOut = n * sizeof(*p);
-        using T = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
-        return sizeOnly ? std::vector<uint8_t>() : pack(download(static_cast<const T*>(p), n, s));
-    };
+    auto tap = [&](const auto* p, size_t n) { return TapField{p, n * sizeof(*p)}; };
     switch (field) {
-    case AG2D_DYN_SORTED: return get(w.dynTree.vals.p, uint32_t(w.dynTree.n));
+    case AG2D_DYN_SORTED: return tap(w.dynTree.vals.p, uint32_t(w.dynTree.n));
     case AG2D_DYN_MORTON:
-        return get(w.nWorlds > 1 ? w.dynTree.sortedKey.p : w.dynTree.keys.p, uint32_t(w.dynTree.n));
-    case AG2D_PAIRS: return get(w.pairs.p, std::min(devCount(&w.dCounters.p->pairs), w.pairCap));
-    case AG2D_MANIFOLDS: return get(w.manifolds.p, devCount(w.nManifolds.p));
-    case AG2D_PREV_MANIFOLDS: w.compactPrev(); return get(w.prevManifolds.p, devCount(w.nPrev.p));
-    case AG2D_SOLVE_ORDER: return get(w.order.p, devCount(w.nManifolds.p));
-    case AG2D_COLOR_STARTS: return get(w.colorStart.p, devCount(&w.dCounters.p->colors) + 1);
-    case AG2D_ISLAND_MANIFOLDS: return get(w.isle.p, devCount(w.nIsle.p));
-    case AG2D_ISLAND_IDS: return get(w.isleId.p, devCount(w.nIsle.p));
+        return tap(w.nWorlds > 1 ? w.dynTree.sortedKey.p : w.dynTree.keys.p, uint32_t(w.dynTree.n));
+    case AG2D_PAIRS: return tap(w.pairs.p, std::min(devCount(&w.dCounters.p->pairs), w.pairCap));
+    case AG2D_MANIFOLDS: return tap(w.manifolds.p, devCount(w.nManifolds.p));
+    case AG2D_PREV_MANIFOLDS: w.compactPrev(); return tap(w.prevManifolds.p, devCount(w.nPrev.p));
+    case AG2D_SOLVE_ORDER: return tap(w.order.p, devCount(w.nManifolds.p));
+    case AG2D_COLOR_STARTS: return tap(w.colorStart.p, devCount(&w.dCounters.p->colors) + 1);
+    case AG2D_ISLAND_MANIFOLDS: return tap(w.isle.p, devCount(w.nIsle.p));
+    case AG2D_ISLAND_IDS: return tap(w.isleId.p, devCount(w.nIsle.p));
     default: throw ApiError(AG2D_ERR_INVALID_ARG, "unknown field " + std::to_string(field));
     }
+}
+static std::vector<uint8_t> read_field(ag2d_world& w, int32_t field)
+{
+    const TapField t = tap_field(w, field);
+    std::vector<uint8_t> out(t.bytes);
+    copy_to_host(w, out.data(), t.src, t.bytes);
+    return out;
+}
+
+// One spatial query (k_query_select); up to 'capacity' results into out / dist. Returns the number found.
+static uint32_t query_select(ag2d_world& w, uint32_t kind, float4 shape, uint32_t trees, uint32_t* out, float* dist,
+                             uint32_t capacity, uint32_t* outCount)
+{
+    CK(cudaSetDevice(w.settings.device));
+    w.ensureUploaded();
+    *outCount = 0;
+    const uint32_t n = w.nColliders;
+    if (n == 0 || !w.aabbValid || (trees & AG2D_TREE_ALL) == 0) return 0;
+    const cudaStream_t s = w.stream;
+    const uint32_t tiles = div_up(n, QUERY_SELECT_THREADS);
+    if (tiles != w.selectTiles) {   // first query, or another number of colliders: both sets of states cleared
+        for (auto& b : w.selectState) {
+            b.reserve(size_t(tiles) + 1);
+            CK(cudaMemsetAsync(b.p, 0, (size_t(tiles) + 1) * sizeof(uint32_t), s));
+        }
+        w.selectTiles = tiles;
+    }
+    w.queryList.reserve(n);
+    if (kind == QUERY_SELECT_CONTACTS) w.queryListDist.reserve(n);
+    if (!w.queryStatus.p) {
+        w.queryStatus.reserve(1);
+        CK(cudaMemsetAsync(w.queryStatus.p, 0, sizeof(uint32_t), s));
+    }
+    w.queryHost.reserve((2 + 2 * size_t(ag2d_world::QUERY_HOST)) * sizeof(uint32_t));
+    uint32_t* const host = reinterpret_cast<uint32_t*>(w.queryHost.p);
+    const QuerySelect q{kind, trees & AG2D_TREE_ALL, shape, w.selectState[w.selectTurn].p,
+                        w.selectState[w.selectTurn ^ 1].p, w.queryList.p, w.queryListDist.p, host,
+                        ag2d_world::QUERY_HOST, w.queryStatus.p};
+    w.selectTurn ^= 1;
+    const uint32_t grid = std::min(tiles, uint32_t(std::max(w.dev.sms, 1)) * 8);
+    k_query_select<<<grid, QUERY_SELECT_THREADS, 0, s>>>(w.view(), q);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(s));
+    if (host[1]) {
+        w.selectTiles = 0;
+        CK(cudaMemsetAsync(w.queryStatus.p, 0, sizeof(uint32_t), s));
+        throw ApiError(AG2D_ERR_TIMEOUT, "a bounded device-side wait timed out");
+    }
+    const uint32_t count = host[0], m = std::min(count, capacity);
+    if (!m) return count;
+    if (count <= ag2d_world::QUERY_HOST) {
+        std::memcpy(out, host + 2, size_t(m) * sizeof(uint32_t));
+        if (dist) std::memcpy(dist, host + 2 + ag2d_world::QUERY_HOST, size_t(m) * sizeof(float));
+    } else {
+        CK(cudaMemcpyAsync(out, w.queryList.p, size_t(m) * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        if (dist) CK(cudaMemcpyAsync(dist, w.queryListDist.p, size_t(m) * sizeof(float), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+    }
+    return count;
 }
 
 extern "C" {
@@ -4018,35 +4112,11 @@ int32_t ag2d_world_query_shape(ag2d_world* world, int32_t shape, const float* pa
         if (shape != AG2D_QUERY_AABB && shape != AG2D_QUERY_CIRCLE)
             throw ApiError(AG2D_ERR_INVALID_ARG, "unknown query shape");
         if (capacity && !out_colliders) throw ApiError(AG2D_ERR_INVALID_ARG, "null output with a capacity");
-        CK(cudaSetDevice(world->settings.device));
-        ag2d_world& w = *world;
-        w.ensureUploaded();
-        *out_count = 0;
-        const uint32_t n = w.nColliders;
-        if (n == 0 || !w.aabbValid || (trees & AG2D_TREE_ALL) == 0) return;
-        const cudaStream_t s = w.stream;
-        w.queryFlag.reserve(n);
-        w.queryOffset.reserve(n);
-        w.queryList.reserve(n);
-        w.queryCount.reserve(1);
-        w.scanner.reserve(std::max({w.pairCap, w.nColliders, w.nBodies}));
-        const float4 q = shape == AG2D_QUERY_AABB ? make_float4(params[0], params[1], params[2], params[3])
-                                                   : make_float4(params[0], params[1], params[2], 0.0f);
-        k_query_shape<<<w.gridFor(n), 256, 0, s>>>(w.caabb.p, w.cbody.p, w.bstate.p, n, uint32_t(shape), q,
-                                                   trees & AG2D_TREE_ALL, w.queryFlag.p);
-        CK(cudaGetLastError());
-        w.scanner.run(w.queryFlag.p, w.queryOffset.p, n, w.queryCount.p, s);
-        k_scatter_list<<<w.gridFor(n), 256, 0, s>>>(w.queryFlag.p, w.queryOffset.p, n, w.queryList.p);
-        CK(cudaGetLastError());
-        uint32_t count = 0;
-        CK(cudaMemcpyAsync(&count, w.queryCount.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        const uint32_t m = std::min(count, capacity);
-        if (m) {
-            CK(cudaMemcpyAsync(out_colliders, w.queryList.p, size_t(m) * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-        }
-        *out_count = count;
+        const bool aabb = shape == AG2D_QUERY_AABB;
+        const float4 q = aabb ? make_float4(params[0], params[1], params[2], params[3])
+                              : make_float4(params[0], params[1], params[2], 0.0f);
+        *out_count = query_select(*world, aabb ? QUERY_SELECT_AABB : QUERY_SELECT_CIRCLE, q, trees, out_colliders, nullptr,
+                                  capacity, out_count);
     });
 }
 
@@ -4058,37 +4128,8 @@ int32_t ag2d_world_query_circle_contacts(ag2d_world* world, float x, float y, fl
         if (!world || !out_count) throw ApiError(AG2D_ERR_INVALID_ARG, "null argument");
         if (capacity && (!out_colliders || !out_distance))
             throw ApiError(AG2D_ERR_INVALID_ARG, "null output with a capacity");
-        CK(cudaSetDevice(world->settings.device));
-        ag2d_world& w = *world;
-        w.ensureUploaded();
-        *out_count = 0;
-        const uint32_t n = w.nColliders;
-        if (n == 0 || !w.aabbValid || (trees & AG2D_TREE_ALL) == 0) return;
-        const cudaStream_t s = w.stream;
-        w.queryFlag.reserve(n);
-        w.queryOffset.reserve(n);
-        w.queryList.reserve(n);
-        w.queryDist.reserve(n);
-        w.queryListDist.reserve(n);
-        w.queryCount.reserve(1);
-        w.scanner.reserve(std::max({w.pairCap, w.nColliders, w.nBodies}));
-        k_circle_contacts<<<w.gridFor(n), 256, 0, s>>>(w.view(), x, y, radius, trees & AG2D_TREE_ALL, w.queryFlag.p,
-                                                       w.queryDist.p);
-        CK(cudaGetLastError());
-        w.scanner.run(w.queryFlag.p, w.queryOffset.p, n, w.queryCount.p, s);
-        k_scatter_contacts<<<w.gridFor(n), 256, 0, s>>>(w.queryFlag.p, w.queryOffset.p, w.queryDist.p, n,
-                                                        w.queryList.p, w.queryListDist.p);
-        CK(cudaGetLastError());
-        uint32_t count = 0;
-        CK(cudaMemcpyAsync(&count, w.queryCount.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        const uint32_t m = std::min(count, capacity);
-        if (m) {
-            CK(cudaMemcpyAsync(out_colliders, w.queryList.p, size_t(m) * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            CK(cudaMemcpyAsync(out_distance, w.queryListDist.p, size_t(m) * sizeof(float), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-        }
-        *out_count = count;
+        *out_count = query_select(*world, QUERY_SELECT_CONTACTS, make_float4(x, y, radius, 0.0f), trees, out_colliders,
+                                  out_distance, capacity, out_count);
     });
 }
 
@@ -4110,12 +4151,11 @@ int32_t ag2d_world_read(ag2d_world* world, int32_t field, void* dst, uint64_t ca
             }
             return;
         }
-        uint64_t size = 0;
-        const auto bytes = read_field(*world, field, dst == nullptr, &size);
-        if (out_bytes) *out_bytes = size;
+        const TapField t = tap_field(*world, field);
+        if (out_bytes) *out_bytes = t.bytes;
         if (dst) {
-            if (cap < bytes.size()) throw ApiError(AG2D_ERR_INVALID_ARG, "destination too small");
-            if (!bytes.empty()) std::memcpy(dst, bytes.data(), bytes.size());
+            if (cap < t.bytes) throw ApiError(AG2D_ERR_INVALID_ARG, "destination too small");
+            copy_to_host(*world, dst, t.src, t.bytes);
         }
     });
 }
@@ -4513,8 +4553,7 @@ int32_t ag2d_batch_read(ag2d_batch* batch, uint32_t world, int32_t field, void* 
         }
         std::vector<uint8_t> out;
         if (field == AG2D_MANIFOLDS || field == AG2D_PREV_MANIFOLDS) {
-            uint64_t size = 0;
-            const std::vector<uint8_t> all = read_field(e, field, false, &size);
+            const std::vector<uint8_t> all = read_field(e, field);
             const Manifold* m = reinterpret_cast<const Manifold*>(all.data());
             const size_t n = all.size() / sizeof(Manifold);
             std::vector<Manifold> mine;
@@ -4529,9 +4568,8 @@ int32_t ag2d_batch_read(ag2d_batch* batch, uint32_t world, int32_t field, void* 
             if (!mine.empty()) std::memcpy(out.data(), mine.data(), out.size());
         } else if (field == AG2D_ISLAND_MANIFOLDS || field == AG2D_ISLAND_IDS) {
             // The world's stored records (collider indices and island roots made world-local).
-            uint64_t size = 0;
-            const std::vector<uint8_t> rec = read_field(e, AG2D_ISLAND_MANIFOLDS, false, &size);
-            const std::vector<uint8_t> ids = read_field(e, AG2D_ISLAND_IDS, false, &size);
+            const std::vector<uint8_t> rec = read_field(e, AG2D_ISLAND_MANIFOLDS);
+            const std::vector<uint8_t> ids = read_field(e, AG2D_ISLAND_IDS);
             const Manifold* m = reinterpret_cast<const Manifold*>(rec.data());
             const uint32_t* id = reinterpret_cast<const uint32_t*>(ids.data());
             const size_t n = rec.size() / sizeof(Manifold);

@@ -118,20 +118,17 @@ __global__ void k_fill_u32(uint32_t* __restrict__ out, uint32_t n, uint32_t valu
 __global__ void k_extract(const void* __restrict__ src, uint32_t lo, uint32_t n, uint32_t kind, uint32_t comp,
                           uint32_t bias, void* __restrict__ out)
 {
+    if (kind == EXTRACT_F4_XYZ) {   // a word a thread: whole lines are written, which host memory needs
+        for (size_t j = blockIdx.x * size_t(blockDim.x) + threadIdx.x; j < 3 * size_t(n); j += size_t(gridDim.x) * blockDim.x)
+            static_cast<float*>(out)[j] = static_cast<const float*>(src)[4 * (lo + j / 3) + j % 3];
+        return;
+    }
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const uint32_t i = lo + e;
         switch (kind) {
         case EXTRACT_F4_COMP:
             static_cast<float*>(out)[e] = static_cast<const float*>(src)[4 * size_t(i) + comp];
             break;
-        case EXTRACT_F4_XYZ: {
-            const float4 v = static_cast<const float4*>(src)[i];
-            float* o = static_cast<float*>(out) + 3 * size_t(e);
-            o[0] = v.x;
-            o[1] = v.y;
-            o[2] = v.z;
-            break;
-        }
         case EXTRACT_F2_COMP:
             static_cast<float*>(out)[e] = static_cast<const float*>(src)[2 * size_t(i) + comp];
             break;
@@ -146,6 +143,19 @@ __global__ void k_extract(const void* __restrict__ src, uint32_t lo, uint32_t n,
         default:
             break;
         }
+    }
+}
+
+// Copies of 16-byte aligned sections, grid-stride over each.
+__global__ void k_copy_sections(SectionCopies a)
+{
+    const uint64_t first = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x, stride = uint64_t(gridDim.x) * blockDim.x;
+    for (uint32_t k = 0; k < a.count; k++) {
+        const SectionCopy c = a.c[k];
+        const uint64_t quads = c.bytes / 16;
+        for (uint64_t i = first; i < quads; i += stride)
+            reinterpret_cast<uint4*>(c.dst)[i] = reinterpret_cast<const uint4*>(c.src)[i];
+        if (first < c.bytes - 16 * quads) c.dst[16 * quads + first] = c.src[16 * quads + first];
     }
 }
 
