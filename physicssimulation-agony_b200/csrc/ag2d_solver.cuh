@@ -340,6 +340,7 @@ constexpr uint32_t COLOR_SLOTS = 2 * MAX_COLORS + 4;
 // Colours 0..63 are chosen first-fit from a body's 64-bit mask of neighbouring colours; a manifold whose bodies see
 // all 64 taken gets colour 64 + its round (unique to the round, so still conflict-free).
 constexpr uint32_t MAX_ROUNDS = MAX_COLORS - 64;
+constexpr uint32_t ONE_BLOCK_ROUND = 4096;   // uncoloured manifolds that one block of a grid finishes
 
 // Solver records in global memory, structure of arrays: field f of record c at q[f * stride + c], so that a warp that
 // takes 32 consecutive records reads every field as four full lines. (As 128-byte structures a lane apart, each
@@ -419,10 +420,12 @@ struct SolveScratch {
 // Team barriers. ld() reads a colour counter written by other team members before the last barrier: global memory
 // through L2 for the grid, shared memory for one CTA.
 struct BlockSync {
+    static constexpr bool GRID = false;
     __device__ __forceinline__ bool operator()() const { __syncthreads(); return true; }
     static __device__ __forceinline__ uint32_t ld(const uint32_t* p) { return *static_cast<const volatile uint32_t*>(p); }
 };
 struct GridSync {
+    static constexpr bool GRID = true;
     uint32_t* bar;
     uint32_t* status;
     __device__ __forceinline__ bool operator()() const { return grid_barrier(bar, status); }
@@ -607,6 +610,16 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
                                 uint32_t* __restrict__ outColors, uint32_t* __restrict__ status, uint32_t& ncolOut)
 {
     for (uint32_t c = rank; c < COLOR_SLOTS; c += size) s.colorCount[c] = 0;
+    // A grid counts per block in shared memory first: one atomic a manifold on the fourteen counters of a pile's colours
+    // took 30 us of its colouring and again 35 us of its ordering (128,000 manifolds).
+    __shared__ uint32_t blockCount[Sync::GRID ? 2 * MAX_COLORS : 1];
+    auto clear_block_counts = [&] {
+        if constexpr (Sync::GRID) {
+            for (uint32_t c = threadIdx.x; c < 2 * MAX_COLORS; c += blockDim.x) blockCount[c] = 0u;
+            __syncthreads();
+        }
+    };
+    clear_block_counts();
     uint32_t* const nColors = s.colorCount + MAX_COLORS + 3;
     // Each manifold's two bodies and whether they are dynamic, looked up once for all colouring rounds; kept
     // colours are counted and marked around their bodies here.
@@ -621,14 +634,23 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
         const bool kept = hw != NO_COLOR && h < 64 && age + 1 < COLOR_KEEP_STEPS;
         if (kept) {
             s.color[i] = h | (age + 1) << COLOR_AGE_SHIFT;
-            atomicAdd(s.colorCount + h, 1u);
+            atomicAdd(Sync::GRID ? blockCount + h : s.colorCount + h, 1u);
             keptTop = max(keptTop, h + 1);
             if (dA) atomicOr(B.maskWord(bA), 1ull << h);
             if (dB) atomicOr(B.maskWord(bB), 1ull << h);
         }
         s.pairBodies[i] = make_uint2(bA | (dA ? DYN : 0u) | (kept ? KEPT : 0u), bB | (dB ? DYN : 0u) | (m[i].count != 1u ? PAIR_TWO : 0u));
     }
-    if (s.hint) {
+    if constexpr (Sync::GRID) {
+        if (s.hint) {
+            __syncthreads();
+            for (uint32_t c = threadIdx.x; c < 64; c += blockDim.x)
+                if (blockCount[c]) {
+                    atomicAdd(s.colorCount + c, blockCount[c]);
+                    atomicMax(nColors, c + 1);
+                }
+        }
+    } else if (s.hint) {
         for (int o = 16; o > 0; o >>= 1) keptTop = max(keptTop, __shfl_xor_sync(0xffffffffu, keptTop, o));
         if ((threadIdx.x & 31) == 0 && keptTop) atomicMax(nColors, keptTop);
     }
@@ -643,34 +665,35 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
         return make_uint4(j, s.prio ? s.prio[j] : priority_hash(j), pb.x, pb.y);
     };
     constexpr uint32_t BATCH = 4;   // records loaded together per thread (independent loads in flight)
-    for (uint32_t r = 0; r < MAX_ROUNDS && len > 0; r++) {
+    // Round r, by 'sz' threads of which this is number rk; false when the barrier gave up.
+    auto round = [&](uint32_t r, uint32_t rk, uint32_t sz, auto barrier) {
         uint4* out = (r & 1) ? s.listB : s.listA;
         uint32_t* outLen = s.colorCount + MAX_COLORS + 1 + (r & 1);
         // This counter was last read before the barrier that ended the previous round.
-        if (rank == 0) *outLen = 0;
+        if (rk == 0) *outLen = 0;
         const unsigned long long tag = static_cast<unsigned long long>(r + 1) << 32;
-        for (uint32_t j0 = rank; j0 < len; j0 += BATCH * size) {
+        for (uint32_t j0 = rk; j0 < len; j0 += BATCH * sz) {
             uint4 e[BATCH];
 #pragma unroll
-            for (uint32_t u = 0; u < BATCH; u++) e[u] = j0 + u * size < len ? rec(j0 + u * size) : make_uint4(0, 0, 0, 0);
+            for (uint32_t u = 0; u < BATCH; u++) e[u] = j0 + u * sz < len ? rec(j0 + u * sz) : make_uint4(0, 0, 0, 0);
 #pragma unroll
             for (uint32_t u = 0; u < BATCH; u++) {
-                if (j0 + u * size >= len) break;
+                if (j0 + u * sz >= len) break;
                 if (e[u].z & KEPT) continue;
                 const unsigned long long key = tag | e[u].y;
                 if (e[u].z & DYN) atomicMax(B.maxWord(e[u].z & PAIR_BODY), key);
                 if (e[u].w & DYN) atomicMax(B.maxWord(e[u].w & PAIR_BODY), key);
             }
         }
-        if (!sync()) return false;
+        if (!barrier()) return false;
         uint32_t top = 0;
-        for (uint32_t j0 = rank; j0 < len; j0 += BATCH * size) {
+        for (uint32_t j0 = rk; j0 < len; j0 += BATCH * sz) {
             uint4 e[BATCH];
 #pragma unroll
-            for (uint32_t u = 0; u < BATCH; u++) e[u] = j0 + u * size < len ? rec(j0 + u * size) : make_uint4(0, 0, 0, 0);
+            for (uint32_t u = 0; u < BATCH; u++) e[u] = j0 + u * sz < len ? rec(j0 + u * sz) : make_uint4(0, 0, 0, 0);
 #pragma unroll
             for (uint32_t u = 0; u < BATCH; u++) {
-                if (j0 + u * size >= len) break;
+                if (j0 + u * sz >= len) break;
                 if (e[u].z & KEPT) continue;
                 const uint32_t i = e[u].x;
                 const unsigned long long key = tag | e[u].y;
@@ -694,9 +717,26 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
         }
         for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
         if ((threadIdx.x & 31) == 0 && top) atomicMax(nColors, top);
-        if (!sync()) return false;
+        if (!barrier()) return false;
         len = Sync::ld(outLen);
         in = out;
+        return true;
+    };
+    uint32_t r = 0;
+    for (; r < MAX_ROUNDS && len > 0 && !(Sync::GRID && r > 0 && len <= ONE_BLOCK_ROUND); r++)
+        if (!round(r, rank, size, sync)) return false;
+    if constexpr (Sync::GRID) {
+        // The few manifolds that are left after the first rounds are finished by one block: a round is then two block
+        // barriers, not two of the grid (10 us a round on 148 blocks).
+        if (len > 0) {
+            if (blockIdx.x == 0) {
+                auto block = [] { __threadfence(); __syncthreads(); return true; };
+                for (; r < MAX_ROUNDS && len > 0; r++) round(r, threadIdx.x, blockDim.x, block);
+                if (rank == 0) s.colorCount[MAX_COLORS + 1] = len;
+            }
+            if (!sync()) return false;
+            len = Sync::ld(s.colorCount + MAX_COLORS + 1);
+        }
     }
     if (len > 0) { if (rank == 0) atomicOr(status, STATUS_COLOR_OVERFLOW); return false; }
     const uint32_t ncol = ncolOut = Sync::ld(nColors);
@@ -709,6 +749,27 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
     if (!sync()) return false;
     // Within a colour (independent contacts, any order) two-point contacts come first and one-point contacts last, so
     // that few warps run both solves.
+    if constexpr (Sync::GRID) {
+        // Places within the block, then the blocks' ranges (front counter c, back counter MAX_COLORS + c).
+        uint32_t* const place = reinterpret_cast<uint32_t*>(s.listA);   // the uncoloured lists are done with
+        clear_block_counts();
+        for (uint32_t i = rank; i < n; i += size)
+            place[i] = atomicAdd(blockCount + (s.color[i] & COLOR_MASK) + (s.pairBodies[i].y & PAIR_TWO ? 0u : MAX_COLORS),
+                                 1u);
+        __syncthreads();
+        for (uint32_t c = threadIdx.x; c < 2 * MAX_COLORS; c += blockDim.x)
+            if (blockCount[c])
+                blockCount[c] = atomicAdd(s.colorCount + (c < MAX_COLORS ? c : c + 4), blockCount[c]);
+        __syncthreads();
+        for (uint32_t i = rank; i < n; i += size) {
+            const uint32_t c = s.color[i] & COLOR_MASK;
+            const uint32_t at = s.pairBodies[i].y & PAIR_TWO
+                                    ? __ldcg(s.colorStart + c) + blockCount[c] + place[i]
+                                    : __ldcg(s.colorStart + c + 1) - 1u - blockCount[MAX_COLORS + c] - place[i];
+            s.order[at] = i;
+        }
+        return sync();
+    }
     for (uint32_t i = rank; i < n; i += size) {
         const uint32_t c = s.color[i] & COLOR_MASK;
         const uint32_t at = s.pairBodies[i].y & PAIR_TWO

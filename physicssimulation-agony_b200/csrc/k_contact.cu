@@ -297,9 +297,23 @@ __device__ __forceinline__ bool flow_wait(const FlowEnd& a, const FlowEnd& b, fl
 {
     bool ra = a.at == nullptr, rb = b.at == nullptr;
     for (uint32_t spins = 0;; spins++) {
-        if (!ra) { va = flow_load(a.at); ra = __float_as_uint(va.w) == a.need; }
-        if (!rb) { vb = flow_load(b.at); rb = __float_as_uint(vb.w) == b.need; }
-        if (__all_sync(0xffffffffu, ra && rb)) return true;
+        uint32_t gap = 0;   // updates still missing on the body that lacks most
+        if (!ra) {
+            va = flow_load(a.at);
+            gap = a.need - __float_as_uint(va.w);
+            ra = gap == 0;
+        }
+        if (!rb) {
+            vb = flow_load(b.at);
+            const uint32_t missing = b.need - __float_as_uint(vb.w);
+            rb = missing == 0;
+            gap = max(gap, missing);
+        }
+        gap = __reduce_max_sync(0xffffffffu, gap);
+        if (gap == 0) return true;
+        // The missing updates follow one another, half a microsecond each at least: a warp that lacks several sleeps
+        // instead of loading the L2 with its polls (all waiting warps polling: 2.5 us a hop).
+        if (gap > 1u) __nanosleep(min(gap - 1u, 8u) * 300u);
         if ((spins & 1023u) == 1023u) {
             const bool gone = (*status & STATUS_BARRIER_TIMEOUT) != 0;
             if (__any_sync(0xffffffffu, gone)) return false;
@@ -511,7 +525,7 @@ __device__ __forceinline__ uint32_t team_find(uint32_t* par, uint32_t x)
     uint32_t px = p[x];
     for (uint32_t guard = 0; px != x && guard < (1u << 20); guard++) {
         const uint32_t gp = p[px];
-        if (gp != px) atomicCAS(par + x, px, gp);   // path halving, benign races
+        if (gp != px) p[x] = gp;   // path halving: x is no root, and any ancestor is a good parent
         x = px;
         px = gp;
     }

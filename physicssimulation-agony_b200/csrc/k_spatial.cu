@@ -997,15 +997,15 @@ __device__ __forceinline__ bool strict_overlap(const float4& a, const float4& b)
     return a.x < b.z && a.z > b.x && a.y < b.w && a.w > b.y;
 }
 
-// All pairs of dynamic collider rank i, in traversal order; emit(k, pair) receives the k-th. Returns the count.
+// All pair partners of dynamic collider rank i, in traversal order; emit(k, collider) receives the k-th. Returns the
+// count.
 template <class Emit>
 __device__ __forceinline__ uint32_t query_one(const TreeView& dyn, const TreeView& other,
-                                              const uint32_t* __restrict__ cbody, int i, Emit emit,
+                                              const uint32_t* __restrict__ cbody, int i, uint32_t me, Emit emit,
                                               uint32_t* __restrict__ status)
 {
     const int n = dyn.n;
     const float4 q = dyn.leafAabb[i];
-    const uint32_t me = dyn.vals[i];
     const uint32_t myBody = cbody[me];
     // This collider's world: the segments of both trees it is tested against.
     int dlo = 0, dhi = n, olo = 0, ohi = other.n;
@@ -1035,8 +1035,8 @@ __device__ __forceinline__ uint32_t query_one(const TreeView& dyn, const TreeVie
                 const int last = side == 0 ? r.last.x : r.last.y;
                 if (last <= i || !strict_overlap(q, r.box[side])) continue;   // every leaf below ranks <= i
                 if (ch < 0) {
-                    const uint32_t other_c = dyn.vals[~ch];
-                    if (cbody[other_c] != myBody) emit(count++, make_uint2(me, other_c));
+                    const uint32_t c = dyn.vals[~ch];
+                    if (cbody[c] != myBody) emit(count++, c);
                 } else if (sp < QUERY_STACK) {
                     stack[sp++] = ch;
                 } else {
@@ -1047,7 +1047,7 @@ __device__ __forceinline__ uint32_t query_one(const TreeView& dyn, const TreeVie
     }
     // Cross pairs against the static + sleeping tree.
     if (ohi - olo == 1) {
-        if (strict_overlap(q, other.leafAabb[olo])) emit(count++, make_uint2(me, other.vals[olo]));
+        if (strict_overlap(q, other.leafAabb[olo])) emit(count++, other.vals[olo]);
     } else if (ohi - olo > 1 && strict_overlap(q, other.nodeAabb[olo])) {
         int sp = 0;
         stack[sp++] = olo;
@@ -1058,7 +1058,7 @@ __device__ __forceinline__ uint32_t query_one(const TreeView& dyn, const TreeVie
             for (int side = 0; side < 2; side++) {
                 const int ch = side == 0 ? r.child.x : r.child.y;
                 if (!strict_overlap(q, r.box[side])) continue;
-                if (ch < 0) emit(count++, make_uint2(me, other.vals[~ch]));
+                if (ch < 0) emit(count++, other.vals[~ch]);
                 else if (sp < QUERY_STACK) stack[sp++] = ch;
                 else atomicOr(status, STATUS_STACK_OVERFLOW);
             }
@@ -1082,7 +1082,7 @@ __global__ void __launch_bounds__(QUERY_MAX_THREADS) k_query(TreeView dyn, TreeV
                                                              uint32_t* __restrict__ tileState,
                                                              uint32_t* __restrict__ tileCounter)
 {
-    __shared__ uint2 kept[QUERY_STASH * QUERY_MAX_THREADS];   // [k][thread]
+    __shared__ uint32_t kept[QUERY_STASH * QUERY_MAX_THREADS];   // [k][thread]
     __shared__ uint32_t warpBase[QUERY_MAX_THREADS / 32];
     __shared__ uint32_t tileSlot, tileBase;
     const uint32_t n = uint32_t(dyn.n);
@@ -1095,9 +1095,10 @@ __global__ void __launch_bounds__(QUERY_MAX_THREADS) k_query(TreeView dyn, TreeV
         if (tile >= tiles) return;
         const uint32_t i = tile * blockDim.x + threadIdx.x;
         uint32_t count = 0;
+        const uint32_t me = i < n ? dyn.vals[i] : 0u;
         if (i < n)
-            count = query_one(dyn, other, cbody, int(i), [&](uint32_t k, uint2 pr) {
-                if (k < QUERY_STASH) kept[k * blockDim.x + threadIdx.x] = pr;
+            count = query_one(dyn, other, cbody, int(i), me, [&](uint32_t k, uint32_t c) {
+                if (k < QUERY_STASH) kept[k * blockDim.x + threadIdx.x] = c;
             }, status);
         // Block scan of the counts: lane prefix within the warp, then the warps' totals.
         uint32_t incl = count;
@@ -1137,10 +1138,10 @@ __global__ void __launch_bounds__(QUERY_MAX_THREADS) k_query(TreeView dyn, TreeV
         const uint32_t out = tileBase + warpBase[warp] + incl - count;
         const uint32_t keptCount = min(count, QUERY_STASH);
         for (uint32_t k = 0; k < keptCount; k++)
-            if (out + k < pairCap) pairs[out + k] = kept[k * blockDim.x + threadIdx.x];
+            if (out + k < pairCap) pairs[out + k] = make_uint2(me, kept[k * blockDim.x + threadIdx.x]);
         if (count > QUERY_STASH)
-            query_one(dyn, other, cbody, int(i), [&](uint32_t k, uint2 pr) {
-                if (k >= QUERY_STASH && out + k < pairCap) pairs[out + k] = pr;
+            query_one(dyn, other, cbody, int(i), me, [&](uint32_t k, uint32_t c) {
+                if (k >= QUERY_STASH && out + k < pairCap) pairs[out + k] = make_uint2(me, c);
             }, status);
         __syncthreads();   // tileSlot, tileBase, warpBase and the stash are reused by the next tile
     }
