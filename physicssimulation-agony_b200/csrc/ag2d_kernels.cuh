@@ -13,7 +13,7 @@ constexpr uint32_t SCAN_THREADS = 256;
 constexpr uint32_t SCAN_ITEMS = 8;
 constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 constexpr int QUERY_STACK = 64;
-constexpr uint32_t QUERY_STASH = 8;   // pairs a query keeps from its counting traversal
+constexpr uint32_t QUERY_STASH = 16;   // pair partners a query keeps from its counting traversal
 constexpr uint32_t MAX_COLORS = 256;
 constexpr uint32_t NO_COLOR = 0xFFFFFFFFu;
 
@@ -335,8 +335,25 @@ __global__ void k_query_select(DeviceWorld w, QuerySelect q);
 // data[k], the motors' accumulated impulses by dense index in motorImpulse. One CTA of JOINT_THREADS threads.
 constexpr uint32_t JOINT_KINDS_DEVICE = 5;
 constexpr uint32_t JOINT_THREADS = 1024;
+// The dataflow schedule (k_joints_flow): the bodies that active constraints name, with how many constraints of each type
+// act on them (dynamic bodies), and per constraint its bodies in that list and its rank among its type's on each.
+struct JointBody {
+    uint32_t body;
+    uint16_t degree[JOINT_KINDS_DEVICE];
+    uint16_t moves;
+};
+static_assert(sizeof(JointBody) == 16, "JointBody is 16 bytes");
+struct JointFlow {
+    uint16_t a, b, rankA, rankB;
+};
+constexpr uint32_t JOINT_FLOW_BODY_BYTES = sizeof(float4) + sizeof(JointBody) + sizeof(float2);
+constexpr uint32_t JOINT_FLOW_BODIES = 5600;   // 40 B of shared memory each
 struct JointLaunch {
     const JointRec* rec[JOINT_KINDS_DEVICE];
+    const JointFlow* flow[JOINT_KINDS_DEVICE];
+    const JointBody* body;
+    uint32_t bodies;
+    uint32_t* status;
     JointData* data[JOINT_KINDS_DEVICE];
     const uint32_t* levelStart[JOINT_KINDS_DEVICE];
     uint32_t count[JOINT_KINDS_DEVICE];
@@ -347,6 +364,9 @@ struct JointLaunch {
     float* motorImpulse;
 };
 __global__ void k_joints(DeviceWorld w, JointLaunch L);
+__global__ void k_joints_flow(DeviceWorld w, JointLaunch L);
+// Host side: raises the dataflow kernel's dynamic shared-memory limit (once per device).
+cudaError_t joints_init();
 // Island links of the active constraints' body pairs (edges[i] = {a, b}), as k_island_union links manifolds.
 __global__ void k_island_union_edges(DeviceWorld w, const uint2* edges, uint32_t n, uint32_t* parent);
 

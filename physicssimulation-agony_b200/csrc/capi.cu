@@ -395,6 +395,7 @@ static DeviceInfo probe_device(int device)
     CK(cudaDeviceGetAttribute(&dev.sms, cudaDevAttrMultiProcessorCount, device));
     CK(block_solver_init());
     CK(tree_segments_init());
+    CK(joints_init());
     int perSm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_color_solve_flow, FLOW_THREADS, 0));
     dev.flowBlocks = std::max(1, perSm) * dev.sms;
@@ -531,6 +532,9 @@ struct ag2d_world {
     DBuf<JointRec> jointRec[JOINT_KINDS];
     DBuf<JointData> jointData[JOINT_KINDS];
     DBuf<uint32_t> jointLevel[JOINT_KINDS];
+    DBuf<JointFlow> jointFlow[JOINT_KINDS];   // the dataflow schedule; jointBodies 0: too large for it
+    DBuf<JointBody> jointBody;
+    uint32_t jointBodies = 0;
     DBuf<float> motorImpulse, snapMotorImpulse;
     DBuf<uint2> jointEdges;
     // Collision events: per-collider opt-in and the step's event ring.
@@ -2200,6 +2204,16 @@ struct ag2d_world {
         auto st = [&](uint32_t b) -> uint8_t { return b < state.size() ? state[b] : uint8_t(STATE_DESTROYED); };
         std::vector<uint32_t> last(std::max<uint32_t>(nBodies, 1));
         std::vector<uint2> edges;
+        std::vector<uint32_t> local(std::max<uint32_t>(nBodies, 1), 0xFFFFFFFFu);   // place in 'bodies'
+        std::vector<JointBody> bodies;
+        bool flowFits = true;
+        auto place = [&](uint32_t b) {
+            if (local[b] == 0xFFFFFFFFu) {
+                local[b] = uint32_t(bodies.size());
+                bodies.push_back(JointBody{b, {}, uint16_t(st(b) == STATE_DYNAMIC)});
+            }
+            return local[b];
+        };
         for (uint32_t k = 0; k < JOINT_KINDS; k++) {
             JointSystem& js = objects.jointSystems[k];
             std::vector<uint64_t> handles;
@@ -2234,8 +2248,16 @@ struct ag2d_world {
             for (uint32_t l = 1; l <= levels + 1; l++) start[l] += start[l - 1];
             std::vector<uint32_t> fill(start.begin(), start.end());
             std::vector<JointRec> recs(end - begin);
+            std::vector<JointFlow> flow(end - begin);
             for (uint32_t i = begin; i < end; i++) {
                 const HJoint& j = js.joints[i];
+                const uint32_t a = place(j.bodyA), b = j.bodyB == NO_BODY ? a : place(j.bodyB);
+                JointFlow f{uint16_t(a), uint16_t(b), bodies[a].degree[k], bodies[b].degree[k]};
+                if (bodies[a].moves) bodies[a].degree[k]++;
+                if (b != a && bodies[b].moves) bodies[b].degree[k]++;
+                flowFits = flowFits && bodies.size() <= JOINT_FLOW_BODIES && bodies[a].degree[k] != 0xFFFFu &&
+                           bodies[b].degree[k] != 0xFFFFu && (k == JOINT_MOTOR || b != a);
+                flow[fill[level[i - begin]]] = f;
                 JointRec r{};
                 r.bodyA = j.bodyA; r.bodyB = j.bodyB == NO_BODY ? j.bodyA : j.bodyB; r.index = i;
                 r.ax = j.anchorAx; r.ay = j.anchorAy; r.bx = j.anchorBx; r.by = j.anchorBy;
@@ -2253,9 +2275,12 @@ struct ag2d_world {
             jointLevels[k] = levels;
             jointLevelHost[k].assign(start.begin() + 1, start.end());   // level l (from 1) starts at [l - 1]
             jointRec[k].upload(recs.data(), recs.size(), s);
+            jointFlow[k].upload(flow.data(), flow.size(), s);
             jointLevel[k].upload(jointLevelHost[k].data(), jointLevelHost[k].size(), s);
             jointData[k].reserve(std::max<size_t>(recs.size(), 1));
         }
+        jointBodies = flowFits ? uint32_t(bodies.size()) : 0u;
+        jointBody.upload(bodies.data(), flowFits ? bodies.size() : 0u, s);
         auto& motors = objects.jointSystems[JOINT_MOTOR].joints;
         std::vector<float> imp(motors.size());
         for (size_t i = 0; i < motors.size(); i++) imp[i] = motors[i].impulse;
@@ -2272,6 +2297,7 @@ struct ag2d_world {
         uint32_t maxIt = 0;
         for (uint32_t k = 0; k < JOINT_KINDS; k++) {
             L.rec[k] = jointRec[k].p;
+            L.flow[k] = jointFlow[k].p;
             L.data[k] = jointData[k].p;
             L.levelStart[k] = jointLevel[k].p;
             L.count[k] = jointActive[k];
@@ -2282,7 +2308,13 @@ struct ag2d_world {
         L.maxIterations = maxIt;
         L.dt = settings.dt;
         L.motorImpulse = motorImpulse.p;
-        k_joints<<<1, JOINT_THREADS, 0, stream>>>(view(), L);
+        L.body = jointBody.p;
+        L.bodies = jointBodies;
+        L.status = &dCounters.p->status;
+        if (jointBodies)
+            k_joints_flow<<<1, JOINT_THREADS, jointBodies * JOINT_FLOW_BODY_BYTES, stream>>>(view(), L);
+        else
+            k_joints<<<1, JOINT_THREADS, 0, stream>>>(view(), L);
         CK(cudaGetLastError());
         launches++;
     }

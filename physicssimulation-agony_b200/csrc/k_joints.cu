@@ -210,22 +210,20 @@ __device__ void motor_data(const DeviceWorld& w, const JointRec& r, float dt, fl
 }
 
 // Applies a point impulse to both bodies, as the spring and revolute solvers do (A gains, B loses).
-__device__ __forceinline__ void apply_pair(const DeviceWorld& w, uint32_t a, uint32_t b, float4 vA, float4 vB,
-                                           float iIA, float iIB, const JointData& d, float ix, float iy)
+__device__ __forceinline__ void apply_pair(float4& vA, float4& vB, float iIA, float iIB, const JointData& d, float ix,
+                                           float iy)
 {
     if (vA.w > 0.0f) {
         vA.x = vA.x + ix * vA.w;
         vA.y = vA.y + iy * vA.w;
         const float tA = d.rAx * iy - d.rAy * ix;
         vA.z = vA.z + tA * iIA;
-        w.bvel[a] = vA;
     }
     if (vB.w > 0.0f) {
         vB.x = vB.x - ix * vB.w;
         vB.y = vB.y - iy * vB.w;
         const float tB = d.rBx * iy - d.rBy * ix;
         vB.z = vB.z - tB * iIB;
-        w.bvel[b] = vB;
     }
 }
 
@@ -237,38 +235,36 @@ __device__ __forceinline__ float2 anchor_relative_velocity(float4 vA, float4 vB,
     return make_float2((vB.x + aBx) - (vA.x + aAx), (vB.y + aBy) - (vA.y + aAy));
 }
 
-__device__ void spring_solve(const DeviceWorld& w, const JointRec& r, const JointData& d)
+// The solves work on the two bodies' velocities in registers (vx, vy, w, inverse mass) and leave a body of infinite mass
+// as it is.
+__device__ __forceinline__ void spring_solve(const JointData& d, float4& vA, float4& vB, float iIA, float iIB)
 {
     if (d.s[2] == 0.0f) return;
-    const float4 vA = w.bvel[r.bodyA], vB = w.bvel[r.bodyB];
-    const float iIA = w.bpos[r.bodyA].w, iIB = w.bpos[r.bodyB].w;
     const float2 rv = anchor_relative_velocity(vA, vB, d);
     const float cdot = rv.x * d.s[0] + rv.y * d.s[1];
     const float mag = (cdot + d.s[3]) * d.s[2];
-    apply_pair(w, r.bodyA, r.bodyB, vA, vB, iIA, iIB, d, d.s[0] * mag, d.s[1] * mag);
+    apply_pair(vA, vB, iIA, iIB, d, d.s[0] * mag, d.s[1] * mag);
 }
 
-__device__ void revolute_solve(const DeviceWorld& w, const JointRec& r, const JointData& d)
+__device__ __forceinline__ void revolute_solve(const JointData& d, float4& vA, float4& vB, float iIA, float iIB)
 {
     if (d.s[4] == 0.0f && d.s[5] == 0.0f && d.s[6] == 0.0f) return;
-    const float4 vA = w.bvel[r.bodyA], vB = w.bvel[r.bodyB];
-    const float iIA = w.bpos[r.bodyA].w, iIB = w.bpos[r.bodyB].w;
     const float2 rv = anchor_relative_velocity(vA, vB, d);
     const float hx = rv.x + d.s[0], hy = rv.y + d.s[1];
     const float ix = d.s[4] * hx + d.s[5] * hy;
     const float iy = d.s[5] * hx + d.s[6] * hy;
-    apply_pair(w, r.bodyA, r.bodyB, vA, vB, iIA, iIB, d, ix, iy);
+    apply_pair(vA, vB, iIA, iIB, d, ix, iy);
 }
 
 // One velocity iteration of a prismatic (PrismaticJointSolver.cpp:160-255) or slider joint (SliderJointSolver.cpp:
 // 132-220): the perpendicular block, then the axis limit with its accumulated, one-sided impulse.
-__device__ void axis_joint_solve(const DeviceWorld& w, const JointRec& r, JointData& d, bool slider)
+__device__ __forceinline__ void axis_joint_solve(JointData& d, float4& vA0, float4& vB0, float iIA, float iIB,
+                                                 bool slider)
 {
     const bool block = slider ? d.s[8] > 0.0f : d.s[11] != 0.0f;
     if (!block && d.s[16] == 0.0f) return;
-    float4 vA = w.bvel[r.bodyA], vB = w.bvel[r.bodyB];
+    float4 vA = vA0, vB = vB0;
     const float imA = vA.w, imB = vB.w;
-    const float iIA = w.bpos[r.bodyA].w, iIB = w.bpos[r.bodyB].w;
     if (block) {
         const float pX = d.s[2], pY = d.s[3], s1 = d.s[4], s2 = d.s[5];
         const float cdot1 = (pX * (vB.x - vA.x) + pY * (vB.y - vA.y)) + s2 * vB.z - s1 * vA.z;
@@ -307,51 +303,44 @@ __device__ void axis_joint_solve(const DeviceWorld& w, const JointRec& r, JointD
         vB.x = vB.x + Px * imB; vB.y = vB.y + Py * imB;
         vB.z = vB.z + LB * iIB;
     }
-    if (imA > 0.0f) w.bvel[r.bodyA] = vA;
-    if (imB > 0.0f) w.bvel[r.bodyB] = vB;
+    if (imA > 0.0f) vA0 = vA;
+    if (imB > 0.0f) vB0 = vB;
 }
 
-__device__ void motor_warm(const DeviceWorld& w, const JointRec& r, const JointData& d)
+__device__ __forceinline__ void motor_warm(const JointData& d, float4& v)
 {
     if (d.s[0] == 0.0f) return;
-    float4 v = w.bvel[r.bodyA];
     v.z = v.z + d.s[4] * d.s[0];
-    w.bvel[r.bodyA] = v;
 }
 
-__device__ void motor_solve(const DeviceWorld& w, const JointRec& r, JointData& d, float* impulses)
+__device__ __forceinline__ void motor_solve(uint32_t index, JointData& d, float4& v, float* impulses)
 {
     if (d.s[0] == 0.0f) return;
-    float4 v = w.bvel[r.bodyA];
     const float lambda = (d.s[2] - v.z) * d.s[1];
     const float oldImpulse = d.s[4];
     const float newImpulse = glm_clamp(oldImpulse + lambda, -d.s[3], d.s[3]);
     d.s[4] = newImpulse;
-    impulses[r.index] = newImpulse;
+    impulses[index] = newImpulse;
     v.z = v.z + (newImpulse - oldImpulse) * d.s[0];
-    w.bvel[r.bodyA] = v;
 }
 
-__device__ __forceinline__ void solve_one(const DeviceWorld& w, uint32_t k, const JointRec& r, JointData& d,
-                                          float* impulses)
+__device__ __forceinline__ void solve_one(uint32_t k, uint32_t index, JointData& d, float4& vA, float4& vB, float iIA,
+                                          float iIB, float* impulses)
 {
     switch (k) {
-    case K_SPRING: spring_solve(w, r, d); break;
-    case K_REVOLUTE: revolute_solve(w, r, d); break;
-    case K_PRISMATIC: axis_joint_solve(w, r, d, false); break;
-    case K_SLIDER: axis_joint_solve(w, r, d, true); break;
-    default: motor_solve(w, r, d, impulses); break;
+    case K_SPRING: spring_solve(d, vA, vB, iIA, iIB); break;
+    case K_REVOLUTE: revolute_solve(d, vA, vB, iIA, iIB); break;
+    case K_PRISMATIC: axis_joint_solve(d, vA, vB, iIA, iIB, false); break;
+    case K_SLIDER: axis_joint_solve(d, vA, vB, iIA, iIB, true); break;
+    default: motor_solve(index, d, vA, impulses); break;
     }
 }
 
-}  // namespace
-
-__global__ void __launch_bounds__(JOINT_THREADS) k_joints(DeviceWorld w, JointLaunch L)
+// Compute tick: every type's constraint data, read-only on the bodies.
+__device__ __forceinline__ void compute_tick(const DeviceWorld& w, const JointLaunch& L)
 {
-    const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    // Compute tick: every type's constraint data, read-only on the bodies.
     for (uint32_t k = 0; k < JOINT_KINDS_DEVICE; k++)
-        for (uint32_t i = tid; i < L.count[k]; i += nt) {
+        for (uint32_t i = threadIdx.x; i < L.count[k]; i += blockDim.x) {
             JointData d;
             const JointRec r = L.rec[k][i];
             switch (k) {
@@ -363,11 +352,138 @@ __global__ void __launch_bounds__(JOINT_THREADS) k_joints(DeviceWorld w, JointLa
             }
             L.data[k][i] = d;
         }
+}
+
+// A body's velocity and version in one 16-byte word of shared memory, read and written whole.
+__device__ __forceinline__ float4 word_load(const float4* p)
+{
+    unsigned long long lo, hi;
+    const uint32_t a = uint32_t(__cvta_generic_to_shared(p));
+    asm volatile("{\n\t.reg .b128 d;\n\tld.relaxed.cta.shared.b128 d, [%2];\n\tmov.b128 {%0, %1}, d;\n\t}"
+                 : "=l"(lo), "=l"(hi) : "r"(a) : "memory");
+    return make_float4(__uint_as_float(uint32_t(lo)), __uint_as_float(uint32_t(lo >> 32)),
+                       __uint_as_float(uint32_t(hi)), __uint_as_float(uint32_t(hi >> 32)));
+}
+__device__ __forceinline__ void word_store(float4* p, float x, float y, float z, uint32_t version)
+{
+    const unsigned long long lo = uint64_t(__float_as_uint(x)) | uint64_t(__float_as_uint(y)) << 32;
+    const unsigned long long hi = uint64_t(__float_as_uint(z)) | uint64_t(version) << 32;
+    const uint32_t a = uint32_t(__cvta_generic_to_shared(p));
+    asm volatile("{\n\t.reg .b128 s;\n\tmov.b128 s, {%1, %2};\n\tst.relaxed.cta.shared.b128 [%0], s;\n\t}"
+                 :: "r"(a), "l"(lo), "l"(hi) : "memory");
+}
+
+}  // namespace
+
+// The schedule as a dataflow over per-body versions, for constraint sets whose bodies fit shared memory. A body's
+// constraints act on it in one order: iteration after iteration, type after type, dense order within a type. The body
+// carries the number of updates made so far in the same word as its velocity; a constraint waits until each of its
+// moving bodies has had all the updates before its own (whole types of the body's degree, then its rank among the
+// type's constraints on it) and nothing else, so iterations follow one another down a chain like waves. Threads take
+// constraints in that order and all are resident, so the oldest one can always go. The order of every body's updates
+// is the dense order's, the results are the same bit for bit.
+// Bound: the longest chain of updates, a few hundred cycles each in shared memory. With a block barrier after every
+// level of every type and iteration, and the velocities in global memory, 960 revolute joints in chains of twelve,
+// 240 motors and 316 springs (eight iterations: 130 levels) took 350 us a step.
+__global__ void __launch_bounds__(JOINT_THREADS) k_joints_flow(DeviceWorld w, JointLaunch L)
+{
+    extern __shared__ float4 jointSmem[];
+    float4* const vel = jointSmem;                                            // [bodies] vx, vy, w, version
+    JointBody* const body = reinterpret_cast<JointBody*>(vel + L.bodies);     // [bodies]
+    float2* const mass = reinterpret_cast<float2*>(body + L.bodies);          // [bodies] inverse mass, inverse inertia
+    compute_tick(w, L);
+    for (uint32_t i = threadIdx.x; i < L.bodies; i += blockDim.x) {
+        const JointBody b = L.body[i];
+        const float4 v = w.bvel[b.body];
+        body[i] = b;
+        mass[i] = make_float2(v.w, w.bpos[b.body].w);
+        vel[i] = make_float4(v.x, v.y, v.z, __uint_as_float(0u));
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t done[JOINT_KINDS_DEVICE], rest[JOINT_KINDS_DEVICE];   // iterations made, and the interleaving's remainder
+    for (uint32_t k = 0; k < JOINT_KINDS_DEVICE; k++) { done[k] = 0; rest[k] = 0; }
+    bool gone = false;
+    // One type's pass: this warp's stretches of 32 constraints.
+    auto pass = [&](uint32_t k, bool warm) {
+        for (uint32_t first = threadIdx.x & ~31u; first < L.count[k] && !gone; first += blockDim.x) {
+            const uint32_t i = first + lane;
+            bool todo = i < L.count[k];
+            JointFlow f{};
+            JointData d;
+            uint32_t index = 0, needA = 0, needB = 0;
+            bool dynA = false, dynB = false;
+            float2 mA = make_float2(0.0f, 0.0f), mB = mA;
+            if (todo) {
+                f = L.flow[k][i];
+                d = L.data[k][i];
+                if (k == K_MOTOR) index = L.rec[k][i].index;
+                const JointBody bA = body[f.a], bB = body[f.b];
+                mA = mass[f.a];
+                mB = mass[f.b];
+                dynA = bA.moves != 0;
+                dynB = bB.moves != 0 && k != K_MOTOR;
+                needA = f.rankA;
+                needB = f.rankB;
+                for (uint32_t t = 0; t < JOINT_KINDS_DEVICE; t++) {
+                    needA += done[t] * bA.degree[t];
+                    needB += done[t] * bB.degree[t];
+                }
+            }
+            for (uint32_t spins = 0; __any_sync(0xffffffffu, todo); spins++) {
+                if (todo) {
+                    float4 vA = word_load(vel + f.a), vB = word_load(vel + f.b);
+                    if ((!dynA || __float_as_uint(vA.w) == needA) && (!dynB || __float_as_uint(vB.w) == needB)) {
+                        vA.w = mA.x;
+                        vB.w = mB.x;
+                        if (warm) motor_warm(d, vA);
+                        else solve_one(k, index, d, vA, vB, mA.y, mB.y, L.motorImpulse);
+                        if (dynA) word_store(vel + f.a, vA.x, vA.y, vA.z, needA + 1u);
+                        if (dynB) word_store(vel + f.b, vB.x, vB.y, vB.z, needB + 1u);
+                        if (!warm && k == K_MOTOR) L.data[k][i].s[4] = d.s[4];
+                        if (k == K_PRISMATIC || k == K_SLIDER) L.data[k][i].s[17] = d.s[17];
+                        todo = false;
+                    }
+                }
+                if (spins > SPIN_LIMIT) {
+                    atomicOr(L.status, STATUS_BARRIER_TIMEOUT);
+                    gone = true;
+                    break;
+                }
+            }
+        }
+    };
+    // Warm start: the motors (the one type with a warm start); then the velocity iterations, the types interleaved in
+    // ConstraintType order.
+    pass(K_MOTOR, true);
+    done[K_MOTOR] = 1;
+    for (uint32_t it = 0; it < L.maxIterations && !gone; it++)
+        for (uint32_t k = 0; k < JOINT_KINDS_DEVICE; k++) {
+            rest[k] += L.iterations[k];
+            if (L.count[k] == 0 || rest[k] < L.maxIterations) continue;
+            rest[k] -= L.maxIterations;
+            pass(k, false);
+            done[k]++;
+        }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < L.bodies; i += blockDim.x)
+        if (body[i].moves) w.bvel[body[i].body] = make_float4(vel[i].x, vel[i].y, vel[i].z, mass[i].x);
+}
+
+// Larger sets: a block barrier after every level, velocities in global memory.
+__global__ void __launch_bounds__(JOINT_THREADS) k_joints(DeviceWorld w, JointLaunch L)
+{
+    const uint32_t tid = threadIdx.x, nt = blockDim.x;
+    compute_tick(w, L);
     __syncthreads();
     // Warm start: the motors (the one type with a warm start), level by level.
     for (uint32_t l = 0; l < L.levels[K_MOTOR]; l++) {
-        for (uint32_t i = L.levelStart[K_MOTOR][l] + tid; i < L.levelStart[K_MOTOR][l + 1]; i += nt)
-            motor_warm(w, L.rec[K_MOTOR][i], L.data[K_MOTOR][i]);
+        for (uint32_t i = L.levelStart[K_MOTOR][l] + tid; i < L.levelStart[K_MOTOR][l + 1]; i += nt) {
+            const uint32_t b = L.rec[K_MOTOR][i].bodyA;
+            float4 v = w.bvel[b];
+            motor_warm(L.data[K_MOTOR][i], v);
+            w.bvel[b] = v;
+        }
         __syncthreads();
     }
     // Velocity iterations, the types interleaved in ConstraintType order.
@@ -377,11 +493,22 @@ __global__ void __launch_bounds__(JOINT_THREADS) k_joints(DeviceWorld w, JointLa
             if (L.count[k] == 0 || (uint64_t(it + 1) * n) / L.maxIterations == (uint64_t(it) * n) / L.maxIterations)
                 continue;
             for (uint32_t l = 0; l < L.levels[k]; l++) {
-                for (uint32_t i = L.levelStart[k][l] + tid; i < L.levelStart[k][l + 1]; i += nt)
-                    solve_one(w, k, L.rec[k][i], L.data[k][i], L.motorImpulse);
+                for (uint32_t i = L.levelStart[k][l] + tid; i < L.levelStart[k][l + 1]; i += nt) {
+                    const uint32_t a = L.rec[k][i].bodyA, b = L.rec[k][i].bodyB;
+                    float4 vA = w.bvel[a], vB = w.bvel[b];
+                    solve_one(k, L.rec[k][i].index, L.data[k][i], vA, vB, w.bpos[a].w, w.bpos[b].w, L.motorImpulse);
+                    if (k == K_MOTOR || vA.w > 0.0f) w.bvel[a] = vA;
+                    if (k != K_MOTOR && vB.w > 0.0f) w.bvel[b] = vB;
+                }
                 __syncthreads();
             }
         }
+}
+
+cudaError_t joints_init()
+{
+    return cudaFuncSetAttribute(k_joints_flow, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(JOINT_FLOW_BODIES * JOINT_FLOW_BODY_BYTES));
 }
 
 }  // namespace ag2d
