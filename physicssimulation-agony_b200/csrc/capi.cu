@@ -2206,6 +2206,9 @@ struct ag2d_world {
         std::vector<uint2> edges;
         std::vector<uint32_t> local(std::max<uint32_t>(nBodies, 1), 0xFFFFFFFFu);   // place in 'bodies'
         std::vector<JointBody> bodies;
+        std::vector<JointRec> recsOf[JOINT_KINDS];
+        std::vector<JointFlow> flowOf[JOINT_KINDS];
+        std::vector<uint32_t> levelMajor[JOINT_KINDS];   // level-major order, dense order within a level
         bool flowFits = true;
         auto place = [&](uint32_t b) {
             if (local[b] == 0xFFFFFFFFu) {
@@ -2242,13 +2245,13 @@ struct ag2d_world {
                 levels = std::max(levels, l);
                 if (k != JOINT_MOTOR) edges.push_back(make_uint2(j.bodyA, j.bodyB));
             }
-            // Level-major order, dense order within a level.
             std::vector<uint32_t> start(levels + 2, 0);
             for (const uint32_t l : level) start[l + 1]++;
             for (uint32_t l = 1; l <= levels + 1; l++) start[l] += start[l - 1];
             std::vector<uint32_t> fill(start.begin(), start.end());
-            std::vector<JointRec> recs(end - begin);
-            std::vector<JointFlow> flow(end - begin);
+            std::vector<JointRec>& recs = recsOf[k];   // dense order
+            std::vector<JointFlow>& flow = flowOf[k];
+            std::vector<uint32_t>& at = levelMajor[k];
             for (uint32_t i = begin; i < end; i++) {
                 const HJoint& j = js.joints[i];
                 const uint32_t a = place(j.bodyA), b = j.bodyB == NO_BODY ? a : place(j.bodyB);
@@ -2257,7 +2260,7 @@ struct ag2d_world {
                 if (b != a && bodies[b].moves) bodies[b].degree[k]++;
                 flowFits = flowFits && bodies.size() <= JOINT_FLOW_BODIES && bodies[a].degree[k] != 0xFFFFu &&
                            bodies[b].degree[k] != 0xFFFFu && (k == JOINT_MOTOR || b != a);
-                flow[fill[level[i - begin]]] = f;
+                flow.push_back(f);
                 JointRec r{};
                 r.bodyA = j.bodyA; r.bodyB = j.bodyB == NO_BODY ? j.bodyA : j.bodyB; r.index = i;
                 r.ax = j.anchorAx; r.ay = j.anchorAy; r.bx = j.anchorBx; r.by = j.anchorBy;
@@ -2269,17 +2272,27 @@ struct ag2d_world {
                     r.p[4] = j.lowerLimit; r.p[5] = j.upperLimit; r.p[6] = j.referenceAngle;
                     r.flags = j.enableLimit ? 1u : 0u;
                 }
-                recs[fill[level[i - begin]]++] = r;
+                recs.push_back(r);
+                at.push_back(fill[level[i - begin]]++);
             }
             jointActive[k] = end - begin;
             jointLevels[k] = levels;
             jointLevelHost[k].assign(start.begin() + 1, start.end());   // level l (from 1) starts at [l - 1]
-            jointRec[k].upload(recs.data(), recs.size(), s);
-            jointFlow[k].upload(flow.data(), flow.size(), s);
             jointLevel[k].upload(jointLevelHost[k].data(), jointLevelHost[k].size(), s);
             jointData[k].reserve(std::max<size_t>(recs.size(), 1));
         }
+        // The dataflow takes constraints in dense order (a warp's are then neighbours in a user's chains and grids, so
+        // that early links run ahead into the next iteration); the barriers take whole levels.
         jointBodies = flowFits ? uint32_t(bodies.size()) : 0u;
+        for (uint32_t k = 0; k < JOINT_KINDS; k++) {
+            if (!jointBodies) {
+                std::vector<JointRec> byLevel(recsOf[k].size());
+                for (size_t i = 0; i < byLevel.size(); i++) byLevel[levelMajor[k][i]] = recsOf[k][i];
+                recsOf[k].swap(byLevel);
+            }
+            jointRec[k].upload(recsOf[k].data(), recsOf[k].size(), s);
+            jointFlow[k].upload(flowOf[k].data(), jointBodies ? flowOf[k].size() : 0, s);
+        }
         jointBody.upload(bodies.data(), flowFits ? bodies.size() : 0u, s);
         auto& motors = objects.jointSystems[JOINT_MOTOR].joints;
         std::vector<float> imp(motors.size());

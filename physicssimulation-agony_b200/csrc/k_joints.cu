@@ -20,6 +20,8 @@
 // s2 target speed, s3 max impulse, s4 impulse.
 #include "ag2d_kernels.cuh"
 
+#include <type_traits>
+
 namespace ag2d {
 
 namespace {
@@ -382,16 +384,19 @@ __device__ __forceinline__ void word_store(float4* p, float x, float y, float z,
 // type's constraints on it) and nothing else, so iterations follow one another down a chain like waves. Threads take
 // constraints in that order and all are resident, so the oldest one can always go. The order of every body's updates
 // is the dense order's, the results are the same bit for bit.
-// Bound: the longest chain of updates, a few hundred cycles each in shared memory. With a block barrier after every
-// level of every type and iteration, and the velocities in global memory, 960 revolute joints in chains of twelve,
-// 240 motors and 316 springs (eight iterations: 130 levels) took 350 us a step.
+// Bound: the longest chain of updates, some 700 cycles each (a poll, the two words, the solve, two stores). Measured on
+// 80 chains of 12 revolute joints with 240 motors and 316 springs between neighbouring chains, eight iterations (92
+// levels an iteration), a step's constraints: 350 us with a block barrier after every level and the velocities in
+// global memory; 222 us as a dataflow in level order, a warp's share of one type far from its share of the next, so
+// that iterations followed one another end to end; 104 us in dense order and equal shares of each type. Sleeping in the
+// polls gave nothing.
 __global__ void __launch_bounds__(JOINT_THREADS) k_joints_flow(DeviceWorld w, JointLaunch L)
 {
     extern __shared__ float4 jointSmem[];
     float4* const vel = jointSmem;                                            // [bodies] vx, vy, w, version
     JointBody* const body = reinterpret_cast<JointBody*>(vel + L.bodies);     // [bodies]
     float2* const mass = reinterpret_cast<float2*>(body + L.bodies);          // [bodies] inverse mass, inverse inertia
-    compute_tick(w, L);
+    compute_tick(w, L);   // the block's barrier below hands the data to the warps that solve with it
     for (uint32_t i = threadIdx.x; i < L.bodies; i += blockDim.x) {
         const JointBody b = L.body[i];
         const float4 v = w.bvel[b.body];
@@ -400,15 +405,18 @@ __global__ void __launch_bounds__(JOINT_THREADS) k_joints_flow(DeviceWorld w, Jo
         vel[i] = make_float4(v.x, v.y, v.z, __uint_as_float(0u));
     }
     __syncthreads();
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t done[JOINT_KINDS_DEVICE], rest[JOINT_KINDS_DEVICE];   // iterations made, and the interleaving's remainder
-    for (uint32_t k = 0; k < JOINT_KINDS_DEVICE; k++) { done[k] = 0; rest[k] = 0; }
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    uint32_t done[JOINT_KINDS_DEVICE] = {}, rest[JOINT_KINDS_DEVICE] = {};   // iterations made; interleaving's remainder
     bool gone = false;
-    // One type's pass: this warp's stretches of 32 constraints.
-    auto pass = [&](uint32_t k, bool warm) {
-        for (uint32_t first = threadIdx.x & ~31u; first < L.count[k] && !gone; first += blockDim.x) {
+    // One type's pass: this warp's share of the dense order. Every type is split in the same proportions, so that what
+    // one warp waits for in one type is near what it waits for in the next, and a warp at the head of a long chain can
+    // be iterations ahead of one at its tail.
+    auto pass = [&](auto kind, bool warm) {
+        constexpr uint32_t k = kind.value;
+        const uint32_t end = uint32_t(uint64_t(L.count[k]) * (warp + 1u) / warps);
+        for (uint32_t first = uint32_t(uint64_t(L.count[k]) * warp / warps); first < end && !gone; first += 32u) {
             const uint32_t i = first + lane;
-            bool todo = i < L.count[k];
+            bool todo = i < end;
             JointFlow f{};
             JointData d;
             uint32_t index = 0, needA = 0, needB = 0;
@@ -425,6 +433,7 @@ __global__ void __launch_bounds__(JOINT_THREADS) k_joints_flow(DeviceWorld w, Jo
                 dynB = bB.moves != 0 && k != K_MOTOR;
                 needA = f.rankA;
                 needB = f.rankB;
+#pragma unroll
                 for (uint32_t t = 0; t < JOINT_KINDS_DEVICE; t++) {
                     needA += done[t] * bA.degree[t];
                     needB += done[t] * bB.degree[t];
@@ -455,16 +464,24 @@ __global__ void __launch_bounds__(JOINT_THREADS) k_joints_flow(DeviceWorld w, Jo
     };
     // Warm start: the motors (the one type with a warm start); then the velocity iterations, the types interleaved in
     // ConstraintType order.
-    pass(K_MOTOR, true);
+    pass(std::integral_constant<uint32_t, K_MOTOR>{}, true);
     done[K_MOTOR] = 1;
-    for (uint32_t it = 0; it < L.maxIterations && !gone; it++)
-        for (uint32_t k = 0; k < JOINT_KINDS_DEVICE; k++) {
-            rest[k] += L.iterations[k];
-            if (L.count[k] == 0 || rest[k] < L.maxIterations) continue;
-            rest[k] -= L.maxIterations;
-            pass(k, false);
-            done[k]++;
-        }
+    auto turn = [&](auto kind) {
+        constexpr uint32_t k = kind.value;
+        rest[k] += L.iterations[k];
+        if (L.count[k] == 0 || rest[k] < L.maxIterations) return;
+        rest[k] -= L.maxIterations;
+        pass(kind, false);
+        done[k]++;
+    };
+    static_assert(K_SPRING == 0 && K_REVOLUTE == 1 && K_PRISMATIC == 2 && K_SLIDER == 3 && K_MOTOR == 4, "order");
+    for (uint32_t it = 0; it < L.maxIterations && !gone; it++) {
+        turn(std::integral_constant<uint32_t, K_SPRING>{});
+        turn(std::integral_constant<uint32_t, K_REVOLUTE>{});
+        turn(std::integral_constant<uint32_t, K_PRISMATIC>{});
+        turn(std::integral_constant<uint32_t, K_SLIDER>{});
+        turn(std::integral_constant<uint32_t, K_MOTOR>{});
+    }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < L.bodies; i += blockDim.x)
         if (body[i].moves) w.bvel[body[i].body] = make_float4(vel[i].x, vel[i].y, vel[i].z, mass[i].x);
