@@ -7,8 +7,9 @@
 namespace ag2d {
 
 constexpr uint32_t SORT_THREADS = 256;
-constexpr uint32_t SORT_ITEMS = 16;
-constexpr uint32_t SORT_TILE = SORT_THREADS * SORT_ITEMS;   // keys per onesweep tile
+// Keys a thread of the sort: few while that leaves an SM at most a few tiles, many above (fewer tiles to look back over).
+constexpr uint32_t SORT_ITEMS_SMALL = 4, SORT_ITEMS_LARGE = 16;
+constexpr uint32_t SORT_SMALL_MAX = 300000;
 constexpr uint32_t SCAN_THREADS = 256;
 constexpr uint32_t SCAN_ITEMS = 8;
 constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
@@ -101,29 +102,32 @@ __global__ void k_collider_pose(DeviceWorld w, const uint32_t* list, const uint8
                                 const uint32_t* worldMask, WarmTable insert);
 __global__ void k_bounds_init(uint32_t* bounds, uint32_t worlds);
 __global__ void k_bounds(const float4* aabb, const uint32_t* list, uint32_t n, const uint32_t* colWorld,
-                         uint32_t* bounds);
+                         uint32_t* bounds, float4* parts, uint32_t* clear, uint32_t clearWords);
 __global__ void k_count_world(const uint32_t* list, uint32_t n, const uint32_t* elemWorld, uint32_t* counts);
 __global__ void k_simd_flags(const uint32_t* list, uint32_t n, const uint32_t* offsets, uint32_t nElems,
                              const uint32_t* elemWorld, const uint32_t* worldStart, uint32_t worlds, uint8_t* simd);
 __global__ void k_morton(const float4* aabb, const uint32_t* list, uint32_t n, const uint32_t* colWorld,
-                         const uint32_t* bounds, uint32_t* keys, uint32_t* vals, uint32_t* keyOf);
-__global__ void k_world_keys(const uint32_t* vals, uint32_t n, const uint32_t* colWorld, uint32_t* keys);
+                         const uint32_t* bounds, const float4* parts, uint32_t nParts, uint32_t* keys, uint32_t* vals,
+                         uint32_t* keyOf, uint32_t* hist, uint32_t* done);
+__global__ void k_world_keys(const uint32_t* vals, uint32_t n, const uint32_t* colWorld, uint32_t* keys, uint32_t* hist,
+                             uint32_t* done);
 __global__ void k_seg_starts(const uint32_t* offsets, const uint32_t* worldStart, uint32_t worlds, uint32_t nElems,
                              const uint32_t* total, uint32_t* segStart);
 __global__ void k_manifold_segments(const Manifold* m, const uint32_t* nM, const uint32_t* cbody,
                                     const uint32_t* bodyWorld, uint32_t worlds, uint32_t* segStart);
 __global__ void k_tree_gather(const uint32_t* vals, uint32_t n, const uint32_t* keyOf, const uint32_t* colWorld,
                               const float4* caabb, uint32_t* sortedKey, uint32_t* sortedWorld, float4* leafAabb);
-__global__ void k_sort_histogram(const uint32_t* keys, uint32_t n, uint32_t* hist);
-__global__ void k_sort_digit_scan(uint32_t* hist);
-__global__ void k_sort_pass(const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut, uint32_t* valsOut,
-                            uint32_t n, uint32_t shift, const uint32_t* digitBase, uint32_t* tileState,
-                            uint32_t* tileCounter, uint32_t* status);
+// Host side: tiles of a sort pass over n keys, and one pass. digitBase: the digits' exclusive scan; tileState [tiles x
+// 256] and tileCounter zeroed before the launch.
+uint32_t sort_tiles(uint32_t n);
+cudaError_t launch_sort_pass(const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut, uint32_t* valsOut,
+                             uint32_t n, uint32_t shift, const uint32_t* digitBase, uint32_t* tileState,
+                             uint32_t* tileCounter, uint32_t* status, cudaStream_t stream);
 // Trees of up to TREE_SEGMENT_MAX leaves are built by one CTA each (k_tree_segments), in size classes.
 constexpr uint32_t TREE_SEGMENT_MAX = 16384;
-// A single tree of more leaves is built by the whole GPU in a dozen launches: 108 us at 6,000 and at 8,000 leaves,
-// where one CTA takes 89 and 113 us (40 against 95 at 2,000).
-constexpr uint32_t TREE_SINGLE_MAX = 7168;
+// A single tree of more leaves is built by the whole GPU in eight launches: 75 us at 6,000 and 77 at 8,000 leaves,
+// where one CTA takes 85 and 113 (57 at 4,000).
+constexpr uint32_t TREE_SINGLE_MAX = 5120;
 struct TreeBuild {
     const float4* caabb;
     const uint32_t* list;       // colliders, world-grouped
@@ -144,7 +148,7 @@ cudaError_t launch_tree_segments(const TreeBuild& t, uint32_t largest, uint32_t 
 // Host side: raises the builders' dynamic shared-memory limit (once per device).
 cudaError_t tree_segments_init();
 __global__ void k_lbvh_build(const uint32_t* keys, const uint32_t* sortedWorld, const uint32_t* segStart, int n,
-                             int2* child, int* parent, int* leafParent, float4* meet, NodeRec* rec);
+                             const uint32_t* vals, const float4* caabb, float4* leafAabb, int2* child, int* parent, int* leafParent, float4* meet, NodeRec* rec);
 __global__ void k_lbvh_refit(int n, const int2* child, const int* parent, const int* leafParent,
                              const float4* leafAabb, float4* nodeAabb, float4* meet, NodeRec* rec);
 // Empty marker of a refit meeting slot (min x bits): a NaN no arithmetic produces.

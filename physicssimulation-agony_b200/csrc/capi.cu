@@ -172,9 +172,15 @@ struct Tree {
     DBuf<float4> leafAabb, nodeAabb;
     DBuf<NodeRec> rec;
     DBuf<float4> meet;   // refit meeting slots: one per internal node, or (one CTA a tree) two per split
-    DBuf<uint32_t> bounds, hist, tileState, tileCounter;
+    DBuf<uint32_t> bounds;
+    DBuf<float4> parts;          // one world: bounds of each block's colliders
+    DBuf<uint32_t> sortWords;    // SortWords
     // World-segmented trees: Morton key per collider, sorted keys / worlds, segment starts (filled with the lists).
     DBuf<uint32_t> keyOf, sortedKey, sortedWorld, segStart;
+    // Words of a build's two sorts (Morton keys, then worlds), zeroed by its first kernel: two sets of four digit
+    // histograms, eight tile counters, two counts of finished blocks, and the tile states of up to eight passes.
+    static constexpr uint32_t SORT_COUNTERS = 2 * 4 * 256, SORT_DONE = SORT_COUNTERS + 8, SORT_HEAD = SORT_DONE + 8;
+    static constexpr uint32_t MAX_PARTS = 1024;
     uint32_t worlds = 1;
     int n = 0;
     void reserve(uint32_t cap, uint32_t nWorlds)
@@ -183,8 +189,10 @@ struct Tree {
         keys.reserve(cap); vals.reserve(cap); keys2.reserve(cap); vals2.reserve(cap);
         child.reserve(cap); parent.reserve(cap); leafParent.reserve(cap);
         leafAabb.reserve(cap); nodeAabb.reserve(cap); meet.reserve(2 * size_t(cap)); rec.reserve(cap);
-        bounds.reserve(4 * size_t(nWorlds)); hist.reserve(4 * 256); tileCounter.reserve(4);
-        tileState.reserve(size_t(div_up(std::max<uint32_t>(cap, 1), SORT_TILE)) * 256 * 4);
+        bounds.reserve(4 * size_t(nWorlds)); parts.reserve(MAX_PARTS);
+        // The most tiles of any size up to the capacity are those of the largest size with small tiles, or its own.
+        const uint32_t tiles = std::max(sort_tiles(std::max<uint32_t>(cap, 1)), sort_tiles(std::min(cap, SORT_SMALL_MAX)));
+        sortWords.reserve(SORT_HEAD + size_t(tiles) * 256 * (nWorlds > 1 ? 8 : 4));
         if (nWorlds > 1) {
             keyOf.reserve(cap); sortedKey.reserve(cap); sortedWorld.reserve(cap); segStart.reserve(nWorlds + 1);
         }
@@ -1795,24 +1803,17 @@ struct ag2d_world {
         launches++;
     }
 
-    // Radix passes over (keys, vals) for the digits [0, passes) with one histogram pass; the result ends in
-    // t.keys / t.vals (buffers swap after an odd number of passes).
-    void sortPasses(Tree& t, uint32_t n, uint32_t passes)
+    // Radix passes over (keys, vals) for the digits [0, passes), whose histograms the kernel before left scanned in the
+    // build's set 'round'; the result ends in t.keys / t.vals (buffers swap after an odd number of passes).
+    void sortPasses(Tree& t, uint32_t n, uint32_t round, uint32_t passes)
     {
-        const cudaStream_t s = stream;
-        CK(cudaMemsetAsync(t.hist.p, 0, 4 * 256 * sizeof(uint32_t), s));
-        k_sort_histogram<<<gridFor(n), 256, 0, s>>>(t.keys.p, n, t.hist.p);
-        k_sort_digit_scan<<<4, 256, 0, s>>>(t.hist.p);
-        CK(cudaGetLastError());
-        const uint32_t tiles = div_up(n, SORT_TILE);
-        CK(cudaMemsetAsync(t.tileState.p, 0, size_t(tiles) * 256 * passes * sizeof(uint32_t), s));
-        CK(cudaMemsetAsync(t.tileCounter.p, 0, 4 * sizeof(uint32_t), s));
+        const uint32_t tiles = sort_tiles(n);
         uint32_t *ki = t.keys.p, *vi = t.vals.p, *ko = t.keys2.p, *vo = t.vals2.p;
         for (uint32_t pass = 0; pass < passes; pass++) {
-            k_sort_pass<<<tiles, SORT_THREADS, 0, s>>>(ki, vi, ko, vo, n, pass * 8, t.hist.p + pass * 256,
-                                                        t.tileState.p + size_t(pass) * tiles * 256,
-                                                        t.tileCounter.p + pass, &dCounters.p->status);
-            CK(cudaGetLastError());
+            const uint32_t slot = 4 * round + pass;
+            CK(launch_sort_pass(ki, vi, ko, vo, n, pass * 8, t.sortWords.p + slot * 256,
+                                t.sortWords.p + Tree::SORT_HEAD + size_t(slot) * tiles * 256,
+                                t.sortWords.p + Tree::SORT_COUNTERS + slot, &dCounters.p->status, stream));
             std::swap(ki, ko);
             std::swap(vi, vo);
         }
@@ -1820,7 +1821,7 @@ struct ag2d_world {
             swap_bufs(t.keys, t.keys2);
             swap_bufs(t.vals, t.vals2);
         }
-        launches += 2 + passes;
+        launches += passes;
     }
 
     // Tree over the colliders of 'list' (Morton keys from the world's bounds, sorted, Karras build, refit). With
@@ -1847,37 +1848,44 @@ struct ag2d_world {
             launches += count;
             return;
         }
-        launches += 5 + (n > 1 ? 1 : 0);
-        k_bounds_init<<<gridFor(W), 256, 0, s>>>(t.bounds.p, W);
-        k_bounds<<<gridFor(n), 256, 0, s>>>(caabb.p, list, n, cw, t.bounds.p);
-        k_morton<<<gridFor(n), 256, 0, s>>>(caabb.p, list, n, cw, t.bounds.p, t.keys.p, t.vals.p,
-                                             seg ? t.keyOf.p : nullptr);
-        CK(cudaGetLastError());
-        if (isDyn) pbegin(12);
-        sortPasses(t, n, 4);
+        // Stable passes on the world id after the Morton ones: order (world, Morton key, collider).
+        uint32_t worldPasses = seg ? 1 : 0;
+        while (seg && worldPasses < 4 && (W - 1) >> (8 * worldPasses)) worldPasses++;
+        const uint32_t parts = seg ? gridFor(n) : std::min<uint32_t>({gridFor(n), 2 * uint32_t(dev.sms), Tree::MAX_PARTS});
+        const uint32_t words = Tree::SORT_HEAD + sort_tiles(n) * 256 * (4 + worldPasses);
         if (seg) {
-            // Stable passes on the world id: order (world, Morton key, collider).
-            uint32_t passes = 1;
-            while (passes < 4 && (W - 1) >> (8 * passes)) passes++;
-            k_world_keys<<<gridFor(n), 256, 0, s>>>(t.vals.p, n, colWorld.p, t.keys.p);
+            k_bounds_init<<<gridFor(W), 256, 0, s>>>(t.bounds.p, W);
+            launches++;
+        }
+        k_bounds<<<parts, 256, 0, s>>>(caabb.p, list, n, cw, t.bounds.p, t.parts.p, t.sortWords.p, words);
+        k_morton<<<gridFor(n), 256, 0, s>>>(caabb.p, list, n, cw, t.bounds.p, t.parts.p, parts, t.keys.p, t.vals.p,
+                                             seg ? t.keyOf.p : nullptr, t.sortWords.p,
+                                             t.sortWords.p + Tree::SORT_DONE);
+        CK(cudaGetLastError());
+        launches += 4;
+        if (isDyn) pbegin(12);
+        sortPasses(t, n, 0, 4);
+        if (seg) {
+            k_world_keys<<<gridFor(n), 256, 0, s>>>(t.vals.p, n, colWorld.p, t.keys.p, t.sortWords.p + 4 * 256,
+                                                     t.sortWords.p + Tree::SORT_DONE + 1);
             CK(cudaGetLastError());
             launches++;
-            sortPasses(t, n, passes);
+            sortPasses(t, n, 1, worldPasses);
         }
         if (isDyn) pend(12);
         if (isDyn) pbegin(13);
-        k_tree_gather<<<gridFor(n), 256, 0, s>>>(t.vals.p, n, seg ? t.keyOf.p : nullptr, cw, caabb.p,
-                                                  seg ? t.sortedKey.p : nullptr, seg ? t.sortedWorld.p : nullptr,
-                                                  t.leafAabb.p);
-        k_lbvh_build<<<gridFor(n), 256, 0, s>>>(seg ? t.sortedKey.p : t.keys.p, seg ? t.sortedWorld.p : nullptr,
-                                                 seg ? t.segStart.p : nullptr, int(n), t.child.p,
-                                                 t.parent.p, t.leafParent.p, t.meet.p, t.rec.p);
-        CK(cudaGetLastError());
-        if (n > 1) {
-            k_lbvh_refit<<<gridFor(n), 256, 0, s>>>(int(n), t.child.p, t.parent.p, t.leafParent.p, t.leafAabb.p,
-                                                     t.nodeAabb.p, t.meet.p, t.rec.p);
-            CK(cudaGetLastError());
+        if (seg) {
+            k_tree_gather<<<gridFor(n), 256, 0, s>>>(t.vals.p, n, t.keyOf.p, cw, caabb.p, t.sortedKey.p,
+                                                      t.sortedWorld.p, t.leafAabb.p);
+            launches++;
         }
+        k_lbvh_build<<<gridFor(n), 256, 0, s>>>(seg ? t.sortedKey.p : t.keys.p, seg ? t.sortedWorld.p : nullptr,
+                                                 seg ? t.segStart.p : nullptr, int(n), t.vals.p, caabb.p,
+                                                 t.leafAabb.p, t.child.p, t.parent.p, t.leafParent.p, t.meet.p,
+                                                 t.rec.p);
+        k_lbvh_refit<<<gridFor(n), 256, 0, s>>>(int(n), t.child.p, t.parent.p, t.leafParent.p, t.leafAabb.p,
+                                                 t.nodeAabb.p, t.meet.p, t.rec.p);
+        CK(cudaGetLastError());
         if (isDyn) pend(13);
     }
 

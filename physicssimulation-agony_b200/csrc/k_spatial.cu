@@ -206,44 +206,47 @@ __global__ void k_collider_pose(DeviceWorld w, const uint32_t* __restrict__ list
 // min/max are order-independent, so a block reduction plus ordered-integer atomics gives the sequential result
 // (up to the sign of a zero bound).
 // ---------------------------------------------------------------------------------------------------------------
-// Per world (4 ordered words each). A warp whose lanes all belong to one world reduces first and issues one atomic
-// per word; a warp that straddles worlds issues per-lane atomics.
+// The union of a block's boxes (blocks of at most 32 warps), valid in thread 0.
+__device__ __forceinline__ float4 block_bounds(float mnx, float mny, float mxx, float mxy)
+{
+    for (int o = 16; o > 0; o >>= 1) {
+        mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
+        mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
+        mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
+        mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+    }
+    __shared__ float4 part[32];
+    const uint32_t warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
+    if ((threadIdx.x & 31) == 0) part[warp] = make_float4(mnx, mny, mxx, mxy);
+    __syncthreads();
+    float4 r = part[0];
+    if (threadIdx.x == 0)
+        for (uint32_t k = 1; k < warps; k++) {
+            const float4 q = part[k];
+            r = make_float4(fminf(r.x, q.x), fminf(r.y, q.y), fmaxf(r.z, q.z), fmaxf(r.w, q.w));
+        }
+    return r;
+}
+
+// One world: every block leaves the bounds of its colliders in parts[block] (k_morton's blocks reduce them). Several
+// worlds: 4 ordered words each; a warp whose lanes all belong to one world reduces first and issues one atomic per
+// word, a warp that straddles worlds issues per-lane atomics. The sort's words are cleared beside it.
 __global__ void k_bounds(const float4* __restrict__ aabb, const uint32_t* __restrict__ list, uint32_t n,
-                         const uint32_t* __restrict__ colWorld, uint32_t* __restrict__ bounds)
+                         const uint32_t* __restrict__ colWorld, uint32_t* __restrict__ bounds,
+                         float4* __restrict__ parts, uint32_t* __restrict__ clear, uint32_t clearWords)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t base0 = blockIdx.x * blockDim.x;
+    for (uint32_t i = base0 + threadIdx.x; i < clearWords; i += stride) clear[i] = 0u;
     if (!colWorld) {
-        // One world: per-thread running bounds over the grid-stride loop, then one block reduction and four
-        // atomics per block (per-warp atomics on four addresses serialise at one L2 slice for large n).
         float mnx = FLT_MAX, mny = FLT_MAX, mxx = -FLT_MAX, mxy = -FLT_MAX;
         for (uint32_t k = base0 + threadIdx.x; k < n; k += stride) {
             const float4 a = aabb[list ? list[k] : k];
             mnx = fminf(mnx, a.x); mny = fminf(mny, a.y); mxx = fmaxf(mxx, a.z); mxy = fmaxf(mxy, a.w);
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-            mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-            mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-            mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-        }
-        __shared__ float4 part[32];
-        const uint32_t warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
-        if ((threadIdx.x & 31) == 0) part[warp] = make_float4(mnx, mny, mxx, mxy);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float4 r = part[0];
-            for (uint32_t k = 1; k < warps; k++) {
-                const float4 q = part[k];
-                r = make_float4(fminf(r.x, q.x), fminf(r.y, q.y), fmaxf(r.z, q.z), fmaxf(r.w, q.w));
-            }
-            if (r.x <= r.z) {   // the block saw at least one collider
-                atomicMin(bounds + 0, float_to_ordered(r.x));
-                atomicMin(bounds + 1, float_to_ordered(r.y));
-                atomicMax(bounds + 2, float_to_ordered(r.z));
-                atomicMax(bounds + 3, float_to_ordered(r.w));
-            }
-        }
+        const float4 r = block_bounds(mnx, mny, mxx, mxy);
+        if (threadIdx.x == 0)   // a block that saw no collider leaves neutral bounds
+            parts[blockIdx.x] = r.x <= r.z ? r : make_float4(FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX);
         return;
     }
     for (uint32_t base = base0; base < n; base += stride) {
@@ -340,28 +343,99 @@ __device__ __forceinline__ uint32_t morton_key(const float4& a, float bminX, flo
     return (part1by1(uint32_t(ty)) << 1) | part1by1(uint32_t(tx));
 }
 
-__global__ void k_morton(const float4* __restrict__ aabb, const uint32_t* __restrict__ list, uint32_t n,
-                         const uint32_t* __restrict__ colWorld, const uint32_t* __restrict__ bounds,
-                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* __restrict__ keyOf)
+// Keys of a radix sort's digit histograms, counted in shared memory ('sh', zeroed, 4 x 256) by blocks of 256 threads and
+// added to 'hist' at the end; the last block to finish turns each histogram into its exclusive scan.
+__device__ __forceinline__ void digits_count(uint32_t* sh, uint32_t k)
 {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    atomicAdd(&sh[0 * 256 + (k & 0xFF)], 1u);
+    atomicAdd(&sh[1 * 256 + ((k >> 8) & 0xFF)], 1u);
+    atomicAdd(&sh[2 * 256 + ((k >> 16) & 0xFF)], 1u);
+    atomicAdd(&sh[3 * 256 + (k >> 24)], 1u);
+}
+__device__ __forceinline__ void digits_end(const uint32_t* sh, uint32_t* hist, uint32_t* done)
+{
+    __shared__ uint32_t warpSum[8], lastBlock;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    __syncthreads();
+    for (uint32_t i = t; i < 4 * 256; i += 256)
+        if (sh[i]) atomicAdd(&hist[i], sh[i]);
+    __threadfence();
+    __syncthreads();
+    if (t == 0) lastBlock = atomicAdd(done, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!lastBlock) return;
+    __threadfence();
+    for (uint32_t j = 0; j < 4; j++) {
+        const uint32_t v = __ldcg(hist + j * 256 + t);
+        uint32_t incl = v;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+        }
+        if (lane == 31) warpSum[warp] = incl;
+        __syncthreads();
+        for (uint32_t k = 0; k < warp; k++) incl += warpSum[k];
+        hist[j * 256 + t] = incl - v;
+        __syncthreads();
+    }
+}
+
+// Morton keys with the digit histograms of their sort (blocks of 256 threads). One world: the bounds are the union of
+// parts[0, nParts), reduced by every block.
+__global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ aabb, const uint32_t* __restrict__ list,
+                                                uint32_t n, const uint32_t* __restrict__ colWorld,
+                                                const uint32_t* __restrict__ bounds,
+                                                const float4* __restrict__ parts, uint32_t nParts,
+                                                uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                uint32_t* __restrict__ keyOf, uint32_t* hist, uint32_t* done)
+{
+    __shared__ uint32_t sh[4 * 256];
+    __shared__ float4 whole;
+    for (uint32_t i = threadIdx.x; i < 4 * 256; i += 256) sh[i] = 0;
+    if (!colWorld) {
+        float mnx = FLT_MAX, mny = FLT_MAX, mxx = -FLT_MAX, mxy = -FLT_MAX;
+        for (uint32_t k = threadIdx.x; k < nParts; k += 256) {
+            const float4 a = parts[k];
+            mnx = fminf(mnx, a.x); mny = fminf(mny, a.y); mxx = fmaxf(mxx, a.z); mxy = fmaxf(mxy, a.w);
+        }
+        const float4 r = block_bounds(mnx, mny, mxx, mxy);
+        if (threadIdx.x == 0) whole = r;
+    }
+    __syncthreads();
+    for (uint32_t k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256) {
         const uint32_t c = list ? list[k] : k;
-        const uint32_t* b = bounds + 4 * (colWorld ? colWorld[c] : 0u);
-        const uint32_t key = morton_key(aabb[c], ordered_to_float(b[0]), ordered_to_float(b[1]), ordered_to_float(b[2]),
-                                        ordered_to_float(b[3]));
+        float4 b;
+        if (colWorld) {
+            const uint32_t* const words = bounds + 4 * colWorld[c];
+            b = make_float4(ordered_to_float(words[0]), ordered_to_float(words[1]), ordered_to_float(words[2]),
+                            ordered_to_float(words[3]));
+        } else {
+            b = whole;
+        }
+        const uint32_t key = morton_key(aabb[c], b.x, b.y, b.z, b.w);
         keys[k] = key;
         vals[k] = c;
         if (keyOf) keyOf[c] = key;
+        digits_count(sh, key);
     }
+    digits_end(sh, hist, done);
 }
 
 // After the Morton passes: the world id of each sorted element becomes the key of the next (stable) passes, so the
 // final order is by (world, Morton key) with ties in collider order.
-__global__ void k_world_keys(const uint32_t* __restrict__ vals, uint32_t n, const uint32_t* __restrict__ colWorld,
-                             uint32_t* __restrict__ keys)
+__global__ void __launch_bounds__(256) k_world_keys(const uint32_t* __restrict__ vals, uint32_t n,
+                                                    const uint32_t* __restrict__ colWorld,
+                                                    uint32_t* __restrict__ keys, uint32_t* hist, uint32_t* done)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        keys[i] = colWorld[vals[i]];
+    __shared__ uint32_t sh[4 * 256];
+    for (uint32_t i = threadIdx.x; i < 4 * 256; i += 256) sh[i] = 0;
+    __syncthreads();
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const uint32_t wd = colWorld[vals[i]];
+        keys[i] = wd;
+        digits_count(sh, wd);
+    }
+    digits_end(sh, hist, done);
 }
 
 // First index of every world's segment of a world-grouped list: segStart[w] = offsets[worldStart[w]] (the exclusive
@@ -390,7 +464,8 @@ __global__ void k_manifold_segments(const Manifold* __restrict__ m, const uint32
     }
 }
 
-// Sorted-order gathers for the tree: Morton key (after the world passes), world id and AABB of every leaf.
+// Sorted-order gathers for the trees of several worlds: Morton key (after the world passes), world id and AABB of every
+// leaf.
 __global__ void k_tree_gather(const uint32_t* __restrict__ vals, uint32_t n, const uint32_t* __restrict__ keyOf,
                               const uint32_t* __restrict__ colWorld, const float4* __restrict__ caabb,
                               uint32_t* __restrict__ sortedKey, uint32_t* __restrict__ sortedWorld,
@@ -398,36 +473,19 @@ __global__ void k_tree_gather(const uint32_t* __restrict__ vals, uint32_t n, con
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t c = vals[i];
-        if (keyOf) sortedKey[i] = keyOf[c];
-        if (colWorld) sortedWorld[i] = colWorld[c];
+        sortedKey[i] = keyOf[c];
+        sortedWorld[i] = colWorld[c];
         leafAabb[i] = caabb[c];
     }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
 // Onesweep LSD radix sort of (key, value) pairs, 8-bit digits, stable: the same permutation as
-// BvhTree::sortByMortonCodes (BvhTree.cpp:282-354). One histogram pass for all four digits, then per digit one
-// kernel that ranks a 4096-key tile (warp match-any ranking, striped so ranks follow input order), resolves the
-// tile's global digit offsets by decoupled look-back over the preceding tiles, reorders the tile in shared
-// memory and writes each digit's run contiguously.
+// BvhTree::sortByMortonCodes (BvhTree.cpp:282-354). The kernel that makes the keys counts all four digits; then per
+// digit one kernel ranks a tile (per warp, striped so ranks follow input order), resolves the tile's global digit
+// offsets by decoupled look-back over the preceding tiles, reorders the tile in shared memory and writes each digit's
+// run contiguously.
 // ---------------------------------------------------------------------------------------------------------------
-__global__ void k_sort_histogram(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* __restrict__ hist)
-{
-    __shared__ uint32_t sh[4 * 256];
-    for (uint32_t i = threadIdx.x; i < 4 * 256; i += blockDim.x) sh[i] = 0;
-    __syncthreads();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t k = keys[i];
-        atomicAdd(&sh[0 * 256 + (k & 0xFF)], 1u);
-        atomicAdd(&sh[1 * 256 + ((k >> 8) & 0xFF)], 1u);
-        atomicAdd(&sh[2 * 256 + ((k >> 16) & 0xFF)], 1u);
-        atomicAdd(&sh[3 * 256 + (k >> 24)], 1u);
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < 4 * 256; i += blockDim.x)
-        if (sh[i]) atomicAdd(&hist[i], sh[i]);
-}
-
 // The lanes of a full warp that hold the same 8-bit digit as this one (among the valid): one ballot a bit. match.any
 // serves one distinct value after the other, and the digits of a warp mostly differ: with it the ranking of 2,000 keys
 // in one CTA took 4,100 cycles a pass.
@@ -443,29 +501,13 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool valid)
     return peers;
 }
 
-// In-place exclusive scan of each 256-bin digit histogram; launched with 4 blocks of 256 threads.
-__global__ void k_sort_digit_scan(uint32_t* hist)
-{
-    __shared__ uint32_t s[256];
-    uint32_t* h = hist + blockIdx.x * 256;
-    const uint32_t t = threadIdx.x;
-    s[t] = h[t];
-    __syncthreads();
-    for (uint32_t o = 1; o < 256; o <<= 1) {
-        const uint32_t v = t >= o ? s[t - o] : 0u;
-        __syncthreads();
-        s[t] += v;
-        __syncthreads();
-    }
-    h[t] = s[t] - h[t];
-}
-
+template <uint32_t SORT_ITEMS>
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
     const uint32_t* __restrict__ keysIn, const uint32_t* __restrict__ valsIn, uint32_t* __restrict__ keysOut,
     uint32_t* __restrict__ valsOut, uint32_t n, uint32_t shift, const uint32_t* __restrict__ digitBase,
     uint32_t* __restrict__ tileState, uint32_t* __restrict__ tileCounter, uint32_t* __restrict__ status)
 {
-    constexpr uint32_t WARPS = SORT_THREADS / 32;
+    constexpr uint32_t WARPS = SORT_THREADS / 32, SORT_TILE = SORT_THREADS * SORT_ITEMS;
     __shared__ uint32_t warpHist[WARPS][256];
     __shared__ uint32_t digitStart[256];     // exclusive scan of the tile's digit counts
     __shared__ uint32_t globalBase[256];     // global output position of the tile's first key of each digit
@@ -587,6 +629,25 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
     }
 }
 
+uint32_t sort_tiles(uint32_t n)
+{
+    const uint32_t tile = SORT_THREADS * (n <= SORT_SMALL_MAX ? SORT_ITEMS_SMALL : SORT_ITEMS_LARGE);
+    return (n + tile - 1) / tile;
+}
+
+cudaError_t launch_sort_pass(const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut, uint32_t* valsOut,
+                             uint32_t n, uint32_t shift, const uint32_t* digitBase, uint32_t* tileState,
+                             uint32_t* tileCounter, uint32_t* status, cudaStream_t stream)
+{
+    if (n <= SORT_SMALL_MAX)
+        k_sort_pass<SORT_ITEMS_SMALL><<<sort_tiles(n), SORT_THREADS, 0, stream>>>(
+            keysIn, valsIn, keysOut, valsOut, n, shift, digitBase, tileState, tileCounter, status);
+    else
+        k_sort_pass<SORT_ITEMS_LARGE><<<sort_tiles(n), SORT_THREADS, 0, stream>>>(
+            keysIn, valsIn, keysOut, valsOut, n, shift, digitBase, tileState, tileCounter, status);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // Karras LBVH over sorted keys (leaf = one collider). Internal node i spans [first, last] of the sorted order and
 // splits at the highest differing bit; equal keys are ordered by index (key ++ index), as the reference's stable
@@ -627,14 +688,16 @@ __device__ __forceinline__ KarrasNode karras_node(int i, Delta delta)
     return KarrasNode{i < j ? i : j, i < j ? j : i, i + s * d + (d < 0 ? -1 : 0)};
 }
 
-// sortedWorld/segStart null: one segment [0, n).
+// sortedWorld/segStart null: one segment [0, n), and the leaf boxes are gathered beside the build.
 __global__ void k_lbvh_build(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ sortedWorld,
-                             const uint32_t* __restrict__ segStart, int n, int2* __restrict__ child,
-                             int* __restrict__ parent, int* __restrict__ leafParent,
+                             const uint32_t* __restrict__ segStart, int n, const uint32_t* __restrict__ vals,
+                             const float4* __restrict__ caabb, float4* __restrict__ leafAabb,
+                             int2* __restrict__ child, int* __restrict__ parent, int* __restrict__ leafParent,
                              float4* __restrict__ meet, NodeRec* __restrict__ rec)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int lo = 0, hi = n;
+        if (!sortedWorld) leafAabb[i] = caabb[vals[i]];
         if (sortedWorld) {
             const uint32_t wd = sortedWorld[i];
             lo = int(segStart[wd]);
