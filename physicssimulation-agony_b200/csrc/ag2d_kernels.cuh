@@ -254,9 +254,18 @@ constexpr uint32_t NARROW_SMEM_PER_THREAD =
     uint32_t(sizeof(Manifold) + sizeof(uint32_t) + 2 * MAX_POLYGON_VERTICES * sizeof(V2) / NARROW_GROUP);
 // Narrow phase + manifold compaction: manifolds of the hit pairs, in pair order, into out; tileState [tiles + 1] and
 // tileCounter zeroed before the launch (tiles: blockDim.x / 32 x perWarp pairs each, perWarp at most 32).
-__global__ void k_narrow(DeviceWorld w, const uint2* pairs, const uint32_t* nPairs, uint32_t pairCap, Manifold* out,
-                         uint32_t manifoldCap, uint32_t* nOut, StepCounters* counters, uint32_t* tileState,
-                         uint32_t* tileCounter, uint32_t perWarp, WarmTable warm, uint32_t* wakeIsland);
+// The narrow phase; lanes: polygon pairs one a lane where a warp has enough of them (blocks of up to
+// NARROW_LANES_THREADS; a form with more registers, so fewer warps an SM for the other pairs).
+constexpr uint32_t NARROW_LANES_THREADS = 256;   // largest block of the one-pair-a-lane form
+// Polygon pairs of a warp from which on each takes its own lane: the lanes together cost what about three rounds of the
+// groups (four pairs each) do.
+constexpr int NARROW_LANES_PAIRS = 10;
+// Host side: raises the narrow phase's dynamic shared-memory limit (once per device).
+cudaError_t narrow_init();
+void launch_narrow(uint32_t blocks, uint32_t threads, cudaStream_t stream, DeviceWorld w, const uint2* pairs,
+                   const uint32_t* nPairs, uint32_t pairCap, Manifold* out, uint32_t manifoldCap, uint32_t* nOut,
+                   StepCounters* counters, uint32_t* tileState, uint32_t* tileCounter, uint32_t perWarp, bool lanes,
+                   WarmTable warm, uint32_t* wakeIsland);
 __global__ void k_warm_insert(WarmTable t);
 __global__ void k_wake(DeviceWorld w, const Manifold* m, const uint32_t* nM, uint32_t* wakeIsland,
                        StepCounters* counters);

@@ -624,6 +624,93 @@ __device__ __forceinline__ bool collide_polygon_polygon_group(const ColliderView
     return true;
 }
 
+// The same search by one lane, for polygons of at most SAT_LANE_VERTICES vertices: both polygons' vertices in registers
+// (vertex 0 again beyond the last, which changes no minimum), every axis of one against all of the other's without a
+// load. A third of the group's instructions a pair where there are pairs enough to fill the lanes (it spends most of
+// its own on shuffles, shared memory and lanes beyond the vertices), but one pair takes several times as long.
+constexpr uint32_t SAT_LANE_VERTICES = 8;
+
+__device__ __forceinline__ bool collide_polygon_polygon_lane(const ColliderView& A, const ColliderView& B,
+                                                             float& depth, uint32_t& edges)
+{
+    constexpr uint32_t N = SAT_LANE_VERTICES;
+    const float cA = A.c, sAn = A.s, cB = B.c, sBn = B.s;
+    const uint32_t nA = A.nv, nB = B.nv;
+    const V2 rightA = v2(cA, sAn), upA = v2(-sAn, cA);
+    const V2 cd = B.pos - A.pos;
+    const V2 bdl = v2(dot(cd, rightA), dot(cd, upA));
+    const float relCos = cA * cB + sAn * sBn;
+    const float relSin = cA * sBn - sAn * cB;
+    V2 a[N], b[N];
+#pragma unroll
+    for (uint32_t k = 0; k < N; k++) a[k] = k == 0 || k < nA ? ld2(A.verts, k) : a[0];
+#pragma unroll
+    for (uint32_t k = 0; k < N; k++) {
+        if (k == 0 || k < nB) {
+            const V2 v = ld2(B.verts, k);
+            b[k] = v2(bdl.x + relCos * v.x - relSin * v.y, bdl.y + relSin * v.x + relCos * v.y);
+        } else {
+            b[k] = b[0];
+        }
+    }
+    float bov = FLT_MAX, bfac = FLT_MAX;
+    uint32_t bord = 0xFFFFFFFFu;
+    bool separated = false;
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) {
+        if (i >= nA) continue;
+        const V2 ax = ld2(A.normals, i);
+        float minB = FLT_MAX;
+#pragma unroll
+        for (uint32_t j = 0; j < N; j++) minB = fminf(minB, dot(b[j], ax));
+        const float overlap = dot(a[i], ax) - minB;
+        if (overlap < 0.0f) separated = true;
+        const float facing = -dot(ax, bdl);
+        if (sat_better(overlap, facing, i, bov, bfac, bord)) { bov = overlap; bfac = facing; bord = i; }
+    }
+    if (separated) return false;
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) {
+        if (i >= nB) continue;
+        const V2 nb = ld2(B.normals, i);
+        const V2 ax = v2(relCos * nb.x - relSin * nb.y, relSin * nb.x + relCos * nb.y);
+        float minA = FLT_MAX;
+#pragma unroll
+        for (uint32_t j = 0; j < N; j++) minA = fminf(minA, dot(a[j], ax));
+        const float overlap = dot(b[i], ax) - minA;
+        if (overlap < 0.0f) separated = true;
+        const float facing = dot(ax, bdl);
+        const uint32_t ord = MAX_POLYGON_VERTICES + i;
+        if (sat_better(overlap, facing, ord, bov, bfac, bord)) { bov = overlap; bfac = facing; bord = ord; }
+    }
+    if (separated || bord == 0xFFFFFFFFu) return false;
+    const bool refIsA = bord < MAX_POLYGON_VERTICES;
+    const uint32_t bestIndex = refIsA ? bord : bord - MAX_POLYGON_VERTICES;
+    V2 nl;
+    if (refIsA) {
+        nl = ld2(A.normals, bestIndex);
+    } else {
+        const V2 nb = ld2(B.normals, bestIndex);
+        nl = -v2(relCos * nb.x - relSin * nb.y, relSin * nb.x + relCos * nb.y);
+    }
+    const uint32_t incCount = refIsA ? nB : nA;
+    const V2 rnl = refIsA ? nl : -nl;
+    const float2* const incNormals = refIsA ? B.normals : A.normals;
+    float bd = FLT_MAX;
+    uint32_t ie = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) {
+        if (i >= incCount) continue;
+        V2 n = ld2(incNormals, i);
+        if (refIsA) n = v2(relCos * n.x - relSin * n.y, relSin * n.x + relCos * n.y);
+        const float d = dot(rnl, n);
+        if (d < bd) { bd = d; ie = i; }
+    }
+    depth = bov;
+    edges = bord | ie << 8;
+    return true;
+}
+
 // The contact points of a pair that collide_polygon_polygon_group found overlapping: the incident edge clipped to the
 // reference edge's sides.
 __device__ __forceinline__ bool collide_polygon_polygon_clip(const ColliderView& A, const ColliderView& B, float depth,

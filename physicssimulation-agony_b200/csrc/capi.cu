@@ -408,7 +408,7 @@ static DeviceInfo probe_device(int device)
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_color_solve_flow, FLOW_THREADS, 0));
     dev.flowBlocks = std::max(1, perSm) * dev.sms;
     // The narrow phase stages polygons in dynamic shared memory: up to 512 threads x NARROW_SMEM_PER_THREAD.
-    CK(cudaFuncSetAttribute(k_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, int(512 * NARROW_SMEM_PER_THREAD)));
+    CK(narrow_init());
     // AG2D_SOLVER=grid forces the whole-grid solver (test hook for that variant).
     if (const char* v = std::getenv("AG2D_SOLVER")) dev.gridOnly = std::string(v) == "grid";
     cache[device] = dev;
@@ -1993,10 +1993,14 @@ struct ag2d_world {
         const uint32_t perWarp = narrowPerWarp();
         const uint32_t gn = std::min(gridFor(uint64_t(pairEstimate()) * 32 / perWarp, narrowThreads),
                                      gridFor(uint64_t(pairCap) * 32 / perWarp, narrowThreads));
+        // Polygon pairs one a lane: where the pairs fill the lanes and half the colliders or more are polygons (3.7 M
+        // pairs of polygons: 1,244 us in groups, 905 in lanes; with one collider in seven a polygon, 128,000
+        // manifolds, 64 against 73).
+        const bool lanes = perWarp == 32 && 2 * uint64_t(nPolygons) >= nColliders;
         pbegin(5);
-        k_narrow<<<gn, narrowThreads, narrowThreads * NARROW_SMEM_PER_THREAD, s>>>(
-            view(), pairs.p, nPairs, pairCap, manifolds.p, manifoldCap, nManifolds.p, dCounters.p, narrowState.p,
-            narrowState.p + narrowTiles(), perWarp, table, begun && anySleeping ? wakeIsland.p : nullptr);
+        launch_narrow(
+            gn, narrowThreads, s, view(), pairs.p, nPairs, pairCap, manifolds.p, manifoldCap, nManifolds.p, dCounters.p, narrowState.p,
+            narrowState.p + narrowTiles(), perWarp, lanes, table, begun && anySleeping ? wakeIsland.p : nullptr);
         CK(cudaGetLastError());
         pend(5);
         launches += 1;
