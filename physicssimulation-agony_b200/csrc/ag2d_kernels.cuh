@@ -255,7 +255,7 @@ constexpr uint32_t NARROW_SMEM_PER_THREAD =
 // Narrow phase + manifold compaction: manifolds of the hit pairs, in pair order, into out; tileState [tiles + 1] and
 // tileCounter zeroed before the launch (tiles: blockDim.x / 32 x perWarp pairs each, perWarp at most 32).
 // The narrow phase; lanes: polygon pairs one a lane where a warp has enough of them (blocks of up to
-// NARROW_LANES_THREADS; a form with more registers, so fewer warps an SM for the other pairs).
+// NARROW_LANES_THREADS).
 constexpr uint32_t NARROW_LANES_THREADS = 256;   // largest block of the one-pair-a-lane form
 // Polygon pairs of a warp from which on each takes its own lane: the lanes together cost what about three rounds of the
 // groups (four pairs each) do.

@@ -656,10 +656,13 @@ __device__ __forceinline__ bool collide_polygon_polygon_lane(const ColliderView&
     float bov = FLT_MAX, bfac = FLT_MAX;
     uint32_t bord = 0xFFFFFFFFu;
     bool separated = false;
+    V2 normals[N];   // loaded together: one latency, not one an axis
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) normals[i] = i < nA ? ld2(A.normals, i) : v2(0.0f, 0.0f);
 #pragma unroll
     for (uint32_t i = 0; i < N; i++) {
         if (i >= nA) continue;
-        const V2 ax = ld2(A.normals, i);
+        const V2 ax = normals[i];
         float minB = FLT_MAX;
 #pragma unroll
         for (uint32_t j = 0; j < N; j++) minB = fminf(minB, dot(b[j], ax));
@@ -670,9 +673,11 @@ __device__ __forceinline__ bool collide_polygon_polygon_lane(const ColliderView&
     }
     if (separated) return false;
 #pragma unroll
+    for (uint32_t i = 0; i < N; i++) normals[i] = i < nB ? ld2(B.normals, i) : v2(0.0f, 0.0f);
+#pragma unroll
     for (uint32_t i = 0; i < N; i++) {
         if (i >= nB) continue;
-        const V2 nb = ld2(B.normals, i);
+        const V2 nb = normals[i];
         const V2 ax = v2(relCos * nb.x - relSin * nb.y, relSin * nb.x + relCos * nb.y);
         float minA = FLT_MAX;
 #pragma unroll
@@ -699,9 +704,11 @@ __device__ __forceinline__ bool collide_polygon_polygon_lane(const ColliderView&
     float bd = FLT_MAX;
     uint32_t ie = 0;
 #pragma unroll
+    for (uint32_t i = 0; i < N; i++) normals[i] = i < incCount ? ld2(incNormals, i) : v2(0.0f, 0.0f);
+#pragma unroll
     for (uint32_t i = 0; i < N; i++) {
         if (i >= incCount) continue;
-        V2 n = ld2(incNormals, i);
+        V2 n = normals[i];
         if (refIsA) n = v2(relCos * n.x - relSin * n.y, relSin * n.x + relCos * n.y);
         const float d = dot(rnl, n);
         if (d < bd) { bd = d; ie = i; }

@@ -1994,8 +1994,8 @@ struct ag2d_world {
         const uint32_t gn = std::min(gridFor(uint64_t(pairEstimate()) * 32 / perWarp, narrowThreads),
                                      gridFor(uint64_t(pairCap) * 32 / perWarp, narrowThreads));
         // Polygon pairs one a lane: where the pairs fill the lanes and half the colliders or more are polygons (3.7 M
-        // pairs of polygons: 1,244 us in groups, 905 in lanes; with one collider in seven a polygon, 128,000
-        // manifolds, 64 against 73).
+        // pairs of polygons: 1,255 us in groups, 830 in lanes; with one collider in seven a polygon, 128,000
+        // manifolds, 69 against 73).
         const bool lanes = perWarp == 32 && 2 * uint64_t(nPolygons) >= nColliders;
         pbegin(5);
         launch_narrow(

@@ -102,10 +102,11 @@ __device__ __forceinline__ void mark_wakes(const DeviceWorld& w, const Manifold&
 // their places: manifolds come out in pair order. The last tile writes the manifold count. Launched with a
 // multiple of 32 threads (at most 1024) and NARROW_SMEM_PER_THREAD bytes of dynamic shared memory per thread.
 // LANES: a warp with more than NARROW_LANES_PAIRS polygon pairs searches and clips them one a lane
-// (collide_polygon_polygon_lane) in place of the groups' rounds: 3.7 M polygon pairs (2.7 M manifolds) 1,244 -> 905 us, a
-// third of the instructions. Bound now by latency: 24 warps an SM, most stalls at the tile's barriers and on loads.
+// (collide_polygon_polygon_lane) in place of the groups' rounds: 3.7 M polygon pairs (2.7 M manifolds) 1,255 -> 830 us, a
+// third of the instructions. Bound now by latency: 32 warps an SM, most stalls at the tile's barriers and on loads (24
+// warps with more registers: 863; normals loaded one an axis: 905; tiles of 128 pairs: 979).
 template <bool LANES>
-__global__ void __launch_bounds__(LANES ? NARROW_LANES_THREADS : 512, LANES ? 3 : 2) k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairs,
+__global__ void __launch_bounds__(LANES ? NARROW_LANES_THREADS : 512, LANES ? 4 : 2) k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairs,
                          uint32_t pairCap, Manifold* __restrict__ out, uint32_t manifoldCap,
                          uint32_t* __restrict__ nOut, StepCounters* counters, uint32_t* __restrict__ tileState,
                          uint32_t* __restrict__ tileCounter, uint32_t perWarp, WarmTable warm,
