@@ -907,6 +907,7 @@ struct FlowScratch {
     float4* pos;       // [bodies] x, y, -, version
     Constraint* cons;  // [manifolds] records, 'pad' the rank and degree of a, of b: one byte each
     float4* posRec;    // [2 x manifolds] position records: normal, penetration base, ranks; masses, bodies
+    uint32_t* parent;  // [bodies] islands to link beside the solve, every body its own; or null
 };
 __global__ void __launch_bounds__(FLOW_THREADS, 1)
 k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, FlowScratch f, uint32_t velIters,

@@ -2503,7 +2503,8 @@ struct ag2d_world {
             }
             flowVel.reserve(nBodies); flowPos.reserve(nBodies); flowPosRec.reserve(2 * size_t(manifoldCap));
             flowCons.reserve(manifoldCap);
-            FlowScratch flow{flowVel.p, flowPos.p, flowCons.p, flowPosRec.p};
+            FlowScratch flow{flowVel.p, flowPos.p, flowCons.p, flowPosRec.p, begun ? ufParent.p : nullptr};
+            islandsLinked = begun;   // the step's first kernel made every body its own island
             uint32_t* barp = bar.p;
             const uint32_t est = std::min<uint32_t>(manifoldCap, lastManifolds + lastManifolds / 2 + 1024);
             const int grid = std::max(1, std::min<int>(dev.flowBlocks, int(div_up(est, 128))));

@@ -373,6 +373,29 @@ __device__ __forceinline__ bool flow_live(uint32_t c, const Constraint& k, uint3
     return false;
 }
 
+// Islands' union-find in global memory (see k_island_union): links the bodies of one pair if both are dynamic.
+__device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t x)
+{
+    uint32_t p = __ldcg(parent + x);
+    while (p != x) {
+        const uint32_t gp = __ldcg(parent + p);
+        if (gp != p) atomicCAS(parent + x, p, gp);   // path halving, benign races
+        x = p;
+        p = gp;
+    }
+    return x;
+}
+__device__ __forceinline__ void uf_link(const DeviceWorld& w, uint32_t* parent, uint32_t a, uint32_t b)
+{
+    if (w.bstate[a] != STATE_DYNAMIC || w.bstate[b] != STATE_DYNAMIC) return;
+    for (uint32_t tries = 0; tries < 1u << 20; tries++) {
+        uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
+        if (ra == rb) break;
+        if (ra < rb) { const uint32_t t = ra; ra = rb; rb = t; }   // link the larger root under the smaller
+        if (atomicCAS(parent + ra, ra, rb) == ra) break;
+    }
+}
+
 // Walks a warp's items of one pass: the manifolds in colour-major order, every colour padded to whole warps, chunk q
 // of 32 to warp q modulo the warps. A chunk has one colour, so its lanes never wait for one another.
 struct FlowWalk {
@@ -413,6 +436,8 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
     uint32_t ncol = 0;
     if (!color_manifolds(w, B, m, n, s, rank, size, sync, &counters->colors, &counters->status, ncol)) return;
     if (ncol > 64u) {
+        if (f.parent)
+            for (uint32_t i = rank; i < n; i += size) uf_link(w, f.parent, w.cbody[m[i].a], w.cbody[m[i].b]);
         solve_colored(w, B, m, n, s, ncol, velIters, posIters, rank, size, sync);
         return;
     }
@@ -554,6 +579,10 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
                 }
             }
         }
+        // The position warps are done before the velocity warps: the islands are linked meanwhile.
+        if (f.parent)
+            for (uint32_t i = q0 * 32u + (threadIdx.x & 31u); i < n; i += qStep * 32u)
+                uf_link(w, f.parent, w.cbody[m[i].a], w.cbody[m[i].b]);
     }
 }
 
@@ -818,18 +847,6 @@ cudaError_t launch_color_solve_teams(uint32_t threads, bool pipelined, uint32_t 
 // most the speed threshold; its timer accumulates while quiet. An island sleeps when every member is quiet and has
 // been for the time threshold.
 // ---------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t x)
-{
-    uint32_t p = __ldcg(parent + x);
-    while (p != x) {
-        const uint32_t gp = __ldcg(parent + p);
-        if (gp != p) atomicCAS(parent + x, p, gp);   // path halving, benign races
-        x = p;
-        p = gp;
-    }
-    return x;
-}
-
 __global__ void k_island_init(DeviceWorld w, uint32_t* __restrict__ parent, uint32_t* __restrict__ flag)
 {
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nBodies; b += gridDim.x * blockDim.x) {
@@ -843,14 +860,7 @@ __global__ void k_island_union(DeviceWorld w, const Manifold* __restrict__ m, co
 {
     const uint32_t n = *nM;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t a = w.cbody[m[i].a], b = w.cbody[m[i].b];
-        if (w.bstate[a] != STATE_DYNAMIC || w.bstate[b] != STATE_DYNAMIC) continue;
-        for (uint32_t tries = 0; tries < 1u << 20; tries++) {
-            uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
-            if (ra == rb) break;
-            if (ra < rb) { const uint32_t t = ra; ra = rb; rb = t; }   // link the larger root under the smaller
-            if (atomicCAS(parent + ra, ra, rb) == ra) break;
-        }
+        uf_link(w, parent, w.cbody[m[i].a], w.cbody[m[i].b]);
     }
 }
 
@@ -859,14 +869,7 @@ __global__ void k_island_union_edges(DeviceWorld w, const uint2* __restrict__ ed
                                      uint32_t* __restrict__ parent)
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t a = edges[i].x, b = edges[i].y;
-        if (w.bstate[a] != STATE_DYNAMIC || w.bstate[b] != STATE_DYNAMIC) continue;
-        for (uint32_t tries = 0; tries < 1u << 20; tries++) {
-            uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
-            if (ra == rb) break;
-            if (ra < rb) { const uint32_t t = ra; ra = rb; rb = t; }
-            if (atomicCAS(parent + ra, ra, rb) == ra) break;
-        }
+        uf_link(w, parent, edges[i].x, edges[i].y);
     }
 }
 
