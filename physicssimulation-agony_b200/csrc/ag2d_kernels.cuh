@@ -97,6 +97,33 @@ struct StepBegin {
     const uint32_t* nIsle;
     StepCounters* counters;
 };
+// A chain of kernels on one stream: launched with chain_launch, a kernel's blocks may be placed while its predecessor
+// still runs, and chain_begin, the first thing they do, waits for its end (and for its writes). Kernels of a small step
+// run about ten microseconds and the gaps between them up to a third of that: 98 -> 90 us a step with 64 bodies,
+// 136 -> 108 with 20,000 in flight. Large ones lose more to the waiting blocks than the gaps cost (900 -> 937 us with
+// 100,000 bodies piled up, 465 -> 489 a pass over a million), so only engines of up to CHAIN_COLLIDERS are chained.
+constexpr uint32_t CHAIN_COLLIDERS = 32768;
+__device__ __forceinline__ void chain_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t chain_launch(bool chained, void (*kernel)(P...), uint32_t blocks, uint32_t threads, size_t smem,
+                                cudaStream_t stream, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 __global__ void k_step_begin(StepBegin a);
 __global__ void k_collider_pose(DeviceWorld w, const uint32_t* list, const uint8_t* listSimd, uint32_t n,
                                 const uint32_t* worldMask, WarmTable insert);
@@ -122,7 +149,7 @@ __global__ void k_tree_gather(const uint32_t* vals, uint32_t n, const uint32_t* 
 uint32_t sort_tiles(uint32_t n);
 cudaError_t launch_sort_pass(const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut, uint32_t* valsOut,
                              uint32_t n, uint32_t shift, const uint32_t* digitBase, uint32_t* tileState,
-                             uint32_t* tileCounter, uint32_t* status, cudaStream_t stream);
+                             uint32_t* tileCounter, uint32_t* status, bool chained, cudaStream_t stream);
 // Trees of up to TREE_SEGMENT_MAX leaves are built by one CTA each (k_tree_segments), in size classes.
 constexpr uint32_t TREE_SEGMENT_MAX = 16384;
 // A single tree of more leaves is built by the whole GPU in eight launches: 75 us at 6,000 and 77 at 8,000 leaves,
@@ -140,6 +167,7 @@ struct TreeBuild {
     int2* child;                // or null, likewise
     NodeRec* rec;
     float4* meet;               // [2 x leaves] meeting boxes of the largest class
+    bool chained;               // one class: launched ahead of its predecessor's end (chain_launch)
 };
 // Host side: builds every segment's tree; 'largest' bounds the segment sizes (at most TREE_SEGMENT_MAX); *launches: the
 // kernels launched.
@@ -262,7 +290,7 @@ constexpr uint32_t NARROW_LANES_THREADS = 256;   // largest block of the one-pai
 constexpr int NARROW_LANES_PAIRS = 10;
 // Host side: raises the narrow phase's dynamic shared-memory limit (once per device).
 cudaError_t narrow_init();
-void launch_narrow(uint32_t blocks, uint32_t threads, cudaStream_t stream, DeviceWorld w, const uint2* pairs,
+cudaError_t launch_narrow(bool chained, uint32_t blocks, uint32_t threads, cudaStream_t stream, DeviceWorld w, const uint2* pairs,
                    const uint32_t* nPairs, uint32_t pairCap, Manifold* out, uint32_t manifoldCap, uint32_t* nOut,
                    StepCounters* counters, uint32_t* tileState, uint32_t* tileCounter, uint32_t perWarp, bool lanes,
                    WarmTable warm, uint32_t* wakeIsland);

@@ -1333,6 +1333,7 @@ struct ag2d_world {
         if (stream) cudaStreamDestroy(stream);
     }
 
+    bool chained() const { return nColliders <= CHAIN_COLLIDERS; }
     uint32_t gridFor(uint64_t n, uint32_t threads = 256) const
     {
         const uint64_t want = (n + threads - 1) / threads;
@@ -1762,8 +1763,9 @@ struct ag2d_world {
         }
         pbegin(1);
         const uint32_t* mask = (full && changedWorlds && nWorlds > 1) ? worldDirty.p : nullptr;
-        k_collider_pose<<<gridFor(std::max(n, insert.keys ? prevCount : 0u)), 256, 0, stream>>>(
-            view(), full ? nullptr : dynCol.p, (full || nWorlds == 1) ? nullptr : dynColSimd.p, n, mask, insert);
+        CK(chain_launch(chained(), k_collider_pose, gridFor(std::max(n, insert.keys ? prevCount : 0u)), 256, 0, stream,
+                        view(), full ? nullptr : dynCol.p, (full || nWorlds == 1) ? nullptr : dynColSimd.p, n, mask,
+                        insert));
         CK(cudaGetLastError());
         pend(1);
         launches++;
@@ -1813,7 +1815,7 @@ struct ag2d_world {
             const uint32_t slot = 4 * round + pass;
             CK(launch_sort_pass(ki, vi, ko, vo, n, pass * 8, t.sortWords.p + slot * 256,
                                 t.sortWords.p + Tree::SORT_HEAD + size_t(slot) * tiles * 256,
-                                t.sortWords.p + Tree::SORT_COUNTERS + slot, &dCounters.p->status, stream));
+                                t.sortWords.p + Tree::SORT_COUNTERS + slot, &dCounters.p->status, chained(), stream));
             std::swap(ki, ko);
             std::swap(vi, vo);
         }
@@ -1840,7 +1842,7 @@ struct ag2d_world {
             // its node boxes and child links; the pair query needs neither.
             const TreeBuild b{caabb.p, list, seg ? t.segStart.p : nullptr, W, n, t.vals.p,
                               seg ? t.sortedKey.p : t.keys.p, seg ? t.sortedWorld.p : nullptr, t.leafAabb.p,
-                              isDyn ? nullptr : t.nodeAabb.p, isDyn ? nullptr : t.child.p, t.rec.p, t.meet.p};
+                              isDyn ? nullptr : t.nodeAabb.p, isDyn ? nullptr : t.child.p, t.rec.p, t.meet.p, !seg};
             uint32_t count = 0;
             if (isDyn) pbegin(13);
             CK(launch_tree_segments(b, seg ? std::min(maxWorldCols, n) : n, uint32_t(std::max(dev.sms, 1)), s, &count));
@@ -1857,10 +1859,11 @@ struct ag2d_world {
             k_bounds_init<<<gridFor(W), 256, 0, s>>>(t.bounds.p, W);
             launches++;
         }
-        k_bounds<<<parts, 256, 0, s>>>(caabb.p, list, n, cw, t.bounds.p, t.parts.p, t.sortWords.p, words);
-        k_morton<<<gridFor(n), 256, 0, s>>>(caabb.p, list, n, cw, t.bounds.p, t.parts.p, parts, t.keys.p, t.vals.p,
-                                             seg ? t.keyOf.p : nullptr, t.sortWords.p,
-                                             t.sortWords.p + Tree::SORT_DONE);
+        CK(chain_launch(chained(), k_bounds, parts, 256, 0, s, caabb.p, list, n, cw, t.bounds.p, t.parts.p,
+                        t.sortWords.p, words));
+        CK(chain_launch(chained(), k_morton, gridFor(n), 256, 0, s, caabb.p, list, n, cw, t.bounds.p, t.parts.p, parts,
+                        t.keys.p, t.vals.p, seg ? t.keyOf.p : nullptr, t.sortWords.p,
+                        t.sortWords.p + Tree::SORT_DONE));
         CK(cudaGetLastError());
         launches += 4;
         if (isDyn) pbegin(12);
@@ -1879,12 +1882,11 @@ struct ag2d_world {
                                                       t.sortedWorld.p, t.leafAabb.p);
             launches++;
         }
-        k_lbvh_build<<<gridFor(n), 256, 0, s>>>(seg ? t.sortedKey.p : t.keys.p, seg ? t.sortedWorld.p : nullptr,
-                                                 seg ? t.segStart.p : nullptr, int(n), t.vals.p, caabb.p,
-                                                 t.leafAabb.p, t.child.p, t.parent.p, t.leafParent.p, t.meet.p,
-                                                 t.rec.p);
-        k_lbvh_refit<<<gridFor(n), 256, 0, s>>>(int(n), t.child.p, t.parent.p, t.leafParent.p, t.leafAabb.p,
-                                                 t.nodeAabb.p, t.meet.p, t.rec.p);
+        CK(chain_launch(chained(), k_lbvh_build, gridFor(n), 256, 0, s, seg ? t.sortedKey.p : t.keys.p,
+                        seg ? t.sortedWorld.p : nullptr, seg ? t.segStart.p : nullptr, int(n), t.vals.p, caabb.p,
+                        t.leafAabb.p, t.child.p, t.parent.p, t.leafParent.p, t.meet.p, t.rec.p));
+        CK(chain_launch(chained(), k_lbvh_refit, gridFor(n), 256, 0, s, int(n), t.child.p, t.parent.p, t.leafParent.p,
+                        t.leafAabb.p, t.nodeAabb.p, t.meet.p, t.rec.p));
         CK(cudaGetLastError());
         if (isDyn) pend(13);
     }
@@ -1943,8 +1945,8 @@ struct ag2d_world {
             queryState.reserve(size_t(tiles) + 1);
             CK(cudaMemsetAsync(queryState.p, 0, (size_t(tiles) + 1) * sizeof(uint32_t), s));
         }
-        k_query<<<gq, queryThreads, 0, s>>>(dynTree.view(), otherTree.view(), cbody.p, pairs.p, pairCap, total,
-                                            &dCounters.p->status, queryState.p, queryState.p + tiles);
+        CK(chain_launch(chained(), k_query, gq, queryThreads, 0, s, dynTree.view(), otherTree.view(), cbody.p, pairs.p,
+                        pairCap, total, &dCounters.p->status, queryState.p, queryState.p + tiles));
         CK(cudaGetLastError());
         pend(4);
     }
@@ -1998,9 +2000,9 @@ struct ag2d_world {
         // manifolds, 69 against 73).
         const bool lanes = perWarp == 32 && 2 * uint64_t(nPolygons) >= nColliders;
         pbegin(5);
-        launch_narrow(
-            gn, narrowThreads, s, view(), pairs.p, nPairs, pairCap, manifolds.p, manifoldCap, nManifolds.p, dCounters.p, narrowState.p,
-            narrowState.p + narrowTiles(), perWarp, lanes, table, begun && anySleeping ? wakeIsland.p : nullptr);
+        CK(launch_narrow(chained(), gn, narrowThreads, s, view(), pairs.p, nPairs, pairCap, manifolds.p, manifoldCap,
+                         nManifolds.p, dCounters.p, narrowState.p, narrowState.p + narrowTiles(), perWarp, lanes, table,
+                         begun && anySleeping ? wakeIsland.p : nullptr));
         CK(cudaGetLastError());
         pend(5);
         launches += 1;
@@ -2535,11 +2537,11 @@ struct ag2d_world {
             launches++;
         }
         islandsLinked = false;
-        k_island_quiet<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p, settings.dt, settings.sleep_speed,
-                                                        settings.sleep_time);
+        CK(chain_launch(chained(), k_island_quiet, gridFor(nBodies), 256, 0, s, w, ufParent.p, ufFlag.p, settings.dt,
+                        settings.sleep_speed, settings.sleep_time));
         // Within a step this is its last kernel: it leaves the counters in page-locked memory.
         const StepEnd end{begun ? hCounters : nullptr, stepDone.p, nManifolds.p, nPrev.p};
-        k_island_sleep<<<gridFor(nBodies), 256, 0, s>>>(w, ufParent.p, ufFlag.p, dCounters.p, end);
+        CK(chain_launch(chained(), k_island_sleep, gridFor(nBodies), 256, 0, s, w, ufParent.p, ufFlag.p, dCounters.p, end));
         CK(cudaGetLastError());
         pend(11);
     }
@@ -3086,9 +3088,8 @@ struct ag2d_world {
             if (newWorldsPending && !fullPose) {
                 // Worlds that joined a server batch: their first step poses every collider, as alone.
                 const DeviceWorld wv = view();
-                k_collider_pose<<<gridFor(nColliders), 256, 0, s>>>(wv, nullptr, nullptr, nColliders,
-                                                                    nWorlds > 1 ? newWorldMask.p : nullptr,
-                                                                    WarmTable{});
+                CK(chain_launch(chained(), k_collider_pose, gridFor(nColliders), 256, 0, s, wv, nullptr, nullptr,
+                                nColliders, nWorlds > 1 ? newWorldMask.p : nullptr, WarmTable{}));
                 CK(cudaGetLastError());
                 launches++;
             }

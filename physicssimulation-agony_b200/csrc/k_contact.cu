@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(LANES ? NARROW_LANES_THREADS : 512, LANES ? 4 
                          uint32_t* __restrict__ tileCounter, uint32_t perWarp, WarmTable warm,
                          uint32_t* __restrict__ wakeIsland)
 {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char narrowSmem[];
     // [blockDim] manifold slots, [blockDim] hit flags, then per group A's vertices and B's (in A's frame).
     Manifold* const slot = reinterpret_cast<Manifold*>(narrowSmem);
@@ -256,18 +257,14 @@ cudaError_t narrow_init()
                                 int(512 * NARROW_SMEM_PER_THREAD));
 }
 
-void launch_narrow(uint32_t blocks, uint32_t threads, cudaStream_t stream, DeviceWorld w, const uint2* pairs,
+cudaError_t launch_narrow(bool chained, uint32_t blocks, uint32_t threads, cudaStream_t stream, DeviceWorld w, const uint2* pairs,
                    const uint32_t* nPairs, uint32_t pairCap, Manifold* out, uint32_t manifoldCap, uint32_t* nOut,
                    StepCounters* counters, uint32_t* tileState, uint32_t* tileCounter, uint32_t perWarp, bool lanes,
                    WarmTable warm, uint32_t* wakeIsland)
 {
-    const size_t smem = size_t(threads) * NARROW_SMEM_PER_THREAD;
-    if (lanes && threads <= NARROW_LANES_THREADS)
-        k_narrow<true><<<blocks, threads, smem, stream>>>(w, pairs, nPairs, pairCap, out, manifoldCap, nOut, counters,
-                                                          tileState, tileCounter, perWarp, warm, wakeIsland);
-    else
-        k_narrow<false><<<blocks, threads, smem, stream>>>(w, pairs, nPairs, pairCap, out, manifoldCap, nOut, counters,
-                                                           tileState, tileCounter, perWarp, warm, wakeIsland);
+    return chain_launch(chained, lanes && threads <= NARROW_LANES_THREADS ? k_narrow<true> : k_narrow<false>, blocks, threads,
+                        size_t(threads) * NARROW_SMEM_PER_THREAD, stream, w, pairs, nPairs, pairCap, out, manifoldCap,
+                        nOut, counters, tileState, tileCounter, perWarp, warm, wakeIsland);
 }
 
 __global__ void k_warm_insert(WarmTable t) { warm_insert(t); }
@@ -615,6 +612,7 @@ __device__ __forceinline__ void team_union(uint32_t* par, uint32_t a, uint32_t b
 template <uint32_t THREADS>
 __global__ void __launch_bounds__(THREADS, 1) k_color_solve_block(BlockSolve a)
 {
+    chain_begin();
     extern __shared__ float4 teamCache[];
     __shared__ uint32_t colorCount[COLOR_SLOTS];
     __shared__ uint32_t colorStart[MAX_COLORS + 1];
@@ -686,10 +684,9 @@ cudaError_t block_solver_init()
 cudaError_t launch_color_solve_block(uint32_t manifolds, cudaStream_t stream, const BlockSolve& a)
 {
     const size_t smem = team_smem_bytes(a.bodyCap, 0);
-    if (manifolds <= 512) k_color_solve_block<128><<<1, 128, smem, stream>>>(a);
-    else if (manifolds <= 4096) k_color_solve_block<512><<<1, 512, smem, stream>>>(a);
-    else k_color_solve_block<1024><<<1, 1024, smem, stream>>>(a);
-    return cudaGetLastError();
+    if (manifolds <= 512) return chain_launch(true, k_color_solve_block<128>, 1, 128, smem, stream, a);
+    if (manifolds <= 4096) return chain_launch(true, k_color_solve_block<512>, 1, 512, smem, stream, a);
+    return chain_launch(true, k_color_solve_block<1024>, 1, 1024, smem, stream, a);
 }
 
 // Batched worlds: each CTA takes the next team of consecutive worlds, whose manifolds are one contiguous range of
@@ -876,6 +873,7 @@ __global__ void k_island_union_edges(DeviceWorld w, const uint2* __restrict__ ed
 __global__ void k_island_quiet(DeviceWorld w, uint32_t* __restrict__ parent, uint32_t* __restrict__ flag, float dt,
                                float speedThreshold, float timeThreshold)
 {
+    chain_begin();
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nBodies; b += gridDim.x * blockDim.x) {
         if (w.bstate[b] != STATE_DYNAMIC) continue;
         const float4 v = w.bvel[b];
@@ -911,6 +909,7 @@ __device__ __forceinline__ void step_end(const StepEnd& e, StepCounters* counter
 __global__ void k_island_sleep(DeviceWorld w, uint32_t* __restrict__ parent, const uint32_t* __restrict__ flag,
                                StepCounters* counters, StepEnd end)
 {
+    chain_begin();
     uint32_t slept = 0;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nBodies; b += gridDim.x * blockDim.x) {
         if (w.bstate[b] != STATE_DYNAMIC) continue;

@@ -171,6 +171,7 @@ __device__ __forceinline__ float4 collider_aabb(const DeviceWorld& w, uint32_t c
 __global__ void k_collider_pose(DeviceWorld w, const uint32_t* __restrict__ list, const uint8_t* __restrict__ listSimd,
                                 uint32_t n, const uint32_t* __restrict__ worldMask, WarmTable insert)
 {
+    chain_begin();
     if (insert.keys) warm_insert(insert);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const uint32_t c = list ? list[k] : k;
@@ -235,6 +236,7 @@ __global__ void k_bounds(const float4* __restrict__ aabb, const uint32_t* __rest
                          const uint32_t* __restrict__ colWorld, uint32_t* __restrict__ bounds,
                          float4* __restrict__ parts, uint32_t* __restrict__ clear, uint32_t clearWords)
 {
+    chain_begin();
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t base0 = blockIdx.x * blockDim.x;
     for (uint32_t i = base0 + threadIdx.x; i < clearWords; i += stride) clear[i] = 0u;
@@ -389,6 +391,7 @@ __global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ aabb,
                                                 uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                                 uint32_t* __restrict__ keyOf, uint32_t* hist, uint32_t* done)
 {
+    chain_begin();
     __shared__ uint32_t sh[4 * 256];
     __shared__ float4 whole;
     for (uint32_t i = threadIdx.x; i < 4 * 256; i += 256) sh[i] = 0;
@@ -507,6 +510,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
     uint32_t* __restrict__ valsOut, uint32_t n, uint32_t shift, const uint32_t* __restrict__ digitBase,
     uint32_t* __restrict__ tileState, uint32_t* __restrict__ tileCounter, uint32_t* __restrict__ status)
 {
+    chain_begin();
     constexpr uint32_t WARPS = SORT_THREADS / 32, SORT_TILE = SORT_THREADS * SORT_ITEMS;
     __shared__ uint32_t warpHist[WARPS][256];
     __shared__ uint32_t digitStart[256];     // exclusive scan of the tile's digit counts
@@ -637,15 +641,11 @@ uint32_t sort_tiles(uint32_t n)
 
 cudaError_t launch_sort_pass(const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut, uint32_t* valsOut,
                              uint32_t n, uint32_t shift, const uint32_t* digitBase, uint32_t* tileState,
-                             uint32_t* tileCounter, uint32_t* status, cudaStream_t stream)
+                             uint32_t* tileCounter, uint32_t* status, bool chained, cudaStream_t stream)
 {
-    if (n <= SORT_SMALL_MAX)
-        k_sort_pass<SORT_ITEMS_SMALL><<<sort_tiles(n), SORT_THREADS, 0, stream>>>(
-            keysIn, valsIn, keysOut, valsOut, n, shift, digitBase, tileState, tileCounter, status);
-    else
-        k_sort_pass<SORT_ITEMS_LARGE><<<sort_tiles(n), SORT_THREADS, 0, stream>>>(
-            keysIn, valsIn, keysOut, valsOut, n, shift, digitBase, tileState, tileCounter, status);
-    return cudaGetLastError();
+    return chain_launch(chained, n <= SORT_SMALL_MAX ? k_sort_pass<SORT_ITEMS_SMALL> : k_sort_pass<SORT_ITEMS_LARGE>, sort_tiles(n),
+                        SORT_THREADS, 0, stream, keysIn, valsIn, keysOut, valsOut, n, shift, digitBase, tileState,
+                        tileCounter, status);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -695,6 +695,7 @@ __global__ void k_lbvh_build(const uint32_t* __restrict__ keys, const uint32_t* 
                              int2* __restrict__ child, int* __restrict__ parent, int* __restrict__ leafParent,
                              float4* __restrict__ meet, NodeRec* __restrict__ rec)
 {
+    chain_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int lo = 0, hi = n;
         if (!sortedWorld) leafAabb[i] = caabb[vals[i]];
@@ -769,8 +770,12 @@ struct TreeSmem {
 template <uint32_t THREADS, uint32_t E, bool MEET_SHARED>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_tree_segments(TreeBuild t, uint32_t minSize, uint32_t maxSize)
 {
-    // The classes work on different segments: the next class's launch need not wait for this one.
-    asm volatile("griddepcontrol.launch_dependents;");
+    if (t.chained) {
+        chain_begin();
+    } else {
+        // The classes work on different segments: the next class's launch need not wait for this one.
+        asm volatile("griddepcontrol.launch_dependents;");
+    }
     using Smem = TreeSmem<THREADS, E, MEET_SHARED>;
     constexpr uint32_t WARPS = Smem::WARPS;
     extern __shared__ float4 treeTile[];
@@ -975,7 +980,7 @@ static cudaError_t launch_tree_class(const TreeBuild& t, uint32_t minSize, uint3
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = *launches > 0 ? 1 : 0;   // beside the class launched before it
+    cfg.numAttrs = *launches > 0 || t.chained ? 1 : 0;   // beside the class launched before it, or chained
     ++*launches;
     return cudaLaunchKernelEx(&cfg, k_tree_segments<THREADS, E, MEET_SHARED>, t, minSize, maxSize);
 }
@@ -1025,6 +1030,7 @@ __global__ void k_lbvh_refit(int n, const int2* __restrict__ child, const int* _
                              const int* __restrict__ leafParent, const float4* __restrict__ leafAabb,
                              float4* __restrict__ nodeAabb, float4* __restrict__ meet, NodeRec* __restrict__ rec)
 {
+    chain_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int node = leafParent[i];   // -1 for the leaf of a one-collider segment
         int self = ~i;              // child encoding of the subtree this thread carries up
@@ -1145,6 +1151,7 @@ __global__ void __launch_bounds__(QUERY_MAX_THREADS) k_query(TreeView dyn, TreeV
                                                              uint32_t* __restrict__ tileState,
                                                              uint32_t* __restrict__ tileCounter)
 {
+    chain_begin();
     __shared__ uint32_t kept[QUERY_STASH * QUERY_MAX_THREADS];   // [k][thread]
     __shared__ uint32_t warpBase[QUERY_MAX_THREADS / 32];
     __shared__ uint32_t tileSlot, tileBase;
