@@ -677,8 +677,8 @@ def run_c4(args, torch, dist, rank, world_size, local, dev):
     phases = e.phase_times()
     msb = mean_shape_bytes(scene_list)
     bytes_by_phase = step_bytes(msb, sums["pairs"], sums["manifolds"], n_bodies - len(scene_list), K)
-    kernel_of = {"solve": "k_color_solve_teams", "narrow": "k_narrow", "integrate": "k_integrate",
-                 "pose": "k_collider_pose", "sort": "k_sort_pass", "query": "k_query_stash + k_query_emit"}
+    kernel_of = {"solve": "k_color_solve_teams", "narrow": "k_narrow", "integrate": "k_step_begin",
+                 "pose": "k_collider_pose", "sort": "k_sort_pass", "query": "k_query"}
     roof = roofline_line(phases, bytes_by_phase, kernel_of, "c4", solve_passes(sums["manifolds"]))
     pose_bytes = e.field_bytes(ag2d.BODY_POSE)
     del batch, e
@@ -800,8 +800,8 @@ def run_c2(args, torch, dist, rank, world_size, local, dev):
     msb = mean_shape_bytes([scene])
     nb, nc = w.counts()
     bytes_by_phase = step_bytes(msb, sums["pairs"], sums["manifolds"], nb - int((scene.mass == 0).sum()), K)
-    kernel_of = {"solve": "k_color_solve_cluster", "narrow": "k_narrow", "integrate": "k_integrate",
-                 "pose": "k_collider_pose", "sort": "k_sort_pass", "query": "k_query_stash + k_query_emit"}
+    kernel_of = {"solve": "k_color_solve_flow", "narrow": "k_narrow", "integrate": "k_step_begin",
+                 "pose": "k_collider_pose", "sort": "k_sort_pass", "query": "k_query"}
     roof = roofline_line(phases, bytes_by_phase, kernel_of, "c2", solve_passes(sums["manifolds"]))
 
     e2e_steps = min(K, 300)

@@ -520,7 +520,7 @@ int32_t ag2d_server_destroy(ag2d_server* server);
  * allocation and no allocating library call. It is for callers that cannot allocate at this point: a host loop
  * that has handed all free device memory to its own pool and runs inside that budget, or code that must not stall
  * a busy device on the implicit synchronisation that cudaMalloc / cudaFree can bring. Its scratch is one fixed
- * static device array of about 3.1 MiB per device, so:
+ * static device array of about 3.4 MiB per device, so:
  *  - at most AG2D_SOLVE_NOALLOC_MAX_MANIFOLDS manifolds and AG2D_SOLVE_NOALLOC_MAX_BODIES bodies per call; larger
  *    sizes return AG2D_ERR_CAPACITY with the limit in the error string, before any launch;
  *  - the array's address belongs to a CUDA context: the first call in each context (the first on a device, and the
