@@ -102,6 +102,8 @@ struct StepBegin {
 // run about ten microseconds and the gaps between them up to a third of that: 98 -> 90 us a step with 64 bodies,
 // 136 -> 108 with 20,000 in flight. Large ones lose more to the waiting blocks than the gaps cost (900 -> 937 us with
 // 100,000 bodies piled up, 465 -> 489 a pass over a million), so only engines of up to CHAIN_COLLIDERS are chained.
+// Such a kernel takes no pointer as __restrict__ and reads nothing through __ldg that an earlier kernel of the chain
+// writes: those loads may move ahead of the wait and need not see the writes.
 constexpr uint32_t CHAIN_COLLIDERS = 32768;
 __device__ __forceinline__ void chain_begin()
 {

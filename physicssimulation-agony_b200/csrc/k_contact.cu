@@ -106,11 +106,11 @@ __device__ __forceinline__ void mark_wakes(const DeviceWorld& w, const Manifold&
 // third of the instructions. Bound now by latency: 32 warps an SM, most stalls at the tile's barriers and on loads (24
 // warps with more registers: 863; normals loaded one an axis: 905; tiles of 128 pairs: 979).
 template <bool LANES>
-__global__ void __launch_bounds__(LANES ? NARROW_LANES_THREADS : 512, LANES ? 4 : 2) k_narrow(DeviceWorld w, const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairs,
-                         uint32_t pairCap, Manifold* __restrict__ out, uint32_t manifoldCap,
-                         uint32_t* __restrict__ nOut, StepCounters* counters, uint32_t* __restrict__ tileState,
-                         uint32_t* __restrict__ tileCounter, uint32_t perWarp, WarmTable warm,
-                         uint32_t* __restrict__ wakeIsland)
+__global__ void __launch_bounds__(LANES ? NARROW_LANES_THREADS : 512, LANES ? 4 : 2) k_narrow(DeviceWorld w, const uint2* pairs, const uint32_t* nPairs,
+                         uint32_t pairCap, Manifold* out, uint32_t manifoldCap,
+                         uint32_t* nOut, StepCounters* counters, uint32_t* tileState,
+                         uint32_t* tileCounter, uint32_t perWarp, WarmTable warm,
+                         uint32_t* wakeIsland)
 {
     chain_begin();
     extern __shared__ __align__(16) unsigned char narrowSmem[];
@@ -870,7 +870,7 @@ __global__ void k_island_union_edges(DeviceWorld w, const uint2* __restrict__ ed
     }
 }
 
-__global__ void k_island_quiet(DeviceWorld w, uint32_t* __restrict__ parent, uint32_t* __restrict__ flag, float dt,
+__global__ void k_island_quiet(DeviceWorld w, uint32_t* parent, uint32_t* flag, float dt,
                                float speedThreshold, float timeThreshold)
 {
     chain_begin();
@@ -906,7 +906,7 @@ __device__ __forceinline__ void step_end(const StepEnd& e, StepCounters* counter
     __threadfence_system();
 }
 
-__global__ void k_island_sleep(DeviceWorld w, uint32_t* __restrict__ parent, const uint32_t* __restrict__ flag,
+__global__ void k_island_sleep(DeviceWorld w, uint32_t* parent, const uint32_t* flag,
                                StepCounters* counters, StepEnd end)
 {
     chain_begin();

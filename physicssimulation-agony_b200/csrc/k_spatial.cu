@@ -49,9 +49,10 @@ __device__ __forceinline__ void integrate_move(const DeviceWorld& w, uint32_t b,
     w.brot[b] = make_float2(c, s);
 }
 
-__global__ void k_integrate(DeviceWorld w, const uint32_t* __restrict__ dynBody, const uint8_t* __restrict__ dynSimd,
+__global__ void k_integrate(DeviceWorld w, const uint32_t* dynBody, const uint8_t* dynSimd,
                             uint32_t nDyn, IntegrateParams ip, uint32_t phase)
 {
+    chain_begin();
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nDyn; k += gridDim.x * blockDim.x) {
         const uint32_t b = dynBody[k];
         const bool simd = dynSimd ? dynSimd[k] != 0 : k < (nDyn & ~7u);
@@ -168,8 +169,8 @@ __device__ __forceinline__ float4 collider_aabb(const DeviceWorld& w, uint32_t c
 
 // insert: the warm-start table filled beside the poses (one launch for two passes that touch nothing in common), or a
 // table without keys.
-__global__ void k_collider_pose(DeviceWorld w, const uint32_t* __restrict__ list, const uint8_t* __restrict__ listSimd,
-                                uint32_t n, const uint32_t* __restrict__ worldMask, WarmTable insert)
+__global__ void k_collider_pose(DeviceWorld w, const uint32_t* list, const uint8_t* listSimd,
+                                uint32_t n, const uint32_t* worldMask, WarmTable insert)
 {
     chain_begin();
     if (insert.keys) warm_insert(insert);
@@ -232,9 +233,9 @@ __device__ __forceinline__ float4 block_bounds(float mnx, float mny, float mxx, 
 // One world: every block leaves the bounds of its colliders in parts[block] (k_morton's blocks reduce them). Several
 // worlds: 4 ordered words each; a warp whose lanes all belong to one world reduces first and issues one atomic per
 // word, a warp that straddles worlds issues per-lane atomics. The sort's words are cleared beside it.
-__global__ void k_bounds(const float4* __restrict__ aabb, const uint32_t* __restrict__ list, uint32_t n,
-                         const uint32_t* __restrict__ colWorld, uint32_t* __restrict__ bounds,
-                         float4* __restrict__ parts, uint32_t* __restrict__ clear, uint32_t clearWords)
+__global__ void k_bounds(const float4* aabb, const uint32_t* list, uint32_t n,
+                         const uint32_t* colWorld, uint32_t* bounds,
+                         float4* parts, uint32_t* clear, uint32_t clearWords)
 {
     chain_begin();
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -384,12 +385,12 @@ __device__ __forceinline__ void digits_end(const uint32_t* sh, uint32_t* hist, u
 
 // Morton keys with the digit histograms of their sort (blocks of 256 threads). One world: the bounds are the union of
 // parts[0, nParts), reduced by every block.
-__global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ aabb, const uint32_t* __restrict__ list,
-                                                uint32_t n, const uint32_t* __restrict__ colWorld,
-                                                const uint32_t* __restrict__ bounds,
-                                                const float4* __restrict__ parts, uint32_t nParts,
-                                                uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                                                uint32_t* __restrict__ keyOf, uint32_t* hist, uint32_t* done)
+__global__ void __launch_bounds__(256) k_morton(const float4* aabb, const uint32_t* list,
+                                                uint32_t n, const uint32_t* colWorld,
+                                                const uint32_t* bounds,
+                                                const float4* parts, uint32_t nParts,
+                                                uint32_t* keys, uint32_t* vals,
+                                                uint32_t* keyOf, uint32_t* hist, uint32_t* done)
 {
     chain_begin();
     __shared__ uint32_t sh[4 * 256];
@@ -455,10 +456,11 @@ __global__ void k_seg_starts(const uint32_t* __restrict__ offsets, const uint32_
 
 // Segment starts of the world-grouped manifold list (world of body a, non-decreasing): the thread at each world
 // change fills the starts of every world in the gap, so worlds without manifolds get empty segments.
-__global__ void k_manifold_segments(const Manifold* __restrict__ m, const uint32_t* __restrict__ nM,
-                                    const uint32_t* __restrict__ cbody, const uint32_t* __restrict__ bodyWorld,
-                                    uint32_t worlds, uint32_t* __restrict__ segStart)
+__global__ void k_manifold_segments(const Manifold* m, const uint32_t* nM,
+                                    const uint32_t* cbody, const uint32_t* bodyWorld,
+                                    uint32_t worlds, uint32_t* segStart)
 {
+    chain_begin();
     const uint32_t n = *nM;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
         const int prev = i == 0 ? -1 : int(bodyWorld[cbody[m[i - 1].a]]);
@@ -506,9 +508,9 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool valid)
 
 template <uint32_t SORT_ITEMS>
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(
-    const uint32_t* __restrict__ keysIn, const uint32_t* __restrict__ valsIn, uint32_t* __restrict__ keysOut,
-    uint32_t* __restrict__ valsOut, uint32_t n, uint32_t shift, const uint32_t* __restrict__ digitBase,
-    uint32_t* __restrict__ tileState, uint32_t* __restrict__ tileCounter, uint32_t* __restrict__ status)
+    const uint32_t* keysIn, const uint32_t* valsIn, uint32_t* keysOut,
+    uint32_t* valsOut, uint32_t n, uint32_t shift, const uint32_t* digitBase,
+    uint32_t* tileState, uint32_t* tileCounter, uint32_t* status)
 {
     chain_begin();
     constexpr uint32_t WARPS = SORT_THREADS / 32, SORT_TILE = SORT_THREADS * SORT_ITEMS;
@@ -689,11 +691,11 @@ __device__ __forceinline__ KarrasNode karras_node(int i, Delta delta)
 }
 
 // sortedWorld/segStart null: one segment [0, n), and the leaf boxes are gathered beside the build.
-__global__ void k_lbvh_build(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ sortedWorld,
-                             const uint32_t* __restrict__ segStart, int n, const uint32_t* __restrict__ vals,
-                             const float4* __restrict__ caabb, float4* __restrict__ leafAabb,
-                             int2* __restrict__ child, int* __restrict__ parent, int* __restrict__ leafParent,
-                             float4* __restrict__ meet, NodeRec* __restrict__ rec)
+__global__ void k_lbvh_build(const uint32_t* keys, const uint32_t* sortedWorld,
+                             const uint32_t* segStart, int n, const uint32_t* vals,
+                             const float4* caabb, float4* leafAabb,
+                             int2* child, int* parent, int* leafParent,
+                             float4* meet, NodeRec* rec)
 {
     chain_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -795,7 +797,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_tree_segments(TreeB
         // Bounds of the segment's boxes.
         float4 bb = make_float4(FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX);
         for (uint32_t i = threadIdx.x; i < n; i += THREADS) {
-            const float4 a = __ldg(t.caabb + __ldg(list + i));
+            const float4 a = t.caabb[__ldg(list + i)];
             bb = make_float4(fminf(bb.x, a.x), fminf(bb.y, a.y), fmaxf(bb.z, a.z), fmaxf(bb.w, a.w));
         }
         for (int o = 16; o > 0; o >>= 1) {
@@ -819,7 +821,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_tree_segments(TreeB
             const uint32_t i = base + k * 32u;
             pos[k] = i;
             key[k] = 0u;
-            if (k < per && i < n) key[k] = morton_key(__ldg(t.caabb + __ldg(list + i)), bb.x, bb.y, bb.z, bb.w);
+            if (k < per && i < n) key[k] = morton_key(t.caabb[__ldg(list + i)], bb.x, bb.y, bb.z, bb.w);
         }
         for (uint32_t shift = 0; shift < 32; shift += 8) {
             for (uint32_t i = threadIdx.x; i < WARPS * 256; i += THREADS) hist[i] = 0u;
@@ -889,7 +891,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_tree_segments(TreeB
             t.vals[lo + i] = c;
             t.keys[lo + i] = k;
             if (t.sortedWorld) t.sortedWorld[lo + i] = w;
-            t.leafAabb[lo + i] = __ldg(t.caabb + c);
+            t.leafAabb[lo + i] = t.caabb[c];
             if (i + 1 < n) {
                 const uint32_t x = k ^ sortKey[i + 1];
                 shared[i] = uint8_t(x ? __clz(x) : 32 + __clz(i ^ (i + 1)));
@@ -1026,9 +1028,9 @@ cudaError_t launch_tree_segments(const TreeBuild& t, uint32_t largest, uint32_t 
 // bounds in with one 16-byte atomic exchange; the first finds the empty marker and stops, the second receives its
 // sibling's bounds in the same operation (no flag, fence or second load on the chain), writes the node's record
 // and bounds and carries on upwards.
-__global__ void k_lbvh_refit(int n, const int2* __restrict__ child, const int* __restrict__ parent,
-                             const int* __restrict__ leafParent, const float4* __restrict__ leafAabb,
-                             float4* __restrict__ nodeAabb, float4* __restrict__ meet, NodeRec* __restrict__ rec)
+__global__ void k_lbvh_refit(int n, const int2* child, const int* parent,
+                             const int* leafParent, const float4* leafAabb,
+                             float4* nodeAabb, float4* meet, NodeRec* rec)
 {
     chain_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1144,12 +1146,12 @@ __device__ __forceinline__ uint32_t query_one(const TreeView& dyn, const TreeVie
 // has published its prefix. The pairs come out ordered by query rank, then traversal order; the last tile writes
 // the pair count.
 __global__ void __launch_bounds__(QUERY_MAX_THREADS) k_query(TreeView dyn, TreeView other,
-                                                             const uint32_t* __restrict__ cbody,
-                                                             uint2* __restrict__ pairs, uint32_t pairCap,
-                                                             uint32_t* __restrict__ total,
-                                                             uint32_t* __restrict__ status,
-                                                             uint32_t* __restrict__ tileState,
-                                                             uint32_t* __restrict__ tileCounter)
+                                                             const uint32_t* cbody,
+                                                             uint2* pairs, uint32_t pairCap,
+                                                             uint32_t* total,
+                                                             uint32_t* status,
+                                                             uint32_t* tileState,
+                                                             uint32_t* tileCounter)
 {
     chain_begin();
     __shared__ uint32_t kept[QUERY_STASH * QUERY_MAX_THREADS];   // [k][thread]
