@@ -953,7 +953,7 @@ struct TeamLaunch {
                           // smallest body index) into this array, initialised to parent[b] = b before the launch
 };
 // Host side: launches the team solver with 'threads' per CTA; returns the launch error.
-cudaError_t launch_color_solve_teams(uint32_t threads, bool pipelined, uint32_t grid, cudaStream_t stream,
+cudaError_t launch_color_solve_teams(bool chained, uint32_t threads, bool pipelined, uint32_t grid, cudaStream_t stream,
                                      const TeamLaunch& a);
 // Host side: co-resident CTAs per SM of the team solver at this CTA size and shared-memory capacities. Also raises
 // the kernel's dynamic shared-memory limit to TEAM_SMEM_MAX (the limit is per kernel, shared by every engine in the

@@ -1671,8 +1671,8 @@ struct ag2d_world {
 
     void integrateHalves(uint32_t phase)
     {
-        k_integrate<<<gridFor(nDynBody), 256, 0, stream>>>(view(), dynBody.p, nWorlds > 1 ? dynSimd.p : nullptr, nDynBody,
-                                                          integrateParams(), phase);
+        CK(chain_launch(chained(), k_integrate, gridFor(nDynBody), 256, 0, stream, view(), dynBody.p,
+                        nWorlds > 1 ? dynSimd.p : nullptr, nDynBody, integrateParams(), phase));
         CK(cudaGetLastError());
         launches++;
     }
@@ -1787,8 +1787,8 @@ struct ag2d_world {
         if (nWorlds > 1) {
             prevSeg.reserve(nWorlds + 1);
             if (!prevSegValid) {
-                k_manifold_segments<<<gridFor(manifoldCap), 256, 0, stream>>>(prevManifolds.p, nPrev.p, cbody.p,
-                                                                              bodyWorld.p, nWorlds, prevSeg.p);
+                CK(chain_launch(chained(), k_manifold_segments, gridFor(manifoldCap), 256, 0, stream, prevManifolds.p,
+                                nPrev.p, cbody.p, bodyWorld.p, nWorlds, prevSeg.p));
                 CK(cudaGetLastError());
                 launches++;
                 prevSegValid = true;
@@ -2021,7 +2021,7 @@ struct ag2d_world {
             k_wake<<<gridFor(manifoldCap), 256, 0, s>>>(view(), manifolds.p, nManifolds.p, wakeIsland.p, dCounters.p);
             launches++;
         }
-        k_wake_apply<<<gridFor(nBodies), 256, 0, s>>>(view(), wakeIsland.p, dCounters.p);
+        CK(chain_launch(chained(), k_wake_apply, gridFor(nBodies), 256, 0, s, view(), wakeIsland.p, dCounters.p));
         CK(cudaGetLastError());
         pend(8);
         launches++;
@@ -2339,7 +2339,8 @@ struct ag2d_world {
         L.bodies = jointBodies;
         L.status = &dCounters.p->status;
         if (jointBodies)
-            k_joints_flow<<<1, JOINT_THREADS, jointBodies * JOINT_FLOW_BODY_BYTES, stream>>>(view(), L);
+            CK(chain_launch(chained(), k_joints_flow, 1, JOINT_THREADS, jointBodies * JOINT_FLOW_BODY_BYTES, stream,
+                            view(), L));
         else
             k_joints<<<1, JOINT_THREADS, 0, stream>>>(view(), L);
         CK(cudaGetLastError());
@@ -2466,8 +2467,8 @@ struct ag2d_world {
                 launches++;
             }
             islandsLinked = true;
-            k_manifold_segments<<<gridFor(manifoldCap), 256, 0, s>>>(mm, nm, cbody.p, bodyWorld.p, nWorlds,
-                                                                      manSeg.p);
+            CK(chain_launch(chained(), k_manifold_segments, gridFor(manifoldCap), 256, 0, s, mm, nm, cbody.p,
+                            bodyWorld.p, nWorlds, manSeg.p));
             scratch.prio = prio.p;
             if (nBigTeams) {
                 // Worlds larger than a team: their own wide CTAs on the side stream, overlapping the small teams.
@@ -2475,7 +2476,7 @@ struct ag2d_world {
                 CK(cudaStreamWaitEvent(sideStream, forkEvent, 0));
                 const TeamLaunch big{w, mm, manSeg.p, teamWorld.p, teamOrder.p + nTeams, nBigTeams, bigBodyCap,
                                      bigConsCap, scratch, vi, pi, nextWorld.p + 1, ctr, ufParent.p};
-                CK(launch_color_solve_teams(bigThreads, bigPipelined, std::min(nBigTeams, bigBlocks), sideStream,
+                CK(launch_color_solve_teams(false, bigThreads, bigPipelined, std::min(nBigTeams, bigBlocks), sideStream,
                                             big));
                 launches++;
             }
@@ -2483,7 +2484,7 @@ struct ag2d_world {
                 const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(nTeams, teamBlocks));
                 const TeamLaunch args{w, mm, manSeg.p, teamWorld.p, teamOrder.p, nTeams, teamBodyCap, teamConsCap,
                                       scratch, vi, pi, nextWorld.p, ctr, ufParent.p};
-                CK(launch_color_solve_teams(teamThreads, false, grid, s, args));
+                CK(launch_color_solve_teams(chained() && !nBigTeams, teamThreads, false, grid, s, args));
             }
             if (nBigTeams) {
                 CK(cudaEventRecord(joinEvent, sideStream));

@@ -281,8 +281,9 @@ __global__ void k_wake(DeviceWorld w, const Manifold* __restrict__ m, const uint
         mark_wakes(w, m[i], wakeIsland);
 }
 
-__global__ void k_wake_apply(DeviceWorld w, const uint32_t* __restrict__ wakeIsland, StepCounters* counters)
+__global__ void k_wake_apply(DeviceWorld w, const uint32_t* wakeIsland, StepCounters* counters)
 {
+    chain_begin();
     uint32_t woke = 0;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nBodies; b += gridDim.x * blockDim.x) {
         if (w.bstate[b] == STATE_SLEEPING && w.sleepIsland[b] < w.nBodies && wakeIsland[w.sleepIsland[b]]) {
@@ -700,6 +701,7 @@ cudaError_t launch_color_solve_block(uint32_t manifolds, cudaStream_t stream, co
 template <uint32_t THREADS, bool PIPELINED>
 __global__ void __launch_bounds__(THREADS, PIPELINED ? 1 : 1024 / THREADS) k_color_solve_teams(TeamLaunch a)
 {
+    chain_begin();
     // [bodyCap] velocities, [bodyCap] poses, then 2 x [bodyCap] u64 colouring words, overwritten after colouring by
     // the constraint records (team_smem_bytes).
     extern __shared__ float4 teamCache[];
@@ -816,25 +818,25 @@ cudaError_t team_solver_blocks_per_sm(uint32_t threads, bool pipelined, uint32_t
 }
 
 template <uint32_t THREADS>
-static void launch_teams(bool pipelined, uint32_t grid, size_t smem, cudaStream_t stream, const TeamLaunch& a)
+static cudaError_t launch_teams(bool chained, bool pipelined, uint32_t grid, size_t smem, cudaStream_t stream,
+                                const TeamLaunch& a)
 {
-    if (pipelined) k_color_solve_teams<THREADS, true><<<grid, THREADS, smem, stream>>>(a);
-    else k_color_solve_teams<THREADS, false><<<grid, THREADS, smem, stream>>>(a);
+    return chain_launch(chained, pipelined ? k_color_solve_teams<THREADS, true> : k_color_solve_teams<THREADS, false>,
+                        grid, THREADS, smem, stream, a);
 }
 
-cudaError_t launch_color_solve_teams(uint32_t threads, bool pipelined, uint32_t grid, cudaStream_t stream,
+cudaError_t launch_color_solve_teams(bool chained, uint32_t threads, bool pipelined, uint32_t grid, cudaStream_t stream,
                                      const TeamLaunch& a)
 {
     const size_t smem = team_smem_bytes(a.bodyCap, a.consCap);
     if (smem > TEAM_SMEM_MAX) return cudaErrorInvalidValue;
     switch (threads) {
-    case 64: launch_teams<64>(pipelined, grid, smem, stream, a); break;
-    case 128: launch_teams<128>(pipelined, grid, smem, stream, a); break;
-    case 256: launch_teams<256>(pipelined, grid, smem, stream, a); break;
-    case 512: launch_teams<512>(pipelined, grid, smem, stream, a); break;
+    case 64: return launch_teams<64>(chained, pipelined, grid, smem, stream, a);
+    case 128: return launch_teams<128>(chained, pipelined, grid, smem, stream, a);
+    case 256: return launch_teams<256>(chained, pipelined, grid, smem, stream, a);
+    case 512: return launch_teams<512>(chained, pipelined, grid, smem, stream, a);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -392,6 +392,7 @@ __device__ __forceinline__ void word_store(float4* p, float x, float y, float z,
 // polls gave nothing.
 __global__ void __launch_bounds__(JOINT_THREADS) k_joints_flow(DeviceWorld w, JointLaunch L)
 {
+    chain_begin();
     extern __shared__ float4 jointSmem[];
     float4* const vel = jointSmem;                                            // [bodies] vx, vy, w, version
     JointBody* const body = reinterpret_cast<JointBody*>(vel + L.bodies);     // [bodies]
