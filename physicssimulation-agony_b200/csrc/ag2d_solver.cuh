@@ -597,9 +597,10 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
 // Colouring with carried colours: a manifold whose collider pair was solved last step (its hint) keeps that
 // step's colour when it was a first-fit one (< 64) and has been kept for fewer than COLOR_KEEP_STEPS steps in a
 // row (so each contact's place in the solving order is revisited regularly). Two kept manifolds of one colour
-// cannot share a dynamic body: their predecessors were coloured together last step, and a body's dynamic flag
-// (finite mass) does not change between steps. The other manifolds run the Jones-Plassmann rounds around the kept
-// colours. With no hints every manifold runs the rounds. s.color holds colour | age << COLOR_AGE_SHIFT.
+// cannot share a dynamic body (of finite mass): their predecessors were coloured together last step, and a body that
+// turned dynamic since has no coloured manifolds (the host drops their colours when a command gives it a mass). The
+// other manifolds run the Jones-Plassmann rounds around the kept colours. With no hints every manifold runs the
+// rounds. s.color holds colour | age << COLOR_AGE_SHIFT.
 // s.pairBodies words: body index | PAIR_DYNAMIC (finite mass) | PAIR_KEPT (first word: colour carried over) or
 // PAIR_TWO (second word: not a one-point contact).
 constexpr uint32_t PAIR_DYNAMIC = 0x80000000u, PAIR_KEPT = 0x40000000u, PAIR_TWO = 0x40000000u, PAIR_BODY = 0x3FFFFFFFu;

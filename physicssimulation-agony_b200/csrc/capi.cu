@@ -19,6 +19,7 @@
 #include <thread>
 #include <stdexcept>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 using namespace ag2d;
@@ -2678,9 +2679,11 @@ struct ag2d_world {
         // ObjectManager.cpp:678-687, and destroyColliderInternal): their colliders count as edited.
         std::vector<uint8_t> editedBody(nBodies, 0);
         bool anyEdited = false;
+        std::unordered_map<uint32_t, float> massBefore;   // inverse masses of the bodies given another, as stepped with
         // applyBodyMass (ObjectManager.cpp:867-905).
         auto applyMass = [&](uint32_t b, float m) {
             HBody& hb = o.bodies[b];
+            massBefore.emplace(b, vel[b].w);
             const float newMass = std::fmax(0.0f, m);
             const float oldMass = hb.mass;
             if (newMass > 0.0f) {
@@ -2949,6 +2952,12 @@ struct ag2d_world {
         jointCommands.clear();
         if (jointTotal()) jointsDirty = true;   // body states may have changed: constraint groups with them
         restoreWokenIslands(state, timer, island, wokenRoots, editedBody, anyEdited);
+        std::vector<uint8_t> freed(nBodies, 0);
+        bool anyFreed = false;
+        for (const auto& [b, w] : massBefore)
+            if (!(w > 0.0f) && vel[b].w > 0.0f) freed[b] = anyFreed = true;
+        if (anyFreed) forgetColours(freed);
+        hintsReady = false;   // a narrow phase run before the commands took its hints from the list as it was
         if (nBodies) {
             CK(cudaMemcpyAsync(bvel.p, vel.data(), nBodies * sizeof(float4), cudaMemcpyHostToDevice, s));
             CK(cudaMemcpyAsync(bpos.p, pos.data(), nBodies * sizeof(float4), cudaMemcpyHostToDevice, s));
@@ -2963,6 +2972,26 @@ struct ag2d_world {
         listsDirty = true;
         otherDirty = true;
         fullPose = true;
+    }
+
+    // The warm-start manifolds on bodies that were of infinite mass until now lose their colours. Contacts around such
+    // a body may share a colour (nothing moves it), around a movable one they may not, so they are coloured anew; the
+    // others' colours are those of a colouring in which they met no contact of their colour.
+    void forgetColours(const std::vector<uint8_t>& freed)
+    {
+        const cudaStream_t s = stream;
+        uint32_t np = 0;
+        CK(cudaMemcpyAsync(&np, nPrev.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (np == 0) return;
+        const std::vector<Manifold> prev = download(prevManifolds.p, np, s);
+        const std::vector<uint32_t> owner = download(cbody.p, nColliders, s);
+        std::vector<uint32_t> col = download(prevColor.p, np, s);
+        for (uint32_t i = 0; i < np; i++)
+            for (const uint32_t c : {prev[i].a, prev[i].b})
+                if (c < nColliders && freed[owner[c]]) col[i] = NO_COLOR;
+        CK(cudaMemcpyAsync(prevColor.p, col.data(), np * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+        CK(cudaStreamSynchronize(s));
     }
 
     // The command path's part of Simulation::flushCommands (Simulation.cpp:454-461): islands touching an edited
