@@ -334,8 +334,8 @@ constexpr uint32_t COLOR_AGE_SHIFT = 24;
 constexpr uint32_t COLOR_MASK = (1u << COLOR_AGE_SHIFT) - 1u;
 constexpr uint32_t COLOR_KEEP_STEPS = 16;
 
-// Colour counters: one per colour, then the lengths of the two uncoloured lists, then the colour count, then a second
-// counter per colour (one-point contacts placed from the colour's end).
+// Colour counters: one per colour, then whether kept colours clash, the lengths of the two uncoloured lists and the
+// colour count, then a second counter per colour (one-point contacts placed from the colour's end).
 constexpr uint32_t COLOR_SLOTS = 2 * MAX_COLORS + 4;
 // Colours 0..63 are chosen first-fit from a body's 64-bit mask of neighbouring colours; a manifold whose bodies see
 // all 64 taken gets colour 64 + its round (unique to the round, so still conflict-free).
@@ -600,7 +600,8 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
 // cannot share a dynamic body (of finite mass): their predecessors were coloured together last step, and a body that
 // turned dynamic since has no coloured manifolds (the host drops their colours when a command gives it a mass). The
 // other manifolds run the Jones-Plassmann rounds around the kept colours. With no hints every manifold runs the
-// rounds. s.color holds colour | age << COLOR_AGE_SHIFT.
+// rounds. Hints that two manifolds on one dynamic body share (from a checkpoint that was not saved so) end the routine
+// with STATUS_COLOR_CLASH before anything moves. s.color holds colour | age << COLOR_AGE_SHIFT.
 // s.pairBodies words: body index | PAIR_DYNAMIC (finite mass) | PAIR_KEPT (first word: colour carried over) or
 // PAIR_TWO (second word: not a one-point contact).
 constexpr uint32_t PAIR_DYNAMIC = 0x80000000u, PAIR_KEPT = 0x40000000u, PAIR_TWO = 0x40000000u, PAIR_BODY = 0x3FFFFFFFu;
@@ -627,6 +628,7 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
     constexpr uint32_t DYN = PAIR_DYNAMIC, KEPT = PAIR_KEPT;
     if (s.hint && !sync()) return false;   // the counters are zeroed before kept colours are counted
     uint32_t keptTop = 0;
+    bool clash = false;
     for (uint32_t i = rank; i < n; i += size) {
         const uint32_t bA = w.cbody[m[i].a], bB = w.cbody[m[i].b];
         const bool dA = B.invMass(bA) > 0.0f, dB = B.invMass(bB) > 0.0f;
@@ -637,8 +639,10 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
             s.color[i] = h | (age + 1) << COLOR_AGE_SHIFT;
             atomicAdd(Sync::GRID ? blockCount + h : s.colorCount + h, 1u);
             keptTop = max(keptTop, h + 1);
-            if (dA) atomicOr(B.maskWord(bA), 1ull << h);
-            if (dB) atomicOr(B.maskWord(bB), 1ull << h);
+            const unsigned long long bit = 1ull << h;
+            const unsigned long long taken = (dA ? atomicOr(B.maskWord(bA), bit) : 0ull) |
+                                             (dB ? atomicOr(B.maskWord(bB), bit) : 0ull);
+            clash |= (taken & bit) != 0;
         }
         s.pairBodies[i] = make_uint2(bA | (dA ? DYN : 0u) | (kept ? KEPT : 0u), bB | (dB ? DYN : 0u) | (m[i].count != 1u ? PAIR_TWO : 0u));
     }
@@ -655,7 +659,13 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
         for (int o = 16; o > 0; o >>= 1) keptTop = max(keptTop, __shfl_xor_sync(0xffffffffu, keptTop, o));
         if ((threadIdx.x & 31) == 0 && keptTop) atomicMax(nColors, keptTop);
     }
+    uint32_t* const clashes = s.colorCount + MAX_COLORS;   // the team's own word: every thread reads the same
+    if (clash) {
+        atomicExch(clashes, 1u);
+        atomicOr(status, STATUS_COLOR_CLASH);
+    }
     if (!sync()) return false;
+    if (s.hint && Sync::ld(clashes)) return false;
     uint32_t len = n;
     const uint4* in = nullptr;   // round 0 visits every manifold; later rounds the uncoloured records
     // Record j of this round: {manifold, priority, body A | dynamic bit, body B | dynamic bit}. In round 0 a kept

@@ -27,6 +27,7 @@ enum StatusBits : uint32_t {
     STATUS_HASH_FULL = 1u << 5,
     STATUS_STACK_OVERFLOW = 1u << 6,
     STATUS_EVENT_OVERFLOW = 1u << 7,
+    STATUS_COLOR_CLASH = 1u << 8,   // two contacts on one movable body were to keep the same colour
 };
 
 // Counters written by the kernels and read back by the host after each step (one 64-byte transfer).

@@ -1416,6 +1416,7 @@ struct ag2d_world {
             CK(cudaStreamSynchronize(stream));
             swap_bufs(prevColor, nb);
         }
+        if (color.n < manifoldCap) hintsReady = false;   // the hints go with the buffer
         color.reserve(manifoldCap);
         order.reserve(manifoldCap);
         prio.reserve(manifoldCap);
@@ -3080,6 +3081,12 @@ struct ag2d_world {
         prevSegValid = false;
     }
 
+    void dropHints()
+    {
+        hintsReady = false;
+        if (prevCount) CK(cudaMemsetAsync(prevColor.p, 0xFF, sizeof(uint32_t) * prevCount, stream));
+    }
+
     // One fixed step (Simulation::physicsStep order, Simulation.cpp:255-351).
     void stepOnce()
     {
@@ -3133,6 +3140,17 @@ struct ag2d_world {
             phaseIslands();
             readCounters();
             const uint32_t st = hCounters->status;
+            // Colours to keep that clash (a checkpoint's that was not saved so), or that may have made a wait run out: the
+            // next attempt or step colours every contact anew.
+            if (st & (STATUS_COLOR_CLASH | STATUS_BARRIER_TIMEOUT)) dropHints();
+            if (st == STATUS_COLOR_CLASH) {
+                snapshot(true);
+                if (nWorlds > 1) CK(cudaMemsetAsync(worldDirty.p, 0, sizeof(uint32_t) * nWorlds, s));
+                fullPose = fullPoseThisStep;
+                otherDirty = true;
+                CK(cudaStreamSynchronize(s));
+                continue;
+            }
             if (st & STATUS_EVENT_OVERFLOW) {
                 // The ring was too small for this step's events: grow it and step again from the saved state.
                 snapshot(true);
@@ -3163,7 +3181,7 @@ struct ag2d_world {
                 CK(cudaStreamSynchronize(s));
                 throw ApiError(AG2D_ERR_TIMEOUT, "a bounded device-side wait timed out (status " + std::to_string(st) + ")");
             }
-            if (st & (STATUS_COLOR_OVERFLOW | STATUS_HASH_FULL | STATUS_STACK_OVERFLOW)) {
+            if (st) {
                 snapshot(true);
                 CK(cudaStreamSynchronize(s));
                 throw ApiError(AG2D_ERR_CAPACITY, "capacity limit (colours, hash or traversal stack), status " + std::to_string(st));
@@ -4337,6 +4355,7 @@ int32_t ag2d_world_write(ag2d_world* world, int32_t field, const void* src, uint
             if (n > w.manifoldCap) w.reserveCapacities(std::max(n, w.pairCap), n);
             const bool prev = field == AG2D_PREV_MANIFOLDS;
             w.islandsLinked = false;   // the solver's links are not this list's
+            if (!prev) w.hintsReady = false;   // nor are the colours found for the list before it
             if (n) CK(cudaMemcpyAsync(prev ? w.prevManifolds.p : w.manifolds.p, src, bytes, cudaMemcpyHostToDevice, s));
             CK(cudaMemcpyAsync(prev ? w.nPrev.p : w.nManifolds.p, &n, 4, cudaMemcpyHostToDevice, s));
             if (prev) {
