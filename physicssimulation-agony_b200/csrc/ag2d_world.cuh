@@ -28,6 +28,7 @@ enum StatusBits : uint32_t {
     STATUS_STACK_OVERFLOW = 1u << 6,
     STATUS_EVENT_OVERFLOW = 1u << 7,
     STATUS_COLOR_CLASH = 1u << 8,   // two contacts on one movable body were to keep the same colour
+    STATUS_SOLVER_STATE = 1u << 9,  // the grid solver met a record or a body version that it cannot have made
 };
 
 // Counters written by the kernels and read back by the host after each step (one 64-byte transfer).

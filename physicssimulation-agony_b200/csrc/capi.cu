@@ -459,6 +459,8 @@ static void* kernel_reach(const void* p, size_t align)
     return a.devicePointer;
 }
 
+constexpr const char* SOLVER_STATE_ERROR = "the grid solver met a record or a body version that it cannot have made";
+
 // Transfers up to this size go between page-locked host memory and the device inside a kernel (packed reads, small
 // checkpoints): a copy operation adds about eight microseconds to a kernel that is there anyway, and above it the copy
 // engine's bandwidth counts.
@@ -3142,7 +3144,7 @@ struct ag2d_world {
             const uint32_t st = hCounters->status;
             // Colours to keep that clash (a checkpoint's that was not saved so), or that may have made a wait run out: the
             // next attempt or step colours every contact anew.
-            if (st & (STATUS_COLOR_CLASH | STATUS_BARRIER_TIMEOUT)) dropHints();
+            if (st & (STATUS_COLOR_CLASH | STATUS_BARRIER_TIMEOUT | STATUS_SOLVER_STATE)) dropHints();
             if (st == STATUS_COLOR_CLASH) {
                 snapshot(true);
                 if (nWorlds > 1) CK(cudaMemsetAsync(worldDirty.p, 0, sizeof(uint32_t) * nWorlds, s));
@@ -3180,6 +3182,11 @@ struct ag2d_world {
                 snapshot(true);
                 CK(cudaStreamSynchronize(s));
                 throw ApiError(AG2D_ERR_TIMEOUT, "a bounded device-side wait timed out (status " + std::to_string(st) + ")");
+            }
+            if (st & STATUS_SOLVER_STATE) {
+                snapshot(true);
+                CK(cudaStreamSynchronize(s));
+                throw ApiError(AG2D_ERR_CUDA, SOLVER_STATE_ERROR);
             }
             if (st) {
                 snapshot(true);
@@ -4498,6 +4505,7 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
         w.readCounters();
         if (w.hCounters->status & (STATUS_BARRIER_TIMEOUT | STATUS_LOOKBACK_TIMEOUT))
             throw ApiError(AG2D_ERR_TIMEOUT, "a bounded device-side wait timed out");
+        if (w.hCounters->status & STATUS_SOLVER_STATE) throw ApiError(AG2D_ERR_CUDA, SOLVER_STATE_ERROR);
         if (w.hCounters->status) throw ApiError(AG2D_ERR_CAPACITY, "phase status " + std::to_string(w.hCounters->status));
     });
 }

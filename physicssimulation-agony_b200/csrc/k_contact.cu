@@ -326,7 +326,8 @@ __device__ __forceinline__ void flow_store(float4* p, const float4& v)
 }
 
 // One end of a constraint in the dataflow: waits until its body's version is 'need' (a body without a version, of
-// infinite mass, is always ready). Polled by a whole warp; false when the wait ran out somewhere on the grid.
+// infinite mass, is always ready). Polled by a whole warp; false when the wait ran out somewhere on the grid, or when a
+// body is past the version waited for, which then never comes.
 struct FlowEnd {
     const float4* at;   // null: nothing to wait for
     uint32_t need;
@@ -350,24 +351,25 @@ __device__ __forceinline__ bool flow_wait(const FlowEnd& a, const FlowEnd& b, fl
         }
         gap = __reduce_max_sync(0xffffffffu, gap);
         if (gap == 0) return true;
+        if (int32_t(gap) < 0) { atomicOr(statusOut, STATUS_SOLVER_STATE); return false; }
         // The missing updates follow one another, half a microsecond each at least: a warp that lacks several sleeps
         // instead of loading the L2 with its polls (all waiting warps polling: 2.5 us a hop).
         if (gap > 1u) __nanosleep(min(gap - 1u, 8u) * 300u);
         if ((spins & 1023u) == 1023u) {
-            const bool gone = (*status & STATUS_BARRIER_TIMEOUT) != 0;
+            const bool gone = (*status & (STATUS_BARRIER_TIMEOUT | STATUS_SOLVER_STATE)) != 0;
             if (__any_sync(0xffffffffu, gone)) return false;
             if (spins > SPIN_LIMIT) { atomicOr(statusOut, STATUS_BARRIER_TIMEOUT); return false; }
         }
     }
 }
 
-// Whether slot c holds a record to solve. A record that names no body of the world is not one that the build above
-// wrote: it is reported and skipped, and the waits on it end.
+// Whether slot c holds a record to solve. Every slot below a colour's end has one, made by the lane that reads it, with
+// bodies of the world; any other is reported as what it is and skipped, and the waits on it end.
 __device__ __forceinline__ bool flow_live(uint32_t c, const Constraint& k, uint32_t nBodies, uint32_t* status)
 {
     if (c == 0xFFFFFFFFu) return false;
     if (k.bodyA < nBodies && k.bodyB < nBodies) return true;
-    atomicOr(status, STATUS_BARRIER_TIMEOUT);
+    atomicOr(status, STATUS_SOLVER_STATE);
     return false;
 }
 
