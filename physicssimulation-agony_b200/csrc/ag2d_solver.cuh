@@ -913,11 +913,13 @@ cudaError_t block_solver_init();
 // versions instead of barriers (k_color_solve_flow).
 constexpr uint32_t FLOW_VEL_WARPS = 16, FLOW_POS_WARPS = 4;   // warps of a CTA: velocity passes, position passes
 constexpr uint32_t FLOW_THREADS = 32 * (FLOW_VEL_WARPS + FLOW_POS_WARPS);
+constexpr uint32_t FLOW_HIGH = MAX_COLORS / 64 - 1;
 struct FlowScratch {
     float4* vel;       // [bodies] vx, vy, w, version
     float4* pos;       // [bodies] x, y, -, version
-    Constraint* cons;  // [manifolds] records, 'pad' the rank and degree of a, of b: one byte each
+    Constraint* cons;  // [manifolds] records, 'pad' the rank of a and its degree less one, those of b: one byte each
     float4* posRec;    // [2 x manifolds] position records: normal, penetration base, ranks; masses, bodies
+    unsigned long long* high;   // [FLOW_HIGH x bodies] colours above the first-fit 64 around each body, written on use
     uint32_t* parent;  // [bodies] islands to link beside the solve, every body its own; or null
 };
 __global__ void __launch_bounds__(FLOW_THREADS, 1)

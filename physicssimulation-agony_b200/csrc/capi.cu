@@ -590,6 +590,7 @@ struct ag2d_world {
     DBuf<unsigned long long> bodyMax, bodyMask;
     DBuf<float4> flowVel, flowPos, flowPosRec;   // grid solver (FlowScratch)
     DBuf<Constraint> flowCons;
+    DBuf<unsigned long long> flowHigh;
     // Manifolds of sleeping islands (k_islands.cu): world-grouped records and the island (root body) of each, with
     // the back buffers the sleep pass scatters into. isleUpper bounds the count as the host knows it (0: empty).
     DBuf<Manifold> isle, bk_isle;
@@ -2510,7 +2511,8 @@ struct ag2d_world {
             }
             flowVel.reserve(nBodies); flowPos.reserve(nBodies); flowPosRec.reserve(2 * size_t(manifoldCap));
             flowCons.reserve(manifoldCap);
-            FlowScratch flow{flowVel.p, flowPos.p, flowCons.p, flowPosRec.p, begun ? ufParent.p : nullptr};
+            flowHigh.reserve(FLOW_HIGH * size_t(nBodies));
+            FlowScratch flow{flowVel.p, flowPos.p, flowCons.p, flowPosRec.p, flowHigh.p, begun ? ufParent.p : nullptr};
             islandsLinked = begun;   // the step's first kernel made every body its own island
             uint32_t* barp = bar.p;
             const uint32_t est = std::min<uint32_t>(manifoldCap, lastManifolds + lastManifolds / 2 + 1024);

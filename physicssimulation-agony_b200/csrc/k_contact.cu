@@ -373,6 +373,14 @@ __device__ __forceinline__ bool flow_live(uint32_t c, const Constraint& k, uint3
     return false;
 }
 
+// From a body's byte pair (rank, degree less one): the version its constraint waits for in pass p, and whether the
+// constraint is the body's last one.
+__device__ __forceinline__ uint32_t flow_need(uint32_t pass, uint32_t pair)
+{
+    return pass * (((pair >> 8) & 255u) + 1u) + (pair & 255u);
+}
+__device__ __forceinline__ bool flow_last(uint32_t pair) { return (pair & 255u) == ((pair >> 8) & 255u); }
+
 // Islands' union-find in global memory (see k_island_union): links the bodies of one pair if both are dynamic.
 __device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t x)
 {
@@ -414,7 +422,7 @@ struct FlowWalk {
 // Colouring and solve of a large single world on a cooperative grid. The passes have no barriers: a body's constraints
 // act on it in colour order, pass after pass, so its k-th update must follow its (k - 1)-th and nothing else. Every
 // body carries a version (the updates made so far) in the same 16-byte word as its velocity, and a constraint, the
-// r-th of the d around a body (both from the body's mask of colours), waits in pass p for version p d + r of each of
+// r-th of the d around a body (both from the body's masks of colours), waits in pass p for version p d + r of each of
 // its moving bodies. Warps take the constraints in colour order within a pass and the passes in order, all warps are
 // resident, so the oldest unfinished constraint can always run. Velocity passes (warm start first) and position passes
 // touch different state and run on warps of their own. The order of the updates of every body is that of the
@@ -422,7 +430,9 @@ struct FlowWalk {
 // Bound: the chain of updates along the contacts (a pass costs about one hop a colour, a hop one L2 round trip for
 // the store, half a poll and the arithmetic). With a grid barrier a colour instead, and on the sixteen SMs that one
 // thread-block cluster has, a pass over the pile of 100,000 bodies (128,000 manifolds, 14 colours) took 8 us a colour.
-// A colouring beyond the 64 first-fit colours has no rank in the masks: its passes run with the grid barrier.
+// Colours beyond the 64 first-fit ones, which a body with that many contacts brings, have masks of their own, filled
+// only then. With a grid barrier a colour instead, 7,200 compound bodies of 16 boxes (53,000 manifolds, 108 colours) took
+// 5,528 us a solve, 1,793 here.
 __global__ void __launch_bounds__(FLOW_THREADS, 1)
 k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, FlowScratch f, uint32_t velIters,
                    uint32_t posIters, uint32_t* bar, StepCounters* counters)
@@ -435,13 +445,20 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
     const GridSync sync{bar, &counters->status};
     uint32_t ncol = 0;
     if (!color_manifolds(w, B, m, n, s, rank, size, sync, &counters->colors, &counters->status, ncol)) return;
-    if (ncol > 64u) {
-        if (f.parent)
-            for (uint32_t i = rank; i < n; i += size) uf_link(w, f.parent, w.cbody[m[i].a], w.cbody[m[i].b]);
-        solve_colored(w, B, m, n, s, ncol, velIters, posIters, rank, size, sync);
-        return;
+    if (ncol > 64u) {   // the colours above the first-fit ones, around each body
+        for (uint32_t i = rank; i < FLOW_HIGH * w.nBodies; i += size) f.high[i] = 0ull;
+        if (!sync()) return;
+        for (uint32_t i = rank; i < n; i += size) {
+            const uint32_t c = s.color[i] & COLOR_MASK;
+            if (c < 64u) continue;
+            const uint2 q = s.pairBodies[i];
+            for (const uint32_t b : {q.x, q.y})
+                if (b & PAIR_DYNAMIC)
+                    atomicOr(f.high + FLOW_HIGH * (b & PAIR_BODY) + (c >> 6) - 1u, 1ull << (c & 63u));
+        }
+        if (!sync()) return;
     }
-    __shared__ uint32_t start[65], chunk[65];
+    __shared__ uint32_t start[MAX_COLORS + 1], chunk[MAX_COLORS + 1];
     for (uint32_t c = threadIdx.x; c <= ncol; c += blockDim.x) start[c] = __ldcg(s.colorStart + c);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -464,16 +481,23 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
             const uint32_t mi = __ldcg(s.order + c);
             Constraint k;
             prep_constraint(w, B, m[mi], mi, k);
-            const unsigned long long below = (1ull << walk.col) - 1ull;
-            uint32_t ranks = 0;   // rank and degree of a, of b: one byte each
-            if (k.imA > 0.0f) {
-                const unsigned long long mask = __ldcg(s.bodyMask + k.bodyA);
-                ranks |= uint32_t(__popcll(mask & below)) | uint32_t(__popcll(mask)) << 8;
-            }
-            if (k.imB > 0.0f) {
-                const unsigned long long mask = __ldcg(s.bodyMask + k.bodyB);
-                ranks |= uint32_t(__popcll(mask & below)) << 16 | uint32_t(__popcll(mask)) << 24;
-            }
+            // A movable body's byte pair: this colour's rank among those around it, and their number less one.
+            auto place = [&](uint32_t b) {
+                const unsigned long long below = (1ull << (walk.col & 63u)) - 1ull, first = __ldcg(s.bodyMask + b);
+                uint32_t r = __popcll(walk.col < 64u ? first & below : first), d = __popcll(first);
+                if (ncol > 64u)
+                    for (uint32_t j = 0; j < FLOW_HIGH; j++) {
+                        const unsigned long long mask = __ldcg(f.high + FLOW_HIGH * b + j);
+                        const uint32_t word = walk.col >> 6;   // 0: the first-fit colours
+                        if (j + 1u < word) r += __popcll(mask);
+                        else if (j + 1u == word) r += __popcll(mask & below);
+                        d += __popcll(mask);
+                    }
+                return r | (d - 1u) << 8;
+            };
+            uint32_t ranks = 0;
+            if (k.imA > 0.0f) ranks |= place(k.bodyA);
+            if (k.imB > 0.0f) ranks |= place(k.bodyB) << 16;
             k.pad = __uint_as_float(ranks);
             f.cons[c] = k;
             f.posRec[2 * size_t(c)] = make_float4(k.nx, k.ny, k.penBase, __uint_as_float(ranks));
@@ -510,8 +534,8 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
                 const BlockMatrix bm = block_matrix(k);   // needs no body: done before the wait
                 const uint32_t ranks = live ? __float_as_uint(k.pad) : 0u;
                 const bool mA = live && k.imA > 0.0f, mB = live && k.imB > 0.0f;
-                const FlowEnd a{mA ? f.vel + k.bodyA : nullptr, pass * ((ranks >> 8) & 255u) + (ranks & 255u)};
-                const FlowEnd b{mB ? f.vel + k.bodyB : nullptr, pass * (ranks >> 24) + ((ranks >> 16) & 255u)};
+                const FlowEnd a{mA ? f.vel + k.bodyA : nullptr, flow_need(pass, ranks)};
+                const FlowEnd b{mB ? f.vel + k.bodyB : nullptr, flow_need(pass, ranks >> 16)};
                 float4 vA = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vB = vA;
                 if (live && !mA) vA = w.bvel[k.bodyA];
                 if (live && !mB) vB = w.bvel[k.bodyB];
@@ -527,11 +551,11 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
                     }
                     if (mA) {
                         flow_store(f.vel + k.bodyA, make_float4(vA.x, vA.y, vA.z, __uint_as_float(a.need + 1u)));
-                        if (pass == velIters && (ranks & 255u) + 1u == ((ranks >> 8) & 255u)) w.bvel[k.bodyA] = vA;
+                        if (pass == velIters && flow_last(ranks)) w.bvel[k.bodyA] = vA;
                     }
                     if (mB) {
                         flow_store(f.vel + k.bodyB, make_float4(vB.x, vB.y, vB.z, __uint_as_float(b.need + 1u)));
-                        if (pass == velIters && ((ranks >> 16) & 255u) + 1u == ranks >> 24) w.bvel[k.bodyB] = vB;
+                        if (pass == velIters && flow_last(ranks >> 16)) w.bvel[k.bodyB] = vB;
                     }
                     if (pass == velIters) {
                         Manifold& d = m[k.manifold];
@@ -558,8 +582,8 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
                 }
                 const bool live = flow_live(c, k, w.nBodies, &counters->status);
                 const bool mA = live && k.imA > 0.0f, mB = live && k.imB > 0.0f;
-                const FlowEnd a{mA ? f.pos + k.bodyA : nullptr, pass * ((ranks >> 8) & 255u) + (ranks & 255u)};
-                const FlowEnd b{mB ? f.pos + k.bodyB : nullptr, pass * (ranks >> 24) + ((ranks >> 16) & 255u)};
+                const FlowEnd a{mA ? f.pos + k.bodyA : nullptr, flow_need(pass, ranks)};
+                const FlowEnd b{mB ? f.pos + k.bodyB : nullptr, flow_need(pass, ranks >> 16)};
                 float4 pA = make_float4(0.0f, 0.0f, 0.0f, 0.0f), pB = pA;
                 if (live && !mA) pA = w.bpos[k.bodyA];
                 if (live && !mB) pB = w.bpos[k.bodyB];
@@ -568,12 +592,12 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
                     position_solve(k, pA, pB);
                     if (mA) {
                         flow_store(f.pos + k.bodyA, make_float4(pA.x, pA.y, 0.0f, __uint_as_float(a.need + 1u)));
-                        if (pass + 1u == posIters && (ranks & 255u) + 1u == ((ranks >> 8) & 255u))
+                        if (pass + 1u == posIters && flow_last(ranks))
                             *reinterpret_cast<float2*>(w.bpos + k.bodyA) = make_float2(pA.x, pA.y);
                     }
                     if (mB) {
                         flow_store(f.pos + k.bodyB, make_float4(pB.x, pB.y, 0.0f, __uint_as_float(b.need + 1u)));
-                        if (pass + 1u == posIters && ((ranks >> 16) & 255u) + 1u == ranks >> 24)
+                        if (pass + 1u == posIters && flow_last(ranks >> 16))
                             *reinterpret_cast<float2*>(w.bpos + k.bodyB) = make_float2(pB.x, pB.y);
                     }
                 }
