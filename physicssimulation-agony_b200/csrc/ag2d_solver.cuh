@@ -918,7 +918,8 @@ struct FlowScratch {
     float4* vel;       // [bodies] vx, vy, w, version
     float4* pos;       // [bodies] x, y, -, version
     Constraint* cons;  // [manifolds] records, 'pad' the rank of a and its degree less one, those of b: one byte each
-    float4* posRec;    // [2 x manifolds] position records: normal, penetration base, ranks; masses, bodies
+    float4 *posA, *posB;   // [manifolds] position records: normal, penetration base, ranks; masses, bodies. They may lie
+                           // over the lists of uncoloured manifolds, which are done with by then
     unsigned long long* high;   // [FLOW_HIGH x bodies] colours above the first-fit 64 around each body, written on use
     uint32_t* parent;  // [bodies] islands to link beside the solve, every body its own; or null
 };

@@ -588,8 +588,7 @@ struct ag2d_world {
     bool hintsReady = false;   // this step's lookup wrote the hints
     DBuf<uint4> listA, listB;
     DBuf<unsigned long long> bodyMax, bodyMask;
-    DBuf<float4> flowVel, flowPos, flowPosRec;   // grid solver (FlowScratch)
-    DBuf<Constraint> flowCons;
+    DBuf<float4> flowVel, flowPos;   // grid solver (FlowScratch); its records lie in consQ, listA and listB
     DBuf<unsigned long long> flowHigh;
     // Manifolds of sleeping islands (k_islands.cu): world-grouped records and the island (root body) of each, with
     // the back buffers the sleep pass scatters into. isleUpper bounds the count as the host knows it (0: empty).
@@ -769,6 +768,7 @@ struct ag2d_world {
         bodyMax.reserve(nBodies);
         bodyMask.reserve(nBodies);
         ufParent.reserve(nBodies); ufFlag.reserve(nBodies); wakeIsland.reserve(nBodies);
+        reserveGridSolver();
         const uint32_t cap = std::max<uint32_t>(INITIAL_PAIRS_PER_COLLIDER * nColliders, 4096);
         if (!capsKnown && (cap > pairCap || cap > manifoldCap))
             reserveCapacities(std::max(pairCap + pairCap / 2, cap), std::max(manifoldCap + manifoldCap / 2, cap));
@@ -1534,6 +1534,7 @@ struct ag2d_world {
         bodyMax.reserve(nBodies);
         bodyMask.reserve(nBodies);
         ufParent.reserve(nBodies); ufFlag.reserve(nBodies); wakeIsland.reserve(nBodies);
+        reserveGridSolver();
         const uint32_t cap = std::max<uint32_t>(INITIAL_PAIRS_PER_COLLIDER * nColliders, 4096);
         reserveCapacities(std::max(pairCap, cap), std::max(manifoldCap, cap));
         CK(cudaMemsetAsync(nPrev.p, 0, sizeof(uint32_t), s));
@@ -2449,6 +2450,15 @@ struct ag2d_world {
     // A single world small enough for one CTA's solver.
     bool blockSolver() const { return nWorlds == 1 && nBodies <= BLOCK_SOLVE_BODIES && !dev.gridOnly; }
 
+    // The grid solver's words per body, with the other buffers of the bodies: a step does not allocate.
+    void reserveGridSolver()
+    {
+        if (nWorlds > 1 || blockSolver()) return;
+        flowVel.reserve(nBodies);
+        flowPos.reserve(nBodies);
+        flowHigh.reserve(FLOW_HIGH * size_t(nBodies));
+    }
+
     void phaseSolve()
     {
         const cudaStream_t s = stream;
@@ -2509,10 +2519,11 @@ struct ag2d_world {
                 CK(cudaMemsetAsync(bodyMask.p, 0, sizeof(unsigned long long) * nBodies, s));
                 CK(cudaMemsetAsync(bar.p, 0, 2 * sizeof(uint32_t), s));
             }
-            flowVel.reserve(nBodies); flowPos.reserve(nBodies); flowPosRec.reserve(2 * size_t(manifoldCap));
-            flowCons.reserve(manifoldCap);
-            flowHigh.reserve(FLOW_HIGH * size_t(nBodies));
-            FlowScratch flow{flowVel.p, flowPos.p, flowCons.p, flowPosRec.p, flowHigh.p, begun ? ufParent.p : nullptr};
+            reserveGridSolver();
+            static_assert(sizeof(Constraint) == ConsRecords::FIELDS * sizeof(float4), "records of either form fit consQ");
+            FlowScratch flow{flowVel.p, flowPos.p, reinterpret_cast<Constraint*>(consQ.p),
+                             reinterpret_cast<float4*>(listA.p), reinterpret_cast<float4*>(listB.p), flowHigh.p,
+                             begun ? ufParent.p : nullptr};
             islandsLinked = begun;   // the step's first kernel made every body its own island
             uint32_t* barp = bar.p;
             const uint32_t est = std::min<uint32_t>(manifoldCap, lastManifolds + lastManifolds / 2 + 1024);

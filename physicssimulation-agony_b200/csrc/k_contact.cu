@@ -500,8 +500,8 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
             if (k.imB > 0.0f) ranks |= place(k.bodyB) << 16;
             k.pad = __uint_as_float(ranks);
             f.cons[c] = k;
-            f.posRec[2 * size_t(c)] = make_float4(k.nx, k.ny, k.penBase, __uint_as_float(ranks));
-            f.posRec[2 * size_t(c) + 1] = make_float4(k.imA, k.imB, __uint_as_float(k.bodyA), __uint_as_float(k.bodyB));
+            f.posA[c] = make_float4(k.nx, k.ny, k.penBase, __uint_as_float(ranks));
+            f.posB[c] = make_float4(k.imA, k.imB, __uint_as_float(k.bodyA), __uint_as_float(k.bodyB));
         }
     }
     for (uint32_t b = rank; b < w.nBodies; b += size) {
@@ -576,7 +576,7 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
                 uint32_t ranks = 0;
                 k.imA = k.imB = 0.0f;
                 if (c != 0xFFFFFFFFu) {
-                    const float4 r0 = __ldcg(f.posRec + 2 * size_t(c)), r1 = __ldcg(f.posRec + 2 * size_t(c) + 1);
+                    const float4 r0 = __ldcg(f.posA + c), r1 = __ldcg(f.posB + c);
                     k.nx = r0.x; k.ny = r0.y; k.penBase = r0.z; ranks = __float_as_uint(r0.w);
                     k.imA = r1.x; k.imB = r1.y; k.bodyA = __float_as_uint(r1.z); k.bodyB = __float_as_uint(r1.w);
                 }
