@@ -5,6 +5,7 @@
 #include "host_objects.hpp"
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -288,6 +289,18 @@ struct CkptHeader {
     uint64_t totalBytes;
     uint64_t off[NCK], len[NCK];
 };
+
+// The bytes of every section for the header's counts.
+std::array<uint64_t, NCK> checkpoint_lengths(const CkptHeader& h)
+{
+    const uint64_t b = h.nBodies, c = h.nColliders, m = h.nPrev, wp = uint64_t(std::max<uint32_t>(h.nWorlds, 1)) + 1,
+                   si = h.nIsle;
+    return {b * 16, b * 16, b * 8, b * 4, b * 4, b * 4, b, b * 4,
+            c * 4, c * 4, c * 4, c * 16, c * 16, c * 16, c * 4, c * 4,
+            uint64_t(h.nCircles) * 4, uint64_t(h.nBoxes) * 8, uint64_t(h.nPolygons) * 4, uint64_t(h.nPolygons) * 4,
+            uint64_t(h.nPolyVerts) * 8, uint64_t(h.nPolyVerts) * 8, uint64_t(h.nMaterialRows) * 16, m * sizeof(Manifold),
+            m * 4, wp * 4, wp * 4, si * sizeof(Manifold), si * 4};
+}
 
 // One world's state in the upload format (host arrays), and the warm-start manifolds.
 struct PackedArrays {
@@ -1173,13 +1186,7 @@ struct ag2d_world {
         CK(cudaMemcpyAsync(&h.nPrev, nPrev.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
         CK(cudaMemcpyAsync(&h.nIsle, nIsle.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
-        const uint64_t b = nBodies, c = nColliders, m = h.nPrev, wp = uint64_t(nWorlds) + 1, si = h.nIsle;
-        const uint64_t len[NCK] = {
-            b * 16, b * 16, b * 8, b * 4, b * 4, b * 4, b, b * 4,
-            c * 4, c * 4, c * 4, c * 16, c * 16, c * 16, c * 4, c * 4,
-            uint64_t(nCircles) * 4, uint64_t(nBoxes) * 8, uint64_t(nPolygons) * 4, uint64_t(nPolygons) * 4,
-            uint64_t(nPolyVerts) * 8, uint64_t(nPolyVerts) * 8, uint64_t(nMaterialRows) * 16, m * sizeof(Manifold),
-            m * 4, wp * 4, wp * 4, si * sizeof(Manifold), si * 4};
+        const auto len = checkpoint_lengths(h);
         uint64_t at = (sizeof(CkptHeader) + 255) & ~uint64_t(255);
         for (uint32_t k = 0; k < NCK; k++) {
             h.off[k] = at;
@@ -1225,7 +1232,9 @@ struct ag2d_world {
         nWorlds = std::max<uint32_t>(h.nWorlds, 1);
         // A small page-locked checkpoint goes over in one kernel that reads the sections where they lie, a large or
         // pageable one in a copy a section.
-        const void* const mapped = h.totalBytes <= 4 * HOST_DIRECT_BYTES ? kernel_reach(src, 16) : nullptr;
+        // The kernel moves 16 bytes at a time; saved sections lie at multiples of 256.
+        const bool aligned = std::all_of(h.off, h.off + NCK, [](uint64_t o) { return o % 16 == 0; });
+        const void* const mapped = aligned && h.totalBytes <= 4 * HOST_DIRECT_BYTES ? kernel_reach(src, 16) : nullptr;
         SectionCopies sections{};
         auto put = [&](void* dst, uint32_t k) {
             if (!h.len[k]) return;
@@ -4766,10 +4775,9 @@ static CkptHeader checked_checkpoint(const void* src, uint64_t bytes)
     for (uint32_t k = 0; k < NCK; k++)
         if (h.off[k] > h.totalBytes || h.len[k] > h.totalBytes - h.off[k])
             throw ApiError(AG2D_ERR_INVALID_ARG, "checkpoint section out of range");
-    if (h.len[CK_WBODY] != (uint64_t(std::max<uint32_t>(h.nWorlds, 1)) + 1) * 4 ||
-        h.len[CK_WCOL] != h.len[CK_WBODY] || h.len[CK_VEL] != uint64_t(h.nBodies) * 16 ||
-        h.len[CK_CBODY] != uint64_t(h.nColliders) * 4 || h.len[CK_ISLE] != uint64_t(h.nIsle) * sizeof(Manifold) ||
-        h.len[CK_ISLEID] != uint64_t(h.nIsle) * 4 || h.len[CK_PREV] != uint64_t(h.nPrev) * sizeof(Manifold))
+    // Each section fills a buffer of its count, whichever way it goes over.
+    const auto len = checkpoint_lengths(h);
+    if (!std::equal(len.begin(), len.end(), h.len))
         throw ApiError(AG2D_ERR_INVALID_ARG, "checkpoint sizes inconsistent");
     return h;
 }
