@@ -23,6 +23,8 @@
 #include <unordered_map>
 #include <vector>
 
+#include <cuda.h>
+
 using namespace ag2d;
 
 namespace {
@@ -449,27 +451,62 @@ static float reference_angle(float rotA, float rotB)
     return a;
 }
 
-// Host memory the device can copy into directly: page-locked by cudaHostAlloc or cudaHostRegister (any CUDA runtime
-// of the process; the driver tracks it).
-static bool page_locked(const void* p)
+// The page-locked allocation or registration that holds host address p (by any CUDA runtime of the process; the driver
+// tracks them); size 0: none.
+struct HostRange {
+    uintptr_t start = 0;
+    size_t size = 0;
+    void* device = nullptr;   // p as the device reaches it
+    int access = 0;           // CU_POINTER_ATTRIBUTE_ACCESS_FLAG_*
+};
+static HostRange host_range(const void* p)
 {
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeHost;
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &found) != cudaSuccess) {
+            (void)cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<Query>(fn);
+    }();
+    unsigned type = 0;
+    CUdeviceptr device = 0, start = 0;
+    size_t size = 0;
+    int access = 0, managed = 0;
+    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                   CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, CU_POINTER_ATTRIBUTE_IS_MANAGED};
+    void* out[] = {&type, &device, &start, &size, &access, &managed};
+    if (!query || query(6, which, out, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST ||
+        managed)
+        return {};
+    return {uintptr_t(start), size, reinterpret_cast<void*>(device), access};
 }
-// Where kernels reach page-locked host memory that is aligned to 'align' bytes; null for any other memory.
-static void* kernel_reach(const void* p, size_t align)
+
+// Whether the device can copy to and from host memory [p, p + bytes) directly. Memory whose front alone is page-locked
+// is refused: the copy would be, and a kernel would fault. (A range over several registrations is the copy's to judge.)
+static bool page_locked(const void* p, size_t bytes)
 {
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        (void)cudaGetLastError();
+    const HostRange r = host_range(p);
+    if (!r.size) return false;
+    const uintptr_t end = r.start + r.size;
+    if (reinterpret_cast<uintptr_t>(p) + bytes > end && !host_range(reinterpret_cast<const void*>(end)).size)
+        throw ApiError(AG2D_ERR_CUDA, "host memory is page-locked only in part");
+    return true;
+}
+// Where kernels reach page-locked host memory [p, p + bytes) that is aligned to 'align' bytes and lies in one allocation
+// or registration, to read it or ('write') to write it; null for any other memory.
+static void* kernel_reach(const void* p, size_t bytes, size_t align, bool write)
+{
+    const HostRange r = host_range(p);
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    const int need = write ? CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE : CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READ;
+    if (!r.size || r.device != p || at % align || at < r.start || bytes > r.start + r.size - at ||
+        (r.access & need) != need)
         return nullptr;
-    }
-    if (a.type != cudaMemoryTypeHost || reinterpret_cast<uintptr_t>(a.devicePointer) % align) return nullptr;
-    return a.devicePointer;
+    return r.device;
 }
 
 constexpr const char* SOLVER_STATE_ERROR = "the grid solver met a record or a body version that it cannot have made";
@@ -1227,14 +1264,16 @@ struct ag2d_world {
     {
         ensureDevice();
         const cudaStream_t s = stream;
-        nBodies = h.nBodies; nColliders = h.nColliders; nCircles = h.nCircles; nBoxes = h.nBoxes;
-        nPolygons = h.nPolygons; nPolyVerts = h.nPolyVerts; nMaterialRows = h.nMaterialRows; nStatic = h.nStatic;
-        nWorlds = std::max<uint32_t>(h.nWorlds, 1);
         // A small page-locked checkpoint goes over in one kernel that reads the sections where they lie, a large or
         // pageable one in a copy a section.
         // The kernel moves 16 bytes at a time; saved sections lie at multiples of 256.
         const bool aligned = std::all_of(h.off, h.off + NCK, [](uint64_t o) { return o % 16 == 0; });
-        const void* const mapped = aligned && h.totalBytes <= 4 * HOST_DIRECT_BYTES ? kernel_reach(src, 16) : nullptr;
+        const void* const mapped =
+            aligned && h.totalBytes <= 4 * HOST_DIRECT_BYTES ? kernel_reach(src, h.totalBytes, 16, false) : nullptr;
+        if (!mapped) (void)page_locked(src, h.totalBytes);   // refused if page-locked in part, before anything changes
+        nBodies = h.nBodies; nColliders = h.nColliders; nCircles = h.nCircles; nBoxes = h.nBoxes;
+        nPolygons = h.nPolygons; nPolyVerts = h.nPolyVerts; nMaterialRows = h.nMaterialRows; nStatic = h.nStatic;
+        nWorlds = std::max<uint32_t>(h.nWorlds, 1);
         SectionCopies sections{};
         auto put = [&](void* dst, uint32_t k) {
             if (!h.len[k]) return;
@@ -4067,7 +4106,7 @@ static void copy_to_host(ag2d_world& w, void* dst, const void* src, size_t bytes
 {
     const cudaStream_t s = w.stream;
     if (!bytes) return;
-    if (page_locked(dst)) {
+    if (page_locked(dst, bytes)) {
         CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         return;
@@ -4100,7 +4139,7 @@ static uint64_t read_packed(ag2d_world& w, const FieldSpec& f, uint32_t lo, uint
     const uint64_t bytes = uint64_t(n) * f.outBytes;
     if (!bytes) return 0;
     const void* src = static_cast<const uint8_t*>(f.src) + size_t(lo) * f.outBytes;
-    void* const mapped = f.kind != EXTRACT_DIRECT && bytes <= HOST_DIRECT_BYTES ? kernel_reach(dst, 4) : nullptr;
+    void* const mapped = f.kind != EXTRACT_DIRECT && bytes <= HOST_DIRECT_BYTES ? kernel_reach(dst, bytes, 4, true) : nullptr;
     if (mapped) {
         k_extract<<<w.gridFor(n), 256, 0, w.stream>>>(f.src, lo, n, f.kind, f.comp, bias, mapped);
         CK(cudaGetLastError());
@@ -4309,7 +4348,7 @@ int32_t ag2d_world_read_async(ag2d_world* world, int32_t field, void* dst, uint6
         const uint64_t bytes = uint64_t(n) * f.outBytes;
         if (out_bytes) *out_bytes = bytes;
         if (!dst || cap < bytes) throw ApiError(AG2D_ERR_INVALID_ARG, "destination missing or too small");
-        if (!page_locked(dst))
+        if (!page_locked(dst, bytes))
             throw ApiError(AG2D_ERR_INVALID_ARG, "asynchronous reads need a page-locked destination (ag2d_host_alloc)");
         read_async(*world, f, 0, n, 0, dst);
     });
