@@ -4467,6 +4467,7 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
         CK(cudaSetDevice(w.settings.device));
         w.ensureUploaded();
         if (w.listsDirty) w.rebuildLists();
+        bool counted = false;   // the phase has read the counters
         switch (phase) {
         case AG2D_PHASE_INTEGRATE:
             CK(cudaMemsetAsync(w.wrapCount.p, 0, sizeof(float) * std::max<uint32_t>(w.nBodies, 1), w.stream));
@@ -4516,9 +4517,12 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
             }
             if (w.collideExec) { CK(cudaGraphExecDestroy(w.collideExec)); w.collideExec = nullptr; }
             if (!std::equal(key, key + 10, w.collideSeen)) {
-                // A new shape: one pass as it is (it may grow buffers or rebuild the static tree), remembered.
+                // A new shape: one pass as it is (it may grow buffers or rebuild the static tree), remembered with the
+                // counts it found, which size the next pass.
                 pass();
+                w.readCounters();
                 shape(w.collideSeen);
+                counted = true;
                 break;
             }
             // The second pass of a shape: captured (nothing left to allocate), then replayed while the shape holds.
@@ -4563,7 +4567,7 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
             break;
         default: throw ApiError(AG2D_ERR_INVALID_ARG, "unknown phase");
         }
-        w.readCounters();
+        if (!counted) w.readCounters();
         if (w.hCounters->status & (STATUS_BARRIER_TIMEOUT | STATUS_LOOKBACK_TIMEOUT))
             throw ApiError(AG2D_ERR_TIMEOUT, "a bounded device-side wait timed out");
         if (w.hCounters->status & STATUS_SOLVER_STATE) throw ApiError(AG2D_ERR_CUDA, SOLVER_STATE_ERROR);
