@@ -1360,6 +1360,7 @@ struct ag2d_world {
         newWorldsPending = false;
         manSegFresh = false;
         hintsReady = false;
+        islandsLinked = false;
         lastManifolds = h.lastManifolds;
     }
 
@@ -1595,6 +1596,8 @@ struct ag2d_world {
         jointsDirty = jointTotal() > 0;
         CK(cudaStreamSynchronize(s));
         hostDirty = false;
+        hintsReady = false;
+        islandsLinked = false;
         listsDirty = true;
         fullPose = true;
         aabbValid = false;
@@ -3022,6 +3025,7 @@ struct ag2d_world {
             if (!(w > 0.0f) && vel[b].w > 0.0f) freed[b] = anyFreed = true;
         if (anyFreed) forgetColours(freed);
         hintsReady = false;   // a narrow phase run before the commands took its hints from the list as it was
+        islandsLinked = false;
         if (nBodies) {
             CK(cudaMemcpyAsync(bvel.p, vel.data(), nBodies * sizeof(float4), cudaMemcpyHostToDevice, s));
             CK(cudaMemcpyAsync(bpos.p, pos.data(), nBodies * sizeof(float4), cudaMemcpyHostToDevice, s));
@@ -4468,6 +4472,9 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
         w.ensureUploaded();
         if (w.listsDirty) w.rebuildLists();
         bool counted = false;   // the phase has read the counters
+        // The solver's island links hold until something other than the islands phase runs (a wake adds bodies and
+        // manifolds; events change nothing).
+        if (phase != AG2D_PHASE_ISLANDS && phase != AG2D_PHASE_EVENTS) w.islandsLinked = false;
         switch (phase) {
         case AG2D_PHASE_INTEGRATE:
             CK(cudaMemsetAsync(w.wrapCount.p, 0, sizeof(float) * std::max<uint32_t>(w.nBodies, 1), w.stream));
