@@ -638,8 +638,7 @@ struct ag2d_world {
     bool hintsReady = false;   // this step's lookup wrote the hints
     DBuf<uint4> listA, listB;
     DBuf<unsigned long long> bodyMax, bodyMask;
-    DBuf<float4> flowVel, flowPos;   // grid solver (FlowScratch); its records lie in consQ, listA and listB
-    DBuf<unsigned long long> flowHigh;
+    DBuf<float4> flowWords;   // grid solver (FlowScratch): vel, pos, high; its records lie in consQ, listA and listB
     // Manifolds of sleeping islands (k_islands.cu): world-grouped records and the island (root body) of each, with
     // the back buffers the sleep pass scatters into. isleUpper bounds the count as the host knows it (0: empty).
     DBuf<Manifold> isle, bk_isle;
@@ -2505,9 +2504,7 @@ struct ag2d_world {
     void reserveGridSolver()
     {
         if (nWorlds > 1 || blockSolver()) return;
-        flowVel.reserve(nBodies);
-        flowPos.reserve(nBodies);
-        flowHigh.reserve(FLOW_HIGH * size_t(nBodies));
+        flowWords.reserve(2 * size_t(nBodies) + (FLOW_HIGH * size_t(nBodies) + 1) / 2);
     }
 
     void phaseSolve()
@@ -2572,8 +2569,10 @@ struct ag2d_world {
             }
             reserveGridSolver();
             static_assert(sizeof(Constraint) == ConsRecords::FIELDS * sizeof(float4), "records of either form fit consQ");
-            FlowScratch flow{flowVel.p, flowPos.p, reinterpret_cast<Constraint*>(consQ.p),
-                             reinterpret_cast<float4*>(listA.p), reinterpret_cast<float4*>(listB.p), flowHigh.p,
+            float4* const words = flowWords.p;
+            FlowScratch flow{words, words + nBodies, reinterpret_cast<Constraint*>(consQ.p),
+                             reinterpret_cast<float4*>(listA.p), reinterpret_cast<float4*>(listB.p),
+                             reinterpret_cast<unsigned long long*>(words + 2 * size_t(nBodies)),
                              begun ? ufParent.p : nullptr};
             islandsLinked = begun;   // the step's first kernel made every body its own island
             uint32_t* barp = bar.p;
