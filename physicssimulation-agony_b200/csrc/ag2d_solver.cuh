@@ -51,7 +51,7 @@ struct SharedBodies {
     __device__ __forceinline__ void setP(uint32_t b, const float4& x) const { pos[b - base] = x; }
     __device__ __forceinline__ float invMass(uint32_t b) const
     {
-        return gvel ? __ldg(&gvel[b].w) : vel[b - base].w;
+        return gvel ? gvel[b].w : vel[b - base].w;
     }
     // Loads the body cache over the colouring words (lazy only); the caller synchronises the team after it.
     __device__ __forceinline__ bool stage(uint32_t rank, uint32_t size) const
@@ -607,9 +607,9 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
 constexpr uint32_t PAIR_DYNAMIC = 0x80000000u, PAIR_KEPT = 0x40000000u, PAIR_TWO = 0x40000000u, PAIR_BODY = 0x3FFFFFFFu;
 
 template <class Sync, class Bodies>
-__device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Manifold* __restrict__ m, uint32_t n,
+__device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Manifold* m, uint32_t n,
                                 const SolveScratch& s, uint32_t rank, uint32_t size, Sync sync,
-                                uint32_t* __restrict__ outColors, uint32_t* __restrict__ status, uint32_t& ncolOut)
+                                uint32_t* outColors, uint32_t* status, uint32_t& ncolOut)
 {
     for (uint32_t c = rank; c < COLOR_SLOTS; c += size) s.colorCount[c] = 0;
     // A grid counts per block in shared memory first: one atomic a manifold on the fourteen counters of a pile's colours
@@ -793,7 +793,7 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
 
 // The colour-major solve of coloured manifolds (s.order, s.colorStart), with the team's barrier between colours.
 template <class Sync, class Bodies, bool PIPELINED = false>
-__device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* __restrict__ m, uint32_t n,
+__device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* m, uint32_t n,
                               const SolveScratch& s, uint32_t ncol, uint32_t velIters, uint32_t posIters,
                               uint32_t rank, uint32_t size, Sync sync, ConsSmem cs = ConsSmem{})
 {
@@ -879,10 +879,10 @@ __device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* _
 }
 
 template <class Sync, class Bodies, bool PIPELINED = false>
-__device__ __forceinline__ bool color_and_solve(const DeviceWorld& w, const Bodies& B, Manifold* __restrict__ m,
+__device__ __forceinline__ bool color_and_solve(const DeviceWorld& w, const Bodies& B, Manifold* m,
                                                 uint32_t n, const SolveScratch& s, uint32_t velIters,
                                                 uint32_t posIters, uint32_t rank, uint32_t size, Sync sync,
-                                                uint32_t* __restrict__ outColors, uint32_t* __restrict__ status,
+                                                uint32_t* outColors, uint32_t* status,
                                                 ConsSmem cs = ConsSmem{})
 {
     uint32_t ncol = 0;
