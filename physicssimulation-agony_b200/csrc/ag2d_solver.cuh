@@ -891,8 +891,14 @@ __device__ __forceinline__ bool color_and_solve(const DeviceWorld& w, const Bodi
 }
 
 // Single worlds whose bodies fit one CTA's shared memory (32 B each, up to BLOCK_SOLVE_BODIES): one CTA colours,
-// solves and links the islands, __syncthreads between colours.
+// solves and links the islands, __syncthreads between colours. With more than BLOCK_SOLVE_MANIFOLDS contacts, and more
+// than BLOCK_SOLVE_PER_COLOR of them a colour, the grid solves them all the same: one CTA pays per manifold, the grid per
+// colour. A step's solve, one CTA against the grid: piles of 2,609 manifolds 167 and 183 us, 3,503: 208 and 191, 4,727: 237
+// and 189, 9,269: 431 and 207; compound bodies of 9 and 16 boxes with 5,110 manifolds in 20 colours 348 and 358, 8,346 in
+// 61: 927 and 1,086, 16,909 in 87: 1,282 and 1,259, 35,542 in 103: 2,219 and 1,670.
 constexpr uint32_t BLOCK_SOLVE_BODIES = 6912;
+constexpr uint32_t BLOCK_SOLVE_MANIFOLDS = 4096;
+constexpr uint32_t BLOCK_SOLVE_PER_COLOR = 192;
 struct BlockSolve {
     DeviceWorld w;
     Manifold* m;
@@ -904,12 +910,12 @@ struct BlockSolve {
     uint32_t* ufFlag;          // [bodies] set to 1
     StepCounters* counters;
 };
-// Host side: launches the one-CTA solver for about 'manifolds' manifolds.
-cudaError_t launch_color_solve_block(uint32_t manifolds, cudaStream_t stream, const BlockSolve& a);
+// Host side: launches the one-CTA solver for about 'perColor' manifolds a colour.
+cudaError_t launch_color_solve_block(uint32_t perColor, cudaStream_t stream, const BlockSolve& a);
 // Host side: raises the one-CTA solver's dynamic shared-memory limit (once per device).
 cudaError_t block_solver_init();
 
-// Larger single worlds: a cooperative grid colours the manifolds, then solves them as a dataflow over per-body
+// Other single worlds: a cooperative grid colours the manifolds, then solves them as a dataflow over per-body
 // versions instead of barriers (k_color_solve_flow).
 constexpr uint32_t FLOW_VEL_WARPS = 16, FLOW_POS_WARPS = 4;   // warps of a CTA: velocity passes, position passes
 constexpr uint32_t FLOW_THREADS = 32 * (FLOW_VEL_WARPS + FLOW_POS_WARPS);

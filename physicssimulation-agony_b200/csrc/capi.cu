@@ -578,6 +578,9 @@ struct ag2d_world {
     uint32_t nDestroyed = 0;   // bodies removed by destroy commands (still in the arrays, in no list)
     uint32_t pairCap = 0, manifoldCap = 0, hashCap = 0;
     uint32_t lastManifolds = 0;
+    bool manifoldsKnown = false;   // lastManifolds is a step's count of the bodies as they are
+    static constexpr uint32_t USUAL_COLORS = 8;
+    uint32_t lastColors = USUAL_COLORS;   // solver colours of the last step
     uint32_t lastPairs = 0;   // candidate pairs of the last step
     uint32_t pairsSeen = 0;   // candidate pairs of the last pass that found any (pairEstimate)
     uint32_t prevCount = 0;   // manifolds in prevManifolds (the warm-start source), as the host knows them
@@ -1024,6 +1027,8 @@ struct ag2d_world {
         fullPose = false;
         manSegFresh = false;
         lastManifolds = prevCount;
+        manifoldsKnown = false;
+        lastColors = USUAL_COLORS;
     }
 
     // The final body state (velocity, pose, state) of the given resident worlds, concatenated in that order: one
@@ -1297,6 +1302,8 @@ struct ag2d_world {
         // Buffers sized from the saved engine's last step (three times its pairs and manifolds: above the growth
         // threshold of twice the count), not from the first-upload guess of pairs a collider.
         const bool known = h.lastPairs > 0;
+        manifoldsKnown = known;
+        lastColors = USUAL_COLORS;
         if (known) {
             lastManifolds = h.lastManifolds;
             lastPairs = h.lastPairs;
@@ -1596,6 +1603,8 @@ struct ag2d_world {
         aabbValid = false;
         otherDirty = true;
         lastManifolds = 0;
+        manifoldsKnown = false;
+        lastColors = USUAL_COLORS;
         prevCount = 0;
     }
 
@@ -2491,10 +2500,19 @@ struct ag2d_world {
         }
     }
 
-    // A single world small enough for one CTA's solver.
-    bool blockSolver() const { return nWorlds == 1 && nBodies <= BLOCK_SOLVE_BODIES && !dev.gridOnly; }
+    // Manifolds to size the solver for: the last step's, or one a collider before the first.
+    uint32_t manifoldGuess() const { return manifoldsKnown ? lastManifolds : std::max(nColliders, prevCount); }
 
-    // The grid solver's words per body, with the other buffers of the bodies: a step does not allocate.
+    // A single world small enough for one CTA's solver.
+    bool blockSolver() const
+    {
+        const uint32_t m = manifoldGuess();
+        return nWorlds == 1 && nBodies <= BLOCK_SOLVE_BODIES && !dev.gridOnly &&
+               (m <= BLOCK_SOLVE_MANIFOLDS || m / lastColors <= BLOCK_SOLVE_PER_COLOR);
+    }
+
+    // The grid solver's words per body, with the other buffers of the bodies: a step does not allocate (but the one after
+    // which a smaller world's contacts first outgrow one CTA).
     void reserveGridSolver()
     {
         if (nWorlds > 1 || blockSolver()) return;
@@ -2551,7 +2569,7 @@ struct ag2d_world {
         } else if (blockSolver()) {
             // One CTA, bodies in shared memory; it also links the islands.
             const BlockSolve args{w, mm, nm, scratch, std::max<uint32_t>(nBodies, 1), vi, pi, ufParent.p, ufFlag.p, ctr};
-            CK(launch_color_solve_block(lastManifolds, s, args));
+            CK(launch_color_solve_block(manifoldGuess() / lastColors, s, args));
             islandsLinked = true;
         } else {
             // Whole-grid cooperative launch: about a warp of manifolds on each of a CTA's first four warps before a
@@ -2570,7 +2588,7 @@ struct ag2d_world {
                              begun ? ufParent.p : nullptr};
             islandsLinked = begun;   // the step's first kernel made every body its own island
             uint32_t* barp = bar.p;
-            const uint32_t est = std::min<uint32_t>(manifoldCap, lastManifolds + lastManifolds / 2 + 1024);
+            const uint32_t guess = manifoldGuess(), est = std::min<uint32_t>(manifoldCap, guess + guess / 2 + 1024);
             const int grid = std::max(1, std::min<int>(dev.flowBlocks, int(div_up(est, 128))));
             void* args[] = {&w, &mm, &nm, &scratch, &flow, &vi, &pi, &barp, &ctr};
             CK(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_color_solve_flow), dim3(grid), dim3(FLOW_THREADS),
@@ -3263,6 +3281,8 @@ struct ag2d_world {
                 prevSegValid = true;
             }
             lastManifolds = hCounters->manifolds;
+            manifoldsKnown = true;
+            lastColors = std::max<uint32_t>(hCounters->colors, 1);
             lastPairs = hCounters->pairs;
             prevCount = std::min(lastManifolds, manifoldCap);
             // The store as the step began (the restore reads it, the sleep pass rewrites it).

@@ -708,11 +708,14 @@ cudaError_t block_solver_init()
     return cudaSuccess;
 }
 
-cudaError_t launch_color_solve_block(uint32_t manifolds, cudaStream_t stream, const BlockSolve& a)
+cudaError_t launch_color_solve_block(uint32_t perColor, cudaStream_t stream, const BlockSolve& a)
 {
     const size_t smem = team_smem_bytes(a.bodyCap, 0);
-    if (manifolds <= 512) return chain_launch(true, k_color_solve_block<128>, 1, 128, smem, stream, a);
-    if (manifolds <= 4096) return chain_launch(true, k_color_solve_block<512>, 1, 512, smem, stream, a);
+    // The threads that a colour's steps use, for each one more is slower at the barriers: 122 manifolds in 7 colours take
+    // 48 us with 128 threads and 51 with 512, 157 in 5: 52 and 49; 554 in 7: 63 with 512 and 66 with 1,024, 2,086 in 36:
+    // 385 and 410, 1,042 in 7: 93 and 91, 3,301 in 9: 202 and 187.
+    if (perColor <= 24) return chain_launch(true, k_color_solve_block<128>, 1, 128, smem, stream, a);
+    if (perColor <= 128) return chain_launch(true, k_color_solve_block<512>, 1, 512, smem, stream, a);
     return chain_launch(true, k_color_solve_block<1024>, 1, 1024, smem, stream, a);
 }
 
