@@ -99,9 +99,12 @@ struct StepBegin {
 };
 // A chain of kernels on one stream: launched with chain_launch, a kernel's blocks may be placed while its predecessor
 // still runs, and chain_begin, the first thing they do, waits for its end (and for its writes). Kernels of a small step
-// run about ten microseconds and the gaps between them up to a third of that: 98 -> 90 us a step with 64 bodies,
-// 136 -> 108 with 20,000 in flight. Large ones lose more to the waiting blocks than the gaps cost (900 -> 937 us with
-// 100,000 bodies piled up, 465 -> 489 a pass over a million), so only engines of up to CHAIN_COLLIDERS are chained.
+// run about ten microseconds and the gaps between them up to a third of that. Unchained against chained, a step of 64
+// bodies 98 and 90 us; of n bodies in flight: 5,000: 112 and 105, 20,000: 130 and 110, 40,000: 134 and 114, 80,000: 148 and
+// 132; of n still falling into a pile: 20,000: 236 and 215, 80,000: 277 and 256; a detection pass over n: 20,000: 115 and
+// 112, 60,000: 131 and 127. Large kernels lose more to the waiting blocks than the gaps cost: a pass over 80,000: 138 and 145,
+// over a million: 465 and 489, a step of 100,000 bodies piled up: 900 and 937. Engines of up to CHAIN_COLLIDERS are
+// chained, half of the 60,000 up to which nothing measured loses.
 // Such a kernel takes no pointer as __restrict__ and reads nothing through __ldg that an earlier kernel of the chain
 // writes: those loads may move ahead of the wait and need not see the writes.
 constexpr uint32_t CHAIN_COLLIDERS = 32768;
