@@ -338,8 +338,12 @@ constexpr uint32_t COLOR_KEEP_STEPS = 16;
 // colour count, then a second counter per colour (one-point contacts placed from the colour's end).
 constexpr uint32_t COLOR_SLOTS = 2 * MAX_COLORS + 4;
 // Colours 0..63 are chosen first-fit from a body's 64-bit mask of neighbouring colours; a manifold whose bodies see
-// all 64 taken gets colour 64 + its round (unique to the round, so still conflict-free).
-constexpr uint32_t MAX_ROUNDS = MAX_COLORS - 64;
+// all 64 taken gets colour 64 + its round (unique to the round, so still conflict-free). What is left after the last
+// round (a body with more contacts than that, a ground that was given a mass) is the tail, the last colour: its manifolds
+// may share bodies and are solved one after the other in list order.
+constexpr uint32_t TAIL_COLOR = MAX_COLORS - 1;
+constexpr uint32_t MAX_ROUNDS = TAIL_COLOR - 64;
+constexpr uint32_t TAIL_MAX = 16384;   // manifolds of a tail; more: STATUS_COLOR_OVERFLOW
 constexpr uint32_t ONE_BLOCK_ROUND = 4096;   // uncoloured manifolds that one block of a grid finishes
 
 // Solver records in global memory, structure of arrays: field f of record c at q[f * stride + c], so that a warp that
@@ -557,12 +561,17 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
         return p == 0 ? PHASE_WARM : (p <= velIters ? PHASE_VELOCITY : PHASE_POSITION);
     };
     constexpr uint32_t NO_REC = 0xFFFFFFFFu;
+    // This thread's first record of a colour, or NO_REC; the tail is the first thread's alone, one after the other.
+    auto first = [&](uint32_t col) {
+        const uint32_t c = Sync::ld(s.colorStart + col) + rank;
+        return c < Sync::ld(s.colorStart + col + 1) && (col != TAIL_COLOR || rank == 0) ? c : NO_REC;
+    };
     Constraint nxt;
     BlockMatrix nxtBm;
     uint32_t cNext = NO_REC;
     if (nPhase) {
-        const uint32_t c0 = Sync::ld(s.colorStart) + rank;
-        if (c0 < Sync::ld(s.colorStart + 1)) { s.cons.load(c0, kindOf(0), nxt, nxtBm); cNext = c0; }
+        cNext = first(0);
+        if (cNext != NO_REC) s.cons.load(cNext, kindOf(0), nxt, nxtBm);
     }
     for (uint32_t ph = 0; ph < nPhase; ph++) {
         const uint32_t col = ph % ncol, kind = kindOf(ph);
@@ -573,14 +582,14 @@ __device__ bool solve_passes_pipelined(const Bodies& B, const SolveScratch& s, u
         cNext = NO_REC;
         if (ph + 1 < nPhase) {
             const uint32_t col2 = (ph + 1) % ncol;
-            const uint32_t c2 = Sync::ld(s.colorStart + col2) + rank;
-            if (c2 < Sync::ld(s.colorStart + col2 + 1)) { s.cons.load(c2, kindOf(ph + 1), nxt, nxtBm); cNext = c2; }
+            cNext = first(col2);
+            if (cNext != NO_REC) s.cons.load(cNext, kindOf(ph + 1), nxt, nxtBm);
         }
         while (c < end) {
             solve_record(B, s.cons, c, kind, k, bm);
             // One colour: the next phase's record is this one, loaded before this phase's impulses.
             if (cNext == c) { nxt.jn0 = k.jn0; nxt.jt0 = k.jt0; nxt.jn1 = k.jn1; nxt.jt1 = k.jt1; }
-            c += size;   // a colour larger than the team
+            c += col == TAIL_COLOR ? 1u : size;   // a colour larger than the team
             if (c < end) s.cons.load(c, kind, k, bm);
         }
         if (!sync()) return false;
@@ -749,7 +758,12 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
             len = Sync::ld(s.colorCount + MAX_COLORS + 1);
         }
     }
-    if (len > 0) { if (rank == 0) atomicOr(status, STATUS_COLOR_OVERFLOW); return false; }
+    if (len > TAIL_MAX) { if (rank == 0) atomicOr(status, STATUS_COLOR_OVERFLOW); return false; }
+    if (rank == 0 && len > 0) {
+        s.colorCount[TAIL_COLOR] = len;
+        atomicMax(nColors, MAX_COLORS);
+    }
+    if (len > 0 && !sync()) return false;
     const uint32_t ncol = ncolOut = Sync::ld(nColors);
     if (rank == 0) {
         uint32_t run = 0;
@@ -758,6 +772,17 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
         atomicMax(outColors, ncol);
     }
     if (!sync()) return false;
+    if (len > 0) {   // the tail in list order: a manifold's place is the number of the tail's below it
+        const uint4* const tail = (MAX_ROUNDS - 1u) & 1u ? s.listB : s.listA;
+        for (uint32_t j = rank; j < len; j += size) {
+            const uint32_t i = tail[j].x;
+            uint32_t below = 0;
+            for (uint32_t k = 0; k < len; k++) below += tail[k].x < i;
+            s.color[i] = TAIL_COLOR;
+            s.order[Sync::ld(s.colorStart + TAIL_COLOR) + below] = i;
+        }
+        if (!sync()) return false;
+    }
     // Within a colour (independent contacts, any order) two-point contacts come first and one-point contacts last, so
     // that few warps run both solves.
     if constexpr (Sync::GRID) {
@@ -765,7 +790,7 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
         uint32_t* const place = reinterpret_cast<uint32_t*>(s.listA);   // the uncoloured lists are done with
         clear_block_counts();
         for (uint32_t i = rank; i < n; i += size)
-            place[i] = atomicAdd(blockCount + (s.color[i] & COLOR_MASK) + (s.pairBodies[i].y & PAIR_TWO ? 0u : MAX_COLORS),
+            if ((s.color[i] & COLOR_MASK) != TAIL_COLOR) place[i] = atomicAdd(blockCount + (s.color[i] & COLOR_MASK) + (s.pairBodies[i].y & PAIR_TWO ? 0u : MAX_COLORS),
                                  1u);
         __syncthreads();
         for (uint32_t c = threadIdx.x; c < 2 * MAX_COLORS; c += blockDim.x)
@@ -774,6 +799,7 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
         __syncthreads();
         for (uint32_t i = rank; i < n; i += size) {
             const uint32_t c = s.color[i] & COLOR_MASK;
+            if (c == TAIL_COLOR) continue;
             const uint32_t at = s.pairBodies[i].y & PAIR_TWO
                                     ? __ldcg(s.colorStart + c) + blockCount[c] + place[i]
                                     : __ldcg(s.colorStart + c + 1) - 1u - blockCount[MAX_COLORS + c] - place[i];
@@ -783,6 +809,7 @@ __device__ bool color_manifolds(const DeviceWorld& w, const Bodies& B, const Man
     }
     for (uint32_t i = rank; i < n; i += size) {
         const uint32_t c = s.color[i] & COLOR_MASK;
+        if (c == TAIL_COLOR) continue;
         const uint32_t at = s.pairBodies[i].y & PAIR_TWO
                                 ? Sync::ld(s.colorStart + c) + atomicAdd(s.colorCount + c, 1u)
                                 : Sync::ld(s.colorStart + c + 1) - 1u - atomicAdd(s.colorCount + MAX_COLORS + 4 + c, 1u);
@@ -817,10 +844,14 @@ __device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* m
             passesDone = true;
         }
     }
+    // The tail is the first thread's alone, one after the other.
+    auto takes = [&](uint32_t col) { return col != TAIL_COLOR || rank == 0; };
+    auto step = [&](uint32_t col) { return col == TAIL_COLOR ? 1u : size; };
     if (!passesDone) {
         for (uint32_t col = 0; col < ncol; col++) {
             const uint32_t end = Sync::ld(s.colorStart + col + 1);
-            for (uint32_t c = Sync::ld(s.colorStart + col) + rank; c < end; c += size) {
+            const uint32_t begin = Sync::ld(s.colorStart + col);
+            for (uint32_t c = begin + rank; takes(col) && c < end; c += step(col)) {
                 Constraint k;
                 BlockMatrix bm;
                 if (onChip) cs.load(c, k);
@@ -839,7 +870,7 @@ __device__ bool solve_colored(const DeviceWorld& w, const Bodies& B, Manifold* m
                 const uint32_t begin = Sync::ld(s.colorStart + col), count = Sync::ld(s.colorStart + col + 1) - begin;
                 const uint32_t posBase = vel ? (count + 31u) & ~31u : 0u;   // a warp does one kind of step
                 const uint32_t total = pos ? posBase + count : count;
-                for (uint32_t j = rank; j < total; j += size) {
+                for (uint32_t j = rank; takes(col) && j < total; j += step(col)) {
                     Constraint k;
                     BlockMatrix bm;
                     if (vel && j < count) {

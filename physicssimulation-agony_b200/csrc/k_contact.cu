@@ -432,7 +432,7 @@ struct FlowWalk {
 // thread-block cluster has, a pass over the pile of 100,000 bodies (128,000 manifolds, 14 colours) took 8 us a colour.
 // Colours beyond the 64 first-fit ones, which a body with that many contacts brings, have masks of their own, filled
 // only then. With a grid barrier a colour instead, 7,200 compound bodies of 16 boxes (53,000 manifolds, 108 colours) took
-// 5,528 us a solve, 1,793 here.
+// 5,528 us a solve, 1,793 here. Only a colouring with a tail is solved that way.
 __global__ void __launch_bounds__(FLOW_THREADS, 1)
 k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch s, FlowScratch f, uint32_t velIters,
                    uint32_t posIters, uint32_t* bar, StepCounters* counters)
@@ -445,6 +445,12 @@ k_color_solve_flow(DeviceWorld w, Manifold* m, const uint32_t* nM, SolveScratch 
     const GridSync sync{bar, &counters->status};
     uint32_t ncol = 0;
     if (!color_manifolds(w, B, m, n, s, rank, size, sync, &counters->colors, &counters->status, ncol)) return;
+    if (ncol > TAIL_COLOR) {   // a tail: no order by colours
+        if (f.parent)
+            for (uint32_t i = rank; i < n; i += size) uf_link(w, f.parent, w.cbody[m[i].a], w.cbody[m[i].b]);
+        solve_colored(w, B, m, n, s, ncol, velIters, posIters, rank, size, sync);
+        return;
+    }
     if (ncol > 64u) {   // the colours above the first-fit ones, around each body
         for (uint32_t i = rank; i < FLOW_HIGH * w.nBodies; i += size) f.high[i] = 0ull;
         if (!sync()) return;
