@@ -101,3 +101,41 @@ def test_batches_of_such_worlds(big_mode, on_chip):
     for k, want in enumerate(alone):
         for f, a in zip(MOVED, want):
             assert np.array_equal(batch.read(k, f).view(np.uint32), a), (sizes[k], f)
+
+
+@pytest.mark.parametrize("n,steps", [(800, 260), (7200, 120)])
+def test_a_settled_pile_whose_ground_gets_a_mass(n, steps):
+    """With sleepers on the ground in the smaller pile: they wake and bring their stored contacts."""
+    worlds = []
+    for _ in range(2):
+        w = ag2d.World()
+        side = 1.6 * float(np.sqrt(n))
+        handles = w.add_scene(scenes.make_c1(n, seed=n, width=side, height=side))
+        w.step(steps)
+        w.set_body_mass(int(handles[0]), 5000.0)
+        worlds.append(w)
+    w, other = worlds
+    ground = int(np.argmin(w.read(ag2d.BODY_INV_MASS)))
+    w.flush_commands()
+    w.run_phase(ag2d.PHASE_INTEGRATE)
+    for phase in (ag2d.PHASE_SPATIAL_FULL, ag2d.PHASE_BROAD, ag2d.PHASE_NARROW, ag2d.PHASE_WAKE):
+        w.run_phase(phase)
+    m_in = _to_oracle(w.read(ag2d.MANIFOLDS))
+    ora, d = _oracle(w)
+    body = d["col.bodyIndex"]
+    assert d["body.invMass"][ground] > 0
+    assert np.count_nonzero((body[m_in["a"]] == ground) | (body[m_in["b"]] == ground)) > 20
+    w.run_phase(ag2d.PHASE_SOLVE)
+    order = w.read(ag2d.SOLVE_ORDER).astype(np.int64)
+    assert np.array_equal(np.sort(order), np.arange(m_in.size))
+    rep = ora.solve(m_in, order)
+    ours = _to_oracle(w.read(ag2d.MANIFOLDS))
+    assert parity.mismatches(ours["jn"], rep["jn"]) == 0
+    for field, ref in zip(MOVED, ("velX", "velY", "angVel", "comX", "comY")):
+        assert parity.mismatches(w.read(field), ora.a[ref]) == 0, ref
+    other.step(1)
+    assert other.counters()["status"] == 0
+    for f in MOVED:
+        assert parity.mismatches(w.read(f), other.read(f)) == 0
+    other.step(10)
+    assert other.counters()["status"] == 0
