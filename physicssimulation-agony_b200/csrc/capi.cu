@@ -742,8 +742,8 @@ struct ag2d_world {
     // The collision-detection pass (AG2D_PHASE_COLLIDE) as a captured CUDA graph, replayed while its launch shapes
     // hold (list sizes, capacities, block sizes, whether the static tree is rebuilt).
     cudaGraphExec_t collideExec = nullptr;
-    uint64_t collideKey[10] = {};
-    uint64_t collideSeen[10] = {};  // the shape of the last pass run without a graph
+    std::array<uint64_t, 15> collideKey{};
+    std::array<uint64_t, 15> collideSeen{};   // the shape of the last pass run without a graph
     uint64_t collideLaunches = 0;
     cudaEvent_t ev[NPHASE][2] = {};
     bool evPending[NPHASE] = {};
@@ -4498,28 +4498,30 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
                 pass();
                 break;
             }
-            // The pass's launches depend on these only; the kernels read their counts on the device.
-            auto shape = [&](uint64_t* k) {
-                // Any device reallocation (a buffer a captured kernel points at) changes the allocation count.
-                const uint64_t v[10] = {w.nDynCol, w.nOther, w.pairCap, w.manifoldCap, w.queryThreads,
-                                       w.narrowThreads, uint64_t(w.otherDirty), uint64_t(w.nColliders),
-                                       g_deviceAllocs.load(std::memory_order_relaxed), w.pairEstimate()};
-                std::copy(v, v + 10, k);
+            // The pass's launches depend on these only; the kernels read their counts on the device. Any reallocation of
+            // a buffer that a captured kernel points at changes the allocation count; a step trades the manifold lists
+            // and an odd number of sort passes the trees' buffers.
+            using Key = decltype(w.collideKey);
+            auto shape = [&] {
+                auto at = [](const void* p) { return uint64_t(reinterpret_cast<uintptr_t>(p)); };
+                return Key{w.nDynCol, w.nOther, w.pairCap, w.manifoldCap, w.queryThreads, w.narrowThreads,
+                           uint64_t(w.otherDirty), uint64_t(w.nColliders), g_deviceAllocs.load(std::memory_order_relaxed),
+                           w.pairEstimate(), at(w.manifolds.p), at(w.dynTree.keys.p), at(w.dynTree.vals.p),
+                           at(w.otherTree.keys.p), at(w.otherTree.vals.p)};
             };
-            uint64_t key[10];
-            shape(key);
-            if (w.collideExec && std::equal(key, key + 10, w.collideKey)) {
+            const Key key = shape();
+            if (w.collideExec && key == w.collideKey) {
                 CK(cudaGraphLaunch(w.collideExec, w.stream));
                 w.launches += w.collideLaunches;
                 break;
             }
             if (w.collideExec) { CK(cudaGraphExecDestroy(w.collideExec)); w.collideExec = nullptr; }
-            if (!std::equal(key, key + 10, w.collideSeen)) {
+            if (key != w.collideSeen) {
                 // A new shape: one pass as it is (it may grow buffers or rebuild the static tree), remembered with the
                 // counts it found, which size the next pass.
                 pass();
                 w.readCounters();
-                shape(w.collideSeen);
+                w.collideSeen = shape();
                 counted = true;
                 break;
             }
@@ -4539,7 +4541,7 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
             cudaGraphDestroy(graph);
             CK(ie);
             w.collideLaunches = w.launches - before;
-            std::copy(key, key + 10, w.collideKey);
+            w.collideKey = shape();   // with the buffers as the pass leaves them, which is how a replay leaves them too
             CK(cudaGraphLaunch(w.collideExec, w.stream));
             break;
         }
