@@ -729,6 +729,7 @@ struct ag2d_world {
     uint32_t selectTurn = 0, selectTiles = 0;
     DBuf<GatherSeg> gatherSegs;
     bool newWorldsPending = false;   // joined worlds take a full pose pass in their first step
+    std::vector<uint32_t> newWorlds;   // which of the resident worlds those are, as of the last repack
     // Shape table sizes of the last upload.
     uint32_t nCircles = 0, nBoxes = 0, nPolygons = 0, nPolyVerts = 0, nMaterialRows = 0;
     // Counters.
@@ -1009,12 +1010,15 @@ struct ag2d_world {
             CK(cudaMemsetAsync(worldDirty.p, 0, sizeof(uint32_t) * nWorlds, s));
             setTeams(teamColliders, teamThreads);
         }
-        // Joining worlds: a full pose pass in their first step (as a freshly uploaded world has).
+        // Joining worlds: a full pose pass in their first step (as a freshly uploaded world has), which a round without
+        // steps (a request for none) leaves to the next one.
         newWorldMask.reserve(nWorlds);
         std::vector<uint32_t> mask(nWorlds, 0u);
-        for (size_t j = keep.size(); j < next.size(); j++) mask[j] = 1u;
+        for (size_t j = 0; j < next.size(); j++)
+            mask[j] = j >= keep.size() || (newWorldsPending && newWorlds[keep[j]]) ? 1u : 0u;
         newWorldMask.upload(mask.data(), mask.size(), s);
-        newWorldsPending = next.size() > keep.size();
+        newWorldsPending = std::count(mask.begin(), mask.end(), 1u) > 0;
+        newWorlds = mask;
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(s));
         mark("partition");
