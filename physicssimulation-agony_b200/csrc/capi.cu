@@ -1433,6 +1433,7 @@ struct ag2d_world {
         stepDone.reserve(4);
         colorCount.reserve(COLOR_SLOTS);
         colorStart.reserve(MAX_COLORS + 1);
+        CK(cudaMemsetAsync(dCounters.p, 0, sizeof(StepCounters), stream));   // a phase run first reads them back
         CK(cudaMemsetAsync(nPrev.p, 0, sizeof(uint32_t), stream));
         CK(cudaMemsetAsync(nManifolds.p, 0, sizeof(uint32_t), stream));
         CK(cudaMemsetAsync(nIsle.p, 0, sizeof(uint32_t), stream));
