@@ -743,8 +743,8 @@ struct ag2d_world {
     // The collision-detection pass (AG2D_PHASE_COLLIDE) as a captured CUDA graph, replayed while its launch shapes
     // hold (list sizes, capacities, block sizes, whether the static tree is rebuilt).
     cudaGraphExec_t collideExec = nullptr;
-    std::array<uint64_t, 15> collideKey{};
-    std::array<uint64_t, 15> collideSeen{};   // the shape of the last pass run without a graph
+    std::array<uint64_t, 16> collideKey{};
+    std::array<uint64_t, 16> collideSeen{};   // the shape of the last pass run without a graph
     uint64_t collideLaunches = 0;
     cudaEvent_t ev[NPHASE][2] = {};
     bool evPending[NPHASE] = {};
@@ -3191,6 +3191,7 @@ struct ag2d_world {
             if (listsDirty) rebuildLists();
             const cudaStream_t s = stream;
             const bool fullPoseThisStep = fullPose;
+            if (fullPose) otherDirty = true;   // a collision pass or a phase may have built the tree before the poses
             const bool otherDirtyThisStep = otherDirty;
             struct Begun {   // an error on the way leaves no step begun
                 bool& b;
@@ -4493,8 +4494,14 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
             break;
         case AG2D_PHASE_NARROW: w.phaseNarrow(); break;
         case AG2D_PHASE_COLLIDE: {
+            // Static and sleeping colliders that no step has posed since they came or were edited.
+            const bool poseOthers = w.fullPose && w.nOther > 0;
             auto pass = [&] {
                 CK(cudaMemsetAsync(w.dCounters.p, 0, sizeof(StepCounters), w.stream));
+                if (poseOthers) {
+                    w.phasePose(true);
+                    w.otherDirty = true;
+                }
                 w.phasePose(false);
                 w.phaseBroad();
                 w.phaseNarrow(false);
@@ -4512,7 +4519,7 @@ int32_t ag2d_world_run_phase(ag2d_world* world, int32_t phase)
                 return Key{w.nDynCol, w.nOther, w.pairCap, w.manifoldCap, w.queryThreads, w.narrowThreads,
                            uint64_t(w.otherDirty), uint64_t(w.nColliders), g_deviceAllocs.load(std::memory_order_relaxed),
                            w.pairEstimate(), at(w.manifolds.p), at(w.dynTree.keys.p), at(w.dynTree.vals.p),
-                           at(w.otherTree.keys.p), at(w.otherTree.vals.p)};
+                           at(w.otherTree.keys.p), at(w.otherTree.vals.p), uint64_t(poseOthers)};
             };
             const Key key = shape();
             if (w.collideExec && key == w.collideKey) {

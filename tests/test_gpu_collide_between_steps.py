@@ -87,3 +87,33 @@ def test_passes_of_a_batch_with_one_world_pass():
         x.step(2)
     for f in STATE:
         assert plain.engine.read(f).tobytes() == b.engine.read(f).tobytes()
+
+
+@pytest.mark.parametrize("n", [40, 3000])
+@pytest.mark.parametrize("edit", [False, True])
+def test_a_pass_before_the_first_step(n, edit):
+    """The static colliders have no poses yet (or a static body was moved since): the pass poses them, and the step after it
+    does not take over a tree from before. 'edit': the pass follows a command on the ground instead of the creation."""
+    def world():
+        b = scenes._Builder([scenes.FRICTION_MATERIAL])
+        b.add(scenes.BOX, 0.0, -0.5, width=3.0 * n, height=1.0, mass=0.0)
+        for k in range(n):
+            b.add(scenes.BOX, 1.1 * (k - 0.5 * n), 0.499, width=1.0, height=1.0, mass=1.0)
+        w = ag2d.World(sleep_time=1.0e6)
+        ground = int(w.add_scene(b.build("row"))[0])
+        if edit:
+            w.step(2)
+            w.set_body_position(ground, 0.0, -0.45)
+            w.flush_commands()
+        return w
+    plain, phases, w = world(), world(), world()
+    for phase in (ag2d.PHASE_SPATIAL_FULL, ag2d.PHASE_SPATIAL_DYNAMIC, ag2d.PHASE_BROAD):
+        phases.run_phase(phase)
+    for _ in range(3):
+        w.run_phase(ag2d.PHASE_COLLIDE)
+        assert np.array_equal(w.read(ag2d.PAIRS), phases.read(ag2d.PAIRS))
+    assert w.read(ag2d.MANIFOLDS).size >= n   # every box on the ground
+    for x in (plain, w):
+        x.step(6)
+    for f in STATE:
+        assert plain.read(f).tobytes() == w.read(f).tobytes()
