@@ -2269,6 +2269,39 @@ struct ag2d_world {
         motorsOnDevice = 0;
         jointsDirty = true;
     }
+    // Regroups a batch's constraints of one kind world by world, as each world alone would: its own constraints change
+    // places among themselves only. The groups stay world after world.
+    template <class Regroup>
+    void regroupWorlds(JointSystem& js, Regroup regroup)
+    {
+        std::vector<JointSystem> own(nWorlds);
+        std::vector<std::vector<uint32_t>> slots(nWorlds);   // the batch's slots of a world's constraints
+        for (uint32_t g = 0; g < 3; g++) {
+            for (uint32_t i = js.starts[g]; i < js.starts[g + 1]; i++) {
+                const uint32_t w = uint32_t(std::upper_bound(hBodyStart.begin(), hBodyStart.end(), js.joints[i].bodyA) -
+                                            hBodyStart.begin()) - 1;
+                HJoint j = js.joints[i];
+                slots[w].push_back(j.handleSlot);
+                j.handleSlot = uint32_t(own[w].joints.size());
+                own[w].slotIndex.push_back(j.handleSlot);
+                own[w].slotGeneration.push_back(0);
+                own[w].joints.push_back(j);
+            }
+            for (JointSystem& s : own) s.starts[g + 1] = uint32_t(s.joints.size());
+        }
+        js.joints.clear();
+        for (JointSystem& s : own) regroup(s);
+        for (uint32_t g = 0; g < 3; g++) {
+            for (uint32_t w = 0; w < nWorlds; w++)
+                for (uint32_t i = own[w].starts[g]; i < own[w].starts[g + 1]; i++) {
+                    HJoint j = own[w].joints[i];
+                    j.handleSlot = slots[w][j.handleSlot];
+                    js.slotIndex[j.handleSlot] = uint32_t(js.joints.size());
+                    js.joints.push_back(j);
+                }
+            js.starts[g + 1] = uint32_t(js.joints.size());
+        }
+    }
     // Regroups every constraint by its bodies' states (Sleeping when a body sleeps, Inactive when no body moves,
     // else Active: ObjectManager.cpp:1207-1220, 1330-1360), then uploads each kind's active constraints grouped by
     // level: level(j) = 1 + the highest level of the earlier active constraints of the kind (dense order) that
@@ -2297,17 +2330,22 @@ struct ag2d_world {
         };
         for (uint32_t k = 0; k < JOINT_KINDS; k++) {
             JointSystem& js = objects.jointSystems[k];
-            std::vector<uint64_t> handles;
-            for (uint32_t i = 0; i < js.joints.size(); i++) handles.push_back(js.handleOf(i));
-            for (const uint64_t h : handles) {
-                const uint32_t i = js.indexOf(h);
-                const HJoint& j = js.joints[i];
-                const uint8_t sa = st(j.bodyA), sb = j.bodyB == NO_BODY ? uint8_t(STATE_STATIC) : st(j.bodyB);
-                const bool sleeping = sa == STATE_SLEEPING || sb == STATE_SLEEPING;
-                const bool moves = sa == STATE_DYNAMIC || sb == STATE_DYNAMIC;
-                const uint32_t g = sleeping ? JGROUP_SLEEPING : (moves ? JGROUP_ACTIVE : JGROUP_INACTIVE);
-                if (js.groupOf(i) != g) js.moveToGroup(i, g);
-            }
+            // In ascending dense order; the swaps of a move decide the order of the others.
+            auto regroup = [&](JointSystem& s) {
+                std::vector<uint64_t> handles;
+                for (uint32_t i = 0; i < s.joints.size(); i++) handles.push_back(s.handleOf(i));
+                for (const uint64_t h : handles) {
+                    const uint32_t i = s.indexOf(h);
+                    const HJoint& j = s.joints[i];
+                    const uint8_t sa = st(j.bodyA), sb = j.bodyB == NO_BODY ? uint8_t(STATE_STATIC) : st(j.bodyB);
+                    const bool sleeping = sa == STATE_SLEEPING || sb == STATE_SLEEPING;
+                    const bool moves = sa == STATE_DYNAMIC || sb == STATE_DYNAMIC;
+                    const uint32_t g = sleeping ? JGROUP_SLEEPING : (moves ? JGROUP_ACTIVE : JGROUP_INACTIVE);
+                    if (s.groupOf(i) != g) s.moveToGroup(i, g);
+                }
+            };
+            if (nWorlds <= 1) regroup(js);
+            else regroupWorlds(js, regroup);
             const uint32_t begin = js.starts[JGROUP_ACTIVE], end = js.starts[JGROUP_UNUSED];
             std::fill(last.begin(), last.end(), 0u);
             std::vector<uint32_t> level(end - begin);
