@@ -165,7 +165,8 @@ enum ag2d_phase {
     AG2D_PHASE_NARROW,             /* narrow phase on AG2D_PAIRS, warm start from AG2D_PREV_MANIFOLDS */
     AG2D_PHASE_SOLVE,              /* colouring + solver on AG2D_MANIFOLDS */
     AG2D_PHASE_ISLANDS,            /* islands + sleep flags from AG2D_MANIFOLDS */
-    AG2D_PHASE_COLLIDE,            /* collision detection alone: dynamic poses + AABBs, broad, narrow (no warm start) */
+    AG2D_PHASE_COLLIDE,            /* collision detection alone: dynamic poses + AABBs (the others' too while no step has
+                                      posed them), broad, narrow (no warm start) */
     AG2D_PHASE_CCD,                /* continuous collision: sweep fast dynamic colliders against static ones, move
                                       hit bodies back (uses the poses AG2D_PHASE_INTEGRATE recorded) */
     AG2D_PHASE_WAKE,               /* wake the sleeping islands AG2D_MANIFOLDS touch, then bring their stored
